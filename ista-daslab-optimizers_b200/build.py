@@ -1,4 +1,4 @@
-"""Builds libmicroadam_b200.so (sm_100a) in-tree with nvcc.
+"""Builds libmicroadam_b200.so (sm_100a) in-tree with nvcc, and the native host side of the step with g++.
 
     python build.py [--verbose] [--force]
 
@@ -17,6 +17,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, 'csrc')
 OUT_DIR = os.path.join(HERE, 'ista_daslab_optimizers_b200', 'lib')
 LIB_PATH = os.path.join(OUT_DIR, 'libmicroadam_b200.so')
+HOST_SRC = os.path.join(HERE, 'csrc_host', 'step_plan.cpp')
+HOST_PATH = os.path.join(HERE, 'ista_daslab_optimizers_b200', '_step_plan.so')      # a Python module next to its users
 INCLUDE = os.path.join(os.path.dirname(HERE), 'include')
 
 
@@ -32,16 +34,28 @@ def sources():
 
 
 def _inputs():
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
+    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [HOST_SRC]
     deps += [os.path.join(INCLUDE, f) for f in os.listdir(INCLUDE)]
     return deps
 
 
 def up_to_date() -> bool:
-    if not os.path.exists(LIB_PATH):
+    if not (os.path.exists(LIB_PATH) and os.path.exists(HOST_PATH)):
         return False
-    t = os.path.getmtime(LIB_PATH)
+    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(HOST_PATH))
     return all(os.path.getmtime(p) <= t for p in _inputs())
+
+
+def host_command():
+    """The g++ line of the extension that walks the optimizer's tensors (it reads torch's tensors directly)."""
+    import sysconfig
+    import torch
+    base = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    return [os.environ.get('CXX', 'g++'), '-O2', '-std=c++17', '-fPIC', '-shared', '-I', INCLUDE, '-I', os.path.join(base, 'include'),
+            '-I', os.path.join(base, 'include', 'torch', 'csrc', 'api', 'include'), '-I', os.path.join(cuda, 'include'),
+            '-I', sysconfig.get_paths()['include'], HOST_SRC, '-o', HOST_PATH, '-L', os.path.join(base, 'lib'),
+            '-ltorch_python', '-lc10_cuda', '-lc10', '-ltorch_cpu']
 
 
 def build(verbose: bool = False, force: bool = False) -> str:
@@ -57,7 +71,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
         common += ['-Xptxas', '-v']
     if os.environ.get('MAB_STATS'):
         common += ['-DMAB_STATS']       # development-only tile statistics
-    procs = []
+    procs = [(HOST_SRC, subprocess.Popen(host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True))]
     for src in sources():
         obj = os.path.join(obj_dir, os.path.basename(src)[:-3] + '.o')
         objs.append(obj)
@@ -70,7 +84,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
             sys.stderr.write(f'--- {os.path.basename(src)}\n{out}\n')
         failed |= p.returncode != 0
     if failed:
-        raise RuntimeError('nvcc failed')
+        raise RuntimeError('a compiler failed')
     link = [_nvcc(), '-shared', '-cudart', 'static', '-gencode', 'arch=compute_100a,code=sm_100a', '-o', LIB_PATH] + objs
     subprocess.run(link, check=True)
     return LIB_PATH

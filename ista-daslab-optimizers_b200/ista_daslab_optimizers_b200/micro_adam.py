@@ -28,6 +28,7 @@ There is no CPU path: parameters must live on a CUDA device and the native libra
 from __future__ import annotations
 
 import ctypes
+import importlib
 import math
 import time
 from typing import Dict, List, Optional, Tuple
@@ -35,6 +36,7 @@ from typing import Dict, List, Optional, Tuple
 import torch
 
 from . import _native as N
+from . import _step_plan
 from .tools import CopyDirection, block_split, get_first_device
 
 
@@ -45,6 +47,20 @@ class _Entry:
     def __init__(self, p, st, lo, hi, group):
         self.p, self.st, self.lo, self.hi, self.fused, self.group = p, st, lo, hi, False, group
         self.window_fused = False       # second half of the step (window -> update -> parameters) on the fused kernel
+
+
+# torch's registries of the hooks that run around every optimizer's step (None: this torch keeps them elsewhere)
+_TORCH_OPTIMIZER = importlib.import_module('torch.optim.optimizer')
+_GLOBAL_HOOKS = [getattr(_TORCH_OPTIMIZER, name, None) for name in ('_global_optimizer_pre_hooks', '_global_optimizer_post_hooks')]
+
+
+def _step_is_observed(opt) -> bool:
+    """Whether anything would notice that torch's wrapper around `step` is left out: a hook of the optimizer, a hook of
+    all optimizers, or a running profiler."""
+    before, after = _GLOBAL_HOOKS
+    if before is None or after is None or before or after:
+        return True
+    return bool(opt._optimizer_step_pre_hooks or opt._optimizer_step_post_hooks) or torch.autograd._profiler_enabled()
 
 
 class MicroAdam(torch.optim.Optimizer):
@@ -100,6 +116,7 @@ class MicroAdam(torch.optim.Optimizer):
         self._descs = {}          # descriptor arrays of the fused step, one per group of entries
         self._workspace: Optional[torch.Tensor] = None
         self._window_workspace: Optional[torch.Tensor] = None
+        self._plan = None         # native form of the step over `_entries` (csrc_host/step_plan.cpp), None = not laid out
         # set to a list to have every fused step append [start, between the two kernels, end] CUDA events
         self.kernel_events: Optional[list] = None
 
@@ -195,6 +212,7 @@ class MicroAdam(torch.optim.Optimizer):
         if steps is not None:
             self.steps = int(steps)
         self._entries_key = None
+        self._plan = None
 
     @staticmethod
     def _check_window_indices(st):
@@ -213,14 +231,36 @@ class MicroAdam(torch.optim.Optimizer):
             raise ValueError("optimizer state 'I' holds an index outside its top-k block")
 
     # ------------------------------------------------------------------------------ step
-    @torch.no_grad()
     def step(self, closure=None):
+        # torch wraps `step` of every optimizer class to run its step hooks under a profiler label, which costs more
+        # host time (about 18 us) than the rest of a small step; the label and the hooks are only gone through here
+        # when there is a profiler or a hook to see them.  (A subclass with a step of its own is wrapped as usual.)
+        if type(self).step is _OWN_STEP and _step_is_observed(self):
+            return _observed_step(self, closure)
+        return self._step(closure)
+
+    step.hooked = True            # tells torch.optim.Optimizer that this class runs the hooks itself
+
+    def _step(self, closure=None):
         self.steps += 1                                                                                # micro_adam.py:98
         loss = None
         if closure is not None:
             with torch.enable_grad():
                 loss = closure()
+        if self._plan is not None and self.log_fn is None and self.kernel_events is None:
+            status = _step_plan.plan_step(self._plan, self.param_groups, self.steps, self.quant_block_size, self.alpha,
+                                          self.beta1, self.beta2, self.eps)
+            if status == N.MAB_OK:
+                self._after_update()
+                return loss
+            if status < 0:
+                N.check(status, 'mab_fused_step')
+            self._plan = None     # something about the parameters has changed: look at them again
+        self._step_entries()
+        return loss
 
+    @torch.no_grad()
+    def _step_entries(self):
         self._refresh_entries()
         probe = self._probe_begin()
         fused = [e for e in self._entries if e.fused]
@@ -238,7 +278,27 @@ class MicroAdam(torch.optim.Optimizer):
             ev = torch.cuda.Event(enable_timing=True)   # end of whatever _after_update enqueued
             ev.record()
             self.kernel_events[-1].append(ev)
-        return loss
+        if self._plan is None and len(fused) == len(self._entries) > 0:
+            self._lay_out_plan()
+
+    def _lay_out_plan(self):
+        """Hands the entries to the native host side, which takes the next steps while nothing about them changes."""
+        descs = self._descs.get(0)
+        if descs is None or any('lr' not in g or 'weight_decay' not in g for g in self.param_groups):
+            return
+        entry_of = {id(e.p): e for e in self._entries}
+        groups = []
+        for group in self.param_groups:
+            rows = []
+            for p in group['params']:
+                e = entry_of.get(id(p))
+                sl = self._slice_of(p)
+                kind = 2 if e is not None else 0 if sl is None or sl[0] == sl[1] else 1     # step_plan.cpp, Kind
+                rows.append((p, kind, e.st if e else None, e.lo if e else 0))
+            groups.append((group, rows))
+        ws, fn = self._workspace, ctypes.cast(N.load().mab_fused_step, ctypes.c_void_p).value
+        self._plan = _step_plan.plan_new(groups, ctypes.addressof(descs), len(descs), self.m, self._entries[0].p.device.index,
+                                         fn, ws.data_ptr(), ws.numel())
 
     # ------------------------------------------------------------------------------ logging probes
     def _probe_begin(self) -> Optional[dict]:
@@ -326,6 +386,7 @@ class MicroAdam(torch.optim.Optimizer):
         self._entries = entries
         self._entries_key = key
         self._descs = {}
+        self._plan = None
         if self.use_fused and entries:
             args = self._step_args()
             for e in entries:
@@ -489,3 +550,7 @@ class MicroAdam(torch.optim.Optimizer):
             grad.zero_()
             N.asymm_block_quant_inv(d, qbs, error, min_vals, max_vals, grad, 1.0)
             probe['norm_e'] += float(grad.float().norm(p=2) ** 2)
+
+
+_OWN_STEP = MicroAdam.step        # (as defined: torch puts its wrapper in its place if it does not find `hooked`)
+_observed_step = torch.optim.Optimizer.profile_hook_step(MicroAdam._step)

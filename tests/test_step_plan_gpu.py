@@ -1,0 +1,74 @@
+"""The native host side of the step (csrc_host/step_plan.cpp) against the Python side it stands in for: the same bits,
+and the Python side again whenever something about the parameters changes between steps."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _optimizer(dtype, **hyper):
+    from ista_daslab_optimizers_b200 import MicroAdam
+    gen = torch.Generator(device='cuda').manual_seed(3)
+    params = [torch.nn.Parameter(torch.empty(n, device='cuda').normal_(0, 0.02, generator=gen).to(dtype)) for n in (7, 4096, 29056 + 72, 300)]
+    opt = MicroAdam([{'params': params[:3]}, {'params': params[3:], 'lr': 5e-4}], m=4, lr=1e-3, quant_block_size=64, weight_decay=0.1, **hyper)
+    return opt, params
+
+
+def _same(a, b, pa, pb):
+    for p, q in zip(pa, pb):
+        assert torch.equal(p.detach(), q.detach())
+        assert a.state[p].get('index') == b.state[q].get('index')
+        for key in ('I', 'V', 'error', 'min_vals', 'max_vals'):
+            if key in a.state[p]:
+                assert torch.equal(a.state[p][key], b.state[q][key]), key
+    assert a.steps == b.steps
+
+
+@pytest.mark.parametrize('dtype,hyper', [(torch.float32, {}), (torch.bfloat16, {}), (torch.float32, {'alpha': 0.5})])
+def test_native_step_follows_every_change(dtype, hyper):
+    """Gradients that come, go and move, a learning rate that becomes a tensor, a parameter added, state loaded back."""
+    (a, pa), (b, pb) = _optimizer(dtype, **hyper), _optimizer(dtype, **hyper)
+    gen = torch.Generator(device='cuda').manual_seed(4)
+    native = 0
+    for t in range(9):
+        for i, (p, q) in enumerate(zip(pa, pb)):
+            g = torch.empty(p.shape, device='cuda').normal_(0, 1e-3, generator=gen).to(dtype)
+            skip = t in (3, 4) and i == 1
+            p.grad, q.grad = (None, None) if skip else (g, g.clone())
+        if t == 2:
+            a.param_groups[1]['lr'] = b.param_groups[1]['lr'] = torch.tensor(2e-4)
+        if t == 6:
+            extra = torch.empty(1000, device='cuda').normal_(0, 0.02, generator=gen).to(dtype)
+            for opt, ps in ((a, pa), (b, pb)):
+                ps.append(torch.nn.Parameter(extra.clone()))
+                ps[-1].grad = extra.clone()
+                opt.add_param_group({'params': [ps[-1]]})
+        if t == 8:
+            a.load_state_dict(a.state_dict())
+        plan = a._plan
+        a.step()
+        native += plan is not None and a._plan is plan
+        b._plan = None                   # the Python side every time
+        b.step()
+        torch.cuda.synchronize()
+        _same(a, b, pa, pb)
+    assert native >= 3                   # steps 1, 2, 4 and 7 find the parameters as the step before left them
+
+
+def test_step_hooks_and_non_contiguous_gradients():
+    """Hooks registered on the optimizer run around the native step as well; what the Python side refuses stays refused."""
+    from ista_daslab_optimizers_b200 import _native as N
+    opt, params = _optimizer(torch.float32)
+    seen = []
+    for p in params:
+        p.grad = torch.ones_like(p)
+    opt.step()
+    assert opt._plan is not None
+    handle = opt.register_step_post_hook(lambda *a: seen.append(opt.steps))
+    opt.step()
+    handle.remove()
+    opt.step()
+    assert seen == [2] and opt.steps == 3
+    params[1].grad = torch.ones(2 * params[1].numel(), device='cuda')[::2]
+    with pytest.raises(N.NativeError, match='contiguous'):
+        opt.step()
