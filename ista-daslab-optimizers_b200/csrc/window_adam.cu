@@ -14,6 +14,7 @@
 //    sub-range of a block with dense accumulators (window.cuh).
 #include "common.cuh"
 #include "window.cuh"
+#include "codec_fast.cuh"
 #include "fused.cuh"
 #include "async_copy.cuh"
 
@@ -82,13 +83,6 @@ template <> struct Octet<uint16_t> {
     }
 };
 
-// Two floats -> two bf16 (round to nearest even) in one conversion; low half = first value.
-__device__ __forceinline__ uint32_t cvt_bf16x2_rne(float a, float b) {
-    uint32_t d;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(b), "f"(a));
-    return d;
-}
-
 // p <- round_p(round_p(p * decay) - lr * u) for 8 values, two per instruction (packed f32x2
 // operations round each component like the scalar ones).
 // HAS_U = false: only the decay (the caller updates the few touched elements afterwards).
@@ -100,7 +94,7 @@ __device__ __forceinline__ void update_octet(float (&pv)[8], const float (&u)[8]
         if (do_decay) {
             x = __fmul2_rn(x, decay2);
             if (sizeof(TP) == 2) {                       // the decayed value is stored as bf16 before the update reads it
-                const uint32_t w = cvt_bf16x2_rne(x.x, x.y);
+                const uint32_t w = pack_bf16x2_rne(x.x, x.y);
                 x = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
             }
         }
@@ -114,6 +108,9 @@ template <typename T> struct RawOctet;
 template <> struct RawOctet<float> {
     float4 a, b;
     __device__ __forceinline__ void load(const float* p) { a = reinterpret_cast<const float4*>(p)[0]; b = reinterpret_cast<const float4*>(p)[1]; }
+    __device__ __forceinline__ void load_unaligned(const float* p) {
+        a = make_float4(p[0], p[1], p[2], p[3]); b = make_float4(p[4], p[5], p[6], p[7]);
+    }
     __device__ __forceinline__ void unpack(float (&v)[8]) const {
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     }
@@ -121,6 +118,10 @@ template <> struct RawOctet<float> {
 template <> struct RawOctet<uint16_t> {
     uint4 a;
     __device__ __forceinline__ void load(const uint16_t* p) { a = reinterpret_cast<const uint4*>(p)[0]; }
+    __device__ __forceinline__ void load_unaligned(const uint16_t* p) {
+        a.x = p[0] | ((uint32_t)p[1] << 16); a.y = p[2] | ((uint32_t)p[3] << 16);
+        a.z = p[4] | ((uint32_t)p[5] << 16); a.w = p[6] | ((uint32_t)p[7] << 16);
+    }
     __device__ __forceinline__ void unpack(float (&v)[8]) const {
         v[0] = __uint_as_float(a.x << 16); v[1] = __uint_as_float(a.x & 0xFFFF0000u);
         v[2] = __uint_as_float(a.y << 16); v[3] = __uint_as_float(a.y & 0xFFFF0000u);
@@ -261,93 +262,157 @@ __device__ __forceinline__ void stream_range(const mab_tensor& T, const WindowAr
         }
         return;
     }
+    // The two forms that read the error feedback.  Octets that are whole (ALPHA 1: of whole quantisation blocks, whose
+    // lanes combine their extremes by shuffles) take the octet-wide codec, with the loads of a thread's next octet in
+    // flight while the current one is worked on; the rest of a ragged tensor goes element by element.
     const bool g_bf16 = (T.grad_dtype == MAB_BF16);
-    if (ALPHA == 2) {
-        // alpha == -2 (micro_adam.py:238-273), with a = the residual kernel A left in quant_err and e = the new codes:
-        //   p <- decay(p);  p <- p - a;  p <- p + Qinv(e);  quant_err <- a - Qinv(e);  then p <- p - lr * u
-        TP* qe = reinterpret_cast<TP*>(T.quant_err) + e0;
-        const bool vec_q = aligned16(qe);
-        for (int o = threadIdx.x; o < n_oct; o += NT) {
-            const int n = min(8, len - o * 8);
-            const int64_t ge = e0 + (int64_t)o * 8;
-            const int64_t qb = ge / a.qbs;
-            const QParams q = qparams(T.min_vals[qb], T.max_vals[qb]);
-            uint32_t codes = 0;
-            const uint8_t* ef = T.error + (ge >> 1);
-#pragma unroll
-            for (int b = 0; b < 4; ++b) if (2 * b < n) codes |= (uint32_t)ef[b] << (8 * b);
-            float pv[8], av[8], uo[8];
-            Octet<TP>::load(p + o * 8, pv, vec && n == 8, n);
-            Octet<TP>::load(qe + o * 8, av, vec_q && n == 8, n);
-            src.load(o, uo);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const uint32_t code = (codes >> (8 * (e >> 1) + ((e & 1) ? 0 : 4))) & 0xFu;
-                const float x = round_as(__fadd_rn(0.0f, qinv(code, q)), g_bf16);             // grad.zero_(); grad += Qinv(e)
-                float v = pv[e];
-                if (do_decay) v = Elem<TP>::round(__fmul_rn(v, decay));
-                v = Elem<TP>::round(__fsub_rn(v, av[e]));                                     // p.add_(grad, alpha=-1)
-                v = Elem<TP>::round(__fadd_rn(v, x));                                         // p.add_(grad)
-                av[e] = Elem<TP>::round(__fsub_rn(av[e], x));                                 // quant_err.sub_(grad)
-                pv[e] = fmaf(neg_lr, uo[e], v);
-                if (probing && e < n) {
-                    pr.sum_u2 = fmaf(uo[e], uo[e], pr.sum_u2); pr.zeros_u += (uo[e] == 0.0f) ? 1 : 0;
-                    pr.sum_qe2 = fmaf(av[e], av[e], pr.sum_qe2); pr.zeros_qe += (av[e] == 0.0f) ? 1 : 0;
-                }
-            }
-            Octet<TP>::store(p + o * 8, pv, vec && n == 8, n);
-            Octet<TP>::store(qe + o * 8, av, vec_q && n == 8, n);
-        }
-        return;
-    }
-    // alpha > 0: u += alpha * Qinv(e); p update; e <- Q((1 - alpha) * Qinv(e)) with fresh statistics
-    const int lanes = a.lanes_per_qb;
-    const int n_oct_pad = (n_oct + 31) & ~31;
-    for (int o = threadIdx.x; o < n_oct_pad; o += NT) {
-        const int n = max(0, min(8, len - o * 8));
-        const int64_t ge = e0 + (int64_t)o * 8;        // global element index of the octet
+    const int cshift = 31 - __clz(a.lanes_per_qb);           // octets per quantisation block, as a shift
+    uint8_t* ef = T.error + (e0 >> 1);
+    uint32_t* ef32 = reinterpret_cast<uint32_t*>(ef);
+    const bool ef_al4 = (reinterpret_cast<uintptr_t>(ef) & 3) == 0;
+    const int64_t qb0 = e0 >> (cshift + 3);
+    uint16_t* mins = T.min_vals + qb0;
+    uint16_t* maxs = T.max_vals + qb0;
+    TP* qe = ALPHA == 2 ? reinterpret_cast<TP*>(T.quant_err) + e0 : nullptr;
+    const bool vec_q = ALPHA == 2 && aligned16(qe);
+    const float2 decay2 = make_float2(decay, decay), neg_lr2 = make_float2(neg_lr, neg_lr);
+    const int whole = !ef_al4 ? 0 : ALPHA == 2 ? len >> 3 : (len >> (cshift + 3)) << cshift;
+    struct In { RawOctet<TP> p, q; uint32_t codes; uint16_t mn, mx; };
+    auto fetch = [&](int o, In& in) {
+        if (vec) in.p.load(p + o * 8); else in.p.load_unaligned(p + o * 8);
+        if (ALPHA == 2) { if (vec_q) in.q.load(qe + o * 8); else in.q.load_unaligned(qe + o * 8); }
+        in.codes = ef32[o];
+        in.mn = mins[o >> cshift]; in.mx = maxs[o >> cshift];
+    };
+    auto round2 = [](float2 v) {                             // two values as bf16 would hold them
+        const uint32_t w = pack_bf16x2_rne(v.x, v.y);
+        return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+    };
+    In cur;
+    if (threadIdx.x < whole) fetch(threadIdx.x, cur);
+    const int n_pad = (whole + 31) & ~31;                    // whole warps meet in the shuffles
+    for (int o = threadIdx.x; o < n_pad; o += NT) {
+        In nxt = cur;
+        if (o + NT < whole) fetch(o + NT, nxt);
+        const bool on = o < whole;
         float xs[8];
-        float lo = INFINITY, hi = -INFINITY;
-        int64_t qb = 0;
-        if (n > 0) {
-            qb = ge / a.qbs;
-            const QParams q = qparams(T.min_vals[qb], T.max_vals[qb]);
-            uint32_t codes = 0;
-            const uint8_t* ef = T.error + (ge >> 1);
+        if (on) {
+            float pv[8], uo[8], x1[8], av[8];
+            decode_octet(cur.codes, qparams(cur.mn, cur.mx), x1);
+            cur.p.unpack(pv);
+            src.load(o, uo);
+            if (ALPHA == 2) cur.q.unpack(av);
 #pragma unroll
-            for (int b = 0; b < 4; ++b) if (2 * b < n) codes |= (uint32_t)ef[b] << (8 * b);
-            float pv[8], uo[8];
+            for (int b = 0; b < 8; b += 2) {
+                float2 v = make_float2(pv[b], pv[b + 1]), u = make_float2(uo[b], uo[b + 1]);
+                const float2 x = make_float2(x1[b], x1[b + 1]), zero = make_float2(0.0f, 0.0f);
+                if (do_decay) { v = __fmul2_rn(v, decay2); if (sizeof(TP) == 2) v = round2(v); }
+                if (ALPHA == 2) {
+                    // alpha == -2 (micro_adam.py:238-273), with a = the residual kernel A left in quant_err and e = the new codes:
+                    //   p <- decay(p);  p <- p - a;  p <- p + Qinv(e);  quant_err <- a - Qinv(e);  then p <- p - lr * u
+                    float2 y = __fadd2_rn(zero, x);                                      // grad.zero_(); grad += Qinv(e)
+                    if (g_bf16) y = round2(y);
+                    float2 r = make_float2(av[b], av[b + 1]);
+                    v = __fadd2_rn(v, make_float2(-r.x, -r.y));                          // p.add_(grad, alpha=-1)
+                    if (sizeof(TP) == 2) v = round2(v);
+                    v = __fadd2_rn(v, y);                                                // p.add_(grad)
+                    if (sizeof(TP) == 2) v = round2(v);
+                    r = __fadd2_rn(r, make_float2(-y.x, -y.y));                          // quant_err.sub_(grad)
+                    if (sizeof(TP) == 2) r = round2(r);
+                    av[b] = r.x; av[b + 1] = r.y;
+                } else {
+                    // alpha > 0: u += alpha * Qinv(e); p update; e <- Q((1 - alpha) * Qinv(e)) with fresh statistics
+                    u = __fadd2_rn(u, __fmul2_rn(make_float2(a.alpha, a.alpha), x));
+                    float2 y = __fadd2_rn(zero, __fmul2_rn(make_float2(a.one_minus_alpha, a.one_minus_alpha), x));
+                    if (g_bf16) { u = round2(u); y = round2(y); }
+                    xs[b] = y.x; xs[b + 1] = y.y;
+                }
+                if (probing) {
+                    pr.sum_u2 = fmaf(u.x, u.x, fmaf(u.y, u.y, pr.sum_u2));
+                    pr.zeros_u += (u.x == 0.0f ? 1 : 0) + (u.y == 0.0f ? 1 : 0);
+                    if (ALPHA == 2) {
+                        pr.sum_qe2 = fmaf(av[b], av[b], fmaf(av[b + 1], av[b + 1], pr.sum_qe2));
+                        pr.zeros_qe += (av[b] == 0.0f ? 1 : 0) + (av[b + 1] == 0.0f ? 1 : 0);
+                    }
+                }
+                v = __ffma2_rn(neg_lr2, u, v);
+                pv[b] = v.x; pv[b + 1] = v.y;
+            }
+            Octet<TP>::store(p + o * 8, pv, vec, 8);
+            if (ALPHA == 2) Octet<TP>::store(qe + o * 8, av, vec_q, 8);
+        }
+        if (ALPHA == 1) {
+            // bf16 rounding is monotone and odd: the block's statistics are the maximum of the rounded (-min, max) pairs
+            float lo = INFINITY, hi = -INFINITY;
+            if (on) octet_min_max(xs, lo, hi);
+            uint32_t st = pack_bf16x2_rne(-lo, hi);
+            for (int off = 1; off < a.lanes_per_qb; off <<= 1) st = max_bf16x2(st, __shfl_xor_sync(0xffffffffu, st, off));
+            if (on) {
+                const uint16_t mn_b = (uint16_t)((st & 0xFFFFu) ^ 0x8000u), mx_b = (uint16_t)(st >> 16);
+                if ((o & (a.lanes_per_qb - 1)) == 0) { mins[o >> cshift] = mn_b; maxs[o >> cshift] = mx_b; }
+                const QParams q2 = qparams(mn_b, mx_b);
+                ef32[o] = (q2.u >= CODEC_U_MIN && q2.u <= CODEC_U_MAX) ? encode_octet_div_f32<true>(xs, div_consts(q2))
+                                                                       : encode_octet_exact(xs, q2, 8);
+            }
+        }
+        cur = nxt;
+    }
+    // the rest: octets of a short last block, or a tensor whose codes are not word-aligned
+    const int rest = n_oct - whole;
+    for (int o = whole + threadIdx.x; o < whole + ((rest + 31) & ~31); o += NT) {
+        const int n = max(0, min(8, len - o * 8));
+        float xs[8], lo = INFINITY, hi = -INFINITY;
+        const int qb = o >> cshift;
+        if (n > 0) {
+            const QParams q = qparams(mins[qb], maxs[qb]);
+            uint32_t codes = 0;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) if (2 * b < n) codes |= (uint32_t)ef[o * 4 + b] << (8 * b);
+            float pv[8], uo[8], av[8];
             Octet<TP>::load(p + o * 8, pv, vec && n == 8, n);
+            if (ALPHA == 2) Octet<TP>::load(qe + o * 8, av, vec_q && n == 8, n);
             src.load(o, uo);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 const uint32_t code = (codes >> (8 * (e >> 1) + ((e & 1) ? 0 : 4))) & 0xFu;
                 const float x1 = qinv(code, q);
-                const float u = round_as(__fadd_rn(uo[e], __fmul_rn(a.alpha, x1)), g_bf16);
-                if (probing && e < n) { pr.sum_u2 = fmaf(u, u, pr.sum_u2); pr.zeros_u += (u == 0.0f) ? 1 : 0; }
-                float x = pv[e];
-                if (do_decay) x = Elem<TP>::round(__fmul_rn(x, decay));
-                pv[e] = fmaf(neg_lr, u, x);
-                xs[e] = round_as(__fadd_rn(0.0f, __fmul_rn(a.one_minus_alpha, x1)), g_bf16);
-                if (e < n) { lo = fminf(lo, xs[e]); hi = fmaxf(hi, xs[e]); }
+                float v = pv[e], u = uo[e];
+                if (do_decay) v = Elem<TP>::round(__fmul_rn(v, decay));
+                if (ALPHA == 2) {
+                    const float x = round_as(__fadd_rn(0.0f, x1), g_bf16);
+                    v = Elem<TP>::round(__fsub_rn(v, av[e]));
+                    v = Elem<TP>::round(__fadd_rn(v, x));
+                    av[e] = Elem<TP>::round(__fsub_rn(av[e], x));
+                } else {
+                    u = round_as(__fadd_rn(u, __fmul_rn(a.alpha, x1)), g_bf16);
+                    xs[e] = round_as(__fadd_rn(0.0f, __fmul_rn(a.one_minus_alpha, x1)), g_bf16);
+                    if (e < n) { lo = fminf(lo, xs[e]); hi = fmaxf(hi, xs[e]); }
+                }
+                if (probing && e < n) {
+                    pr.sum_u2 = fmaf(u, u, pr.sum_u2); pr.zeros_u += (u == 0.0f) ? 1 : 0;
+                    if (ALPHA == 2) { pr.sum_qe2 = fmaf(av[e], av[e], pr.sum_qe2); pr.zeros_qe += (av[e] == 0.0f) ? 1 : 0; }
+                }
+                pv[e] = fmaf(neg_lr, u, v);
             }
             Octet<TP>::store(p + o * 8, pv, vec && n == 8, n);
+            if (ALPHA == 2) Octet<TP>::store(qe + o * 8, av, vec_q && n == 8, n);
         }
-        for (int off = 1; off < lanes; off <<= 1) {
-            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, off));
-            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, off));
-        }
-        if (n > 0) {
-            const uint16_t mn_b = f32_to_bf16_bits_rne(lo), mx_b = f32_to_bf16_bits_rne(hi);
-            if ((ge % a.qbs) == 0) { T.min_vals[qb] = mn_b; T.max_vals[qb] = mx_b; }
-            const QParams q2 = qparams(mn_b, mx_b);
-            uint8_t* ef = T.error + (ge >> 1);
+        if (ALPHA == 1) {
+            for (int off = 1; off < a.lanes_per_qb; off <<= 1) {
+                lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+                hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+            }
+            if (n > 0) {
+                const uint16_t mn_b = f32_to_bf16_bits_rne(lo), mx_b = f32_to_bf16_bits_rne(hi);
+                if ((o & (a.lanes_per_qb - 1)) == 0) { mins[qb] = mn_b; maxs[qb] = mx_b; }
+                const QParams q2 = qparams(mn_b, mx_b);
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                if (2 * b < n) {
-                    const uint32_t c0 = qcode_exact(xs[2 * b], q2);
-                    const uint32_t c1 = (2 * b + 1 < n) ? qcode_exact(xs[2 * b + 1], q2) : 0u;
-                    ef[b] = (uint8_t)((c0 << 4) | c1);
+                for (int b = 0; b < 4; ++b) {
+                    if (2 * b < n) {
+                        const uint32_t c0 = qcode_exact(xs[2 * b], q2);
+                        const uint32_t c1 = (2 * b + 1 < n) ? qcode_exact(xs[2 * b + 1], q2) : 0u;
+                        ef[o * 4 + b] = (uint8_t)((c0 << 4) | c1);
+                    }
                 }
             }
         }
@@ -648,7 +713,7 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
 // NT threads per CTA: 256 while four CTAs fit an SM; windows whose arrays leave room for two CTAs or one get 512 or
 // 1024 threads instead, so that an SM always has 32 warps to hide the latency of the barrier-separated phases.
 template <typename TP, int MODE, int ALPHA, int NT>
-__global__ void __launch_bounds__(NT, ALPHA == 0 ? 1024 / NT : 1)
+__global__ void __launch_bounds__(NT, ALPHA == 0 ? 1024 / NT : 3)
 window_tile_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int max_k,
                    const __grid_constant__ WindowArgs a) {
     window_tile_body<TP, MODE, ALPHA, NT>(tensors, n_tensors, total_units, max_k, a);
@@ -764,7 +829,7 @@ window_resident_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, in
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
                     const float2 x = __fmul2_rn(make_float2(__uint_as_float(in[b] << 16), __uint_as_float(in[b] & 0xFFFF0000u)), decay2);
-                    out[b] = cvt_bf16x2_rne(x.x, x.y);
+                    out[b] = pack_bf16x2_rne(x.x, x.y);
                 }
                 tile4[o] = make_uint4(out[0], out[1], out[2], out[3]);         // (positions past n_blk of a ragged tile are never stored)
             }
@@ -856,7 +921,7 @@ window_wide_single_kernel(const __grid_constant__ mab_tensor t, int total_units,
 
 // ------------------------------------------------------------------------------------ launch
 
-// `single` != nullptr: one tensor passed by value; else n_tensors descriptors in device memory.
+// MODE_WRITE_UPDATE: one tensor, passed by value (`single`); MODE_STEP: n_tensors descriptors in device memory.
 // units_tile / units_wide are the unit counts of the two variants; rows * max_k (the largest
 // k_block_size of the launch) decides which one runs.
 template <typename TP, int MODE, int ALPHA>
@@ -871,28 +936,28 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
         const int grid = (int)std::min<int64_t>(units_tile, (int64_t)sms * per_sm);
         // fewer resident CTAs (large windows) get more threads each; the forms with the alpha term keep 256
         const int nt = (ALPHA != 0 || per_sm >= 4) ? 256 : per_sm >= 2 ? 512 : 1024;
-        auto run = [&](auto kern_single, auto kern_multi, int threads) -> int {
-            if (single) {
-                MAB_CUDA_TRY(cudaFuncSetAttribute(kern_single, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-                kern_single<<<grid, threads, smem, s>>>(*single, units_tile, max_k, a);
-            } else {
-                MAB_CUDA_TRY(cudaFuncSetAttribute(kern_multi, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-                kern_multi<<<grid, threads, smem, s>>>(dev_tensors, n_tensors, units_tile, max_k, a);
-            }
+        auto run = [&](auto kern, int threads) -> int {
+            MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            if constexpr (MODE == MODE_WRITE_UPDATE) kern<<<grid, threads, smem, s>>>(*single, units_tile, max_k, a);
+            else kern<<<grid, threads, smem, s>>>(dev_tensors, n_tensors, units_tile, max_k, a);
             return MAB_OK;
         };
         int rc;
-        if constexpr (ALPHA == 0) {
-            if (nt == 1024) rc = run(window_tile_single_kernel<TP, MODE, 0, 1024>, window_tile_kernel<TP, MODE, 0, 1024>, 1024);
-            else if (nt == 512) rc = run(window_tile_single_kernel<TP, MODE, 0, 512>, window_tile_kernel<TP, MODE, 0, 512>, 512);
-            else rc = run(window_tile_single_kernel<TP, MODE, 0, 256>, window_tile_kernel<TP, MODE, 0, 256>, 256);
+        if constexpr (MODE == MODE_WRITE_UPDATE) {
+            if (nt == 1024) rc = run(window_tile_single_kernel<TP, MODE, 0, 1024>, 1024);
+            else if (nt == 512) rc = run(window_tile_single_kernel<TP, MODE, 0, 512>, 512);
+            else rc = run(window_tile_single_kernel<TP, MODE, 0, 256>, 256);
+        } else if constexpr (ALPHA == 0) {
+            if (nt == 1024) rc = run(window_tile_kernel<TP, MODE, 0, 1024>, 1024);
+            else if (nt == 512) rc = run(window_tile_kernel<TP, MODE, 0, 512>, 512);
+            else rc = run(window_tile_kernel<TP, MODE, 0, 256>, 256);
         } else {
-            rc = run(window_tile_single_kernel<TP, MODE, ALPHA, 256>, window_tile_kernel<TP, MODE, ALPHA, 256>, 256);
+            rc = run(window_tile_kernel<TP, MODE, ALPHA, 256>, 256);
         }
         if (rc) return rc;
     } else {
         const int grid = (int)std::min<int64_t>(units_wide, (int64_t)sms * 2);
-        if (single) {
+        if constexpr (MODE == MODE_WRITE_UPDATE) {
             auto kern = window_wide_single_kernel<TP, MODE, ALPHA>;
             MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WIN_SMEM_BYTES));
             kern<<<grid, WIN_THREADS, WIN_SMEM_BYTES, s>>>(*single, units_wide, a);
@@ -908,16 +973,13 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
     return MAB_OK;
 }
 
-// `single` != nullptr: one tensor passed by value; else n_tensors descriptors in device memory.
-// units_tile / units_wide are the unit counts of the two variants; rows * max_k (the largest
-// k_block_size of the launch) decides which one runs.
 template <typename TP, int MODE>
 static int launch_window(const mab_tensor* dev_tensors, const mab_tensor* single, int n_tensors, int units_tile,
                          int units_wide, int max_k, const WindowArgs& a, cudaStream_t s) {
-    if (MODE == MODE_STEP && a.alpha == -2.0f)
-        return launch_window_impl<TP, MODE, 2>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, s);
-    if (MODE == MODE_STEP && a.alpha != 0.0f)
-        return launch_window_impl<TP, MODE, 1>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, s);
+    if constexpr (MODE == MODE_STEP) {
+        if (a.alpha == -2.0f) return launch_window_impl<TP, MODE, 2>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, s);
+        if (a.alpha != 0.0f) return launch_window_impl<TP, MODE, 1>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, s);
+    }
     return launch_window_impl<TP, MODE, 0>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, s);
 }
 
