@@ -6,53 +6,107 @@
 //
 // Both results are reproducible bit for bit: fixed assignment of entries to threads, fixed
 // reduction trees, rows accumulated in row order.
+#include <cooperative_groups.h>
 #include "common.cuh"
+#include "codec_fast.cuh"
 #include "window.cuh"
 
 namespace mab {
 
-constexpr int SPR_SR = 7296;          // elements of a block one CTA accumulates at a time (57 * 128)
-constexpr int SPR_THREADS = 512;
+constexpr int SPR_SR = 14592;         // elements of a block one CTA accumulates at a time (57 * 256): a 29 056-element block is two ranges
+constexpr int SPR_THREADS = 512;      // three CTAs of 58 KB of accumulators per SM
+constexpr int SPR_AHEAD = 8;          // rows whose entries a thread has in flight
 
-constexpr int SP_THREADS = 1024;
+constexpr int SP_THREADS = 512;
+constexpr int SP_CLUSTER = 8;         // CTAs per row (the portable cluster size)
 
 template <typename T> __device__ __forceinline__ float load_value(const void* p, int64_t i);
 template <> __device__ __forceinline__ float load_value<float>(const void* p, int64_t i) { return reinterpret_cast<const float*>(p)[i]; }
 template <> __device__ __forceinline__ float load_value<uint16_t>(const void* p, int64_t i) { return bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(p)[i]); }
 
-// out[r] = sum_j V[r, j] * g[(j / kbs) * dbs + I[r, j]]: one CTA per row, fp32 products summed per thread in
-// entry order, then over the CTA by a fixed tree.
+// out[0 .. 16 bytes) += v, element by element in out's type.
+template <typename TO> constexpr int SPR_VEC = 16 / (int)sizeof(TO);
+__device__ __forceinline__ void add_vector(float* o, const float* v) {
+    float4 a = *reinterpret_cast<float4*>(o);
+    const float4 b = *reinterpret_cast<const float4*>(v);
+    a.x = __fadd_rn(a.x, b.x); a.y = __fadd_rn(a.y, b.y); a.z = __fadd_rn(a.z, b.z); a.w = __fadd_rn(a.w, b.w);
+    *reinterpret_cast<float4*>(o) = a;
+}
+__device__ __forceinline__ void add_vector(uint16_t* o, const float* v) {
+    uint4 a = *reinterpret_cast<uint4*>(o);
+    const float4 b = reinterpret_cast<const float4*>(v)[0], c = reinterpret_cast<const float4*>(v)[1];
+    auto pair = [](uint32_t w, float x, float y) {
+        return pack_bf16x2_rne(__fadd_rn(__uint_as_float(w << 16), x), __fadd_rn(__uint_as_float(w & 0xFFFF0000u), y));
+    };
+    a.x = pair(a.x, b.x, b.y); a.y = pair(a.y, b.z, b.w); a.z = pair(a.z, c.x, c.y); a.w = pair(a.w, c.z, c.w);
+    *reinterpret_cast<uint4*>(o) = a;
+}
+
+// out[r] = sum_j V[r, j] * g[(j / kbs) * dbs + I[r, j]]: a cluster of 8 CTAs per row (one CTA per row left most of the chip
+// idle: 268 -> 49 us for 32 rows of 256 091 entries).  A warp takes whole top-k blocks, so that an entry's
+// address needs no division and neighbouring lanes gather from neighbouring places; the partial sums of lanes, warps and
+// CTAs (through distributed shared memory) are added in a fixed order.
 template <typename TG, typename TV>
-__global__ void __launch_bounds__(SP_THREADS)
-sparse_rows_dot_kernel(int64_t k, int64_t dbs, int64_t kbs, const TG* __restrict__ g, const int16_t* __restrict__ I,
+__global__ void __cluster_dims__(SP_CLUSTER, 1, 1) __launch_bounds__(SP_THREADS)
+sparse_rows_dot_kernel(int64_t k, int64_t dbs, int kbs, int nfull, int k_few, const TG* __restrict__ g, const int16_t* __restrict__ I,
                        const void* __restrict__ V, float* __restrict__ out) {
     __shared__ float s_part[SP_THREADS / 32];
-    const int r = blockIdx.x;
-    const int16_t* idx = I + (int64_t)r * k;
+    __shared__ float s_cta[SP_CLUSTER];
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int rank = (int)cluster.block_rank();
+    const int64_t r = blockIdx.x / SP_CLUSTER;
+    const int lane = lane_id(), warp = warp_id();
+    const int nblocks = nfull + (k_few > 0 ? 1 : 0);
+    constexpr int U = 4;                                     // entries a lane has in flight
     float acc = 0.0f;
-    for (int64_t j = threadIdx.x; j < k; j += SP_THREADS) {
-        const int64_t e = (j / kbs) * dbs + (int64_t)idx[j];
-        acc = __fadd_rn(acc, __fmul_rn(load_value<TV>(V, (int64_t)r * k + j), Elem<TG>::load(g, e)));
+    for (int blk = rank * (SP_THREADS / 32) + warp; blk < nblocks; blk += SP_CLUSTER * (SP_THREADS / 32)) {
+        const int kcnt = blk < nfull ? kbs : k_few;
+        const int64_t row = r * k + (int64_t)blk * kbs;
+        const TG* gb = g + (int64_t)blk * dbs;
+        for (int j0 = lane; j0 < kcnt; j0 += 32 * U) {
+            int pos[U];
+            float val[U];
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+                const int j = j0 + 32 * i;
+                pos[i] = j < kcnt ? (int)I[row + j] : 0;
+                val[i] = j < kcnt ? load_value<TV>(V, row + j) : 0.0f;
+            }
+            float x[U];
+#pragma unroll
+            for (int i = 0; i < U; ++i) x[i] = j0 + 32 * i < kcnt ? Elem<TG>::load(gb, pos[i]) : 0.0f;
+#pragma unroll
+            for (int i = 0; i < U; ++i) acc = __fadd_rn(acc, __fmul_rn(val[i], x[i]));
+        }
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
-    if (lane_id() == 0) s_part[warp_id()] = acc;
-    __syncthreads();
+    if (lane == 0) s_part[warp] = acc;
+    cluster.sync();                                          // (every CTA of the cluster runs by now: its shared memory may be written)
     if (threadIdx.x == 0) {
         float total = 0.0f;
         for (int w = 0; w < SP_THREADS / 32; ++w) total = __fadd_rn(total, s_part[w]);
+        *cluster.map_shared_rank(&s_cta[rank], 0) = total;
+    }
+    cluster.sync();
+    if (rank == 0 && threadIdx.x == 0) {
+        float total = 0.0f;
+        for (int c = 0; c < SP_CLUSTER; ++c) total = __fadd_rn(total, s_cta[c]);
         out[r] = total;
     }
 }
 
 // out[e] += sum_r M[r] * V[r, j] over the entries (r, j) that address e: one CTA per sub-range of a top-k block
 // with a dense fp32 accumulator in shared memory; rows are added in row order (positions are unique inside a
-// row, so a row needs no atomics).
+// row, so a row needs no atomics, but a barrier).  Bound by the chain of rows: a thread fetches its first entry of
+// SPR_AHEAD rows at once, so that a row costs a shared-memory update and a barrier (25.6 M elements, 32 rows of 1 %: 232 us
+// with one load latency per row and four walks over a block's entries, 98 now).
 template <typename TO, typename TV>
-__global__ void __launch_bounds__(SPR_THREADS)
+__global__ void __launch_bounds__(SPR_THREADS, 3)
 sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int nfull, int k_few, const float* __restrict__ M,
                            const int16_t* __restrict__ I, const void* __restrict__ V, TO* __restrict__ out, int total_units) {
-    __shared__ float acc[SPR_SR];
+    extern __shared__ __align__(16) float acc[];
+    const int t = threadIdx.x;
     const int subs_per_block = (dbs + SPR_SR - 1) / SPR_SR;
     for (int unit = blockIdx.x; unit < total_units; unit += gridDim.x) {
         int blk = unit / subs_per_block, sub = unit - blk * subs_per_block;
@@ -62,21 +116,37 @@ sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int
         const int kcnt = (blk < nfull) ? kbs : k_few;
         const int s0 = sub * SPR_SR;
         const int len = min(SPR_SR, n_blk - s0);
-        for (int i = threadIdx.x; i < len; i += SPR_THREADS) acc[i] = 0.0f;
-        __syncthreads();
-        for (int r = 0; r < rows; ++r) {
-            const int64_t row0 = (int64_t)r * k + (int64_t)blk * kbs;
-            const float coef = M[r];
-            for (int j = threadIdx.x; j < kcnt; j += SPR_THREADS) {
-                const int pos = (int)I[row0 + j] - s0;
-                if (pos >= 0 && pos < len) acc[pos] = __fadd_rn(acc[pos], __fmul_rn(coef, load_value<TV>(V, row0 + j)));
+        const int64_t row0 = (int64_t)blk * kbs;
+        for (int i = t; i < len; i += SPR_THREADS) acc[i] = 0.0f;
+        for (int r0 = 0; r0 < rows; r0 += SPR_AHEAD) {
+            int pos[SPR_AHEAD];
+            float val[SPR_AHEAD];
+#pragma unroll
+            for (int i = 0; i < SPR_AHEAD; ++i) {
+                const bool on = r0 + i < rows && t < kcnt;
+                const int64_t at = (int64_t)(r0 + i) * k + row0 + t;
+                pos[i] = on ? (int)I[at] - s0 : -1;
+                val[i] = on ? __fmul_rn(M[r0 + i], load_value<TV>(V, at)) : 0.0f;
             }
-            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < SPR_AHEAD; ++i) {
+                if (r0 + i < rows) {                             // uniform
+                    __syncthreads();                             // the row before (or the clearing) is done
+                    if (pos[i] >= 0 && pos[i] < len) acc[pos[i]] = __fadd_rn(acc[pos[i]], val[i]);
+                    for (int j = t + SPR_THREADS; j < kcnt; j += SPR_THREADS) {
+                        const int64_t at = (int64_t)(r0 + i) * k + row0 + j;
+                        const int p = (int)I[at] - s0;
+                        if (p >= 0 && p < len) acc[p] = __fadd_rn(acc[p], __fmul_rn(M[r0 + i], load_value<TV>(V, at)));
+                    }
+                }
+            }
         }
-        for (int i = threadIdx.x; i < len; i += SPR_THREADS) {
-            const int64_t e = blk_base + s0 + i;
-            Elem<TO>::store(out, e, __fadd_rn(Elem<TO>::load(out, e), acc[i]));
-        }
+        __syncthreads();
+        TO* o = out + blk_base + s0;
+        const int whole = ((reinterpret_cast<uintptr_t>(o) & 15) == 0) ? len / SPR_VEC<TO> : 0;
+        for (int i = t; i < whole; i += SPR_THREADS) add_vector(o + i * SPR_VEC<TO>, acc + i * SPR_VEC<TO>);
+        for (int i = whole * SPR_VEC<TO> + t; i < len; i += SPR_THREADS)
+            Elem<TO>::store(o, i, __fadd_rn(Elem<TO>::load(o, i), acc[i]));
         __syncthreads();
     }
 }
@@ -108,15 +178,15 @@ extern "C" int mab_sparse_rows_dot(int64_t d, int64_t rows, int64_t k, int64_t d
     MAB_REQUIRE((g_dtype == MAB_F32 || g_dtype == MAB_BF16) && (v_dtype == MAB_F32 || v_dtype == MAB_BF16), MAB_ERR_UNSUPPORTED,
                 "sparse_rows_dot: dtypes %d, %d", g_dtype, v_dtype);
     cudaStream_t s = (cudaStream_t)stream;
-    const int grid = (int)rows;
+    const int grid = (int)rows * SP_CLUSTER, kbs = (int)k_block_size;
     if (g_dtype == MAB_F32 && v_dtype == MAB_BF16)
-        sparse_rows_dot_kernel<float, uint16_t><<<grid, SP_THREADS, 0, s>>>(k, d_block_size, k_block_size, (const float*)g, I, V, out);
+        sparse_rows_dot_kernel<float, uint16_t><<<grid, SP_THREADS, 0, s>>>(k, d_block_size, kbs, nfull, k_few, (const float*)g, I, V, out);
     else if (g_dtype == MAB_F32)
-        sparse_rows_dot_kernel<float, float><<<grid, SP_THREADS, 0, s>>>(k, d_block_size, k_block_size, (const float*)g, I, V, out);
+        sparse_rows_dot_kernel<float, float><<<grid, SP_THREADS, 0, s>>>(k, d_block_size, kbs, nfull, k_few, (const float*)g, I, V, out);
     else if (v_dtype == MAB_BF16)
-        sparse_rows_dot_kernel<uint16_t, uint16_t><<<grid, SP_THREADS, 0, s>>>(k, d_block_size, k_block_size, (const uint16_t*)g, I, V, out);
+        sparse_rows_dot_kernel<uint16_t, uint16_t><<<grid, SP_THREADS, 0, s>>>(k, d_block_size, kbs, nfull, k_few, (const uint16_t*)g, I, V, out);
     else
-        sparse_rows_dot_kernel<uint16_t, float><<<grid, SP_THREADS, 0, s>>>(k, d_block_size, k_block_size, (const uint16_t*)g, I, V, out);
+        sparse_rows_dot_kernel<uint16_t, float><<<grid, SP_THREADS, 0, s>>>(k, d_block_size, kbs, nfull, k_few, (const uint16_t*)g, I, V, out);
     count_launch();
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? MAB_OK : cuda_fail(e, "sparse_rows_dot_kernel launch");
@@ -137,10 +207,13 @@ extern "C" int mab_sparse_rows_combine(int64_t d, int64_t rows, int64_t k, int64
     const int64_t tail = d - (int64_t)nfull * dbs;
     const int64_t units = (int64_t)nfull * subs + (tail > 0 ? (tail + SPR_SR - 1) / SPR_SR : 0);
     if (units == 0) return MAB_OK;
-    const int grid = (int)std::min<int64_t>(units, (int64_t)device_sm_count() * 4);
+    const int grid = (int)std::min<int64_t>(units, (int64_t)device_sm_count() * 3);
+    const int smem = SPR_SR * (int)sizeof(float);
     cudaStream_t s = (cudaStream_t)stream;
-#define MAB_LAUNCH_COMBINE(TO, TV) sparse_rows_combine_kernel<TO, TV><<<grid, SPR_THREADS, 0, s>>>( \
-        d, (int)rows, k, dbs, (int)k_block_size, nfull, k_few, M, I, V, (TO*)out, (int)units)
+#define MAB_LAUNCH_COMBINE(TO, TV) do { \
+        MAB_CUDA_TRY(cudaFuncSetAttribute(sparse_rows_combine_kernel<TO, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
+        sparse_rows_combine_kernel<TO, TV><<<grid, SPR_THREADS, smem, s>>>(d, (int)rows, k, dbs, (int)k_block_size, nfull, k_few, \
+                                                                           M, I, V, (TO*)out, (int)units); } while (0)
     if (out_dtype == MAB_F32 && v_dtype == MAB_BF16) MAB_LAUNCH_COMBINE(float, uint16_t);
     else if (out_dtype == MAB_F32) MAB_LAUNCH_COMBINE(float, float);
     else if (v_dtype == MAB_BF16) MAB_LAUNCH_COMBINE(uint16_t, uint16_t);
