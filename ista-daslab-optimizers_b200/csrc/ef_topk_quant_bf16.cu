@@ -36,8 +36,10 @@ constexpr int S_NT = 256;
 constexpr int S_CTAS = 3;                    // resident CTAs per SM the shared memory is sized for
 constexpr int S_SLOTS = SEL_MAX_TILE / 8 / S_NT;   // octets per thread: 16
 constexpr int S_WPT = SEL_WORDS / S_NT;      // bitmap words per thread: 4
-constexpr int S_CAND_CAP = 1536;
-constexpr int S_WLIST = 128;                 // octets with a candidate, per warp
+constexpr int S_CAND_CAP = 2144;             // what three CTAs per SM leave room for ...
+constexpr int S_MAX_K = 1536;                // ... and the largest k it is tried for: c of 3632 octets at the bound hold about
+                                             //     -3632 ln(1 - c / 3632) candidates, 2003 at c = 1536
+constexpr int S_WLIST = 384;                 // octets with a candidate, per warp
 constexpr int S_QTAB = 512;                  // quantisation blocks whose constants fit the tables
 constexpr int S_MAX_TENSORS = WIN_MAX_TENSORS;   // one limit for every kernel of a fused launch
 static_assert(S_WPT == 4, "a thread owns four consecutive bitmap words");
@@ -63,9 +65,13 @@ struct __align__(16) SmemSel {
             float  r0[S_QTAB];           //   1/u for the encoder, 0 where the defining form must run
         } qt;
     };
-    uint32_t sel_bm[SEL_WORDS];          // selected positions
-    uint16_t sel_before[SEL_WORDS];      // selected positions in lower words
-    uint16_t oct_list[(S_NT / 32) * S_WLIST];
+    union {
+        struct {
+            uint32_t sel_bm[SEL_WORDS];      // selected positions
+            uint16_t sel_before[SEL_WORDS];  // selected positions in lower words
+        };
+        uint16_t oct_list[(S_NT / 32) * S_WLIST];      // before that: octets with a candidate
+    };
     int      hist[256];
     uint32_t member[32];
     int      rot[64];
@@ -440,7 +446,6 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
         if (t == 0) { ss.kmax = 0; ss.n_member = 0; ss.n_cand = 0; ss.ctrl[4] = 0; ss.ctrl[slow_slot ^ 3] = 0; }
         if (t < 64) ss.rot[t] = 0;
         ss.hist[t] = 0;
-        reinterpret_cast<uint4*>(ss.sel_bm)[t] = make_uint4(0u, 0u, 0u, 0u);
         if (staged) {
             if (t == 0 && !issued) {
                 fence_async_smem();
@@ -541,9 +546,12 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
             resolve_selection_regs(gt, tw, 0, ss);
             done = true;
         }
-        if (!done && kmax < 0x7f800000 && k <= n_oct) {
-            // lower bound of the k-th key on octet maxima: at least k octets reach it, at most ~1.5 k
-            const int accept = k + (k >> 1) + 8;
+        if (!done && kmax < 0x7f800000 && k <= n_oct && k <= S_MAX_K) {
+            // lower bound of the k-th key on octet maxima: at least k octets reach it, at most ~1.5 k (fewer where that would
+            // bring more candidates than the list holds).  With room for 1536 candidates and 128 listed octets per warp, k = 5 %
+            // of a tile always, and 2 % sometimes, went to the bisection below: a step of 67 M elements took 700 and 327 us, now
+            // 491 and 287.
+            const int accept = k + (k > 1024 ? 112 : (k >> 1) + 8);
             int lo = 0, hi = kmax + 1, step = 1 << 20;
             int gq = (guess > 0 && guess <= kmax) ? guess : max(1, kmax - (2 << 23));
             bool have_lo = false, have_hi = false;
@@ -616,6 +624,7 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
                 const int n_cand = ss.n_cand;
                 if (n_cand <= S_CAND_CAP && ss.ctrl[4] == 0) {
                     C = n_cand;
+                    reinterpret_cast<uint4*>(ss.sel_bm)[t] = make_uint4(0u, 0u, 0u, 0u);   // (the lists are done with; the barrier below publishes it)
                     // 2. the k-th largest candidate.  The composite values are distinct, so no ties are left to
                     //    break.  256-bin radix levels over the live range, filled by all threads; every warp
                     //    reads the histogram for itself (no barrier for the result); the last <= 32 members
