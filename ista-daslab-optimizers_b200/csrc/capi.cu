@@ -56,16 +56,18 @@ extern "C" const char* mab_last_error(void) { return g_error; }
 extern "C" int64_t mab_kernel_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 
 extern "C" int mab_device_error(void) {
-    int a = 0, b = 0, c = 0;
+    int a = 0, b = 0, c = 0, d = 0;
     if (int rc = copy_timeout_f32(&a, false)) return rc;
+    if (int rc = copy_timeout_f32_split(&d, false)) return rc;
     if (int rc = copy_timeout_bf16(&b, false)) return rc;
     if (int rc = copy_timeout_window(&c, false)) return rc;
-    return (a | b | c) ? 1 : 0;
+    return (a | b | c | d) ? 1 : 0;
 }
 
 extern "C" int mab_device_error_clear(void) {
     int v = 0;
     if (int rc = copy_timeout_f32(&v, true)) return rc;
+    if (int rc = copy_timeout_f32_split(&v, true)) return rc;
     if (int rc = copy_timeout_bf16(&v, true)) return rc;
     return copy_timeout_window(&v, true);
 }
@@ -243,7 +245,7 @@ static int fused_run(mab_tensor* tensors, int n, const mab_step_args* args, void
         for (const Chunk& c : chunks) {
             const LooseArgs la = {qbs, reinterpret_cast<uint32_t*>(ws + L.off_min), reinterpret_cast<uint32_t*>(ws + L.off_max),
                                   reinterpret_cast<const int64_t*>(ws + L.off_first) + c.first};
-            if (int rc = launch_ef_topk_quant(dev + c.first, c.count, c.units_a, c.grad_dtype, qbs, c.max_dbs, s, &la)) return rc;
+            if (int rc = launch_ef_topk_quant(dev + c.first, c.count, c.units_a, c.grad_dtype, qbs, c.max_dbs, c.max_k, s, &la)) return rc;
         }
         for (const Chunk& c : chunks) {
             const LooseArgs la = {qbs, reinterpret_cast<uint32_t*>(ws + L.off_min), reinterpret_cast<uint32_t*>(ws + L.off_max),
@@ -252,7 +254,7 @@ static int fused_run(mab_tensor* tensors, int n, const mab_step_args* args, void
         }
     } else if (what & RUN_A) {
         for (const Chunk& c : chunks)
-            if (int rc = launch_ef_topk_quant(dev + c.first, c.count, c.units_a, c.grad_dtype, args->quant_block_size, c.max_dbs, s)) return rc;
+            if (int rc = launch_ef_topk_quant(dev + c.first, c.count, c.units_a, c.grad_dtype, args->quant_block_size, c.max_dbs, c.max_k, s)) return rc;
     }
     if (what & RUN_B) {
         WindowArgs wa;
@@ -367,7 +369,7 @@ extern "C" int mab_fused_step_static(mab_tensor* tensors, int n, const mab_step_
     // kernel A over every run, then kernel B over every run (the runs are recomputed, not stored)
     for (int first = 0; first < n;) {
         const int end = static_run_end(tensors, n, first, &ua, &ub, &mk, &md);
-        if (int rc = launch_ef_topk_quant(dev + first, end - first, ua, tensors[first].grad_dtype, args->quant_block_size, md, s)) return rc;
+        if (int rc = launch_ef_topk_quant(dev + first, end - first, ua, tensors[first].grad_dtype, args->quant_block_size, md, mk, s)) return rc;
         first = end;
     }
     wa.probe = args->probe_out;

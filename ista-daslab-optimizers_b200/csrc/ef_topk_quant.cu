@@ -459,9 +459,13 @@ ef_topk_quant_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int 
 int units_a_of(const mab_tensor& t) { return t.topk_full_blocks_count + (t.k_block_size_few > 0 ? 1 : 0); }
 
 int launch_ef_topk_quant(const mab_tensor* dev_tensors, int n_tensors, int total_units, int grad_dtype,
-                         int qbs, int max_dbs, cudaStream_t s, const LooseArgs* loose) {
+                         int qbs, int max_dbs, int max_k, cudaStream_t s, const LooseArgs* loose) {
     if (grad_dtype == MAB_BF16) {          // bf16 tiles are small enough for two shared-memory resident CTAs per SM
         const int rc = launch_ef_topk_quant_bf16(dev_tensors, n_tensors, total_units, qbs, max_dbs, s, loose);
+        if (rc <= 0) return rc;
+    }
+    if (grad_dtype == MAB_F32 && loose == nullptr) {   // two CTAs per SM while tile and candidates fit
+        const int rc = launch_ef_topk_quant_f32(dev_tensors, n_tensors, total_units, qbs, max_dbs, max_k, s);
         if (rc <= 0) return rc;
     }
     const int grid = (int)std::min<int64_t>(total_units, (int64_t)device_sm_count());

@@ -63,7 +63,7 @@ __device__ __forceinline__ int loose_block(int r, int qbs, bool big) {
 
 // ef_topk_quant.cu
 int launch_ef_topk_quant(const mab_tensor* dev_tensors, int n_tensors, int total_units, int grad_dtype,
-                         int qbs, int max_dbs, cudaStream_t s, const LooseArgs* loose = nullptr);
+                         int qbs, int max_dbs, int max_k, cudaStream_t s, const LooseArgs* loose = nullptr);
 int units_a_of(const mab_tensor& t);
 
 // requant_loose.cu: statistics (bf16) and codes of the residual kernel A left in the gradient buffers
@@ -74,9 +74,13 @@ int launch_requant_loose(const mab_tensor* dev_tensors, int n_tensors, int total
 int launch_ef_topk_quant_bf16(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, cudaStream_t s,
                               const LooseArgs* loose = nullptr);
 
+// ef_topk_quant_f32.cu: returns 1 (without launching) where the tile or its candidates do not fit
+int launch_ef_topk_quant_f32(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, int max_k, cudaStream_t s);
+
 // Each kernel file keeps its own "a bounded wait gave up" flag (no relocatable device code): these read
 // it into *out and optionally clear it.
 int copy_timeout_f32(int* out, bool clear);      // ef_topk_quant.cu
+int copy_timeout_f32_split(int* out, bool clear);   // ef_topk_quant_f32.cu
 int copy_timeout_bf16(int* out, bool clear);     // ef_topk_quant_bf16.cu
 int copy_timeout_window(int* out, bool clear);   // window_adam.cu
 

@@ -1,0 +1,115 @@
+"""The fp32 kernel A that keeps a tile's first 8192 elements in registers and the rest in shared memory, against the
+CPU oracle where it can go wrong: tiles that end around that border, short octets, buffers that start anywhere, every
+quantisation block size, and selections that leave the fast route."""
+import pytest
+import torch
+
+import cases
+from ista_daslab_optimizers_b200 import synthetic as S
+
+pytestmark = pytest.mark.gpu
+
+DBS = 29056
+SIZES = (8184, 8191, 8192, 8193, 8200, DBS - 1, DBS, DBS + 8192 + 8, 2 * DBS + 8195)
+
+
+def _gradient(kind, n, step):
+    g = S.normal_tensor(31 + step, n, n, 1e-3)
+    if kind == 'ties':                                   # more equal magnitudes than the candidate list holds
+        g[::3] = 2e-3 * torch.sign(g[::3])
+    elif kind == 'border':                               # everything that is selected sits around the border
+        g[8000:8400] *= 100.0
+    elif kind == 'few':
+        g.zero_()
+        g[:: max(1, n // 5)] = -1.5
+    elif kind == 'inf':
+        g[n // 2] = float('inf')
+    return g
+
+
+@pytest.mark.parametrize('kind,qbs,k_init,alpha,skip', [
+    ('normal', 64, 0.01, 0.0, 0), ('normal', 64, 0.01, 0.0, 3), ('normal', 8, 0.02, 0.0, 0), ('normal', 16, 0.005, 0.0, 4),
+    ('normal', 128, 0.05, 0.0, 0), ('normal', 64, 0.0647, 0.0, 0),       # k = 1880, the largest this kernel takes
+    ('normal', 32, 0.01, -2.0, 0), ('ties', 64, 0.02, 0.0, 0), ('ties', 64, 0.05, -2.0, 1), ('border', 64, 0.01, 0.0, 0),
+    ('few', 64, 0.01, 0.0, 0), ('inf', 64, 0.01, 0.0, 0)])
+def test_split_tile_matches_oracle(kind, qbs, k_init, alpha, skip):
+    from ista_daslab_optimizers_b200 import MicroAdam, _native
+    from oracle.microadam_oracle import MicroAdamOracle
+    hyper = dict(m=4, lr=1e-3, quant_block_size=qbs, k_init=k_init, weight_decay=0.1, alpha=int(alpha))
+    buffers = [S.normal_tensor(30, i, n + skip, 0.02).cuda() for i, n in enumerate(SIZES)]
+    params = [torch.nn.Parameter(b[skip:]) for b in buffers]
+    cpu = [p.detach().cpu().clone() for p in params]
+    opt = MicroAdam(params, **hyper)
+    ref = MicroAdamOracle(cpu, d_block_size=opt.d_block_size, **hyper)
+    assert opt.d_block_size == DBS
+    for step in range(1 if kind == 'inf' else 3):
+        grads = [_gradient(kind, n, step) for n in SIZES]
+        for p, g in zip(params, grads):
+            p.grad = torch.empty(g.numel() + skip, device='cuda')[skip:].copy_(g)
+        opt.step()
+        ref.step([g.clone() for g in grads])
+        assert all(e.fused for e in opt._entries)
+        for i, (p, n) in enumerate(zip(params, SIZES)):
+            a, b, used = opt.state[p], ref.state[i], -(-n // qbs)
+            row = step % hyper['m']
+            assert torch.equal(a['I'][row].cpu(), b['I'][row]), (n, step)
+            for key, cut in (('error', None), ('min_vals', used), ('max_vals', used)):
+                assert torch.equal(a[key][:cut].cpu().view(torch.uint8), b[key][:cut].view(torch.uint8)), (n, step, key)
+            assert torch.equal(a['V'][row].cpu().view(torch.int16), b['V'][row].view(torch.int16)), (n, step)
+            if kind != 'inf':                            # the update itself: the tolerance the parameters have everywhere
+                rtol, atol = cases.param_tolerances(torch.float32, hyper['lr'])
+                torch.testing.assert_close(p.detach().cpu(), cpu[i], rtol=rtol, atol=atol)
+    assert _native.device_error() == 0
+
+
+@pytest.mark.parametrize('rows', [8, 9, 17])
+def test_sparse_rows_many_blocks(rows):
+    """More top-k blocks than a cluster has warps, rows around the number fetched ahead."""
+    from ista_daslab_optimizers_b200 import _native as N
+    from oracle import microadam_oracle as O
+    d, k_init = 131 * DBS + 777, 0.003
+    geo = O.Geometry.make(d, DBS, k_init, 64)
+    gen = torch.Generator().manual_seed(rows)
+    few = geo.k - geo.topk_full_blocks_count * geo.k_block_size_many
+    I = torch.empty(rows, geo.k, dtype=torch.int16)
+    for r in range(rows):
+        full = torch.rand(geo.topk_full_blocks_count, DBS, generator=gen).topk(geo.k_block_size_many, dim=1).indices.sort(dim=1).values
+        tail = torch.rand(777, generator=gen).topk(few).indices.sort().values
+        I[r] = torch.cat([full.reshape(-1), tail]).to(torch.int16)
+    V = torch.randn(rows, geo.k, generator=gen).bfloat16()
+    g, M, out = torch.randn(d, generator=gen), torch.randn(rows, generator=gen), torch.randn(d, generator=gen)
+    dots, dots_g, out_g = torch.zeros(rows), torch.zeros(rows, device='cuda'), out.cuda()
+    args = (d, rows, geo.k, geo.d_block_size, geo.k_block_size_many)
+    O.sparse_rows_dot(*args, g, I, V, dots)
+    N.sparse_rows_dot(*args, g.cuda(), I.cuda(), V.cuda(), dots_g)
+    # a sum of k products of unit size in fp32: |error| <= k * 2^-24 * sum |v g| ~ 1e-4 * sqrt(k) for either order
+    torch.testing.assert_close(dots_g.cpu(), dots, rtol=1e-4, atol=1e-4 * geo.k ** 0.5)
+    O.sparse_rows_combine(*args, M, I, V, out)
+    N.sparse_rows_combine(*args, M.cuda(), I.cuda(), V.cuda(), out_g)
+    assert torch.equal(out.view(torch.int32), out_g.cpu().view(torch.int32))
+
+
+@pytest.mark.parametrize('dtype,alpha', [(torch.float32, 0.5), (torch.bfloat16, 0.1), (torch.bfloat16, -2)])
+@pytest.mark.parametrize('skip,qbs', [(1, 64), (3, 128), (4, 8)])
+def test_alpha_forms_on_slices_that_start_anywhere(dtype, alpha, skip, qbs):
+    """The octet-wide alpha forms of the update with unaligned parameters, whole and short last quantisation blocks."""
+    from ista_daslab_optimizers_b200 import MicroAdam
+    from oracle.microadam_oracle import MicroAdamOracle
+    sizes = (7, 200, 4096, DBS + 8 * 5, DBS + 1003)
+    hyper = dict(m=3, lr=1e-3, quant_block_size=qbs, k_init=0.02, weight_decay=0.1, alpha=alpha)
+    params = [torch.nn.Parameter(S.normal_tensor(40, i, n + skip, 0.02).to(dtype).cuda()[skip:]) for i, n in enumerate(sizes)]
+    cpu = [p.detach().cpu().clone() for p in params]
+    opt = MicroAdam(params, **hyper)
+    ref = MicroAdamOracle(cpu, d_block_size=opt.d_block_size, **hyper)
+    for step in range(4):
+        grads = [S.normal_tensor(41 + step, n, n, 1e-3).to(dtype) for n in sizes]
+        for p, g in zip(params, grads):
+            p.grad = torch.empty(g.numel() + skip, dtype=dtype, device='cuda')[skip:].copy_(g)
+        opt.step()
+        ref.step([g.clone() for g in grads])
+        for i, (p, n) in enumerate(zip(params, sizes)):
+            a, b, used = opt.state[p], ref.state[i], -(-n // qbs)
+            for key, cut in (('error', None), ('min_vals', used), ('max_vals', used)):
+                assert torch.equal(a[key][:cut].cpu().view(torch.uint8), b[key][:cut].view(torch.uint8)), (n, step, key)
+            rtol, atol = cases.param_tolerances(dtype, hyper['lr'])
+            torch.testing.assert_close(p.detach().cpu().float(), cpu[i].float(), rtol=rtol, atol=atol)
