@@ -7,13 +7,18 @@
 // other's arithmetic.  The shared-memory part is staged by the bulk copy engine and turned into a = g + Qinv(e) in
 // place; the tile after this one is asked into L2 meanwhile.
 //
-// Thread t owns octets t, t + 512, ...: the first two in registers, the rest in shared memory, so every octet-wise
-// phase (decode, statistics, encode) is the same code for both.  An octet in shared memory is two 16-byte pieces 32
-// bytes apart from the next lane's: lanes 4-7 of every 8 take the second piece first (`h`), so that a quarter warp's
-// 16-byte accesses cover all banks; the code word is rotated by 16 bits to match.
+// Thread t owns octets 2 t and 2 t + 1 (registers) and 1024 + t, 1024 + t + 512, ... (shared memory).  An octet in shared
+// memory is two 16-byte pieces 32 bytes apart from the next lane's: lanes 4-7 of every 8 take the second piece first
+// (`h`), so that a quarter warp's 16-byte accesses cover all banks; the code word is rotated by 16 bits to match.
 //
-// Bound by instruction issue (64 instructions per element, 62 % of the issue slots), not by memory: kernel A on 67.1 M
-// elements 204 us, 1.66 TB/s; a step of one 124.4 M tensor 606 -> 571 us, of 67.1 M with k = 5 % 672 -> 657.
+// Regular tiles (whole blocks of 64, seven whole octets per thread, aligned buffers, every block with a finite positive
+// step: all but a tensor's last tile) take a leaner route: the decode has no branches and writes a with the sixteen
+// 16-byte pieces of every 256-byte row (= one quantisation block) permuted by the row number (piece c of row r sits at
+// c ^ (r & 7)), so that after the selection a thread owns whole rows, consecutive lanes reading different banks, and
+// computes a block's statistics, constants and 32 code bytes without shuffles.
+//
+// Bound by instruction issue and the phases' barriers, not by memory: a step of one 124.4 M tensor takes 606 us with one
+// tile per SM, 571 with two, 499 with the regular route; 67.1 M with k = 5 % 602, 586 and 556.
 #include "common.cuh"
 #include "select.cuh"
 #include "codec_fast.cuh"
@@ -28,6 +33,7 @@ constexpr int F_REG = 2;                     // octets a thread keeps in registe
 constexpr int F_SLOTS = SEL_MAX_TILE / 8 / F_NT;   // octets per thread: 8
 constexpr int F_REG_ELEMS = F_REG * F_NT * 8;      // tile elements that never enter shared memory
 constexpr int F_WPT = SEL_WORDS / F_NT;      // bitmap words per thread: 2
+constexpr int F_FULL = 5;                    // shared-memory octets every thread of a regular tile owns (some own one more)
 constexpr int F_CAND_CAP = 3072;
 constexpr int F_WLIST = 192;                 // shared-memory octets with a candidate, per warp
 constexpr int F_MAX_K = 1880;                // largest k whose candidates fit the list (see launch_ef_topk_quant_f32)
@@ -57,7 +63,7 @@ struct __align__(16) SmemF {
     int rot[64];
     int counters[40];
     int scan[36];
-    int n_member, n_cand, kmax, over;
+    int n_member, n_cand, kmax, over, slow, pad[3];
 };
 constexpr int F_QTAB = F_CAND_CAP * 6 / 8;   // quantisation blocks whose constants fit the table: 2304 (all of a tile's when they have 16 elements or more)
 static_assert(sizeof(uint16_t) * (F_NT / 32) * F_WLIST <= (4 + 2) * SEL_WORDS, "the octet lists reuse the bitmap");
@@ -73,14 +79,22 @@ __device__ __forceinline__ int f32_warp_alloc(int cnt, int* counter) {
     return base + inc - cnt;
 }
 
-// An octet of the shared-memory part; h: which of its two 16-byte pieces comes first in v.
-__device__ __forceinline__ void octet_from_smem(const float4* tile4, int o, int h, float (&v)[8]) {
-    const float4 a = tile4[o * 2 + h], b = tile4[o * 2 + (h ^ 1)];
+// The octet thread t owns in slot j.
+__device__ __forceinline__ int f32_oct(int j) { return j < F_REG ? F_REG * (int)threadIdx.x + j : j * F_NT + (int)threadIdx.x; }
+
+// Where element e of the shared-memory part sits on a permuted (regular) tile.
+__device__ __forceinline__ int f32_phys(int e, bool swz) { return swz ? e ^ (((e >> 6) & 7) << 2) : e; }
+
+// Octet o of the shared-memory part; h: which of its two 16-byte pieces comes first in v.
+__device__ __forceinline__ void octet_from_smem(const float4* tile4, int o, int h, bool swz, float (&v)[8]) {
+    const int at = (o * 2 + h) ^ (swz ? (o >> 3) & 7 : 0);
+    const float4 a = tile4[at], b = tile4[at ^ 1];
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
-__device__ __forceinline__ void octet_to_smem(float4* tile4, int o, int h, const float (&v)[8]) {
-    tile4[o * 2 + h] = make_float4(v[0], v[1], v[2], v[3]);
-    tile4[o * 2 + (h ^ 1)] = make_float4(v[4], v[5], v[6], v[7]);
+__device__ __forceinline__ void octet_to_smem(float4* tile4, int o, int h, bool swz, const float (&v)[8]) {
+    const int at = (o * 2 + h) ^ (swz ? (o >> 3) & 7 : 0);
+    tile4[at] = make_float4(v[0], v[1], v[2], v[3]);
+    tile4[at ^ 1] = make_float4(v[4], v[5], v[6], v[7]);
 }
 __device__ __forceinline__ uint32_t rotate_codes(uint32_t w, int h) { return __funnelshift_l(w, w, h << 4); }
 
@@ -96,6 +110,26 @@ __device__ __noinline__ uint32_t encode_octet_scalar(const float* r, float mn, f
     return w;
 }
 
+__device__ __forceinline__ float octet_max_abs(const float (&v)[8]) {
+    const float m0 = max3(fabsf(v[0]), fabsf(v[1]), fabsf(v[2])), m1 = max3(fabsf(v[3]), fabsf(v[4]), fabsf(v[5]));
+    return max3(m0, m1, fmaxf(fabsf(v[6]), fabsf(v[7])));
+}
+__device__ __forceinline__ void add_octet(float (&v)[8], const float (&x)[8]) {
+#pragma unroll
+    for (int b = 0; b < 8; b += 2) {
+        const float2 s = __fadd2_rn(make_float2(v[b], v[b + 1]), make_float2(x[b], x[b + 1]));
+        v[b] = s.x; v[b + 1] = s.y;
+    }
+}
+// v <- v + Qinv(codes) with the constants (min, u) of a block whose step is finite and positive; returns the largest |v|.
+__device__ __forceinline__ float accumulate_regular(float (&v)[8], uint32_t codes, float2 mu) {
+    const QParams q = {mu.x, mu.y};
+    float x[8];
+    decode_octet_fast(codes, decode_consts(q), x);
+    add_octet(v, x);
+    return octet_max_abs(v);
+}
+
 // v <- v + Qinv(codes), elements from `cnt` on to 0; returns the largest |v|.
 __device__ __forceinline__ float accumulate_octet(float (&v)[8], uint32_t codes, const QParams& q, int cnt) {
     const DecodeConsts dc = decode_consts(q);
@@ -108,21 +142,70 @@ __device__ __forceinline__ float accumulate_octet(float (&v)[8], uint32_t codes,
 #pragma unroll
         for (int e = 0; e < 8; ++e) x[e] = y[e];
     }
-#pragma unroll
-    for (int b = 0; b < 8; b += 2) {
-        const float2 s = __fadd2_rn(make_float2(v[b], v[b + 1]), make_float2(x[b], x[b + 1]));
-        v[b] = s.x; v[b + 1] = s.y;
-    }
+    add_octet(v, x);
     if (cnt < 8) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) if (e >= cnt) v[e] = 0.0f;
     }
-    const float m0 = max3(fabsf(v[0]), fabsf(v[1]), fabsf(v[2])), m1 = max3(fabsf(v[3]), fabsf(v[4]), fabsf(v[5]));
-    return max3(m0, m1, fmaxf(fabsf(v[6]), fabsf(v[7])));
+    return octet_max_abs(v);
+}
+
+// Whether the codes of a block need no clamp: its values lie within half an ulp of bf16 (2^-8 of the larger statistic's
+// magnitude) of [mn, mx], which is less than half a step when that magnitude is at most 125 steps: the quotients then
+// stay in (-0.5, 15.5).
+__device__ __forceinline__ bool codes_in_range(uint16_t mn_b, uint16_t mx_b, const QParams& q) {
+    return fmaxf(fabsf(bf16_bits_to_f32(mn_b)), fabsf(bf16_bits_to_f32(mx_b))) <= 125.0f * q.u;
+}
+__device__ __forceinline__ bool step_in_range(const QParams& q) { return q.u >= CODEC_U_MIN && q.u <= CODEC_U_MAX; }
+
+// The 32 code bytes of row r of a regular tile (one quantisation block, pieces permuted by key = r & 7).
+template <bool CLAMP>
+__device__ __forceinline__ void encode_row(const float4* row, int key, const DivConsts& dc, uint4* dst) {
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+        uint32_t w[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float4 a = row[(half * 8 + 2 * c) ^ key], b = row[(half * 8 + 2 * c + 1) ^ key];
+            const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            w[c] = encode_octet_div_f32<CLAMP>(v, dc);
+        }
+        dst[half] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// Statistics and codes of the shared-memory part of a regular tile: thread t owns rows t, t + F_NT, ...
+__device__ __forceinline__ void stats_encode_rows(const float4* tile4, int n_rows, uint16_t* mn_out, uint16_t* mx_out, uint8_t* ef_out) {
+    for (int r = threadIdx.x; r < n_rows; r += F_NT) {
+        const float4* row = tile4 + (r << 4);
+        const int key = r & 7;
+        float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+            const float4 v = row[c ^ key];
+            lo = min3(min3(lo, v.x, v.y), v.z, v.w);
+            hi = max3(max3(hi, v.x, v.y), v.z, v.w);
+        }
+        const uint16_t mn_b = f32_to_bf16_bits_rne(lo), mx_b = f32_to_bf16_bits_rne(hi);
+        mn_out[r] = mn_b; mx_out[r] = mx_b;
+        const QParams q = qparams(mn_b, mx_b);
+        uint4* dst = reinterpret_cast<uint4*>(ef_out) + (r << 1);
+        if (!step_in_range(q)) {                             // all-equal block (u == 0), subnormal or infinite step
+            for (int o = 0; o < 8; ++o) {
+                float y[8];
+                for (int e = 0; e < 8; ++e) y[e] = reinterpret_cast<const float*>(row)[((o * 8 + e) ^ (key << 2))];
+                reinterpret_cast<uint32_t*>(dst)[o] = encode_octet_scalar(y, q.mn, q.u, 8);
+            }
+        } else if (codes_in_range(mn_b, mx_b, q)) {
+            encode_row<false>(row, key, div_consts(q), dst);
+        } else {
+            encode_row<true>(row, key, div_consts(q), dst);
+        }
+    }
 }
 
 // Number of the tile's keys >= thr (key bits), every thread of the CTA calling; `counter` is zero on entry.
-__device__ __forceinline__ int f32_count_ge(const float (&a)[F_REG][8], const float4* tile4, int n_oct, int thr, int* counter) {
+__device__ __forceinline__ int f32_count_ge(const float (&a)[F_REG][8], const float4* tile4, int n_oct, bool swz, int thr, int* counter) {
     const float thr_f = __int_as_float(thr);
     int c = 0;
 #pragma unroll
@@ -131,7 +214,7 @@ __device__ __forceinline__ int f32_count_ge(const float (&a)[F_REG][8], const fl
         for (int e = 0; e < 8; ++e) c += (fabsf(a[j][e]) >= thr_f) ? 1 : 0;
     for (int o = threadIdx.x + F_REG * F_NT; o < n_oct; o += F_NT) {
         float v[8];
-        octet_from_smem(tile4, o - F_REG * F_NT, 0, v);
+        octet_from_smem(tile4, o - F_REG * F_NT, 0, swz, v);
 #pragma unroll
         for (int e = 0; e < 8; ++e) c += (fabsf(v[e]) >= thr_f) ? 1 : 0;
     }
@@ -175,7 +258,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
     SmemF& ss = *reinterpret_cast<SmemF*>(smem_raw + tile_bytes);
     const int t = threadIdx.x, lane = lane_id(), warp = warp_id();
     for (int i = t; i < n_tensors; i += F_NT) s_first[i] = tensors[i].first_unit_a;
-    if (t == 0) { s_first[n_tensors] = total_units; mbar_init(&s_bar, 1); }
+    if (t == 0) { s_first[n_tensors] = total_units; mbar_init(&s_bar, 1); ss.slow = 0; }
     __syncthreads();
     const int oshift = qshift - 3;              // octets per quantisation block, as a shift
     const int lanes_per_qb = 1 << oshift;
@@ -221,7 +304,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
         float a[F_REG][8];
 #pragma unroll
         for (int j = 0; j < F_REG; ++j) {
-            const int o = t + j * F_NT, cnt = n - o * 8;
+            const int o = f32_oct(j), cnt = n - o * 8;
             if (g_al16 && cnt >= 8) {
                 const float4 x = __ldg(reinterpret_cast<const float4*>(g) + o * 2), y = __ldg(reinterpret_cast<const float4*>(g) + o * 2 + 1);
                 a[j][0] = x.x; a[j][1] = x.y; a[j][2] = x.z; a[j][3] = x.w; a[j][4] = y.x; a[j][5] = y.y; a[j][6] = y.z; a[j][7] = y.w;
@@ -233,18 +316,24 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
         uint32_t cw[F_SLOTS];
         if (ef_al4 && whole) {
 #pragma unroll
-            for (int j = 0; j < F_SLOTS; ++j) { const int o = t + j * F_NT; cw[j] = o < n_oct ? reinterpret_cast<const uint32_t*>(ef)[o] : 0u; }
+            for (int j = 0; j < F_SLOTS; ++j) { const int o = f32_oct(j); cw[j] = o < n_oct ? reinterpret_cast<const uint32_t*>(ef)[o] : 0u; }
         } else {
 #pragma unroll
             for (int j = 0; j < F_SLOTS; ++j) {
-                const int o = t + j * F_NT;
+                const int o = f32_oct(j);
                 uint32_t w = 0;
                 for (int b = 0; b < 4; ++b) if (o * 8 + 2 * b < n) w |= (uint32_t)ef[o * 4 + b] << (8 * b);
                 cw[j] = w;
             }
         }
         if (tables) {
-            for (int b = t; b < n_qb; b += F_NT) { const QParams q = qparams(mn_g[b], mx_g[b]); ss.qtab[b] = make_float2(q.mn, q.u); }
+            bool slow = false;
+            for (int b = t; b < n_qb; b += F_NT) {
+                const QParams q = qparams(mn_g[b], mx_g[b]);
+                ss.qtab[b] = make_float2(q.mn, q.u);
+                slow |= !decode_consts(q).fast;
+            }
+            if (slow) ss.slow = 1;
         }
         if (staged) {
             const bool ok = mbar_wait(&s_bar, parity);
@@ -275,23 +364,46 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
 
         // ---- a = g + Qinv(e) in place; per-octet maxima stay in registers ------------------------------------
         const int h = whole ? (lane >> 2) & 1 : 0;                   // (a short octet needs its elements in order)
+        const int n_so = n_oct - F_REG * F_NT;                       // octets in shared memory
+        // regular tile: see the head of the file; its pieces are permuted from here on
+        const bool swz = staged && qshift == 6 && (n & 63) == 0 && n_so >= F_FULL * F_NT && (reinterpret_cast<uintptr_t>(ef) & 15) == 0 &&
+                         ss.slow == 0 && T.quant_err == nullptr;
         float omax[F_SLOTS];
+        if (swz) {
 #pragma unroll
-        for (int j = 0; j < F_SLOTS; ++j) {
-            const int o = t + j * F_NT;
-            omax[j] = 0.0f;
-            if (o < n_oct) {
-                QParams q;
-                if (tables) { const float2 c = ss.qtab[o >> oshift]; q.mn = c.x; q.u = c.y; }
-                else q = qparams(mn_g[o >> oshift], mx_g[o >> oshift]);
-                const int cnt = whole ? 8 : n - o * 8;
-                if (j < F_REG) {
-                    omax[j] = accumulate_octet(a[j < F_REG ? j : 0], cw[j], q, cnt);
-                } else {
+            for (int j = 0; j < F_REG; ++j) omax[j] = accumulate_regular(a[j], cw[j], ss.qtab[t >> 2]);
+#pragma unroll
+            for (int j = F_REG; j < F_SLOTS; ++j) {
+                const int so = t + (j - F_REG) * F_NT;
+                omax[j] = 0.0f;
+                if (j < F_REG + F_FULL || (so & ~31) < n_so) {       // whole warps: the 8 lanes of a row read it before they write it
+                    const bool on = j < F_REG + F_FULL || so < n_so;
+                    const int at = on ? so : 0;
                     float v[8];
-                    octet_from_smem(tile4, o - F_REG * F_NT, h, v);
-                    omax[j] = accumulate_octet(v, rotate_codes(cw[j], h), q, cnt);
-                    octet_to_smem(tile4, o - F_REG * F_NT, h, v);
+                    octet_from_smem(tile4, at, h, false, v);
+                    const float m = accumulate_regular(v, rotate_codes(cw[j], h), ss.qtab[(at >> 3) + F_REG_ELEMS / 64]);
+                    __syncwarp();
+                    if (on) { octet_to_smem(tile4, so, h, true, v); omax[j] = m; }
+                }
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < F_SLOTS; ++j) {
+                const int o = f32_oct(j);
+                omax[j] = 0.0f;
+                if (o < n_oct) {
+                    QParams q;
+                    if (tables) { const float2 c = ss.qtab[o >> oshift]; q.mn = c.x; q.u = c.y; }
+                    else q = qparams(mn_g[o >> oshift], mx_g[o >> oshift]);
+                    const int cnt = whole ? 8 : n - o * 8;
+                    if (j < F_REG) {
+                        omax[j] = accumulate_octet(a[j < F_REG ? j : 0], cw[j], q, cnt);
+                    } else {
+                        float v[8];
+                        octet_from_smem(tile4, o - F_REG * F_NT, h, false, v);
+                        omax[j] = accumulate_octet(v, rotate_codes(cw[j], h), q, cnt);
+                        octet_to_smem(tile4, o - F_REG * F_NT, h, false, v);
+                    }
                 }
             }
         }
@@ -306,6 +418,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
         }
         __syncthreads();
         const int kmax = ss.kmax;
+        if (t == 0) ss.slow = 0;                                     // (for the next tile)
         bool fast = false;                                           // the selection is described by the candidate list
         int C = 0;
         if (kmax > 0 && kmax < 0x7f800000 && k <= n_oct) {
@@ -349,7 +462,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
                                 for (int e = 0; e < 8; ++e) {
                                     if (mask & (1u << (8 * j + e))) {
                                         if (slot < F_CAND_CAP) {
-                                            const uint32_t bits = __float_as_uint(a[j][e]), pos = (uint32_t)(t + j * F_NT) * 8 + e;
+                                            const uint32_t bits = __float_as_uint(a[j][e]), pos = (uint32_t)f32_oct(j) * 8 + e;
                                             ss.key[slot] = bits & 0x7FFFFFFFu;
                                             ss.meta[slot] = (uint16_t)(((0x7FFFu - pos) << 1) | (bits >> 31));
                                         }
@@ -368,7 +481,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
                     const bool q = omax[j] >= lo_f;
                     const unsigned bal = __ballot_sync(0xffffffffu, q);
                     const int at = n_w + __popc(bal & ((1u << lane) - 1u));
-                    if (q && at < F_WLIST) wlist[at] = (uint16_t)(t + j * F_NT);
+                    if (q && at < F_WLIST) wlist[at] = (uint16_t)f32_oct(j);
                     n_w += __popc(bal);
                 }
                 if (lane == 0 && n_w > F_WLIST) ss.over = 1;
@@ -379,7 +492,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
                     if (e0 + lane < n_w) {
                         o = wlist[e0 + lane];
                         float v[8];
-                        octet_from_smem(tile4, (int)o - F_REG * F_NT, 0, v);
+                        octet_from_smem(tile4, (int)o - F_REG * F_NT, 0, swz, v);
 #pragma unroll
                         for (int e = 0; e < 8; ++e) mask |= (fabsf(v[e]) >= lo_f) ? (1u << e) : 0u;
                     }
@@ -388,7 +501,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
                         const uint32_t pos = (o << 3) + (__ffs(mask) - 1);
                         mask &= mask - 1;
                         if (slot < F_CAND_CAP) {
-                            const uint32_t bits = __float_as_uint(tile[(int)pos - F_REG_ELEMS]);
+                            const uint32_t bits = __float_as_uint(tile[f32_phys((int)pos - F_REG_ELEMS, swz)]);
                             ss.key[slot] = bits & 0x7FFFFFFFu;
                             ss.meta[slot] = (uint16_t)(((0x7FFFu - pos) << 1) | (bits >> 31));
                         }
@@ -477,7 +590,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
                         const int rank = ss.sel_before[w] + __popc(ss.sel_bm[w] & ((1u << (pos & 31)) - 1u));
                         i_out[rank] = (int16_t)pos;
                         v_out[rank] = f32_to_bf16_bits_rne(__uint_as_float(ss.key[i] | ((uint32_t)ss.meta[i] << 31)));
-                        if (pos >= (uint32_t)F_REG_ELEMS) tile[pos - F_REG_ELEMS] = 0.0f;
+                        if (pos >= (uint32_t)F_REG_ELEMS) tile[f32_phys((int)pos - F_REG_ELEMS, swz)] = 0.0f;
                     }
                 }
                 __syncthreads();
@@ -502,13 +615,13 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
                 int Tk = 0;
                 for (int bit = 30; bit >= 0; --bit) {
                     const int c = Tk | (1 << bit);
-                    if (f32_count_ge(a, tile4, n_oct, c, &ss.counters[bit]) >= k) Tk = c;
+                    if (f32_count_ge(a, tile4, n_oct, swz, c, &ss.counters[bit]) >= k) Tk = c;
                 }
-                need = k - f32_count_ge(a, tile4, n_oct, Tk + 1, &ss.counters[32]);
+                need = k - f32_count_ge(a, tile4, n_oct, swz, Tk + 1, &ss.counters[32]);
                 const float Tf = __int_as_float(Tk);
 #pragma unroll
                 for (int j = 0; j < F_SLOTS; ++j) {
-                    const int o = t + j * F_NT;
+                    const int o = f32_oct(j);
                     uint32_t gt = 0u, tie = 0u;
                     if (o < n_oct) {
                         float v[8];
@@ -516,7 +629,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
 #pragma unroll
                             for (int e = 0; e < 8; ++e) v[e] = a[j < F_REG ? j : 0][e];
                         } else {
-                            octet_from_smem(tile4, o - F_REG * F_NT, 0, v);
+                            octet_from_smem(tile4, o - F_REG * F_NT, 0, swz, v);
                         }
 #pragma unroll
                         for (int e = 0; e < 8; ++e) {                // (padding ties with T == 0 only, at the highest positions: never selected)
@@ -546,28 +659,28 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
 
         // ---- a[I] = 0 where that is still to be done; statistics; e = Q(a) ----------------------------------
         const uint8_t* sel_bytes = reinterpret_cast<const uint8_t*>(ss.sel_bm);
-        auto finish_octet = [&](int o, float (&v)[8], int hh) {      // whole warps call: the lanes of a block meet in the shuffles
-            const int cnt = n - o * 8;
-            if (T.quant_err != nullptr && cnt > 0) {                 // alpha == -2: the residual a also goes to the caller's buffer
-                float* qe = reinterpret_cast<float*>(T.quant_err) + base + o * 8;
-                for (int e = 0; e < min(cnt, 8); ++e) qe[e ^ (hh << 2)] = v[e];
-            }
-            float lo = INFINITY, hi = -INFINITY;
+        auto octet_stats = [&](const float (&v)[8], int cnt) {       // as the rounded pair (-min, max): bf16 rounding is monotone and
+            float lo = INFINITY, hi = -INFINITY;                     // odd, so a block's statistics are the maximum of its pairs
             if (cnt >= 8) {
                 octet_min_max(v, lo, hi);
             } else {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) if (e < cnt) { lo = fminf(lo, v[e]); hi = fmaxf(hi, v[e]); }
             }
-            // bf16 rounding is monotone and odd: the block's statistics are the maximum of the rounded (-min, max) pairs
-            uint32_t st = pack_bf16x2_rne(-lo, hi);
-            for (int off = 1; off < lanes_per_qb; off <<= 1) st = max_bf16x2(st, __shfl_xor_sync(0xffffffffu, st, off));
+            return pack_bf16x2_rne(-lo, hi);
+        };
+        auto finish_octet = [&](int o, const float (&v)[8], int hh, uint32_t st) {
+            const int cnt = n - o * 8;
             if (cnt <= 0) return;
+            if (T.quant_err != nullptr) {                            // alpha == -2: the residual a also goes to the caller's buffer
+                float* qe = reinterpret_cast<float*>(T.quant_err) + base + o * 8;
+                for (int e = 0; e < min(cnt, 8); ++e) qe[e ^ (hh << 2)] = v[e];
+            }
             const uint16_t mn_b = (uint16_t)((st & 0xFFFFu) ^ 0x8000u), mx_b = (uint16_t)(st >> 16);
             if ((o & (lanes_per_qb - 1)) == 0) { mn_g[o >> oshift] = mn_b; mx_g[o >> oshift] = mx_b; }
             const QParams q = qparams(mn_b, mx_b);
             uint32_t w;
-            if (cnt >= 8 && q.u >= CODEC_U_MIN && q.u <= CODEC_U_MAX) {
+            if (cnt >= 8 && step_in_range(q)) {
                 w = encode_octet_div_f32<true>(v, div_consts(q));    // values can lie outside statistics rounded to bf16: clamped
             } else {
                 float y[8];
@@ -580,7 +693,8 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
             else
                 for (int b = 0; b < 4; ++b) if (2 * b < cnt) ef[o * 4 + b] = (uint8_t)(w >> (8 * b));
         };
-        auto take_selected = [&](int o, float (&v)[8], uint32_t sel, bool emit) {
+        auto take_selected = [&](int o, float (&v)[8], bool emit) {
+            const uint32_t sel = sel_bytes[o];
             if (!sel) return;
             int p = ss.sel_before[o >> 2] + __popc(ss.sel_bm[o >> 2] & ((1u << (8 * (o & 3))) - 1u));
 #pragma unroll
@@ -590,25 +704,72 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
                     v[e] = 0.0f;
                 }
         };
+        if (swz && fast) {
+            // registers: the four lanes that hold a block's eight octets meet in two shuffles
+            const uint32_t sel2 = reinterpret_cast<const uint16_t*>(sel_bytes)[t];
+            float lo = INFINITY, hi = -INFINITY;
 #pragma unroll
-        for (int j = 0; j < F_REG; ++j) {
-            const int o = t + j * F_NT;
-            if ((o & ~31) < n_oct) {
-                take_selected(o, a[j], sel_bytes[o], !fast);
-                finish_octet(o, a[j], 0);
+            for (int j = 0; j < F_REG; ++j) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) a[j][e] = (sel2 & (1u << (8 * j + e))) ? 0.0f : a[j][e];
+                float l, u;
+                octet_min_max(a[j], l, u);
+                lo = fminf(lo, l); hi = fmaxf(hi, u);
             }
-        }
-#pragma unroll 2
-        for (int o = t + F_REG * F_NT; (o & ~31) < n_oct; o += F_NT) {
-            float v[8];
-            if (o < n_oct) {
-                octet_from_smem(tile4, o - F_REG * F_NT, fast ? h : 0, v);
+            uint32_t st = pack_bf16x2_rne(-lo, hi);
+            st = max_bf16x2(st, __shfl_xor_sync(0xffffffffu, st, 1));
+            st = max_bf16x2(st, __shfl_xor_sync(0xffffffffu, st, 2));
+            const uint16_t mn_b = (uint16_t)((st & 0xFFFFu) ^ 0x8000u), mx_b = (uint16_t)(st >> 16);
+            if ((t & 3) == 0) { mn_g[t >> 2] = mn_b; mx_g[t >> 2] = mx_b; }
+            const QParams q = qparams(mn_b, mx_b);
+            uint2 w;
+            if (step_in_range(q)) {
+                const DivConsts dc = div_consts(q);
+                w.x = encode_octet_div_f32<true>(a[0], dc);
+                w.y = encode_octet_div_f32<true>(a[1], dc);
             } else {
+                float y[F_REG][8];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] = 0.0f;
+                for (int j = 0; j < F_REG; ++j)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) y[j][e] = a[j][e];
+                w.x = encode_octet_scalar(y[0], q.mn, q.u, 8);
+                w.y = encode_octet_scalar(y[1], q.mn, q.u, 8);
             }
-            if (!fast) take_selected(o, v, sel_bytes[o], true);
-            finish_octet(o, v, fast ? h : 0);
+            reinterpret_cast<uint2*>(ef)[t] = w;
+            stats_encode_rows(tile4, n_so >> 3, mn_g + F_REG_ELEMS / 64, mx_g + F_REG_ELEMS / 64, ef + F_REG_ELEMS / 2);
+        } else {
+            {
+                uint32_t st[F_REG];
+#pragma unroll
+                for (int j = 0; j < F_REG; ++j) {
+                    const int o = f32_oct(j);
+                    take_selected(o, a[j], !fast);
+                    st[j] = octet_stats(a[j], n - o * 8);
+                }
+                if (oshift > 0) {                                    // both octets lie in one block
+                    st[0] = max_bf16x2(st[0], st[1]);
+                    for (int off = 1; off < (lanes_per_qb >> 1); off <<= 1) st[0] = max_bf16x2(st[0], __shfl_xor_sync(0xffffffffu, st[0], off));
+                    st[1] = st[0];
+                }
+#pragma unroll
+                for (int j = 0; j < F_REG; ++j) finish_octet(f32_oct(j), a[j], 0, st[j]);
+            }
+#pragma unroll 1
+            for (int o = t + F_REG * F_NT; (o & ~31) < n_oct; o += F_NT) {   // whole warps: the lanes of a block meet in the shuffles
+                float v[8];
+                const int hh = fast ? h : 0;
+                if (o < n_oct) {
+                    octet_from_smem(tile4, o - F_REG * F_NT, hh, swz, v);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[e] = 0.0f;
+                }
+                if (!fast) take_selected(o, v, true);
+                uint32_t st = octet_stats(v, n - o * 8);
+                for (int off = 1; off < lanes_per_qb; off <<= 1) st = max_bf16x2(st, __shfl_xor_sync(0xffffffffu, st, off));
+                finish_octet(o, v, hh, st);
+            }
         }
         __syncthreads();                                             // tile and scratch are overwritten by the next load
     }
