@@ -13,13 +13,12 @@
 // blocks t, t + 256; no shuffles).  For quant_block_size 64 the block tables fit the scratch; other
 // block sizes take general per-block code in the same kernel.
 //
-// Regular tiles (whole blocks of 64, every thread with 14 whole octets, all blocks with a finite
-// positive step) take a leaner route: the decode writes a into the tile with the octets of every
+// Regular tiles (blocks of 64, aligned codes, all blocks with a finite step) take a leaner route: the decode writes a into the tile with the octets of every
 // 128-byte row (= one quantisation block) permuted by the row number (octet o sits at o ^ ((o >> 3) & 7)),
 // so that afterwards a thread can own whole blocks - consecutive lanes own consecutive blocks and read
 // different banks - and computes a block's statistics, its constants and its 32 code bytes from
 // registers, with no tables and no shuffles.  The selection addresses the tile through the same
-// permutation.  Everything else (other block sizes, ragged tiles, degenerate blocks) keeps the
+// permutation.  Everything else (other block sizes, unaligned codes, degenerate blocks) keeps the
 // linear layout and the general code.
 //
 // Results are bit-identical to the register-resident kernel in ef_topk_quant.cu (same arithmetic,
@@ -100,13 +99,17 @@ __device__ __forceinline__ int warp_alloc(int cnt, int* counter) {
     return base + inc - cnt;
 }
 
+// Where octet o of the tile sits: rows of 8 octets are permuted by the row number on regular tiles.
+__device__ __forceinline__ int phys_oct(int o, bool swz) { return swz ? (o ^ ((o >> 3) & 7)) : o; }
+__device__ __forceinline__ int phys_pos(int pos, bool swz) { return (phys_oct(pos >> 3, swz) << 3) | (pos & 7); }
+
 // Number of tile elements with key >= thr (key bits), every thread of the CTA calling.
-__device__ __forceinline__ int tile_count_ge(const uint16_t* tile, int n_oct, int thr, int* counter) {
+__device__ __forceinline__ int tile_count_ge(const uint4* tile4, bool swz, int n_oct, int thr, int* counter) {
     const float thr_f = __int_as_float(thr);
     int c = 0;
     for (int o = threadIdx.x; o < n_oct; o += S_NT) {
         float v[8];
-        unpack8(reinterpret_cast<const uint4*>(tile)[o], v);
+        unpack8(tile4[phys_oct(o, swz)], v);
 #pragma unroll
         for (int e = 0; e < 8; ++e) c += (fabsf(v[e]) >= thr_f) ? 1 : 0;
     }
@@ -162,10 +165,6 @@ __device__ __forceinline__ void store_code_word(uint8_t* ef_g, bool aligned4, in
     for (int b = 0; b < 4; ++b) if (o * 8 + 2 * b < n) ef_g[o * 4 + b] = (uint8_t)(w >> (8 * b));
 }
 
-// Where octet o of the tile sits: rows of 8 octets are permuted by the row number on regular tiles.
-__device__ __forceinline__ int phys_oct(int o, bool swz) { return swz ? (o ^ ((o >> 3) & 7)) : o; }
-__device__ __forceinline__ int phys_pos(int pos, bool swz) { return (phys_oct(pos >> 3, swz) << 3) | (pos & 7); }
-
 // Codes of one octet of bf16 values r (statistics = their exact block minimum and maximum, u in
 // [2^-100, 2^100]): the defining floor(RN(RN((r - mn) / u) + 0.5)) itself, two elements per instruction and
 // without the division and conversion instructions.  The IEEE quotient comes from the correctly rounded
@@ -199,9 +198,10 @@ constexpr int S_FULL = 14;                   // 29 056 values = 3632 octets: eve
 
 // One octet of a = bf16(g + Qinv(e)) in place (positions >= n of a ragged tile stay zero); returns the
 // largest |a| of the octet.
-// RAGGED = false promises a whole octet; `commit` = false computes but leaves the tile as it is.
+// RAGGED = false promises a whole octet; `commit` = false computes but leaves the tile as it is.  SYNC: the warp's lanes
+// meet between their loads and their stores (all of them call).
 // The result goes to octet o_out of the tile (o itself, or its permuted place on a regular tile).
-template <bool FAST, bool RAGGED>
+template <bool FAST, bool RAGGED, bool SYNC = false>
 __device__ __forceinline__ float dequant_octet(uint4* tile4, int o, int o_out, int n, uint32_t codes, const QParams& q, const DecodeConsts& dc, bool commit) {
     float gv[8], x[8];
     unpack8(tile4[o], gv);
@@ -221,6 +221,7 @@ __device__ __forceinline__ float dequant_octet(uint4* tile4, int o, int o_out, i
             if (e0 + 1 >= n) ow[p] = (e0 >= n) ? 0u : (ow[p] & 0xFFFFu);
         }
     }
+    if (SYNC) __syncwarp();
     if (commit) tile4[o_out] = out;
     const uint32_t m2 = maxabs_bf16x2(maxabs_bf16x2(ow[0], ow[1]), maxabs_bf16x2(ow[2], ow[3]));
     return fmaxf(fabsf(__uint_as_float(m2 << 16)), fabsf(__uint_as_float(m2 & 0xFFFF0000u)));
@@ -274,13 +275,30 @@ __device__ __forceinline__ void dequant_phase(uint4* tile4, const SmemSel& ss, b
     }
 }
 
-// The same on a regular tile (see the head of the file): every block's decode is the fast one, the
-// first S_FULL octets of every thread exist, and octet o is written to its permuted place.  The 8
-// lanes that hold a 128-byte row read it in one instruction and write it in a later one, so the
-// permutation inside the row happens in place.
-__device__ __forceinline__ void dequant_phase_regular(uint4* tile4, const SmemSel& ss, int n_oct, const uint32_t (&cw)[S_SLOTS], float (&omax)[S_SLOTS]) {
+// The same on a regular tile (see the head of the file): every block's decode is the fast one, and octet o is written
+// to its permuted place.  The 8 lanes that hold a 128-byte row read it in one instruction and write it in a later one,
+// so the permutation inside the row happens in place.  FULL: the first S_FULL octets of every thread exist and none
+// is short; otherwise the tile may end anywhere (the places a last, short row's missing octets leave are never read).
+template <bool FULL>
+__device__ __forceinline__ void dequant_phase_regular(uint4* tile4, const SmemSel& ss, int n, int n_oct, const uint32_t (&cw)[S_SLOTS], float (&omax)[S_SLOTS]) {
     const int t = threadIdx.x;
     const int t_out = t ^ ((t >> 3) & 7);                   // phys_oct(t + j * S_NT) = t_out + j * S_NT
+    if constexpr (!FULL) {
+#pragma unroll
+        for (int j = 0; j < S_SLOTS; ++j) {
+            omax[j] = 0.0f;
+            const int o = t + j * S_NT;
+            if ((o & ~31) < n_oct) {                         // whole warps
+                const bool on = o < n_oct;
+                const int at = on ? o : n_oct - 1;
+                const float2 c = ss.qt.mu[at >> 3];
+                const QParams q = {c.x, c.y};
+                const float m = dequant_octet<true, true, true>(tile4, at, t_out + j * S_NT, n, cw[j], q, decode_consts(q), on);
+                omax[j] = on ? m : 0.0f;
+            }
+        }
+        return;
+    }
 #pragma unroll
     for (int j = 0; j < S_SLOTS; ++j) {
         omax[j] = 0.0f;
@@ -352,6 +370,31 @@ __device__ __forceinline__ void stats_encode_regular(const uint4* tile4, int n_q
     }
 }
 
+// A regular tile's last, short row (elements [64 b, n)) by the lanes 0..7 of one warp, an octet each; all 32 call.
+__device__ __noinline__ void stats_encode_short_row(const uint4* tile4, int b, int n, uint16_t* mn_out, uint16_t* mx_out, uint8_t* ef_out) {
+    const int c = lane_id() & 7;
+    const int cnt = max(0, min(8, n - b * 64 - c * 8));
+    const uint4 v = tile4[(b << 3) + (c ^ (b & 7))];
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    uint32_t hi2 = 0xFF80FF80u, lo2 = 0x7F807F80u;
+    for (int e = 0; e < cnt; ++e) {
+        const uint32_t x = (w[e >> 1] >> (16 * (e & 1))) & 0xFFFFu;
+        hi2 = max_bf16x2(hi2, x | (x << 16));
+        lo2 = min_bf16x2(lo2, x | (x << 16));
+    }
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) {
+        hi2 = max_bf16x2(hi2, __shfl_xor_sync(0xffffffffu, hi2, d));
+        lo2 = min_bf16x2(lo2, __shfl_xor_sync(0xffffffffu, lo2, d));
+    }
+    if (lane_id() >= 8 || cnt == 0) return;
+    const uint16_t mn_b = (uint16_t)(lo2 & 0xFFFFu), mx_b = (uint16_t)(hi2 & 0xFFFFu);
+    if (c == 0) { mn_out[b] = mn_b; mx_out[b] = mx_b; }
+    float r[8];
+    unpack8(v, r);
+    store_code_word(ef_out, true, b * 8 + c, n, encode_octet_exact(r, qparams(mn_b, mx_b), cnt));
+}
+
 // Codes of the thread's octets from the block tables, written to global memory; octets that came too
 // close to a code boundary (or whose block is degenerate) are left to the caller in `redo`.  The
 // first FS octets of every thread are promised to exist, to be whole and their code words aligned.
@@ -408,10 +451,10 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
 
     for (int unit = blockIdx.x; unit < total_units; unit += gridDim.x) {
         bool issued = false;
-        if (t == 0 && g_next != nullptr && (n_next & 7) == 0 && aligned16(g_next)) {   // same test as `staged` below
+        if (t == 0 && g_next != nullptr && (LOOSE ? (n_next & 7) == 0 : n_next >= 8) && aligned16(g_next)) {   // same test as `staged` below
             fence_async_smem();
-            mbar_arrive_expect_tx(&s_bar, (uint32_t)n_next * 2u);
-            bulk_g2s(smem_raw, g_next, (uint32_t)n_next * 2u, &s_bar);
+            mbar_arrive_expect_tx(&s_bar, (uint32_t)(n_next & ~7) * 2u);
+            bulk_g2s(smem_raw, g_next, (uint32_t)(n_next & ~7) * 2u, &s_bar);
             issued = true;
         }
         const int ti = ti_next >= 0 ? ti_next : find_tensor(s_first, n_tensors, unit);
@@ -429,7 +472,7 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
         // quantisation blocks of the tile; loose ones are at least 72 elements long, so the tables hold those a tile touches
         const int n_oct = (n + 7) >> 3;
         const int n_qb = LOOSE ? loose_block(lrem0 + n - 1, la.qbs, false) + 1 : (n + (1 << qshift) - 1) >> qshift;
-        const bool staged = (n & 7) == 0 && aligned16(g);            // the bulk copy moves whole 16-byte pieces
+        const bool staged = (LOOSE ? (n & 7) == 0 : n >= 8) && aligned16(g);   // the bulk copy moves whole 16-byte pieces
         const bool ef_al4 = (reinterpret_cast<uintptr_t>(ef_in) & 3) == 0;
         const bool tables = (QB64 || LOOSE) && n_qb <= S_QTAB;
         const uint16_t* mn_g = T.min_vals + qb0;
@@ -449,8 +492,12 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
         if (staged) {
             if (t == 0 && !issued) {
                 fence_async_smem();
-                mbar_arrive_expect_tx(&s_bar, (uint32_t)n * 2u);
-                bulk_g2s(tile, g, (uint32_t)n * 2u, &s_bar);
+                mbar_arrive_expect_tx(&s_bar, (uint32_t)(n & ~7) * 2u);
+                bulk_g2s(tile, g, (uint32_t)(n & ~7) * 2u, &s_bar);
+            }
+            if (!LOOSE && (n & 7) != 0 && t < 8) {           // the last, short octet, zero padded
+                const int i = (n & ~7) + t;
+                tile[i] = i < n ? g[i] : (uint16_t)0;
             }
         } else {
             // ragged tile (a tensor's last block, or an unaligned buffer): plain loads, zero padded to whole octets
@@ -513,9 +560,11 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
 
         // ---- a = bf16(g + Qinv(e)) in place; per-octet maxima stay in registers ------------------------
         float omax[S_SLOTS];
-        // regular tile: whole blocks of 64, 14 whole octets per thread, aligned codes, every block with the fast decode
-        const bool swz = !LOOSE && tables && (n & 63) == 0 && n_oct >= S_FULL * S_NT && ef_al4 && ss.ctrl[slow_slot] == 0 && T.quant_err == nullptr;
-        if (swz) dequant_phase_regular(tile4, ss, n_oct, cw, omax);
+        // regular tile: blocks of 64, aligned codes, every block with the fast decode.  (While short tiles took the general
+        // route, a step of 120 ragged tensors, 10.2 M elements, spent 78 us in this kernel: 121 us in all, 69 now.)
+        const bool swz = !LOOSE && tables && ef_al4 && ss.ctrl[slow_slot] == 0;
+        if (swz && (n & 7) == 0 && n_oct >= S_FULL * S_NT) dequant_phase_regular<true>(tile4, ss, n, n_oct, cw, omax);
+        else if (swz) dequant_phase_regular<false>(tile4, ss, n, n_oct, cw, omax);
         else if (LOOSE && tables && (n & 7) == 0 && n_oct >= S_FULL * S_NT && ef_al4)   // a full tile: branch-free first octets
             dequant_phase<S_FULL>(tile4, ss, tables, mn_g, mx_g, cshift, n, n_oct, cw, omax, la.qbs, lrem0);
         else dequant_phase<0>(tile4, ss, tables, mn_g, mx_g, cshift, n, n_oct, cw, omax, LOOSE ? la.qbs : 0, lrem0);
@@ -554,8 +603,15 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
             const int accept = k + (k > 1024 ? 112 : (k >> 1) + 8);
             int lo = 0, hi = kmax + 1, step = 1 << 20;
             int gq = (guess > 0 && guess <= kmax) ? guess : max(1, kmax - (2 << 23));
-            bool have_lo = false, have_hi = false;
-            for (int it = 0; it < 64; ++it) {
+            bool have_lo = false, have_hi = false, search = true;
+            const bool cold = guess <= 0 || guess > kmax;    // no bound from a tile before: the histogram of the maxima gives one
+            if (cold) {
+                const int c = bound_from_histogram(omax, kmax, k, ss.hist, lo, hi);
+                have_lo = c > 0; have_hi = true;
+                search = hi - lo > 1 && !(c > 0 && c <= accept);
+                gq = have_lo ? lo + ((hi - lo) >> 1) : max(hi - step, 1);
+            }
+            for (int it = 0; search && it < 64; ++it) {
                 int mine = 0;
 #pragma unroll
                 for (int j = 0; j < S_SLOTS; ++j) mine += (__float_as_int(omax[j]) >= gq) ? 1 : 0;
@@ -622,6 +678,10 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
                 __syncthreads();
                 MAB_CTICK(10);
                 const int n_cand = ss.n_cand;
+                if (cold) {                                  // the levels below count in the same bins
+                    ss.hist[t] = 0;
+                    __syncthreads();
+                }
                 if (n_cand <= S_CAND_CAP && ss.ctrl[4] == 0) {
                     C = n_cand;
                     reinterpret_cast<uint4*>(ss.sel_bm)[t] = make_uint4(0u, 0u, 0u, 0u);   // (the lists are done with; the barrier below publishes it)
@@ -715,9 +775,9 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
             int Tk = 0;
             for (int bit = 30; bit >= 16; --bit) {          // bf16 keys have 16 zero bits below
                 const int cand = Tk | (1 << bit);
-                if (tile_count_ge(tile, n_oct, cand, &ss.counters[bit]) >= k) Tk = cand;
+                if (tile_count_ge(tile4, swz, n_oct, cand, &ss.counters[bit]) >= k) Tk = cand;
             }
-            const int n_gt = tile_count_ge(tile, n_oct, Tk + 0x10000, &ss.counters[32]);
+            const int n_gt = tile_count_ge(tile4, swz, n_oct, Tk + 0x10000, &ss.counters[32]);
             const int need = k - n_gt;
             const float Tf = __int_as_float(Tk);
             uint32_t gt[S_WPT], tw[S_WPT];                  // the thread's 128 positions = 16 octets
@@ -776,12 +836,12 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
         __syncthreads();
 
         if (T.quant_err != nullptr) {
-            // alpha == -2: the residual a also goes to the caller's buffer (same element type as the gradient; linear tile)
+            // alpha == -2: the residual a also goes to the caller's buffer (same element type as the gradient)
             uint16_t* qe = reinterpret_cast<uint16_t*>(T.quant_err) + base;
             const bool vec = aligned16(qe);
             for (int o = t; o < n_oct; o += S_NT) {
-                if (vec && o * 8 + 8 <= n) reinterpret_cast<uint4*>(qe)[o] = tile4[o];
-                else for (int e = o * 8; e < min(o * 8 + 8, n); ++e) qe[e] = tile[e];
+                if (vec && o * 8 + 8 <= n) reinterpret_cast<uint4*>(qe)[o] = tile4[phys_oct(o, swz)];
+                else for (int e = o * 8; e < min(o * 8 + 8, n); ++e) qe[e] = tile[phys_pos(e, swz)];
             }
         }
         MAB_CTICK(4);
@@ -856,7 +916,8 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
             MAB_CTICK(9);
             __syncthreads();                                 // the tile is overwritten by the next load
         } else if (swz) {
-            stats_encode_regular(tile4, n_qb, mn_out, mx_out, ef_out, (reinterpret_cast<uintptr_t>(ef_out) & 15) == 0);
+            stats_encode_regular(tile4, n >> 6, mn_out, mx_out, ef_out, (reinterpret_cast<uintptr_t>(ef_out) & 15) == 0);
+            if ((n & 63) != 0 && warp == S_NT / 32 - 1) stats_encode_short_row(tile4, n >> 6, n, mn_out, mx_out, ef_out);
             __syncthreads();                                 // the tile is overwritten by the next load
         } else if (tables && (n & 63) == 0) {
             // whole blocks of 64: statistics block by block (a thread's 8 octets, rotated so that a warp's

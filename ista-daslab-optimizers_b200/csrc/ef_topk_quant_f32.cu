@@ -322,7 +322,8 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
             for (int j = 0; j < F_SLOTS; ++j) {
                 const int o = f32_oct(j);
                 uint32_t w = 0;
-                for (int b = 0; b < 4; ++b) if (o * 8 + 2 * b < n) w |= (uint32_t)ef[o * 4 + b] << (8 * b);
+                if (ef_al4 && o * 8 + 8 <= n) w = reinterpret_cast<const uint32_t*>(ef)[o];
+                else for (int b = 0; b < 4; ++b) if (o * 8 + 2 * b < n) w |= (uint32_t)ef[o * 4 + b] << (8 * b);
                 cw[j] = w;
             }
         }
@@ -367,7 +368,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
         const int n_so = n_oct - F_REG * F_NT;                       // octets in shared memory
         // regular tile: see the head of the file; its pieces are permuted from here on
         const bool swz = staged && qshift == 6 && (n & 63) == 0 && n_so >= F_FULL * F_NT && (reinterpret_cast<uintptr_t>(ef) & 15) == 0 &&
-                         ss.slow == 0 && T.quant_err == nullptr;
+                         ss.slow == 0;
         float omax[F_SLOTS];
         if (swz) {
 #pragma unroll
@@ -427,8 +428,15 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
             const int accept = k + (k > 1024 ? 192 : (k >> 1) + 8);
             int lo = 0, hi = kmax + 1, step = 1 << 20;
             int gq = (guess > 0 && guess <= kmax) ? guess : max(1, kmax - (2 << 23));
-            bool have_lo = false, have_hi = false;
-            for (int it = 0; it < 64; ++it) {
+            bool have_lo = false, have_hi = false, search = true;
+            const bool cold = guess <= 0 || guess > kmax;    // no bound from a tile before: the histogram of the maxima gives one
+            if (cold) {
+                const int c = bound_from_histogram(omax, kmax, k, ss.hist, lo, hi);
+                have_lo = c > 0; have_hi = true;
+                search = hi - lo > 1 && !(c > 0 && c <= accept);
+                gq = have_lo ? lo + ((hi - lo) >> 1) : max(hi - step, 1);
+            }
+            for (int it = 0; search && it < 64; ++it) {
                 int mine = 0;
 #pragma unroll
                 for (int j = 0; j < F_SLOTS; ++j) mine += (__float_as_int(omax[j]) >= gq) ? 1 : 0;
@@ -511,6 +519,10 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
                 __syncthreads();
                 C = ss.n_cand;
                 fast = C <= F_CAND_CAP && ss.over == 0;
+                if (cold) {                                          // the levels below count in the same bins
+                    if (t < 256) ss.hist[t] = 0;
+                    __syncthreads();
+                }
             }
             if (fast) {
                 ss.sel_bm[t] = 0u; ss.sel_bm[t + F_NT] = 0u;         // (the octet lists are done with; published by the barriers below)
@@ -715,6 +727,24 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
                 float l, u;
                 octet_min_max(a[j], l, u);
                 lo = fminf(lo, l); hi = fmaxf(hi, u);
+            }
+            if (T.quant_err != nullptr) {                            // alpha == -2: the residual a also goes to the caller's buffer
+                float* qe = reinterpret_cast<float*>(T.quant_err) + base;
+                const bool vec = aligned16(qe);
+#pragma unroll
+                for (int j = 0; j < F_REG; ++j)
+#pragma unroll
+                    for (int e = 0; e < 8; e += 4) {
+                        float* to = qe + f32_oct(j) * 8 + e;
+                        if (vec) *reinterpret_cast<float4*>(to) = make_float4(a[j][e], a[j][e + 1], a[j][e + 2], a[j][e + 3]);
+                        else { to[0] = a[j][e]; to[1] = a[j][e + 1]; to[2] = a[j][e + 2]; to[3] = a[j][e + 3]; }
+                    }
+                for (int c = t; c < n_so * 2; c += F_NT) {
+                    const float4 v = tile4[c ^ ((c >> 4) & 7)];
+                    float* to = qe + F_REG_ELEMS + c * 4;
+                    if (vec) *reinterpret_cast<float4*>(to) = v;
+                    else { to[0] = v.x; to[1] = v.y; to[2] = v.z; to[3] = v.w; }
+                }
             }
             uint32_t st = pack_bf16x2_rne(-lo, hi);
             st = max_bf16x2(st, __shfl_xor_sync(0xffffffffu, st, 1));
