@@ -152,6 +152,30 @@ __device__ __forceinline__ void resolve_selection_regs(const uint32_t (&gt)[S_WP
     __syncthreads();
 }
 
+// 8 bf16 values from any address: both aligned 16-byte pieces that hold some of them must be readable.
+__device__ __forceinline__ uint4 load_octet_anywhere(const uint16_t* p) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+    const uint4* piece = reinterpret_cast<const uint4*>(at & ~(uintptr_t)15);
+    const uint4 x = __ldg(piece), y = (at & 15) ? __ldg(piece + 1) : make_uint4(0u, 0u, 0u, 0u);
+    uint32_t w[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+    if (at & 8) { w[0] = w[2]; w[1] = w[3]; w[2] = w[4]; w[3] = w[5]; w[4] = w[6]; w[5] = w[7]; }
+    if (at & 4) { w[0] = w[1]; w[1] = w[2]; w[2] = w[3]; w[3] = w[4]; w[4] = w[5]; }
+    const int sh = (int)(at & 2) * 8;
+    return make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh), __funnelshift_r(w[2], w[3], sh), __funnelshift_r(w[3], w[4], sh));
+}
+
+// A tile from an unaligned buffer: whole octets from the two aligned 16-byte pieces they lie in, but for the tile's first
+// and last two octets, whose pieces may reach out of the buffer: those element by element, zero padded.  (Element by
+// element throughout, with the update's blocks copied likewise: 67 M elements 592 us a step, now 222; 183 when aligned.)
+__device__ __noinline__ void load_tile_anywhere(uint16_t* tile, const uint16_t* g, int n, int n_oct) {
+    const int t = threadIdx.x;
+    for (int o = t + 1; o < n_oct - 2; o += S_NT) reinterpret_cast<uint4*>(tile)[o] = load_octet_anywhere(g + o * 8);
+    if (t < 24) {
+        const int o = t < 8 ? 0 : n_oct - (t < 16 ? 2 : 1), e = o * 8 + (t & 7);
+        if (o >= 0) tile[e] = e < n ? g[e] : (uint16_t)0;
+    }
+}
+
 // The four code bytes of octet o (elements [8 o, 8 o + 8) of a tile of n elements), missing bytes as 0.
 __device__ __forceinline__ uint32_t load_code_word(const uint8_t* ef_g, bool aligned4, int o, int n) {
     if (aligned4 && o * 8 + 8 <= n) return reinterpret_cast<const uint32_t*>(ef_g)[o];
@@ -297,17 +321,17 @@ __device__ __forceinline__ void dequant_phase_regular(uint4* tile4, const SmemSe
                 omax[j] = on ? m : 0.0f;
             }
         }
-        return;
-    }
+    } else {
 #pragma unroll
-    for (int j = 0; j < S_SLOTS; ++j) {
-        omax[j] = 0.0f;
-        const int o = t + j * S_NT;
-        if (j < S_FULL || o < n_oct) {
-            if (j < S_FULL && j % S_GROUP == 0) asm volatile("" ::: "memory");
-            const float2 c = ss.qt.mu[o >> 3];
-            const QParams q = {c.x, c.y};
-            omax[j] = dequant_octet<true, false>(tile4, o, t_out + j * S_NT, 0, cw[j], q, decode_consts(q), true);
+        for (int j = 0; j < S_SLOTS; ++j) {
+            omax[j] = 0.0f;
+            const int o = t + j * S_NT;
+            if (j < S_FULL || o < n_oct) {
+                if (j < S_FULL && j % S_GROUP == 0) asm volatile("" ::: "memory");
+                const float2 c = ss.qt.mu[o >> 3];
+                const QParams q = {c.x, c.y};
+                omax[j] = dequant_octet<true, false>(tile4, o, t_out + j * S_NT, 0, cw[j], q, decode_consts(q), true);
+            }
         }
     }
 }
@@ -500,8 +524,7 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
                 tile[i] = i < n ? g[i] : (uint16_t)0;
             }
         } else {
-            // ragged tile (a tensor's last block, or an unaligned buffer): plain loads, zero padded to whole octets
-            for (int i = t; i < n_oct * 8; i += S_NT) tile[i] = (i < n) ? g[i] : (uint16_t)0;
+            load_tile_anywhere(tile, g, n, n_oct);
         }
         uint32_t cw[S_SLOTS];
         if (ef_al4 && (n & 7) == 0 && n_oct >= S_FULL * S_NT) {  // a full tile: the first S_FULL words of every thread exist and are whole

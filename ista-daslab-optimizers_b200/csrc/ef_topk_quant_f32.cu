@@ -296,7 +296,11 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
                 bulk_g2s(tile, g + F_REG_ELEMS, (uint32_t)n_smem * 4u, &s_bar);
             }
         } else {
-            for (int i = t; i < n_oct * 8 - F_REG_ELEMS; i += F_NT) tile[i] = (i < n_smem) ? g[F_REG_ELEMS + i] : 0.0f;
+            for (int i = t; i < n_oct * 8 - F_REG_ELEMS; i += F_NT) {
+                if (i < n_smem) cp_async_4(tile + i, g + F_REG_ELEMS + i);
+                else tile[i] = 0.0f;
+            }
+            cp_async_commit();
         }
         if (t == 0) { ss.kmax = 0; ss.n_member = 0; ss.n_cand = 0; ss.over = 0; }
         if (t < 64) ss.rot[t] = 0;
@@ -344,6 +348,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
                 return;
             }
         } else {
+            cp_async_wait_all();
             __syncthreads();
         }
         if (unit + (int)gridDim.x < total_units) {                   // the tile after this one: into L2 while this one is worked on
@@ -367,7 +372,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
         const int h = whole ? (lane >> 2) & 1 : 0;                   // (a short octet needs its elements in order)
         const int n_so = n_oct - F_REG * F_NT;                       // octets in shared memory
         // regular tile: see the head of the file; its pieces are permuted from here on
-        const bool swz = staged && qshift == 6 && (n & 63) == 0 && n_so >= F_FULL * F_NT && (reinterpret_cast<uintptr_t>(ef) & 15) == 0 &&
+        const bool swz = qshift == 6 && (n & 63) == 0 && n_so >= F_FULL * F_NT && (reinterpret_cast<uintptr_t>(ef) & 15) == 0 &&
                          ss.slow == 0;
         float omax[F_SLOTS];
         if (swz) {

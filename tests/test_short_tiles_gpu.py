@@ -29,11 +29,14 @@ def _gradient(kind, n, step, dtype):
 @pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize('kind,k_init,skip,alpha', [
     ('normal', 0.01, 0, 0), ('normal', 0.05, 8, 0), ('normal', 0.01, 1, 0), ('normal', 0.02, 2, 0), ('normal', 0.01, 5, 0),
-    ('normal', 0.01, 0, -2), ('normal', 0.01, 3, -2), ('wide', 0.01, 0, 0), ('tiny', 0.02, 0, 0), ('equal', 0.01, 0, 0), ('sparse', 0.02, 0, 0)])
+    ('normal', 0.01, 0, -2), ('normal', 0.01, 3, -2), ('decay', 0.01, 0, 0), ('decay', 0.01, 3, 0),
+    ('wide', 0.01, 0, 0), ('tiny', 0.02, 0, 0), ('equal', 0.01, 0, 0), ('sparse', 0.02, 0, 0)])
 def test_short_tiles_match_oracle(kind, k_init, skip, alpha, dtype):
     from ista_daslab_optimizers_b200 import MicroAdam, _native
     from oracle.microadam_oracle import MicroAdamOracle
     hyper = dict(m=4, lr=1e-3, quant_block_size=64, k_init=k_init, weight_decay=0.1, alpha=alpha)
+    if kind == 'decay':                                  # a decay that changes bf16 parameters
+        hyper.update(lr=1e-2, weight_decay=0.5)
     params = [torch.nn.Parameter(S.normal_tensor(60, i, n + skip, 0.02).to(dtype).cuda()[skip:]) for i, n in enumerate(SIZES)]
     cpu = [p.detach().cpu().clone() for p in params]
     opt = MicroAdam(params, **hyper)
