@@ -235,6 +235,13 @@ __device__ __forceinline__ uint32_t maxabs_bf16x2(uint32_t a, uint32_t b) {
     return d;
 }
 
+// Lane-wise sum of two packed bf16 pairs, rounded once.
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
 __device__ __forceinline__ uint32_t min_bf16x2(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("min.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));

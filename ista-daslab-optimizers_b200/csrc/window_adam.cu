@@ -32,6 +32,8 @@ __device__ unsigned long long g_stats_b[16];
 
 enum : int { MODE_WRITE_UPDATE = 0, MODE_STEP = 1 };
 
+constexpr int WT_WORDS = 1024;            // bitmap words of a tile (32768 positions)
+
 // 8 consecutive elements of a buffer as floats; vector access when `full`, else element-wise
 // up to `n` (the tensor's last, short octet).
 template <typename T> struct Octet;
@@ -82,6 +84,11 @@ template <> struct Octet<uint16_t> {
         }
     }
 };
+
+// Whether bf16(p * decay) == p for every bf16 p (see the resident-tile kernel).
+__device__ __forceinline__ bool decay_is_identity_bf16(float decay) {
+    return decay <= 1.0f && (1.0f - decay) <= 0.0009765625f;
+}
 
 // p <- round_p(round_p(p * decay) - lr * u) for 8 values, two per instruction (packed f32x2
 // operations round each component like the scalar ones).
@@ -145,6 +152,7 @@ struct DenseU {                 // a dense float array in shared memory, 16-byte
         const float4 a = reinterpret_cast<const float4*>(u + o * 8)[0], b = reinterpret_cast<const float4*>(u + o * 8)[1];
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     }
+    __device__ __forceinline__ void load_warp(int o, bool on, float (&v)[8]) const { if (on) load(o, v); }
 };
 struct SparseU {                // touched positions as a bitmap, their updates compact in slot order
     static constexpr bool has_u = true;
@@ -163,6 +171,35 @@ struct SparseU {                // touched positions as a bitmap, their updates 
             slot += on ? 1 : 0;
         }
     }
+};
+
+// The same, for a stream whose warps walk 32 consecutive octets at a time: the updates of those 256 positions, which are
+// consecutive slots, are scattered into a dense array of the warp's own (a look-up per element through the bitmap was
+// a quarter of the streams' instructions).
+struct WarpU {
+    static constexpr bool has_u = true;
+    const uint32_t* bitmap;
+    const uint16_t* prefix;
+    const uint16_t* spos;       // position of each slot
+    const float2* mv;
+    int touched;
+    float* dense;               // 256 floats per warp, all zero between calls
+    // octet o (those of the lanes are 32 consecutive ones, the first a multiple of 32); all 32 lanes call
+    __device__ __forceinline__ void load_warp(int o, bool on, float (&v)[8]) const {
+        if (dense == nullptr) { if (on) load(o, v); return; }           // (the window left no room for the arrays)
+        const int o0 = o - lane_id();
+        float* d = dense + warp_id() * 256;
+        const int w0 = o0 >> 2;
+        const int first = prefix[w0], last = w0 + 8 < WT_WORDS ? (int)prefix[w0 + 8] : touched;
+        for (int s = first + lane_id(); s < last; s += 32) d[(int)spos[s] - o0 * 8] = mv[s].x;
+        __syncwarp();
+        float4* mine = reinterpret_cast<float4*>(d) + lane_id() * 2;
+        const float4 a = mine[0], b = mine[1];
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+        mine[0] = make_float4(0.0f, 0.0f, 0.0f, 0.0f); mine[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        __syncwarp();
+    }
+    __device__ __forceinline__ void load(int o, float (&v)[8]) const { SparseU{bitmap, prefix, mv}.load(o, v); }
 };
 
 // Per-thread partial sums of the update's logging probes (micro_adam.py:306-308, 272-273); they live across the
@@ -214,6 +251,13 @@ __device__ __forceinline__ void stream_range(const mab_tensor& T, const WindowAr
     }
     const float decay = T.decay_f32, neg_lr = T.neg_lr_f32;
     const bool do_decay = T.weight_decay > 0.0;
+    if (ALPHA == 0 && !USrc::has_u && !vec) {                // the decay of a misaligned tensor
+        if (do_decay) {
+#pragma unroll 4
+            for (int i = threadIdx.x; i < len; i += NT) Elem<TP>::store(p, i, __fmul_rn(Elem<TP>::load(p, i), decay));
+        }
+        return;
+    }
     if (ALPHA == 0) {
         const float2 decay2 = make_float2(decay, decay), neg_lr2 = make_float2(neg_lr, neg_lr);
         constexpr int B = (sizeof(TP) == 2) ? 4 : 2;          // octets per thread and batch
@@ -262,9 +306,11 @@ __device__ __forceinline__ void stream_range(const mab_tensor& T, const WindowAr
         }
         return;
     }
-    // The two forms that read the error feedback.  Octets that are whole (ALPHA 1: of whole quantisation blocks, whose
-    // lanes combine their extremes by shuffles) take the octet-wide codec, with the loads of a thread's next octet in
-    // flight while the current one is worked on; the rest of a ragged tensor goes element by element.
+    // The two forms that read the error feedback.  Octets that are whole (ALPHA 1: of whole quantisation blocks) take the
+    // octet-wide codec, with the loads of a thread's next octet in flight while the current one is worked on; the rest of a
+    // ragged tensor goes element by element.  Bound by instruction issue: alpha = 0.5 on 33.5 M fp32
+    // elements 232 -> 134 us through the octet-wide codec, 14 us less through the warps' dense arrays; alpha == -2 on 54.5 M bf16
+    // elements 295 -> 182, 29 us less through those and the packed bf16 sums.
     const bool g_bf16 = (T.grad_dtype == MAB_BF16);
     const int cshift = 31 - __clz(a.lanes_per_qb);           // octets per quantisation block, as a shift
     uint8_t* ef = T.error + (e0 >> 1);
@@ -275,7 +321,7 @@ __device__ __forceinline__ void stream_range(const mab_tensor& T, const WindowAr
     uint16_t* maxs = T.max_vals + qb0;
     TP* qe = ALPHA == 2 ? reinterpret_cast<TP*>(T.quant_err) + e0 : nullptr;
     const bool vec_q = ALPHA == 2 && aligned16(qe);
-    const float2 decay2 = make_float2(decay, decay), neg_lr2 = make_float2(neg_lr, neg_lr);
+    const float2 neg_lr2 = make_float2(neg_lr, neg_lr);
     const int whole = !ef_al4 ? 0 : ALPHA == 2 ? len >> 3 : (len >> (cshift + 3)) << cshift;
     struct In { RawOctet<TP> p, q; uint32_t codes; uint16_t mn, mx; };
     auto fetch = [&](int o, In& in) {
@@ -290,42 +336,55 @@ __device__ __forceinline__ void stream_range(const mab_tensor& T, const WindowAr
     };
     In cur;
     if (threadIdx.x < whole) fetch(threadIdx.x, cur);
-    const int n_pad = (whole + 31) & ~31;                    // whole warps meet in the shuffles
+    const bool decaying = do_decay && !(sizeof(TP) == 2 && decay_is_identity_bf16(decay));
+    const int lanes = a.lanes_per_qb;
+    const int n_pad = (whole + 31) & ~31;                    // whole warps meet in the exchanges
     for (int o = threadIdx.x; o < n_pad; o += NT) {
         In nxt = cur;
         if (o + NT < whole) fetch(o + NT, nxt);
         const bool on = o < whole;
-        float xs[8];
+        float uo[8];
+        if constexpr (ALPHA != 0) src.load_warp(o, on, uo);
+        const QParams q = on ? qparams(cur.mn, cur.mx) : QParams{0.0f, 0.0f};
+        float x1[8];
         if (on) {
-            float pv[8], uo[8], x1[8], av[8];
-            decode_octet(cur.codes, qparams(cur.mn, cur.mx), x1);
+            float pv[8], av[8];
+            decode_octet(cur.codes, q, x1);
             cur.p.unpack(pv);
-            src.load(o, uo);
-            if (ALPHA == 2) cur.q.unpack(av);
+            if (ALPHA == 2 && sizeof(TP) == 4) cur.q.unpack(av);
+            uint32_t avw[4] = {0u, 0u, 0u, 0u};
+            if constexpr (ALPHA == 2 && sizeof(TP) == 2) { avw[0] = cur.q.a.x; avw[1] = cur.q.a.y; avw[2] = cur.q.a.z; avw[3] = cur.q.a.w; }
 #pragma unroll
             for (int b = 0; b < 8; b += 2) {
                 float2 v = make_float2(pv[b], pv[b + 1]), u = make_float2(uo[b], uo[b + 1]);
                 const float2 x = make_float2(x1[b], x1[b + 1]), zero = make_float2(0.0f, 0.0f);
-                if (do_decay) { v = __fmul2_rn(v, decay2); if (sizeof(TP) == 2) v = round2(v); }
+                // (products that a sum follows are scalar: the compiler merges a packed product and a packed sum into one rounding)
+                if (decaying) { v = make_float2(__fmul_rn(v.x, decay), __fmul_rn(v.y, decay)); if (sizeof(TP) == 2) v = round2(v); }
                 if (ALPHA == 2) {
                     // alpha == -2 (micro_adam.py:238-273), with a = the residual kernel A left in quant_err and e = the new codes:
                     //   p <- decay(p);  p <- p - a;  p <- p + Qinv(e);  quant_err <- a - Qinv(e);  then p <- p - lr * u
-                    float2 y = __fadd2_rn(zero, x);                                      // grad.zero_(); grad += Qinv(e)
-                    if (g_bf16) y = round2(y);
-                    float2 r = make_float2(av[b], av[b + 1]);
-                    v = __fadd2_rn(v, make_float2(-r.x, -r.y));                          // p.add_(grad, alpha=-1)
-                    if (sizeof(TP) == 2) v = round2(v);
-                    v = __fadd2_rn(v, y);                                                // p.add_(grad)
-                    if (sizeof(TP) == 2) v = round2(v);
-                    r = __fadd2_rn(r, make_float2(-y.x, -y.y));                          // quant_err.sub_(grad)
-                    if (sizeof(TP) == 2) r = round2(r);
-                    av[b] = r.x; av[b + 1] = r.y;
+                    const float2 y = __fadd2_rn(zero, x);                                // grad.zero_(); grad += Qinv(e)
+                    if (sizeof(TP) == 2) {
+                        // gradient and parameter are both bf16 here.  A packed bf16 sum rounds once, torch's twice (fp32, then
+                        // bf16); the two agree: the fp32 sum of two bf16 values is exact unless one of them is below 2^-15 of
+                        // the other, and so far from the middle between two bf16 values
+                        const uint32_t yw = pack_bf16x2_rne(y.x, y.y);
+                        uint32_t w = pack_bf16x2_rne(v.x, v.y);
+                        w = add_bf16x2(w, avw[b >> 1] ^ 0x80008000u);                    // p.add_(grad, alpha=-1)
+                        w = add_bf16x2(w, yw);                                           // p.add_(grad)
+                        avw[b >> 1] = add_bf16x2(avw[b >> 1], yw ^ 0x80008000u);         // quant_err.sub_(grad)
+                        v = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+                        if (probing) { av[b] = __uint_as_float(avw[b >> 1] << 16); av[b + 1] = __uint_as_float(avw[b >> 1] & 0xFFFF0000u); }
+                    } else {
+                        float2 r = make_float2(av[b], av[b + 1]);
+                        v = __fadd2_rn(v, make_float2(-r.x, -r.y));
+                        v = __fadd2_rn(v, y);
+                        r = __fadd2_rn(r, make_float2(-y.x, -y.y));
+                        av[b] = r.x; av[b + 1] = r.y;
+                    }
                 } else {
-                    // alpha > 0: u += alpha * Qinv(e); p update; e <- Q((1 - alpha) * Qinv(e)) with fresh statistics
-                    u = __fadd2_rn(u, __fmul2_rn(make_float2(a.alpha, a.alpha), x));
-                    float2 y = __fadd2_rn(zero, __fmul2_rn(make_float2(a.one_minus_alpha, a.one_minus_alpha), x));
-                    if (g_bf16) { u = round2(u); y = round2(y); }
-                    xs[b] = y.x; xs[b + 1] = y.y;
+                    u = __fadd2_rn(u, make_float2(__fmul_rn(a.alpha, x.x), __fmul_rn(a.alpha, x.y)));   // alpha > 0: u += alpha * Qinv(e)
+                    if (g_bf16) u = round2(u);
                 }
                 if (probing) {
                     pr.sum_u2 = fmaf(u.x, u.x, fmaf(u.y, u.y, pr.sum_u2));
@@ -339,17 +398,31 @@ __device__ __forceinline__ void stream_range(const mab_tensor& T, const WindowAr
                 pv[b] = v.x; pv[b + 1] = v.y;
             }
             Octet<TP>::store(p + o * 8, pv, vec, 8);
-            if (ALPHA == 2) Octet<TP>::store(qe + o * 8, av, vec_q, 8);
+            if constexpr (ALPHA == 2 && sizeof(TP) == 2) {
+                if (vec_q) reinterpret_cast<uint4*>(qe + o * 8)[0] = make_uint4(avw[0], avw[1], avw[2], avw[3]);
+                else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) qe[o * 8 + e] = (uint16_t)(avw[e >> 1] >> (16 * (e & 1)));
+                }
+            } else if constexpr (ALPHA == 2) {
+                Octet<TP>::store(qe + o * 8, av, vec_q, 8);
+            }
         }
         if (ALPHA == 1) {
-            // bf16 rounding is monotone and odd: the block's statistics are the maximum of the rounded (-min, max) pairs
-            float lo = INFINITY, hi = -INFINITY;
-            if (on) octet_min_max(xs, lo, hi);
+            // e <- Q((1 - alpha) * Qinv(e)) with fresh statistics.  bf16 rounding is monotone and odd: the block's are the
+            // maximum of the rounded (-min, max) pairs.  (What is quantised takes 16 values per block, and nearly always keeps its
+            // codes; telling that apart from the rest was 7 % slower than encoding everything.)
+            float xs[8], lo = INFINITY, hi = -INFINITY;
+            if (on) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) xs[e] = round_as(__fadd_rn(0.0f, __fmul_rn(a.one_minus_alpha, x1[e])), g_bf16);
+                octet_min_max(xs, lo, hi);
+            }
             uint32_t st = pack_bf16x2_rne(-lo, hi);
-            for (int off = 1; off < a.lanes_per_qb; off <<= 1) st = max_bf16x2(st, __shfl_xor_sync(0xffffffffu, st, off));
+            for (int off = 1; off < lanes; off <<= 1) st = max_bf16x2(st, __shfl_xor_sync(0xffffffffu, st, off));
             if (on) {
                 const uint16_t mn_b = (uint16_t)((st & 0xFFFFu) ^ 0x8000u), mx_b = (uint16_t)(st >> 16);
-                if ((o & (a.lanes_per_qb - 1)) == 0) { mins[o >> cshift] = mn_b; maxs[o >> cshift] = mx_b; }
+                if ((o & (lanes - 1)) == 0) { mins[o >> cshift] = mn_b; maxs[o >> cshift] = mx_b; }
                 const QParams q2 = qparams(mn_b, mx_b);
                 ef32[o] = (q2.u >= CODEC_U_MIN && q2.u <= CODEC_U_MAX) ? encode_octet_div_f32<true>(xs, div_consts(q2))
                                                                        : encode_octet_exact(xs, q2, 8);
@@ -421,7 +494,6 @@ __device__ __forceinline__ void stream_range(const mab_tensor& T, const WindowAr
 
 // ------------------------------------------------------------------------------------ tile kernel
 
-constexpr int WT_WORDS = 1024;            // bitmap words (32768 positions)
 constexpr int WT_MAX_ENTRIES = 16384;     // window entries of one block the compact arrays may hold
 constexpr int WT_KEEP = 6;                // window entries a thread keeps in registers between marking and numbering
 constexpr int WT_NO_SLOT = 0xFFFF;        // slot of a window entry whose index lies outside the block (slots stay below 32768)
@@ -630,7 +702,7 @@ __device__ __forceinline__ int window_tile_moments(const mab_tensor& T, int blk,
 
 template <typename TP, int MODE, int ALPHA, int NT>
 __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units,
-                                                 int max_k, const WindowArgs& a) {
+                                                 int max_k, const WindowArgs& a, int dense_at = 0) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ int s_first[WIN_MAX_TENSORS + 1];
     __shared__ int s_scan[36];
@@ -641,6 +713,8 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
 
     for (int i = t; i < n_tensors; i += NT) s_first[i] = tensors[i].first_unit_a;
     if (t == 0) s_first[n_tensors] = total_units;
+    float* const dense = dense_at > 0 ? reinterpret_cast<float*>(smem_raw + dense_at) : nullptr;   // the streams' arrays of the warps
+    if (dense != nullptr) for (int i = t; i < NT * 8; i += NT) dense[i] = 0.0f;
     __syncthreads();
     const float inv_bc1 = 1.0f / a.bc1, inv_bc2 = 1.0f / a.bc2;
     UpdateProbe pr;
@@ -670,35 +744,56 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
         MAB_BTICK_DECL
         const int touched = window_tile_moments<NT>(T, blk, n_blk, kcnt, a, w, s_scan, s_pos_off, s_val_off);
         MAB_BTICK(9);
-        // 5. moments -> update (rounded to the gradient's element type), slot by slot
-        for (int s = t; s < touched; s += NT) {
-            const float2 acc = w.mv[s];
-            const float u = round_as(adam_update_fast(acc.x, acc.y, inv_bc1, inv_bc2, a.eps), g_bf16);
-            w.mv[s].x = u;
-            if (probing && ALPHA == 0) { pr.sum_u2 = fmaf(u, u, pr.sum_u2); pr.zeros_u -= (u != 0.0f) ? 1 : 0; }   // (the other forms count in the stream)
-        }
-        if (probing && ALPHA == 0 && t == 0) pr.zeros_u += n_blk;       // every position without a non-zero update is a zero of u
-        __syncthreads();
-        MAB_BTICK(5);
-        if (MODE == MODE_STEP && ALPHA == 0) {
-            // 6. without the alpha term only the touched positions get an update: stream the block for the
-            //    weight decay alone (nothing to stream without decay), then update the touched elements
-            //    one by one; fma(-lr, 0, x) == x, so the untouched elements are already final
+        if constexpr (MODE == MODE_STEP && ALPHA == 0) {
+            // 5. without the alpha term only the touched positions get an update: stream the block for the
+            //    weight decay alone (nothing to stream without decay), then turn the moments into updates (rounded to the
+            //    gradient's element type) and apply them one by one; fma(-lr, 0, x) == x, so the untouched elements are
+            //    already final.  A thread has UB of its scattered reads in flight (one at a time, a read that waits for
+            //    the write before it: a step of 124.4 M elements 499 -> 493 us,
+            //    67.1 M with windows of 10 rows of 5 % 556 -> 504).
             if (T.weight_decay > 0.0) {
                 stream_range<TP, MODE, NT, ALPHA>(T, a, NoU{}, blk_base, n_blk, pr);
                 __syncthreads();                               // the decayed values are read back below
             }
             MAB_BTICK(6);
+            constexpr int UB = 4;
             TP* p = reinterpret_cast<TP*>(T.param) + blk_base;
             const float neg_lr = T.neg_lr_f32;
-            for (int s2 = t; s2 < touched; s2 += NT) {
-                const int pos = w.spos[s2];
-                Elem<TP>::store(p, pos, __fmaf_rn(neg_lr, w.mv[s2].x, Elem<TP>::load(p, pos)));
+            for (int s0 = t; s0 < touched; s0 += UB * NT) {
+                int pos[UB];
+                float pv[UB];
+#pragma unroll
+                for (int i = 0; i < UB; ++i) {
+                    pos[i] = s0 + i * NT < touched ? (int)w.spos[s0 + i * NT] : -1;
+                    pv[i] = pos[i] >= 0 ? Elem<TP>::load(p, pos[i]) : 0.0f;
+                }
+#pragma unroll
+                for (int i = 0; i < UB; ++i) {
+                    if (pos[i] >= 0) {
+                        const float2 acc = w.mv[s0 + i * NT];
+                        const float u = round_as(adam_update_fast(acc.x, acc.y, inv_bc1, inv_bc2, a.eps), g_bf16);
+                        Elem<TP>::store(p, pos[i], __fmaf_rn(neg_lr, u, pv[i]));
+                        if (probing) { pr.sum_u2 = fmaf(u, u, pr.sum_u2); pr.zeros_u -= (u != 0.0f) ? 1 : 0; }
+                    }
+                }
             }
+            if (probing && t == 0) pr.zeros_u += n_blk;        // every position without a non-zero update is a zero of u
         } else {
+            // 5. moments -> update (rounded to the gradient's element type), slot by slot
+            for (int s = t; s < touched; s += NT) {
+                const float2 acc = w.mv[s];
+                w.mv[s].x = round_as(adam_update_fast(acc.x, acc.y, inv_bc1, inv_bc2, a.eps), g_bf16);
+            }
+            __syncthreads();
+            MAB_BTICK(5);
             // 6. stream the whole block; each octet finds its updates through the bitmap
-            const SparseU src{w.bitmap, w.prefix, w.mv};
-            stream_range<TP, MODE, NT, ALPHA>(T, a, src, blk_base, n_blk, pr);
+            if constexpr (ALPHA != 0) {
+                const WarpU src{w.bitmap, w.prefix, w.spos, w.mv, touched, dense};
+                stream_range<TP, MODE, NT, ALPHA>(T, a, src, blk_base, n_blk, pr);
+            } else {
+                const SparseU src{w.bitmap, w.prefix, w.mv};
+                stream_range<TP, MODE, NT, ALPHA>(T, a, src, blk_base, n_blk, pr);
+            }
         }
         MAB_BTICK(7);
         __syncthreads();                                       // everything is reused by the next unit
@@ -715,8 +810,8 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
 template <typename TP, int MODE, int ALPHA, int NT>
 __global__ void __launch_bounds__(NT, ALPHA == 0 ? 1024 / NT : 3)
 window_tile_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int max_k,
-                   const __grid_constant__ WindowArgs a) {
-    window_tile_body<TP, MODE, ALPHA, NT>(tensors, n_tensors, total_units, max_k, a);
+                   int dense_at, const __grid_constant__ WindowArgs a) {
+    window_tile_body<TP, MODE, ALPHA, NT>(tensors, n_tensors, total_units, max_k, a, dense_at);
 }
 
 // Single tensor whose descriptor travels as a kernel argument (operator-level entry point).
@@ -744,8 +839,16 @@ constexpr int WR_THREADS = 512;
 // Set when a wait on the copy engine gave up; read through mab_device_error() together with the other kernels' flags.
 __device__ int g_copy_timeout_window;
 
-__device__ __forceinline__ bool decay_is_identity_bf16(float decay) {
-    return decay <= 1.0f && (1.0f - decay) <= 0.0009765625f;
+// The touched elements of a block where they are in global memory (out of line: the blocks the copy engine moves are the
+// ones whose code should stay small).
+__device__ __noinline__ void update_in_place(uint16_t* p, const uint16_t* spos, const float2* mv, int touched, float neg_lr, float inv_bc1,
+                                             float inv_bc2, float eps, bool g_bf16, UpdateProbe* pr) {
+    for (int s = threadIdx.x; s < touched; s += WR_THREADS) {
+        const float u = round_as(adam_update_fast(mv[s].x, mv[s].y, inv_bc1, inv_bc2, eps), g_bf16);
+        uint16_t* at = p + spos[s];
+        *at = f32_to_bf16_bits_rne(__fmaf_rn(neg_lr, u, bf16_bits_to_f32(*at)));
+        if (pr != nullptr) { pr->sum_u2 = fmaf(u, u, pr->sum_u2); pr->zeros_u -= (u != 0.0f) ? 1 : 0; }
+    }
 }
 
 __global__ void __launch_bounds__(WR_THREADS, 2)
@@ -781,6 +884,9 @@ window_resident_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, in
         const int n_blk = (int)min((int64_t)dbs, T.d - blk_base);
         uint16_t* p = reinterpret_cast<uint16_t*>(T.param) + blk_base;
         const bool bulk = (n_blk & 7) == 0 && aligned16(p);                     // the copy engine moves whole 16-byte pieces
+        // a block it cannot move (a tensor's ragged last one, an unaligned slice) and whose decay changes nothing: the touched
+        // elements are updated where they are
+        const bool in_place = !bulk && !(T.weight_decay > 0.0 && !decay_is_identity_bf16(T.decay_f32));
         const int n_oct = (n_blk + 7) >> 3;
 
         MAB_BTICK_DECL
@@ -811,7 +917,7 @@ window_resident_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, in
                 if (t == 0) atomicExch(&g_copy_timeout_window, 1);
                 return;
             }
-        } else {
+        } else if (!in_place) {
             if (t == 0 && store_in_flight) { bulk_wait_read(); store_in_flight = false; }
             __syncthreads();
             for (int i = t; i < n_blk; i += WR_THREADS) tile[i] = p[i];
@@ -839,12 +945,16 @@ window_resident_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, in
         // moments -> update (rounded to the gradient's element type) -> parameter, touched positions only:
         // fma(-lr, 0, x) == x, so the untouched elements are already final
         const float neg_lr = T.neg_lr_f32;
-        for (int s = t; s < touched; s += WR_THREADS) {
-            const float2 acc = w.mv[s];
-            const float u = round_as(adam_update_fast(acc.x, acc.y, inv_bc1, inv_bc2, a.eps), g_bf16);
-            const int pos = w.spos[s];
-            tile[pos] = f32_to_bf16_bits_rne(__fmaf_rn(neg_lr, u, bf16_bits_to_f32(tile[pos])));
-            if (probing) { pr.sum_u2 = fmaf(u, u, pr.sum_u2); pr.zeros_u -= (u != 0.0f) ? 1 : 0; }
+        if (in_place) {
+            update_in_place(p, w.spos, w.mv, touched, neg_lr, inv_bc1, inv_bc2, a.eps, g_bf16, probing ? &pr : nullptr);
+        } else {
+            for (int s = t; s < touched; s += WR_THREADS) {
+                const float2 acc = w.mv[s];
+                const float u = round_as(adam_update_fast(acc.x, acc.y, inv_bc1, inv_bc2, a.eps), g_bf16);
+                const int pos = w.spos[s];
+                tile[pos] = f32_to_bf16_bits_rne(__fmaf_rn(neg_lr, u, bf16_bits_to_f32(tile[pos])));
+                if (probing) { pr.sum_u2 = fmaf(u, u, pr.sum_u2); pr.zeros_u -= (u != 0.0f) ? 1 : 0; }
+            }
         }
         if (probing && t == 0) pr.zeros_u += n_blk;                             // every position without a non-zero update is a zero of u
         MAB_BTICK(7);
@@ -855,8 +965,10 @@ window_resident_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, in
             if (t == 0) { bulk_s2g(p, tile, (uint32_t)n_blk * 2u); store_in_flight = true; }
         } else {
             __syncthreads();
-            for (int i = t; i < n_blk; i += WR_THREADS) p[i] = tile[i];
-            __syncthreads();
+            if (!in_place) {
+                for (int i = t; i < n_blk; i += WR_THREADS) p[i] = tile[i];
+                __syncthreads();
+            }
         }
         MAB_BTICK(8);
 #ifdef MAB_STATS
@@ -931,7 +1043,9 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
     // the tile variant while its compact arrays fit one CTA's shared memory (next to the kernel's static arrays)
     const int smem_tile = (int64_t)a.rows * max_k <= WT_MAX_ENTRIES ? wt_smem_bytes(a.rows, max_k) : 0;
     if (smem_tile > 0 && smem_tile + 4096 <= device_max_optin_smem()) {
-        const int smem = smem_tile;
+        // the forms with the alpha term: a dense array of 256 floats per warp behind the window's arrays, if it fits
+        const int dense_at = ALPHA != 0 && ((smem_tile + 15) & ~15) + 8 * 1024 + 4096 <= device_max_optin_smem() ? (smem_tile + 15) & ~15 : 0;
+        const int smem = dense_at > 0 ? dense_at + 8 * 1024 : smem_tile;
         const int per_sm = std::max(1, std::min(8, (227 * 1024) / (smem + 3072)));
         const int grid = (int)std::min<int64_t>(units_tile, (int64_t)sms * per_sm);
         // fewer resident CTAs (large windows) get more threads each; the forms with the alpha term keep 256
@@ -939,7 +1053,7 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
         auto run = [&](auto kern, int threads) -> int {
             MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
             if constexpr (MODE == MODE_WRITE_UPDATE) kern<<<grid, threads, smem, s>>>(*single, units_tile, max_k, a);
-            else kern<<<grid, threads, smem, s>>>(dev_tensors, n_tensors, units_tile, max_k, a);
+            else kern<<<grid, threads, smem, s>>>(dev_tensors, n_tensors, units_tile, max_k, dense_at, a);
             return MAB_OK;
         };
         int rc;

@@ -90,9 +90,10 @@ def test_sparse_rows_many_blocks(rows):
 
 
 @pytest.mark.parametrize('dtype,alpha', [(torch.float32, 0.5), (torch.bfloat16, 0.1), (torch.bfloat16, -2)])
-@pytest.mark.parametrize('skip,qbs', [(1, 64), (3, 128), (4, 8)])
-def test_alpha_forms_on_slices_that_start_anywhere(dtype, alpha, skip, qbs):
-    """The octet-wide alpha forms of the update with unaligned parameters, whole and short last quantisation blocks."""
+@pytest.mark.parametrize('skip,qbs,offset', [(1, 64, 0.0), (3, 128, 0.0), (4, 8, 0.0), (0, 64, 0.0), (0, 64, 0.2), (2, 32, -1.0)])
+def test_alpha_forms_on_slices_that_start_anywhere(dtype, alpha, skip, qbs, offset):
+    """The octet-wide alpha forms of the update with unaligned parameters, whole and short last quantisation blocks, and
+    residuals far from zero, whose statistics are coarse against a quantisation step (codes then change when they shrink)."""
     from ista_daslab_optimizers_b200 import MicroAdam
     from oracle.microadam_oracle import MicroAdamOracle
     sizes = (7, 200, 4096, DBS + 8 * 5, DBS + 1003)
@@ -102,7 +103,7 @@ def test_alpha_forms_on_slices_that_start_anywhere(dtype, alpha, skip, qbs):
     opt = MicroAdam(params, **hyper)
     ref = MicroAdamOracle(cpu, d_block_size=opt.d_block_size, **hyper)
     for step in range(4):
-        grads = [S.normal_tensor(41 + step, n, n, 1e-3).to(dtype) for n in sizes]
+        grads = [(S.normal_tensor(41 + step, n, n, 1e-3) + (offset if step == 0 else 0.0)).to(dtype) for n in sizes]
         for p, g in zip(params, grads):
             p.grad = torch.empty(g.numel() + skip, dtype=dtype, device='cuda')[skip:].copy_(g)
         opt.step()
