@@ -14,7 +14,7 @@
 namespace mab {
 
 constexpr int SPR_SR = 14592;         // elements of a block one CTA accumulates at a time (57 * 256): a 29 056-element block is two ranges
-constexpr int SPR_THREADS = 512;      // three CTAs of 58 KB of accumulators per SM
+constexpr int SPR_THREADS = 384;      // three CTAs of 58 KB of accumulators per SM, 56 registers a thread (512 threads of 40 spill: 98 us, now 78)
 constexpr int SPR_AHEAD = 8;          // rows whose entries a thread has in flight
 
 constexpr int SP_THREADS = 512;
@@ -100,7 +100,7 @@ sparse_rows_dot_kernel(int64_t k, int64_t dbs, int kbs, int nfull, int k_few, co
 // with a dense fp32 accumulator in shared memory; rows are added in row order (positions are unique inside a
 // row, so a row needs no atomics, but a barrier).  Bound by the chain of rows: a thread fetches its first entry of
 // SPR_AHEAD rows at once, so that a row costs a shared-memory update and a barrier (25.6 M elements, 32 rows of 1 %: 232 us
-// with one load latency per row and four walks over a block's entries, 98 now).
+// with one load latency per row and four walks over a block's entries, 78 now).
 template <typename TO, typename TV>
 __global__ void __launch_bounds__(SPR_THREADS, 3)
 sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int nfull, int k_few, const float* __restrict__ M,
