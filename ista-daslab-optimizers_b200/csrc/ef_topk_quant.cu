@@ -5,6 +5,8 @@
 //   a[I] = 0                   the residual
 //   min / max per quant block  as bf16
 //   e = Q(a)                   requantise the residual
+// It serves what the two-tiles-per-SM kernels do not take: fp32 gradients with loose quantisation blocks, with k above 1880
+// or with tiles above 29 900 elements, and bf16 tiles two of which do not fit an SM.
 // The gradient buffer is only read.  HBM traffic per element: the gradient, one nibble in, one
 // nibble out, plus the per-block statistics and the k selected (index, value) pairs.
 #include "common.cuh"

@@ -21,8 +21,7 @@
 // permutation.  Everything else (other block sizes, unaligned codes, degenerate blocks) keeps the
 // linear layout and the general code.
 //
-// Results are bit-identical to the register-resident kernel in ef_topk_quant.cu (same arithmetic,
-// same tie rule); that kernel keeps serving fp32 gradients.
+// Results are bit-identical to those of the fp32 kernels' arithmetic (ef_topk_quant_f32.cu, ef_topk_quant.cu; same tie rule).
 #include "common.cuh"
 #include "select.cuh"
 #include "codec_fast.cuh"
