@@ -657,6 +657,8 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
             if (T_lo > 0) {
                 const float T_lo_f = __int_as_float(T_lo);
                 const uint32_t T16 = ((uint32_t)T_lo + 0xFFFFu) >> 16;          // the bound as a bf16 magnitude
+                // magnitudes up to infinity's: a NaN is no candidate (it would be selected on top of the k, past the end of the row)
+                const uint32_t span = 0x7F80u - T16;
                 // 1. each warp lists its octets whose maximum reaches the bound and turns their values that
                 //    reach it into candidates (any order)
                 uint16_t* wlist = ss.oct_list + warp * S_WLIST;
@@ -683,8 +685,8 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
                             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                             for (int p = 0; p < 4; ++p) {
-                                mask2[h] |= ((w[p] & 0x7FFFu) >= T16) ? (1u << (2 * p)) : 0u;
-                                mask2[h] |= (((w[p] >> 16) & 0x7FFFu) >= T16) ? (2u << (2 * p)) : 0u;
+                                mask2[h] |= ((w[p] & 0x7FFFu) - T16 <= span) ? (1u << (2 * p)) : 0u;
+                                mask2[h] |= (((w[p] >> 16) & 0x7FFFu) - T16 <= span) ? (2u << (2 * p)) : 0u;
                             }
                         }
                     }
