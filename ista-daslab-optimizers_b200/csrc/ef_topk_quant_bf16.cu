@@ -220,7 +220,7 @@ constexpr int S_GROUP = 2;                   // octets whose instructions the co
 constexpr int S_FULL = 14;                   // 29 056 values = 3632 octets: every thread has 14 whole octets, some a 15th
 
 // One octet of a = bf16(g + Qinv(e)) in place (positions >= n of a ragged tile stay zero); returns the
-// largest |a| of the octet.
+// largest |a| of the octet, never a NaN: the bound search compares bits, and a NaN's would reach every bound.
 // RAGGED = false promises a whole octet; `commit` = false computes but leaves the tile as it is.  SYNC: the warp's lanes
 // meet between their loads and their stores (all of them call).
 // The result goes to octet o_out of the tile (o itself, or its permuted place on a regular tile).
@@ -247,7 +247,7 @@ __device__ __forceinline__ float dequant_octet(uint4* tile4, int o, int o_out, i
     if (SYNC) __syncwarp();
     if (commit) tile4[o_out] = out;
     const uint32_t m2 = maxabs_bf16x2(maxabs_bf16x2(ow[0], ow[1]), maxabs_bf16x2(ow[2], ow[3]));
-    return fmaxf(fabsf(__uint_as_float(m2 << 16)), fabsf(__uint_as_float(m2 & 0xFFFF0000u)));
+    return max3(fabsf(__uint_as_float(m2 << 16)), fabsf(__uint_as_float(m2 & 0xFFFF0000u)), 0.0f);   // (nothing but NaN: 0)
 }
 
 // a = bf16(g + Qinv(e)) in place for the thread's octets t, t + S_NT, ...; per-octet maxima to omax.

@@ -110,9 +110,10 @@ __device__ __noinline__ uint32_t encode_octet_scalar(const float* r, float mn, f
     return w;
 }
 
+// Never a NaN (0 for an octet that holds nothing else): the bound search compares bits, and a NaN's would reach every bound.
 __device__ __forceinline__ float octet_max_abs(const float (&v)[8]) {
     const float m0 = max3(fabsf(v[0]), fabsf(v[1]), fabsf(v[2])), m1 = max3(fabsf(v[3]), fabsf(v[4]), fabsf(v[5]));
-    return max3(m0, m1, fmaxf(fabsf(v[6]), fabsf(v[7])));
+    return max3(m0, m1, max3(fabsf(v[6]), fabsf(v[7]), 0.0f));
 }
 __device__ __forceinline__ void add_octet(float (&v)[8], const float (&x)[8]) {
 #pragma unroll

@@ -50,3 +50,28 @@ def test_nan_is_never_selected(dtype, kind, skip, qbs):
         assert torch.equal(st['V'][0].cpu().view(torch.int16), V.view(torch.int16)), g.numel()
         assert not st['I'][1:].any() and not st['V'][1:].any()          # nothing past the end of the row
     assert _native.device_error() == 0
+
+
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('qbs', [64, 32, 1000])
+def test_nan_octets_do_not_move_the_bound(dtype, qbs):
+    """Tiles with more octets of nothing but NaN than the k that are selected, met by CTAs that come with the bound of a tile
+    before (more tiles than CTAs), and tiles where they leave fewer octets than k."""
+    from ista_daslab_optimizers_b200 import MicroAdam, _native
+    tiles = 148 * 3 + 40
+    g = S.normal_tensor(82, 1, tiles * DBS, 1e-3)
+    t = g.view(tiles, DBS)
+    t[300::3, 4096:8192] = float('nan')                  # 512 octets, k = 291
+    t[301::6, :DBS - 1600] = float('nan')                # 200 octets are left
+    t[302::7, 8:16] = float('nan')
+    g = g.to(dtype)
+    p = torch.nn.Parameter(torch.zeros(g.numel(), dtype=dtype, device='cuda'))
+    opt = MicroAdam([p], m=2, lr=1e-3, quant_block_size=qbs, k_init=0.01)
+    p.grad = g.cuda()
+    opt.step()
+    st = opt.state[p]
+    I, V = _expected_row(g, st)
+    assert torch.equal(st['I'][0].cpu(), I)
+    assert torch.equal(st['V'][0].cpu().view(torch.int16), V.view(torch.int16))
+    assert not st['I'][1].any() and not st['V'][1].any()
+    assert _native.device_error() == 0
