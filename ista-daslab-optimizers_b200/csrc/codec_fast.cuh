@@ -80,7 +80,9 @@ __device__ __forceinline__ uint32_t encode_octet_exact(const float (&r)[8], cons
 // 0 <= r - mn <= mx - mn makes s~ fall in [0.5, 15.5 + 2^-18] by itself.
 // min and max of 8 values with the 3-input min / max of sm_100.
 __device__ __forceinline__ float min3(float a, float b, float c) { float d; asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
+__device__ __forceinline__ float min3_nan(float a, float b, float c) { float d; asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }   // NaN if one of them is
 __device__ __forceinline__ float max3(float a, float b, float c) { float d; asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
+__device__ __forceinline__ float max3_nan(float a, float b, float c) { float d; asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c)); return d; }
 __device__ __forceinline__ void octet_min_max(const float (&v)[8], float& lo, float& hi) {
     lo = fminf(min3(v[0], v[1], v[2]), min3(min3(v[3], v[4], v[5]), v[6], v[7]));
     hi = fmaxf(max3(v[0], v[1], v[2]), max3(max3(v[3], v[4], v[5]), v[6], v[7]));
@@ -114,14 +116,14 @@ __device__ __forceinline__ uint32_t encode_octet_fast(const float (&r)[8], const
         }
         const float2 fl = __fadd2_rn(__fadd2_rd(s, mg2), nmg2);         // floor(s), exact
         const float2 dd = __fadd2_rn(__ffma2_rn(fl, neg1, s), nhalf2);   // (s - floor(s)) - 0.5, exact
-        worst = fmaxf(worst, fmaxf(fabsf(dd.x), fabsf(dd.y)));
+        worst = max3_nan(worst, fabsf(dd.x), fabsf(dd.y));
         f[2 * b] = fl.x; f[2 * b + 1] = fl.y;
         d[2 * b] = dd.x; d[2 * b + 1] = dd.y;
     }
-    if (worst > 0.5f - 1.52587890625e-5f) {
+    if (!(worst <= 0.5f - 1.52587890625e-5f)) {    // (a NaN among the values too: code 0)
 #pragma unroll
         for (int e = 0; e < 8; ++e)
-            if (fabsf(d[e]) > 0.5f - 1.52587890625e-5f) f[e] = static_cast<float>(qcode_exact(r[e], q));
+            if (!(fabsf(d[e]) <= 0.5f - 1.52587890625e-5f)) f[e] = static_cast<float>(qcode_exact(r[e], q));
     }
     // byte b = 16 * code(2b) + code(2b+1), built in float and read from the low mantissa byte
     const uint32_t b0 = __float_as_uint(__fmaf_rn(f[0], 16.0f, f[1]) + 8388608.0f);
@@ -132,7 +134,7 @@ __device__ __forceinline__ uint32_t encode_octet_fast(const float (&r)[8], const
 }
 
 // The same codes without the per-octet branch: `worst` returns the largest |frac(s~) - 0.5| of the
-// octet, and the caller re-codes the octet with encode_octet_fast when it exceeds CODEC_SAFE_FRAC.
+// octet, and the caller re-codes the octet with encode_octet_fast when it exceeds CODEC_SAFE_FRAC or is a NaN.
 // Several octets coded this way in a row overlap in the pipeline.  Requires c.fast.
 constexpr float CODEC_SAFE_FRAC = 0.5f - 1.52587890625e-5f;
 template <bool CLAMP>
@@ -152,7 +154,7 @@ __device__ __forceinline__ uint32_t encode_octet_speculative(const float (&r)[8]
         }
         const float2 fl = __fadd2_rn(__fadd2_rd(s, mg2), nmg2);
         const float2 dd = __fadd2_rn(__ffma2_rn(fl, neg1, s), nhalf2);
-        worst = fmaxf(worst, fmaxf(fabsf(dd.x), fabsf(dd.y)));
+        worst = max3_nan(worst, fabsf(dd.x), fabsf(dd.y));
         f[2 * b] = fl.x; f[2 * b + 1] = fl.y;
     }
     const uint32_t b0 = __float_as_uint(__fmaf_rn(f[0], 16.0f, f[1]) + 8388608.0f);
@@ -177,7 +179,9 @@ __device__ __forceinline__ uint32_t encode_octet(const float (&r)[8], const QPar
 // division).  Values far below half a step, where the residual could underflow, get code 0 from any
 // quotient below 0.5.  floor: adding 2^23 with rounding down leaves the integer in the low mantissa bits.
 // CLAMP: values may lie outside [mn, mn + 15 u] (statistics rounded to bf16): s is clamped to [0, 15.5]
-// before the floor, which gives the codes the defining clamp(floor(s), 0, 15) gives.
+// before the floor, which gives the codes the defining clamp(floor(s), 0, 15) gives, and a NaN the code 0.  Without CLAMP
+// a NaN's bits run into its neighbours' codes: kernel A looks for one first (its block's
+// minimum is then a NaN); the requantisation of loose bf16 blocks does not, NaN being outside the step's contract.
 struct DivConsts { float2 nmn2, r02, nu2; };
 
 __device__ __forceinline__ DivConsts div_consts(const QParams& q) {
@@ -239,6 +243,13 @@ __device__ __forceinline__ uint32_t maxabs_bf16x2(uint32_t a, uint32_t b) {
 __device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
+// Lane-wise minimum that a NaN among the operands makes NaN.
+__device__ __forceinline__ uint32_t min_nan_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("min.NaN.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
 

@@ -403,8 +403,10 @@ ef_topk_quant_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int 
                         if (l_cur >= 0) { atomicMin(&s_qlo[l_cur], l_lo); atomicMax(&s_qhi[l_cur], l_hi); }
                         l_cur = qi; l_lo = 0xFFFFFFFFu; l_hi = 0u;
                     }
-                    l_lo = min(l_lo, ord_key(lo));
-                    l_hi = max(l_hi, ord_key(hi));
+                    if (lo <= hi) {                                      // (not of an octet of nothing but NaN)
+                        l_lo = min(l_lo, ord_key(lo));
+                        l_hi = max(l_hi, ord_key(hi));
+                    }
                 }
                 continue;
             }

@@ -335,9 +335,18 @@ __device__ __forceinline__ void dequant_phase_regular(uint4* tile4, const SmemSe
     }
 }
 
-// Codes of one block of a regular tile with the scalar form of the quantiser: the rare blocks whose step is
-// zero (all values equal), subnormal or infinite.  Kept out of line so that the common path stays small.
-__device__ __noinline__ void encode_block_exact(const uint4* row, int key, uint16_t mn_b, uint16_t mx_b, uint8_t* dst) {
+// Codes of one block of a regular tile with the scalar form of the quantiser: the rare blocks that hold a NaN or whose
+// step is zero (all values equal), subnormal or infinite.  Kept out of line so that the common path stays small.
+__device__ __noinline__ void encode_block_exact(const uint4* row, int key, uint16_t mn_b, uint16_t mx_b, uint16_t* mn_out, uint8_t* dst) {
+    if ((mn_b & 0x7FFFu) > 0x7F80u) {                        // the statistics are those of the other values; the NaN's code is 0
+        uint32_t lo2 = 0x7F807F80u;
+        for (int c = 0; c < 8; ++c) {
+            const uint4 v = row[c];
+            lo2 = min_bf16x2(min_bf16x2(lo2, v.x), min_bf16x2(min_bf16x2(v.y, v.z), v.w));
+        }
+        mn_b = (uint16_t)min_bf16x2(lo2, lo2 >> 16 | lo2 << 16);
+        *mn_out = mn_b;
+    }
     const QParams q2 = qparams(mn_b, mx_b);
     for (int c = 0; c < 8; ++c) {
         float r[8];
@@ -359,16 +368,16 @@ __device__ __forceinline__ void stats_encode_regular(const uint4* tile4, int n_q
         for (int c = 0; c < 8; ++c) {
             const uint4 v = row[c ^ key];
             hi2 = max_bf16x2(max_bf16x2(hi2, v.x), max_bf16x2(max_bf16x2(v.y, v.z), v.w));
-            lo2 = min_bf16x2(min_bf16x2(lo2, v.x), min_bf16x2(min_bf16x2(v.y, v.z), v.w));
+            lo2 = min_nan_bf16x2(min_nan_bf16x2(lo2, v.x), min_nan_bf16x2(min_nan_bf16x2(v.y, v.z), v.w));
         }
         hi2 = max_bf16x2(hi2, hi2 >> 16);
-        lo2 = min_bf16x2(lo2, lo2 >> 16);
+        lo2 = min_nan_bf16x2(lo2, lo2 >> 16);
         const uint16_t mn_b = (uint16_t)(lo2 & 0xFFFFu), mx_b = (uint16_t)(hi2 & 0xFFFFu);
         mn_out[b] = mn_b; mx_out[b] = mx_b;
         const QParams q2 = qparams(mn_b, mx_b);
         uint8_t* dst = ef_out + ((size_t)b << 5);
-        if (!(q2.u >= CODEC_U_MIN && q2.u <= CODEC_U_MAX)) {   // all-equal block (u == 0), subnormal or infinite step
-            encode_block_exact(row, key, mn_b, mx_b, dst);
+        if (!(q2.u >= CODEC_U_MIN && q2.u <= CODEC_U_MAX)) {   // all-equal block (u == 0), subnormal or infinite step, or a NaN in it
+            encode_block_exact(row, key, mn_b, mx_b, mn_out + b, dst);
             continue;
         }
         const float r0 = rcp_rn_normal(q2.u);
@@ -915,8 +924,9 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
             if (t == S_NT - 1 && n_whole < n_oct) {           // the tensor's last, short octet: element by element
                 const int qi = loose_block(lrem0 + n_whole * 8, la.qbs, big);
                 for (int e = n_whole * 8; e < n; ++e) {
-                    const uint32_t key = ord_key(__uint_as_float((uint32_t)tile[e] << 16));
-                    atomicMin(&s_qlo[qi], key); atomicMax(&s_qhi[qi], key);
+                    const float v = __uint_as_float((uint32_t)tile[e] << 16);
+                    if (v != v) continue;                    // (a NaN is in no statistics)
+                    atomicMin(&s_qlo[qi], ord_key(v)); atomicMax(&s_qhi[qi], ord_key(v));
                 }
             }
             {

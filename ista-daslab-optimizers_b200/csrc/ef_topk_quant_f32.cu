@@ -184,14 +184,20 @@ __device__ __forceinline__ void stats_encode_rows(const float4* tile4, int n_row
 #pragma unroll
         for (int c = 0; c < 16; ++c) {
             const float4 v = row[c ^ key];
-            lo = min3(min3(lo, v.x, v.y), v.z, v.w);
+            lo = min3_nan(min3_nan(lo, v.x, v.y), v.z, v.w);
             hi = max3(max3(hi, v.x, v.y), v.z, v.w);
         }
         const uint16_t mn_b = f32_to_bf16_bits_rne(lo), mx_b = f32_to_bf16_bits_rne(hi);
         mn_out[r] = mn_b; mx_out[r] = mx_b;
-        const QParams q = qparams(mn_b, mx_b);
+        QParams q = qparams(mn_b, mx_b);
         uint4* dst = reinterpret_cast<uint4*>(ef_out) + (r << 1);
-        if (!step_in_range(q)) {                             // all-equal block (u == 0), subnormal or infinite step
+        if (!step_in_range(q)) {                             // all-equal block (u == 0), subnormal or infinite step, or a NaN in it
+            if (lo != lo) {                                  // the statistics are those of the other values; the NaN's code is 0
+                lo = INFINITY;
+                for (int i = 0; i < 64; ++i) lo = fminf(lo, reinterpret_cast<const float*>(row)[i]);
+                mn_out[r] = f32_to_bf16_bits_rne(lo);
+                q = qparams(f32_to_bf16_bits_rne(lo), mx_b);
+            }
             for (int o = 0; o < 8; ++o) {
                 float y[8];
                 for (int e = 0; e < 8; ++e) y[e] = reinterpret_cast<const float*>(row)[((o * 8 + e) ^ (key << 2))];

@@ -75,3 +75,41 @@ def test_nan_octets_do_not_move_the_bound(dtype, qbs):
     assert torch.equal(st['V'][0].cpu().view(torch.int16), V.view(torch.int16))
     assert not st['I'][1].any() and not st['V'][1].any()
     assert _native.device_error() == 0
+
+
+@pytest.mark.parametrize('dtype,qbs', [(torch.bfloat16, 64), (torch.bfloat16, 32), (torch.bfloat16, 128),
+                                       (torch.float32, 64), (torch.float32, 32), (torch.float32, 1000)])
+@pytest.mark.parametrize('offset', [0.0, 0.02])
+def test_nan_spoils_no_neighbour(dtype, qbs, offset):
+    """A NaN gets code 0 and is in no statistics: error feedback and window are, bit for bit, those of the operator-level
+    kernels, whose codec is the scalar definition, and no parameter becomes NaN.  (With an offset the statistics are coarse
+    against a quantisation step, and the fp32 kernel clamps.)"""
+    from ista_daslab_optimizers_b200 import MicroAdam, _native
+    sizes = SIZES + (29056 + 64 * 3 + 5, 64, 71)
+    hyper = dict(m=3, lr=1e-3, quant_block_size=qbs, k_init=0.01)
+    pairs = []
+    for use_fused in (True, False):
+        params = [torch.nn.Parameter(S.normal_tensor(83, i, n, 0.02).to(dtype).cuda()) for i, n in enumerate(sizes)]
+        pairs.append((params, MicroAdam(params, use_fused=use_fused, **hyper)))
+    for step in range(4):
+        for i, n in enumerate(sizes):
+            g = S.normal_tensor(84 + step, n, n, 1e-3) + (offset if step == 0 else 0.0)
+            if step < 3:
+                g[3::16 + step] = float('nan')
+                g[n // 2:n // 2 + 10] = float('nan')
+                if n > 4096:
+                    g[1280:1280 + 64 * 5] = float('nan')        # whole quantisation blocks
+            for params, _ in pairs:
+                params[i].grad = g.to(dtype).cuda()
+        for _, opt in pairs:
+            opt.step()
+        for p, q in zip(*(params for params, _ in pairs)):
+            a, b = pairs[0][1].state[p], pairs[1][1].state[q]
+            for key in ('I', 'V', 'error', 'min_vals', 'max_vals'):
+                x, y = a[key], b[key]
+                if key in ('min_vals', 'max_vals'):      # (a block of nothing else: any statistics that decode to NaN)
+                    x, y = x.nan_to_num(0.0, 0.0, 0.0), y.nan_to_num(0.0, 0.0, 0.0)
+                assert torch.equal(x.view(torch.uint8), y.view(torch.uint8)), (step, p.numel(), key)
+            assert torch.isfinite(p).all() and torch.isfinite(q).all()
+    assert any(e.fused for e in pairs[0][1]._entries) and not any(e.fused for e in pairs[1][1]._entries)
+    assert _native.device_error() == 0
