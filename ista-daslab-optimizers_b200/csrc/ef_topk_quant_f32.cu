@@ -231,6 +231,20 @@ __device__ __forceinline__ int f32_count_ge(const float (&a)[F_REG][8], const fl
     return *reinterpret_cast<volatile int*>(counter);
 }
 
+// Whether the tile holds a NaN, every thread of the CTA calling.
+__device__ __forceinline__ bool f32_any_nan(const float (&a)[F_REG][8], const float4* tile4, int n_oct) {
+    bool nan = false;
+#pragma unroll
+    for (int j = 0; j < F_REG; ++j)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) nan |= isnan(a[j][e]);
+    for (int i = threadIdx.x; i < (n_oct - F_REG * F_NT) * 2; i += F_NT) {
+        const float4 v = tile4[i];
+        nan |= isnan(v.x) || isnan(v.y) || isnan(v.z) || isnan(v.w);
+    }
+    return __syncthreads_or(nan);
+}
+
 // sel_bm from gt | (the need_ties lowest positions of tie) of the thread's own two words, and sel_before.  Starts and
 // ends with a barrier.
 __device__ __forceinline__ void f32_resolve(uint32_t (&sel)[F_WPT], uint32_t (&tw)[F_WPT], int need_ties, SmemF& ss) {
@@ -625,7 +639,8 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
             // key bits over the tile, at a cost that does not depend on the data
             uint32_t sel[F_WPT], tw[F_WPT];
             int need = 0;
-            if (kmax == 0) {                                         // every key is zero: the k lowest positions win the ties
+            const bool all_zero = kmax == 0 && !f32_any_nan(a, tile4, n_oct);     // (a NaN leaves no trace in the maxima)
+            if (all_zero) {                                          // every key is zero: the k lowest positions win the ties
 #pragma unroll
                 for (int i = 0; i < F_WPT; ++i) {
                     const int p0 = (t * F_WPT + i) * 32;

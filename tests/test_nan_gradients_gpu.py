@@ -16,6 +16,10 @@ def _gradient(kind, n, step, dtype):
     if kind == 'scattered':                              # one NaN in every second octet, next to values that are selected
         g[3::16] = float('nan')
         g[4::64] *= 20.0
+    elif kind == 'zeros':                                # nothing but zeros next to them
+        g.zero_()
+        g[3::16] = float('nan')
+        g[64:128] = float('nan')
     return g.to(dtype)
 
 
@@ -33,7 +37,7 @@ def _expected_row(g, geo):
     return torch.cat([i for i, _ in idx]).to(torch.int16), g[torch.cat([p for _, p in idx])].bfloat16()
 
 
-@pytest.mark.parametrize('dtype,kind', [(torch.bfloat16, 'scattered'), (torch.float32, 'scattered')])
+@pytest.mark.parametrize('dtype,kind', [(torch.bfloat16, 'scattered'), (torch.float32, 'scattered'), (torch.float32, 'zeros')])
 @pytest.mark.parametrize('skip,qbs', [(0, 64), (1, 64), (0, 32), (0, 1000)])
 def test_nan_is_never_selected(dtype, kind, skip, qbs):
     from ista_daslab_optimizers_b200 import MicroAdam, _native
