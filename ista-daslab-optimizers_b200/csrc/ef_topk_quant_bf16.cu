@@ -217,17 +217,19 @@ __device__ __forceinline__ uint32_t encode_octet_div(const uint4& v, float2 nmn2
 }
 
 constexpr int S_GROUP = 2;                   // octets whose instructions the compiler may interleave (register pressure)
+constexpr int S_AHEAD = 7;                   // octets a thread of a full regular tile reads before its warp meets (with 2 a step of 218 M elements takes
+                                             // 532 us, with 7 528)
 constexpr int S_FULL = 14;                   // 29 056 values = 3632 octets: every thread has 14 whole octets, some a 15th
 
-// One octet of a = bf16(g + Qinv(e)) in place (positions >= n of a ragged tile stay zero); returns the
+// One octet `g8` of a = bf16(g + Qinv(e)) (positions >= n of a ragged tile stay zero); returns the
 // largest |a| of the octet, never a NaN: the bound search compares bits, and a NaN's would reach every bound.
-// RAGGED = false promises a whole octet; `commit` = false computes but leaves the tile as it is.  SYNC: the warp's lanes
-// meet between their loads and their stores (all of them call).
+// RAGGED = false promises a whole octet; `commit` = false computes but leaves the tile as it is.
 // The result goes to octet o_out of the tile (o itself, or its permuted place on a regular tile).
-template <bool FAST, bool RAGGED, bool SYNC = false>
-__device__ __forceinline__ float dequant_octet(uint4* tile4, int o, int o_out, int n, uint32_t codes, const QParams& q, const DecodeConsts& dc, bool commit) {
+template <bool FAST, bool RAGGED>
+__device__ __forceinline__ float dequant_octet(uint4* tile4, const uint4& g8, int o, int o_out, int n, uint32_t codes, const QParams& q, const DecodeConsts& dc,
+                                               bool commit) {
     float gv[8], x[8];
-    unpack8(tile4[o], gv);
+    unpack8(g8, gv);
     if (FAST) decode_octet_fast(codes, dc, x);
     else decode_octet_exact(codes, q, x);
     uint4 out;
@@ -244,7 +246,6 @@ __device__ __forceinline__ float dequant_octet(uint4* tile4, int o, int o_out, i
             if (e0 + 1 >= n) ow[p] = (e0 >= n) ? 0u : (ow[p] & 0xFFFFu);
         }
     }
-    if (SYNC) __syncwarp();
     if (commit) tile4[o_out] = out;
     const uint32_t m2 = maxabs_bf16x2(maxabs_bf16x2(ow[0], ow[1]), maxabs_bf16x2(ow[2], ow[3]));
     return max3(fabsf(__uint_as_float(m2 << 16)), fabsf(__uint_as_float(m2 & 0xFFFF0000u)), 0.0f);   // (nothing but NaN: 0)
@@ -272,7 +273,7 @@ __device__ __forceinline__ void dequant_phase(uint4* tile4, const SmemSel& ss, b
             const float2 c = ss.qt.mu[block_of(o)];
             const QParams q = {c.x, c.y};
             const DecodeConsts dc = decode_consts(q);
-            const float m = dequant_octet<true, false>(tile4, o, o, n, cw[j], q, dc, dc.fast);
+            const float m = dequant_octet<true, false>(tile4, tile4[o], o, o, n, cw[j], q, dc, dc.fast);
             omax[j] = dc.fast ? m : 0.0f;
             slow |= dc.fast ? 0u : (1u << j);
         } else if (o < n_oct) {
@@ -282,7 +283,7 @@ __device__ __forceinline__ void dequant_phase(uint4* tile4, const SmemSel& ss, b
             else q = qparams(mn_g[b], mx_g[b]);
             const DecodeConsts dc = decode_consts(q);
             if (!dc.fast) slow |= 1u << j;
-            else omax[j] = dequant_octet<true, true>(tile4, o, o, n, cw[j], q, dc, true);
+            else omax[j] = dequant_octet<true, true>(tile4, tile4[o], o, o, n, cw[j], q, dc, true);
         }
     }
     if (slow) {
@@ -292,45 +293,48 @@ __device__ __forceinline__ void dequant_phase(uint4* tile4, const SmemSel& ss, b
                 const int o = t + j * S_NT;
                 const int b = block_of(o);
                 const QParams q = qparams(mn_g[b], mx_g[b]);
-                omax[j] = dequant_octet<false, true>(tile4, o, o, n, cw[j], q, decode_consts(q), true);
+                omax[j] = dequant_octet<false, true>(tile4, tile4[o], o, o, n, cw[j], q, decode_consts(q), true);
             }
         }
     }
 }
 
 // The same on a regular tile (see the head of the file): every block's decode is the fast one, and octet o is written
-// to its permuted place.  The 8 lanes that hold a 128-byte row read it in one instruction and write it in a later one,
-// so the permutation inside the row happens in place.  FULL: the first S_FULL octets of every thread exist and none
+// to its permuted place.  The 8 lanes that hold a 128-byte row all read it before one of them writes it (the warp meets in
+// between), so the permutation inside the row happens in place.  FULL: the first S_FULL octets of every thread exist and none
 // is short; otherwise the tile may end anywhere (the places a last, short row's missing octets leave are never read).
 template <bool FULL>
 __device__ __forceinline__ void dequant_phase_regular(uint4* tile4, const SmemSel& ss, int n, int n_oct, const uint32_t (&cw)[S_SLOTS], float (&omax)[S_SLOTS]) {
     const int t = threadIdx.x;
     const int t_out = t ^ ((t >> 3) & 7);                   // phys_oct(t + j * S_NT) = t_out + j * S_NT
-    if constexpr (!FULL) {
+    constexpr int whole = FULL ? S_FULL : 0;
+    static_assert(S_FULL % S_AHEAD == 0, "whole groups");
 #pragma unroll
-        for (int j = 0; j < S_SLOTS; ++j) {
-            omax[j] = 0.0f;
-            const int o = t + j * S_NT;
-            if ((o & ~31) < n_oct) {                         // whole warps
-                const bool on = o < n_oct;
-                const int at = on ? o : n_oct - 1;
-                const float2 c = ss.qt.mu[at >> 3];
-                const QParams q = {c.x, c.y};
-                const float m = dequant_octet<true, true, true>(tile4, at, t_out + j * S_NT, n, cw[j], q, decode_consts(q), on);
-                omax[j] = on ? m : 0.0f;
-            }
+    for (int j0 = 0; j0 < whole; j0 += S_AHEAD) {
+        uint4 g8[S_AHEAD];
+#pragma unroll
+        for (int i = 0; i < S_AHEAD; ++i) g8[i] = tile4[t + (j0 + i) * S_NT];
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < S_AHEAD; ++i) {
+            const int j = j0 + i, o = t + j * S_NT;
+            if (i % S_GROUP == 0) asm volatile("" ::: "memory");
+            const float2 c = ss.qt.mu[o >> 3];
+            const QParams q = {c.x, c.y};
+            omax[j] = dequant_octet<true, false>(tile4, g8[i], o, t_out + j * S_NT, 0, cw[j], q, decode_consts(q), true);
         }
-    } else {
+    }
 #pragma unroll
-        for (int j = 0; j < S_SLOTS; ++j) {
-            omax[j] = 0.0f;
-            const int o = t + j * S_NT;
-            if (j < S_FULL || o < n_oct) {
-                if (j < S_FULL && j % S_GROUP == 0) asm volatile("" ::: "memory");
-                const float2 c = ss.qt.mu[o >> 3];
-                const QParams q = {c.x, c.y};
-                omax[j] = dequant_octet<true, false>(tile4, o, t_out + j * S_NT, 0, cw[j], q, decode_consts(q), true);
-            }
+    for (int j = whole; j < S_SLOTS; ++j) {
+        omax[j] = 0.0f;
+        const int o = t + j * S_NT;
+        const unsigned there = __ballot_sync(0xffffffffu, o < n_oct);
+        if (o < n_oct) {
+            const uint4 g8 = tile4[o];
+            __syncwarp(there);
+            const float2 c = ss.qt.mu[o >> 3];
+            const QParams q = {c.x, c.y};
+            omax[j] = dequant_octet<true, !FULL>(tile4, g8, o, t_out + j * S_NT, n, cw[j], q, decode_consts(q), true);
         }
     }
 }

@@ -57,3 +57,28 @@ def test_short_tiles_match_oracle(kind, k_init, skip, alpha, dtype):
                 rtol, atol = cases.param_tolerances(dtype, hyper['lr'])
                 torch.testing.assert_close(p.detach().cpu().float(), cpu[i].float(), rtol=rtol, atol=atol)
     assert _native.device_error() == 0
+
+
+@pytest.mark.parametrize('qbs', [64, 32])
+def test_full_tiles_that_end_inside_a_row(qbs):
+    """bf16 tiles long enough for the branch-free decode whose last row of eight octets is short: the rows are permuted in
+    place, the last octets of a thread among partly idle warps."""
+    from ista_daslab_optimizers_b200 import MicroAdam, _native
+    from oracle.microadam_oracle import MicroAdamOracle
+    sizes = (28672 + 8, 28672 + 56, 28672 + 256 - 8, 28672 + 264, DBS - 8, 2 * DBS - 40)
+    hyper = dict(m=3, lr=1e-3, quant_block_size=qbs, k_init=0.01)
+    params = [torch.nn.Parameter(S.normal_tensor(62, i, n, 0.02).bfloat16().cuda()) for i, n in enumerate(sizes)]
+    opt = MicroAdam(params, **hyper)
+    ref = MicroAdamOracle([p.detach().cpu().clone() for p in params], d_block_size=opt.d_block_size, **hyper)
+    for step in range(3):
+        grads = [S.normal_tensor(63 + step, n, n, 1e-3).bfloat16() for n in sizes]
+        for p, g in zip(params, grads):
+            p.grad = g.cuda()
+        opt.step()
+        ref.step([g.clone() for g in grads])
+        for i, (p, n) in enumerate(zip(params, sizes)):
+            a, b, used = opt.state[p], ref.state[i], -(-n // qbs)
+            assert torch.equal(a['I'][step].cpu(), b['I'][step]), (n, step)
+            for key, cut in (('V', None), ('error', None), ('min_vals', used), ('max_vals', used)):
+                assert torch.equal(a[key][:cut].cpu().view(torch.uint8), b[key][:cut].view(torch.uint8)), (n, step, key)
+    assert _native.device_error() == 0
