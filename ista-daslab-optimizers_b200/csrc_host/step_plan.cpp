@@ -7,15 +7,17 @@
 // every step it is checked against the optimizer as it stands (same groups, same parameters, a gradient where there was
 // one, the same element types, contiguous CUDA memory), and any difference hands the step back to the Python side,
 // which rebuilds the plan or raises.  Learning rates, weight decays, ring positions, parameter and gradient
-// addresses are read every step.
+// addresses are read every step.  What torch throws on the way becomes the Python exception it stands for.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <memory>
 #include <optional>
 #include <vector>
 
@@ -82,15 +84,15 @@ bool number(PyObject* dict, PyObject* key, double* out) {
 //   groups: [(group dictionary, [(parameter, kind, state dictionary or None, first element of its slice), ...]), ...]
 //   descs: the descriptors of the Active parameters in that order, their fixed fields filled in
 PyObject* plan_new(PyObject*, PyObject* args) {
+    HANDLE_TH_ERRORS
     PyObject* groups;
     unsigned long long descs_at, fn_at, ws_at;
     long long n_descs, ws_bytes;
     int window, device;
     if (!PyArg_ParseTuple(args, "O!KLiiKKL", &PyList_Type, &groups, &descs_at, &n_descs, &window, &device, &fn_at, &ws_at, &ws_bytes))
         return nullptr;
-    auto* plan = new Plan;
-    PyObject* capsule = PyCapsule_New(plan, CAPSULE, destroy_plan);
-    if (capsule == nullptr) { delete plan; return nullptr; }
+    auto owner = std::make_unique<Plan>();
+    Plan* plan = owner.get();
     const auto* d = reinterpret_cast<const mab_tensor*>(static_cast<uintptr_t>(descs_at));
     plan->descs.assign(d, d + n_descs);
     plan->window = window;
@@ -106,7 +108,7 @@ PyObject* plan_new(PyObject*, PyObject* args) {
     int64_t active = 0;
     for (Py_ssize_t gi = 0; gi < PyList_GET_SIZE(groups); ++gi) {
         PyObject *dict, *list;
-        if (!PyArg_ParseTuple(PyList_GET_ITEM(groups, gi), "O!O!", &PyDict_Type, &dict, &PyList_Type, &list)) { Py_DECREF(capsule); return nullptr; }
+        if (!PyArg_ParseTuple(PyList_GET_ITEM(groups, gi), "O!O!", &PyDict_Type, &dict, &PyList_Type, &list)) return nullptr;
         plan->groups.emplace_back();
         Group& g = plan->groups.back();
         g.object = Py_NewRef(dict);
@@ -114,10 +116,9 @@ PyObject* plan_new(PyObject*, PyObject* args) {
             PyObject *object, *state;
             int kind;
             long long first;
-            if (!PyArg_ParseTuple(PyList_GET_ITEM(list, i), "OiOL", &object, &kind, &state, &first)) { Py_DECREF(capsule); return nullptr; }
+            if (!PyArg_ParseTuple(PyList_GET_ITEM(list, i), "OiOL", &object, &kind, &state, &first)) return nullptr;
             if (!THPVariable_Check(object) || kind < 0 || kind > 2 || (kind == 2 && !PyDict_Check(state))) {
                 PyErr_SetString(PyExc_TypeError, "plan_new: a parameter is not a tensor, or has no state dictionary");
-                Py_DECREF(capsule);
                 return nullptr;
             }
             Param p = {};
@@ -138,10 +139,12 @@ PyObject* plan_new(PyObject*, PyObject* args) {
     }
     if (active != n_descs || window < 1) {
         PyErr_SetString(PyExc_ValueError, "plan_new: one descriptor per active parameter");
-        Py_DECREF(capsule);
         return nullptr;
     }
+    PyObject* capsule = PyCapsule_New(plan, CAPSULE, destroy_plan);
+    if (capsule != nullptr) owner.release();
     return capsule;
+    END_HANDLE_TH_ERRORS
 }
 
 // Brings plan.descs up to date.  1: the optimizer no longer looks like the plan, 0: done, -1: a Python error is set.
@@ -187,6 +190,7 @@ int refresh(Plan& plan, PyObject* groups) {
 
 // plan_step(plan, param_groups, steps, quant_block_size, alpha, beta1, beta2, eps) -> 1 stale, <= 0 the library's status
 PyObject* plan_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
     if (n != 8) { PyErr_SetString(PyExc_TypeError, "plan_step takes 8 arguments"); return nullptr; }
     auto* plan = static_cast<Plan*>(PyCapsule_GetPointer(args[0], CAPSULE));
     if (plan == nullptr) return nullptr;
@@ -201,14 +205,15 @@ PyObject* plan_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (PyErr_Occurred()) return nullptr;
     const int state = refresh(*plan, args[1]);
     if (state != 0) return state < 0 ? nullptr : PyLong_FromLong(1);
+    std::optional<c10::cuda::CUDAGuard> guard;           // (the calls that can fail, before anything has changed)
+    if (c10::cuda::current_device() != plan->device) guard.emplace(plan->device);
+    void* stream = c10::cuda::getCurrentCUDAStream(plan->device).stream();
     size_t at = 0;                                       // every position has been read: now they advance (micro_adam.py:211)
     for (Group& g : plan->groups)
         for (Param& p : g.params)
             if (p.kind == Kind::Active && PyDict_SetItem(p.state, plan->key_index, plan->ring_next[plan->descs[at++].ring_index]) < 0) return nullptr;
-    std::optional<c10::cuda::CUDAGuard> guard;
-    if (c10::cuda::current_device() != plan->device) guard.emplace(plan->device);
-    void* stream = c10::cuda::getCurrentCUDAStream(plan->device).stream();
     return PyLong_FromLong(plan->fused_step(plan->descs.data(), static_cast<int>(plan->descs.size()), &a, plan->workspace, plan->workspace_bytes, stream));
+    END_HANDLE_TH_ERRORS
 }
 
 PyMethodDef methods[] = {

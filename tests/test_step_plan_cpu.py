@@ -1,0 +1,51 @@
+"""The native host side of the step (csrc_host/step_plan.cpp) where no GPU is needed: what it does when torch throws."""
+import subprocess
+import sys
+import textwrap
+
+import pytest
+import torch
+
+from conftest import ROOT
+
+_PRELUDE = textwrap.dedent(f"""
+    import ctypes, sys, warnings
+    sys.path.insert(0, {ROOT + '/ista-daslab-optimizers_b200'!r})
+    import torch
+    from ista_daslab_optimizers_b200 import _native as N
+    from ista_daslab_optimizers_b200 import _step_plan as plan
+
+    def step(p, groups):
+        return plan.plan_step(p, groups, 1, 64, 0, 0.9, 0.999, 1e-8)
+""")
+
+
+def _run(body):
+    return subprocess.run([sys.executable, '-c', _PRELUDE + textwrap.dedent(body)], capture_output=True, text=True, timeout=300)
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason='needs a machine where torch finds no CUDA device')
+def test_an_error_of_torch_is_an_exception_and_changes_nothing():
+    """Asking torch for the current device fails here.  The process lives, and the ring position has not moved."""
+    out = _run("""
+        group = {'params': [], 'lr': 0.1, 'weight_decay': 0.0}
+        empty = plan.plan_new([(group, [])], 0, 0, 4, 0, 0, 0, 0)
+        try:
+            step(empty, [group])
+        except RuntimeError as e:
+            print('raised', 'CUDA' in str(e))
+        # a parameter that says it lies on a CUDA device
+        from torch._subclasses.fake_tensor import FakeTensorMode
+        warnings.simplefilter('ignore')
+        with FakeTensorMode(allow_non_fake_inputs=True):
+            p = torch.nn.Parameter(torch.empty(64, device='cuda'))
+            p.grad = torch.empty(64, device='cuda')
+        group, state, desc = {'params': [p], 'lr': 0.1, 'weight_decay': 0.0}, {'index': 2}, (N.MabTensor * 1)()
+        full = plan.plan_new([(group, [(p, 2, state, 0)])], ctypes.addressof(desc), 1, 4, 0, 0, 0, 0)
+        try:
+            step(full, [group])
+        except RuntimeError:
+            print('raised', state)
+    """)
+    assert out.returncode == 0, out.stderr[-2000:]
+    assert out.stdout.split('\n')[:2] == ['raised True', "raised {'index': 2}"]
