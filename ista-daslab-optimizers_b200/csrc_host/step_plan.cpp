@@ -188,6 +188,11 @@ int refresh(Plan& plan, PyObject* groups) {
     return 0;
 }
 
+struct ReleasedInterpreter {
+    PyThreadState* saved = PyEval_SaveThread();
+    ~ReleasedInterpreter() { PyEval_RestoreThread(saved); }
+};
+
 // plan_step(plan, param_groups, steps, quant_block_size, alpha, beta1, beta2, eps) -> 1 stale, <= 0 the library's status
 PyObject* plan_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
@@ -212,7 +217,12 @@ PyObject* plan_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
     for (Group& g : plan->groups)
         for (Param& p : g.params)
             if (p.kind == Kind::Active && PyDict_SetItem(p.state, plan->key_index, plan->ring_next[plan->descs[at++].ring_index]) < 0) return nullptr;
-    return PyLong_FromLong(plan->fused_step(plan->descs.data(), static_cast<int>(plan->descs.size()), &a, plan->workspace, plan->workspace_bytes, stream));
+    long status;
+    {
+        const ReleasedInterpreter other_threads_run;     // the copy of the table and the launches may wait for the GPU
+        status = plan->fused_step(plan->descs.data(), static_cast<int>(plan->descs.size()), &a, plan->workspace, plan->workspace_bytes, stream);
+    }
+    return PyLong_FromLong(status);
     END_HANDLE_TH_ERRORS
 }
 

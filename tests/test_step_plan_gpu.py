@@ -1,5 +1,10 @@
 """The native host side of the step (csrc_host/step_plan.cpp) against the Python side it stands in for: the same bits,
 and the Python side again whenever something about the parameters changes between steps."""
+import ctypes
+import subprocess
+import threading
+import time
+
 import pytest
 import torch
 
@@ -72,3 +77,33 @@ def test_step_hooks_and_non_contiguous_gradients():
     params[1].grad = torch.ones(2 * params[1].numel(), device='cuda')[::2]
     with pytest.raises(N.NativeError, match='contiguous'):
         opt.step()
+
+
+def test_other_threads_run_while_the_library_is_called(tmp_path):
+    """The call into the library may wait for the GPU (a full launch queue, a large descriptor table): Python's global lock is
+    not held meanwhile.  A host function that sleeps stands in for the library."""
+    from ista_daslab_optimizers_b200 import _step_plan
+    src, lib = tmp_path / 'slow.c', tmp_path / 'slow.so'
+    src.write_text('#include <unistd.h>\nint slow(void* t, int n, const void* a, void* w, long long b, void* s) { usleep(400000); return n; }\n')
+    subprocess.run(['gcc', '-shared', '-fPIC', '-o', str(lib), str(src)], check=True)
+    slow = ctypes.CDLL(str(lib)).slow
+    torch.zeros(1, device='cuda')
+    group = {'params': [], 'lr': 0.1, 'weight_decay': 0.0}
+    plan = _step_plan.plan_new([(group, [])], 0, 0, 4, 0, ctypes.cast(slow, ctypes.c_void_p).value, 0, 0)
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(0.005)
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    time.sleep(0.05)
+    begin = time.perf_counter()
+    assert _step_plan.plan_step(plan, [group], 1, 64, 0, 0.9, 0.999, 1e-8) == 0
+    end = time.perf_counter()
+    stop.set()
+    thread.join()
+    assert end - begin >= 0.4
+    assert sum(begin + 0.05 < t < end - 0.05 for t in ticks) >= 10      # of about 60; none with the lock held
