@@ -19,6 +19,7 @@
 
 #include <memory>
 #include <optional>
+#include <utility>
 #include <vector>
 
 #include "microadam_b200.h"
@@ -54,19 +55,54 @@ struct Plan {
     int64_t workspace_bytes = 0;
     PyObject *key_params = nullptr, *key_lr = nullptr, *key_weight_decay = nullptr, *key_index = nullptr;
 
-    ~Plan() {
+    // Every reference the plan owns, for Python's collector: a group or a parameter may refer to the optimizer that holds the plan.
+    template <typename F> int each_reference(F&& visit) {
         for (Group& g : groups) {
-            for (Param& p : g.params) { Py_XDECREF(p.object); Py_XDECREF(p.state); }
-            Py_XDECREF(g.object);
+            for (Param& p : g.params) {
+                if (int rc = visit(p.object)) return rc;
+                if (int rc = visit(p.state)) return rc;
+            }
+            if (int rc = visit(g.object)) return rc;
         }
-        for (PyObject* o : ring_next) Py_XDECREF(o);
-        Py_XDECREF(key_params); Py_XDECREF(key_lr); Py_XDECREF(key_weight_decay); Py_XDECREF(key_index);
+        for (PyObject*& o : ring_next) if (int rc = visit(o)) return rc;
+        for (PyObject** o : {&key_params, &key_lr, &key_weight_decay, &key_index}) if (int rc = visit(*o)) return rc;
+        return 0;
     }
+    ~Plan() { each_reference([](PyObject*& o) { Py_CLEAR(o); return 0; }); }
 };
 
-constexpr const char* CAPSULE = "mab_step_plan";
+// The Python object around a plan.
+struct PlanObject {
+    PyObject_HEAD
+    Plan* plan;                  // nullptr once the collector has cleared it
+};
 
-void destroy_plan(PyObject* capsule) { delete static_cast<Plan*>(PyCapsule_GetPointer(capsule, CAPSULE)); }
+PyTypeObject* g_plan_type = nullptr;     // (the module owns it as well)
+
+int plan_traverse(PyObject* self, visitproc visit, void* arg) {
+    Py_VISIT(Py_TYPE(self));
+    Plan* plan = reinterpret_cast<PlanObject*>(self)->plan;
+    return plan == nullptr ? 0 : plan->each_reference([&](PyObject* o) { Py_VISIT(o); return 0; });
+}
+
+int plan_clear(PyObject* self) {
+    delete std::exchange(reinterpret_cast<PlanObject*>(self)->plan, nullptr);
+    return 0;
+}
+
+void plan_dealloc(PyObject* self) {
+    PyObject_GC_UnTrack(self);
+    plan_clear(self);
+    PyTypeObject* type = Py_TYPE(self);
+    PyObject_GC_Del(self);
+    Py_DECREF(type);
+}
+
+PyType_Slot plan_slots[] = {{Py_tp_traverse, reinterpret_cast<void*>(plan_traverse)},
+                            {Py_tp_clear, reinterpret_cast<void*>(plan_clear)},
+                            {Py_tp_dealloc, reinterpret_cast<void*>(plan_dealloc)},
+                            {0, nullptr}};
+PyType_Spec plan_spec = {"_step_plan.Plan", sizeof(PlanObject), 0, Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_GC | Py_TPFLAGS_DISALLOW_INSTANTIATION, plan_slots};
 
 // A number in a group's dictionary (a float, an int, or anything float() takes, such as a tensor).
 bool number(PyObject* dict, PyObject* key, double* out) {
@@ -141,9 +177,11 @@ PyObject* plan_new(PyObject*, PyObject* args) {
         PyErr_SetString(PyExc_ValueError, "plan_new: one descriptor per active parameter");
         return nullptr;
     }
-    PyObject* capsule = PyCapsule_New(plan, CAPSULE, destroy_plan);
-    if (capsule != nullptr) owner.release();
-    return capsule;
+    auto* object = PyObject_GC_New(PlanObject, g_plan_type);
+    if (object == nullptr) return nullptr;
+    object->plan = owner.release();
+    PyObject_GC_Track(object);
+    return reinterpret_cast<PyObject*>(object);
     END_HANDLE_TH_ERRORS
 }
 
@@ -197,8 +235,9 @@ struct ReleasedInterpreter {
 PyObject* plan_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     if (n != 8) { PyErr_SetString(PyExc_TypeError, "plan_step takes 8 arguments"); return nullptr; }
-    auto* plan = static_cast<Plan*>(PyCapsule_GetPointer(args[0], CAPSULE));
-    if (plan == nullptr) return nullptr;
+    if (!Py_IS_TYPE(args[0], g_plan_type)) { PyErr_SetString(PyExc_TypeError, "plan_step: not a plan"); return nullptr; }
+    Plan* plan = reinterpret_cast<PlanObject*>(args[0])->plan;
+    if (plan == nullptr) return PyLong_FromLong(1);
     mab_step_args a = {};
     a.steps = PyLong_AsLongLong(args[2]);
     a.m = plan->window;
@@ -235,4 +274,10 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_step_plan", "Native host side of 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__step_plan(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__step_plan(void) {
+    PyObject* m = PyModule_Create(&module);
+    if (m == nullptr) return nullptr;
+    g_plan_type = reinterpret_cast<PyTypeObject*>(PyType_FromSpec(&plan_spec));
+    if (g_plan_type == nullptr || PyModule_AddObjectRef(m, "Plan", reinterpret_cast<PyObject*>(g_plan_type)) < 0) { Py_DECREF(m); return nullptr; }
+    return m;
+}

@@ -49,3 +49,35 @@ def test_an_error_of_torch_is_an_exception_and_changes_nothing():
     """)
     assert out.returncode == 0, out.stderr[-2000:]
     assert out.stdout.split('\n')[:2] == ['raised True', "raised {'index': 2}"]
+
+
+def test_a_plan_keeps_no_cycle_alive():
+    """A group or a parameter may refer to the optimizer that holds the plan: Python's collector sees through the plan, as it
+    sees through the optimizer's own dictionaries."""
+    out = _run("""
+        import gc, weakref
+
+        class Holder:
+            pass
+
+        def make(where):
+            h, p, desc = Holder(), torch.nn.Parameter(torch.zeros(8)), (N.MabTensor * 1)()
+            p.grad = torch.zeros(8)
+            group, state = {'params': [p], 'lr': 0.1, 'weight_decay': 0.0}, {'index': 0}
+            h.plan = plan.plan_new([(group, [(p, 2, state, 0)])], ctypes.addressof(desc), 1, 4, 0, 0, 0, 0)
+            h.group = group
+            if where == 'group':
+                group['owner'] = h
+            elif where == 'parameter':
+                p.owner = h
+            elif where == 'state':
+                state['owner'] = h
+            return weakref.ref(h), weakref.ref(p)
+
+        for where in ('nowhere', 'group', 'parameter', 'state'):
+            refs = make(where)
+            gc.collect()
+            print(where, [r() is None for r in refs])
+    """)
+    assert out.returncode == 0, out.stderr[-2000:]
+    assert out.stdout.split('\n')[:4] == [f'{w} [True, True]' for w in ('nowhere', 'group', 'parameter', 'state')]
