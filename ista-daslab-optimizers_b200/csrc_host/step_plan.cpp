@@ -17,6 +17,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <exception>
 #include <memory>
 #include <optional>
 #include <utility>
@@ -116,11 +117,16 @@ bool number(PyObject* dict, PyObject* key, double* out) {
     return true;
 }
 
+// The exception in flight (torch's errors, bad_alloc) as Python's: none may cross the interpreter's C frames.
+PyObject* raise_python() {
+    torch::translate_exception_to_python(std::current_exception());
+    return nullptr;
+}
+
 // plan_new(groups, descs_address, n_descs, m, device_index, fused_step_address, workspace_address, workspace_bytes)
 //   groups: [(group dictionary, [(parameter, kind, state dictionary or None, first element of its slice), ...]), ...]
 //   descs: the descriptors of the Active parameters in that order, their fixed fields filled in
-PyObject* plan_new(PyObject*, PyObject* args) {
-    HANDLE_TH_ERRORS
+PyObject* plan_new(PyObject*, PyObject* args) try {
     PyObject* groups;
     unsigned long long descs_at, fn_at, ws_at;
     long long n_descs, ws_bytes;
@@ -182,7 +188,8 @@ PyObject* plan_new(PyObject*, PyObject* args) {
     object->plan = owner.release();
     PyObject_GC_Track(object);
     return reinterpret_cast<PyObject*>(object);
-    END_HANDLE_TH_ERRORS
+} catch (...) {
+    return raise_python();
 }
 
 // Brings plan.descs up to date.  1: the optimizer no longer looks like the plan, 0: done, -1: a Python error is set.
@@ -232,8 +239,7 @@ struct ReleasedInterpreter {
 };
 
 // plan_step(plan, param_groups, steps, quant_block_size, alpha, beta1, beta2, eps) -> 1 stale, <= 0 the library's status
-PyObject* plan_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    HANDLE_TH_ERRORS
+PyObject* plan_step(PyObject*, PyObject* const* args, Py_ssize_t n) try {
     if (n != 8) { PyErr_SetString(PyExc_TypeError, "plan_step takes 8 arguments"); return nullptr; }
     if (!Py_IS_TYPE(args[0], g_plan_type)) { PyErr_SetString(PyExc_TypeError, "plan_step: not a plan"); return nullptr; }
     Plan* plan = reinterpret_cast<PlanObject*>(args[0])->plan;
@@ -262,7 +268,8 @@ PyObject* plan_step(PyObject*, PyObject* const* args, Py_ssize_t n) {
         status = plan->fused_step(plan->descs.data(), static_cast<int>(plan->descs.size()), &a, plan->workspace, plan->workspace_bytes, stream);
     }
     return PyLong_FromLong(status);
-    END_HANDLE_TH_ERRORS
+} catch (...) {
+    return raise_python();
 }
 
 PyMethodDef methods[] = {
