@@ -251,7 +251,10 @@ class MicroAdam(torch.optim.Optimizer):
             status = _step_plan.plan_step(self._plan, self.param_groups, self.steps, self.quant_block_size, self.alpha,
                                           self.beta1, self.beta2, self.eps)
             if status == N.MAB_OK:
-                self._after_update()
+                after = self._after_update
+                if getattr(after, '__func__', None) is not MicroAdam._after_update:     # (1 us that only a hook needs)
+                    with torch.no_grad():
+                        after()
                 return loss
             if status < 0:
                 N.check(status, 'mab_fused_step')
@@ -353,7 +356,7 @@ class MicroAdam(torch.optim.Optimizer):
         })
 
     def _after_update(self):
-        """Hook for subclasses (the sharded optimizer gathers the updated parameters here)."""
+        """Hook for subclasses (the sharded optimizer gathers the updated parameters here); runs without gradients."""
 
     def _refresh_entries(self):
         active = []

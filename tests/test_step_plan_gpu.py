@@ -107,3 +107,31 @@ def test_other_threads_run_while_the_library_is_called(tmp_path):
     thread.join()
     assert end - begin >= 0.4
     assert sum(begin + 0.05 < t < end - 0.05 for t in ticks) >= 10      # of about 60; none with the lock held
+
+
+def test_after_update_hook_runs_without_gradients():
+    """A subclass may write parameters in `_after_update`, on native steps as on the others; so may a hook set on the object."""
+    from ista_daslab_optimizers_b200 import MicroAdam
+
+    class Halving(MicroAdam):
+        def _after_update(self):
+            assert not torch.is_grad_enabled()
+            for group in self.param_groups:
+                for p in group['params']:
+                    p.mul_(0.5)
+
+    p = torch.nn.Parameter(torch.ones(5000, device='cuda'))
+    opt = Halving([p], m=4, lr=0.0, quant_block_size=64)
+    p.grad = torch.ones_like(p)
+    for _ in range(3):
+        opt.step()
+    assert opt._plan is not None and torch.is_grad_enabled()
+    assert torch.equal(p.detach(), torch.full_like(p, 0.125))
+    q = torch.nn.Parameter(torch.ones(5000, device='cuda'))
+    opt = MicroAdam([q], m=4, lr=0.0, quant_block_size=64)
+    seen = []
+    opt._after_update = lambda: seen.append(torch.is_grad_enabled())
+    q.grad = torch.ones_like(q)
+    for _ in range(3):
+        opt.step()
+    assert seen == [False] * 3
