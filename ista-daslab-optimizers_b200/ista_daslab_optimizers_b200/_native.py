@@ -6,6 +6,7 @@ Torch is used only to obtain device pointers and the current CUDA stream.
 from __future__ import annotations
 
 import ctypes
+import importlib
 import os
 from ctypes import POINTER, Structure, c_char_p, c_double, c_float, c_int, c_int32, c_int64, c_void_p
 
@@ -103,6 +104,21 @@ def load(path: str = LIB_PATH) -> ctypes.CDLL:
             fn.argtypes = argtypes
         _lib = lib
     return _lib
+
+
+_step_plan = None
+
+
+def load_step_plan():
+    """The module of the step's native host side (csrc_host/step_plan.cpp).  Raises if it is not built."""
+    global _step_plan
+    if _step_plan is None:
+        try:
+            _step_plan = importlib.import_module('._step_plan', __package__)
+        except ImportError as e:
+            raise NativeError('the native host side of the step cannot be loaded: build it with '
+                              f'`python ista-daslab-optimizers_b200/build.py` (needs g++ and Python\'s headers): {e}') from e
+    return _step_plan
 
 
 def check(status: int, what: str) -> None:

@@ -36,7 +36,6 @@ from typing import Dict, List, Optional, Tuple
 import torch
 
 from . import _native as N
-from . import _step_plan
 from .tools import CopyDirection, block_split, get_first_device
 
 
@@ -96,7 +95,8 @@ class MicroAdam(torch.optim.Optimizer):
         self.use_fused = bool(use_fused)
         self.log_fn = log_fn      # callable(dict) or None; None (the default) switches the probes off
 
-        N.load()   # fail here, loudly, if the native library is not built
+        N.load()   # fail here, loudly, if the native library or the step's host side is not built
+        self._native_step = N.load_step_plan()
         if d_block_size is None:
             self.blocks = N.get_sm_count() * int(100 / self.shared_memory_carveout)                  # micro_adam.py:40
             self.max_floats = N.get_max_floats_for_shared_memory_per_thread_block()                    # micro_adam.py:43
@@ -248,8 +248,8 @@ class MicroAdam(torch.optim.Optimizer):
             with torch.enable_grad():
                 loss = closure()
         if self._plan is not None and self.log_fn is None and self.kernel_events is None:
-            status = _step_plan.plan_step(self._plan, self.param_groups, self.steps, self.quant_block_size, self.alpha,
-                                          self.beta1, self.beta2, self.eps)
+            status = self._native_step.plan_step(self._plan, self.param_groups, self.steps, self.quant_block_size, self.alpha,
+                                                self.beta1, self.beta2, self.eps)
             if status == N.MAB_OK:
                 after = self._after_update
                 if getattr(after, '__func__', None) is not MicroAdam._after_update:     # (1 us that only a hook needs)
@@ -300,8 +300,8 @@ class MicroAdam(torch.optim.Optimizer):
                 rows.append((p, kind, e.st if e else None, e.lo if e else 0))
             groups.append((group, rows))
         ws, fn = self._workspace, ctypes.cast(N.load().mab_fused_step, ctypes.c_void_p).value
-        self._plan = _step_plan.plan_new(groups, ctypes.addressof(descs), len(descs), self.m, self._entries[0].p.device.index,
-                                         fn, ws.data_ptr(), ws.numel())
+        self._plan = self._native_step.plan_new(groups, ctypes.addressof(descs), len(descs), self.m, self._entries[0].p.device.index,
+                                                fn, ws.data_ptr(), ws.numel())
 
     # ------------------------------------------------------------------------------ logging probes
     def _probe_begin(self) -> Optional[dict]:

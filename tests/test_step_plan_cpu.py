@@ -1,4 +1,6 @@
 """The native host side of the step (csrc_host/step_plan.cpp) where no GPU is needed: what it does when torch throws."""
+import os
+import shutil
 import subprocess
 import sys
 import textwrap
@@ -13,7 +15,7 @@ _PRELUDE = textwrap.dedent(f"""
     sys.path.insert(0, {ROOT + '/ista-daslab-optimizers_b200'!r})
     import torch
     from ista_daslab_optimizers_b200 import _native as N
-    from ista_daslab_optimizers_b200 import _step_plan as plan
+    plan = N.load_step_plan()
 
     def step(p, groups):
         return plan.plan_step(p, groups, 1, 64, 0, 0.9, 0.999, 1e-8)
@@ -81,3 +83,28 @@ def test_a_plan_keeps_no_cycle_alive():
     """)
     assert out.returncode == 0, out.stderr[-2000:]
     assert out.stdout.split('\n')[:4] == [f'{w} [True, True]' for w in ('nowhere', 'group', 'parameter', 'state')]
+
+
+def test_package_without_the_built_files(tmp_path):
+    """A clean checkout: the package imports, what needs no built file works, and an optimizer says how to build."""
+    src = os.path.join(ROOT, 'ista-daslab-optimizers_b200', 'ista_daslab_optimizers_b200')
+    dst = os.path.join(tmp_path, 'ista_daslab_optimizers_b200')
+    shutil.copytree(src, dst, ignore=shutil.ignore_patterns('*.so', '__pycache__'))
+    body = """
+        import sys
+        sys.path.insert(0, {0!r})
+        import torch
+        from ista_daslab_optimizers_b200 import MicroAdam, _native, block_split, sharding, synthetic
+        assert _native.__file__.startswith({0!r})
+        assert block_split(10, 4) == (2, 8) and len(sharding.plan_shards([29056 * 4], 29056, 64, 2)) == 2
+        if {1}:
+            _native.load = lambda *a: None           # the library alone is there
+        try:
+            MicroAdam([torch.nn.Parameter(torch.zeros(4))], m=1, lr=1.0, quant_block_size=64)
+        except _native.NativeError as e:
+            print('build.py' in str(e))
+    """
+    for library_there in (False, True):
+        out = subprocess.run([sys.executable, '-c', textwrap.dedent(body.format(str(tmp_path), library_there))],
+                             capture_output=True, text=True, timeout=300)
+        assert out.stdout == 'True\n', out.stderr[-2000:]

@@ -82,7 +82,8 @@ def test_step_hooks_and_non_contiguous_gradients():
 def test_other_threads_run_while_the_library_is_called(tmp_path):
     """The call into the library may wait for the GPU (a full launch queue, a large descriptor table): Python's global lock is
     not held meanwhile.  A host function that sleeps stands in for the library."""
-    from ista_daslab_optimizers_b200 import _step_plan
+    from ista_daslab_optimizers_b200 import _native
+    _step_plan = _native.load_step_plan()
     src, lib = tmp_path / 'slow.c', tmp_path / 'slow.so'
     src.write_text('#include <unistd.h>\nint slow(void* t, int n, const void* a, void* w, long long b, void* s) { usleep(400000); return n; }\n')
     subprocess.run(['gcc', '-shared', '-fPIC', '-o', str(lib), str(src)], check=True)
