@@ -18,8 +18,18 @@ CSRC = os.path.join(HERE, 'csrc')
 OUT_DIR = os.path.join(HERE, 'ista_daslab_optimizers_b200', 'lib')
 LIB_PATH = os.path.join(OUT_DIR, 'libmicroadam_b200.so')
 HOST_SRC = os.path.join(HERE, 'csrc_host', 'step_plan.cpp')
-HOST_PATH = os.path.join(HERE, 'ista_daslab_optimizers_b200', '_step_plan.so')      # a Python module next to its users
 INCLUDE = os.path.join(os.path.dirname(HERE), 'include')
+
+
+def host_path() -> str:
+    """The extension, next to its users.  It is compiled against the layout of torch's and Python's objects, so its file
+    name carries their versions: for others it does not exist."""
+    sys.path.insert(0, HERE)
+    try:
+        from ista_daslab_optimizers_b200._native import step_plan_path
+    finally:
+        sys.path.remove(HERE)
+    return step_plan_path()
 
 
 def _nvcc() -> str:
@@ -40,9 +50,10 @@ def _inputs():
 
 
 def up_to_date() -> bool:
-    if not (os.path.exists(LIB_PATH) and os.path.exists(HOST_PATH)):
+    built = (LIB_PATH, host_path())
+    if not all(os.path.exists(p) for p in built):
         return False
-    t = min(os.path.getmtime(LIB_PATH), os.path.getmtime(HOST_PATH))
+    t = min(os.path.getmtime(p) for p in built)
     return all(os.path.getmtime(p) <= t for p in _inputs())
 
 
@@ -54,7 +65,7 @@ def host_command():
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
     return [os.environ.get('CXX', 'g++'), '-O2', '-std=c++17', '-fPIC', '-shared', '-I', INCLUDE, '-I', os.path.join(base, 'include'),
             '-I', os.path.join(base, 'include', 'torch', 'csrc', 'api', 'include'), '-I', os.path.join(cuda, 'include'),
-            '-I', sysconfig.get_paths()['include'], HOST_SRC, '-o', HOST_PATH, '-L', os.path.join(base, 'lib'),
+            '-I', sysconfig.get_paths()['include'], HOST_SRC, '-o', host_path(), '-L', os.path.join(base, 'lib'),
             '-ltorch_python', '-lc10_cuda', '-lc10', '-ltorch_cpu']
 
 

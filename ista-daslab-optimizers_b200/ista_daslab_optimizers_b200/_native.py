@@ -6,8 +6,9 @@ Torch is used only to obtain device pointers and the current CUDA stream.
 from __future__ import annotations
 
 import ctypes
-import importlib
+import importlib.util
 import os
+import sys
 from ctypes import POINTER, Structure, c_char_p, c_double, c_float, c_int, c_int32, c_int64, c_void_p
 
 import torch
@@ -109,15 +110,28 @@ def load(path: str = LIB_PATH) -> ctypes.CDLL:
 _step_plan = None
 
 
+def step_plan_path() -> str:
+    """The step's native host side, as built for this torch and this Python (it reads their objects' fields directly, so
+    a file built for others must not be loaded)."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    return os.path.join(here, f'_step_plan.{sys.implementation.cache_tag}.torch-{torch.__version__}.so')
+
+
 def load_step_plan():
     """The module of the step's native host side (csrc_host/step_plan.cpp).  Raises if it is not built."""
     global _step_plan
     if _step_plan is None:
+        path, name = step_plan_path(), __package__ + '._step_plan'
+        hint = 'build it with `python ista-daslab-optimizers_b200/build.py` (needs g++ and Python\'s headers)'
+        if not os.path.exists(path):
+            raise NativeError(f'{path} is missing: {hint}')
         try:
-            _step_plan = importlib.import_module('._step_plan', __package__)
+            spec = importlib.util.spec_from_file_location(name, path)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
         except ImportError as e:
-            raise NativeError('the native host side of the step cannot be loaded: build it with '
-                              f'`python ista-daslab-optimizers_b200/build.py` (needs g++ and Python\'s headers): {e}') from e
+            raise NativeError(f'{path} cannot be loaded ({e}): {hint}') from e
+        _step_plan = module
     return _step_plan
 
 

@@ -108,3 +108,18 @@ def test_package_without_the_built_files(tmp_path):
         out = subprocess.run([sys.executable, '-c', textwrap.dedent(body.format(str(tmp_path), library_there))],
                              capture_output=True, text=True, timeout=300)
         assert out.stdout == 'True\n', out.stderr[-2000:]
+
+
+def test_extension_of_another_torch_is_not_taken(monkeypatch):
+    """The file name carries the versions of torch and Python: for others the build is not up to date, and nothing is loaded."""
+    import build
+    from ista_daslab_optimizers_b200 import _native
+    assert build.host_path() == _native.step_plan_path() and os.path.exists(build.host_path())
+    monkeypatch.setattr(_native, '_step_plan', None)
+    monkeypatch.setattr(torch, '__version__', '0.0.1')
+    assert not build.up_to_date()
+    with pytest.raises(_native.NativeError, match='build.py'):
+        _native.load_step_plan()
+    monkeypatch.undo()
+    monkeypatch.setattr(sys.implementation, 'cache_tag', 'cpython-300')
+    assert not build.up_to_date()
