@@ -28,6 +28,7 @@ There is no CPU path: parameters must live on a CUDA device and the native libra
 from __future__ import annotations
 
 import ctypes
+import functools
 import importlib
 import math
 import time
@@ -231,16 +232,6 @@ class MicroAdam(torch.optim.Optimizer):
             raise ValueError("optimizer state 'I' holds an index outside its top-k block")
 
     # ------------------------------------------------------------------------------ step
-    def step(self, closure=None):
-        # torch wraps `step` of every optimizer class to run its step hooks under a profiler label, which costs more
-        # host time (about 18 us) than the rest of a small step; the label and the hooks are only gone through here
-        # when there is a profiler or a hook to see them.  (A subclass with a step of its own is wrapped as usual.)
-        if type(self).step is _OWN_STEP and _step_is_observed(self):
-            return _observed_step(self, closure)
-        return self._step(closure)
-
-    step.hooked = True            # tells torch.optim.Optimizer that this class runs the hooks itself
-
     def _step(self, closure=None):
         self.steps += 1                                                                                # micro_adam.py:98
         loss = None
@@ -261,6 +252,17 @@ class MicroAdam(torch.optim.Optimizer):
             self._plan = None     # something about the parameters has changed: look at them again
         self._step_entries()
         return loss
+
+    @functools.wraps(_step, assigned=('__doc__',))
+    def step(self, *args, **kwargs):
+        # torch wraps `step` of every optimizer class to run its step hooks under a profiler label, which costs more
+        # host time (about 18 us) than the rest of a small step; the label and the hooks are only gone through here
+        # when there is a profiler or a hook to see them.  (A subclass with a step of its own is wrapped as usual.)
+        if type(self).step is _OWN_STEP and _step_is_observed(self):
+            return _observed_step(self, *args, **kwargs)      # (hooks see the call as it was made)
+        return self._step(*args, **kwargs)
+
+    step.hooked = True            # tells torch.optim.Optimizer that this class runs the hooks itself
 
     @torch.no_grad()
     def _step_entries(self):
