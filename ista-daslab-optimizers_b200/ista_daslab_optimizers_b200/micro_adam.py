@@ -257,12 +257,28 @@ class MicroAdam(torch.optim.Optimizer):
     def step(self, *args, **kwargs):
         # torch wraps `step` of every optimizer class to run its step hooks under a profiler label, which costs more
         # host time (about 18 us) than the rest of a small step; the label and the hooks are only gone through here
-        # when there is a profiler or a hook to see them.  (A subclass with a step of its own is wrapped as usual.)
-        if type(self).step is _OWN_STEP and _step_is_observed(self):
+        # when there is a profiler or a hook to see them, and torch's wrapper around a subclass's step has not done so.
+        if not self._hooks_run and _step_is_observed(self):
             return _observed_step(self, *args, **kwargs)      # (hooks see the call as it was made)
         return self._step(*args, **kwargs)
 
     step.hooked = True            # tells torch.optim.Optimizer that this class runs the hooks itself
+    _hooks_run = False            # inside a call of torch's wrapper
+
+    @staticmethod
+    def profile_hook_step(func):
+        """torch.optim.Optimizer wraps by this what stands in the place of `step`: a subclass's own, or what a program
+        has put around it."""
+        observed = torch.optim.Optimizer.profile_hook_step(func)
+
+        @functools.wraps(func)
+        def wrapper(self, *args, **kwargs):
+            outer, self._hooks_run = self._hooks_run, True
+            try:
+                return observed(self, *args, **kwargs)
+            finally:
+                self._hooks_run = outer
+        return wrapper
 
     @torch.no_grad()
     def _step_entries(self):
@@ -557,5 +573,4 @@ class MicroAdam(torch.optim.Optimizer):
             probe['norm_e'] += float(grad.float().norm(p=2) ** 2)
 
 
-_OWN_STEP = MicroAdam.step        # (as defined: torch puts its wrapper in its place if it does not find `hooked`)
 _observed_step = torch.optim.Optimizer.profile_hook_step(MicroAdam._step)
