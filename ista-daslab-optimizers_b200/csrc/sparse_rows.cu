@@ -18,7 +18,8 @@ constexpr int SPR_THREADS = 384;      // three CTAs of 58 KB of accumulators per
 constexpr int SPR_AHEAD = 8;          // rows whose entries a thread has in flight
 
 constexpr int SP_THREADS = 512;
-constexpr int SP_CLUSTER = 8;         // CTAs per row (the portable cluster size)
+constexpr int SP_CLUSTER = 8;         // CTAs per row (the portable cluster size) ...
+constexpr int SP_ONE_CTA = 2048;      // ... and the longest row one CTA takes (2003 entries: 3.3 us, 3.6 by a cluster; 3005: 3.9 and 3.7)
 
 template <typename T> __device__ __forceinline__ float load_value(const void* p, int64_t i);
 template <> __device__ __forceinline__ float load_value<float>(const void* p, int64_t i) { return reinterpret_cast<const float*>(p)[i]; }
@@ -42,58 +43,88 @@ __device__ __forceinline__ void add_vector(uint16_t* o, const float* v) {
     *reinterpret_cast<uint4*>(o) = a;
 }
 
+// acc + the products of a row's entries [first, end) of one top-k block with that block of g, by one warp.
+template <typename TG, typename TV>
+__device__ __forceinline__ float dot_entries(float acc, const TG* gb, const int16_t* __restrict__ I, const void* __restrict__ V, int64_t row, int first, int end) {
+    constexpr int U = 5;                                     // entries a lane has in flight (32 rows of 1 278 028: 4 124-147 us, 5 111, 6 115, 8 123)
+    for (int j0 = first + lane_id(); j0 < end; j0 += 32 * U) {
+        int pos[U];
+        float val[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            const int j = j0 + 32 * i;
+            pos[i] = j < end ? (int)I[row + j] : 0;
+            val[i] = j < end ? load_value<TV>(V, row + j) : 0.0f;
+        }
+        float x[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) x[i] = j0 + 32 * i < end ? Elem<TG>::load(gb, pos[i]) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < U; ++i) acc = __fadd_rn(acc, __fmul_rn(val[i], x[i]));
+    }
+    return acc;
+}
+
+// The sum of `acc` over the CTAs of a cluster, to *out; lanes, warps and CTAs (through distributed shared memory) in a fixed order.
+template <int CTAS>
+__device__ __forceinline__ void dot_sum(float acc, float* s_part, float* s_cta, float* out) {
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int rank = CTAS > 1 ? (int)cluster.block_rank() : 0;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+    if (lane_id() == 0) s_part[warp_id()] = acc;
+    if constexpr (CTAS > 1) cluster.sync();                  // (every CTA of the cluster runs by now: its shared memory may be written)
+    else __syncthreads();
+    if (threadIdx.x == 0) {
+        float total = 0.0f;
+        for (int w = 0; w < SP_THREADS / 32; ++w) total = __fadd_rn(total, s_part[w]);
+        if constexpr (CTAS > 1) *cluster.map_shared_rank(&s_cta[rank], 0) = total;
+        else *out = total;
+    }
+    if constexpr (CTAS > 1) {
+        cluster.sync();
+        if (rank == 0 && threadIdx.x == 0) {
+            float total = 0.0f;
+            for (int c = 0; c < CTAS; ++c) total = __fadd_rn(total, s_cta[c]);
+            *out = total;
+        }
+    }
+}
+
 // out[r] = sum_j V[r, j] * g[(j / kbs) * dbs + I[r, j]]: a cluster of 8 CTAs per row (one CTA per row left most of the chip
-// idle: 268 -> 49 us for 32 rows of 256 091 entries).  A warp takes whole top-k blocks, so that an entry's
-// address needs no division and neighbouring lanes gather from neighbouring places; the partial sums of lanes, warps and
-// CTAs (through distributed shared memory) are added in a fixed order.
+// idle: 258 -> 38 us for 32 rows of 255 958 entries).  A warp takes whole top-k blocks, so that an entry's
+// address needs no division and neighbouring lanes gather from neighbouring places.
 template <typename TG, typename TV>
 __global__ void __cluster_dims__(SP_CLUSTER, 1, 1) __launch_bounds__(SP_THREADS)
 sparse_rows_dot_kernel(int64_t k, int64_t dbs, int kbs, int nfull, int k_few, const TG* __restrict__ g, const int16_t* __restrict__ I,
                        const void* __restrict__ V, float* __restrict__ out) {
     __shared__ float s_part[SP_THREADS / 32];
     __shared__ float s_cta[SP_CLUSTER];
-    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-    const int rank = (int)cluster.block_rank();
     const int64_t r = blockIdx.x / SP_CLUSTER;
-    const int lane = lane_id(), warp = warp_id();
     const int nblocks = nfull + (k_few > 0 ? 1 : 0);
-    constexpr int U = 4;                                     // entries a lane has in flight
     float acc = 0.0f;
-    for (int blk = rank * (SP_THREADS / 32) + warp; blk < nblocks; blk += SP_CLUSTER * (SP_THREADS / 32)) {
-        const int kcnt = blk < nfull ? kbs : k_few;
-        const int64_t row = r * k + (int64_t)blk * kbs;
-        const TG* gb = g + (int64_t)blk * dbs;
-        for (int j0 = lane; j0 < kcnt; j0 += 32 * U) {
-            int pos[U];
-            float val[U];
-#pragma unroll
-            for (int i = 0; i < U; ++i) {
-                const int j = j0 + 32 * i;
-                pos[i] = j < kcnt ? (int)I[row + j] : 0;
-                val[i] = j < kcnt ? load_value<TV>(V, row + j) : 0.0f;
-            }
-            float x[U];
-#pragma unroll
-            for (int i = 0; i < U; ++i) x[i] = j0 + 32 * i < kcnt ? Elem<TG>::load(gb, pos[i]) : 0.0f;
-#pragma unroll
-            for (int i = 0; i < U; ++i) acc = __fadd_rn(acc, __fmul_rn(val[i], x[i]));
-        }
+    for (int blk = (int)(blockIdx.x % SP_CLUSTER) * (SP_THREADS / 32) + warp_id(); blk < nblocks; blk += SP_CLUSTER * (SP_THREADS / 32))
+        acc = dot_entries<TG, TV>(acc, g + (int64_t)blk * dbs, I, V, r * k + (int64_t)blk * kbs, 0, blk < nfull ? kbs : k_few);
+    dot_sum<SP_CLUSTER>(acc, s_part, s_cta, out + r);
+}
+
+// The same where a row has fewer blocks than the cluster has warps: `parts` parts of `seg` entries of each block, a warp per
+// part (32 rows of 10 002 entries in seven blocks: 11.2 us with a warp per block, 4.1 so), and for the shortest rows one CTA
+// instead of a cluster, whose two meetings take longer than the work (370 entries: 4.3 us, 3.5 with parts, 2.2 so).
+template <typename TG, typename TV, int CTAS>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(SP_THREADS)
+sparse_rows_dot_parts_kernel(int64_t k, int64_t dbs, int kbs, int nfull, int k_few, int parts, int seg, const TG* __restrict__ g,
+                             const int16_t* __restrict__ I, const void* __restrict__ V, float* __restrict__ out) {
+    __shared__ float s_part[SP_THREADS / 32];
+    __shared__ float s_cta[CTAS];
+    const int64_t r = blockIdx.x / CTAS;
+    const int tasks = (nfull + (k_few > 0 ? 1 : 0)) * parts;
+    float acc = 0.0f;
+    for (int task = (int)(blockIdx.x % CTAS) * (SP_THREADS / 32) + warp_id(); task < tasks; task += CTAS * (SP_THREADS / 32)) {
+        const int blk = task / parts, first = (task - blk * parts) * seg;
+        acc = dot_entries<TG, TV>(acc, g + (int64_t)blk * dbs, I, V, r * k + (int64_t)blk * kbs, first, min(first + seg, blk < nfull ? kbs : k_few));
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
-    if (lane == 0) s_part[warp] = acc;
-    cluster.sync();                                          // (every CTA of the cluster runs by now: its shared memory may be written)
-    if (threadIdx.x == 0) {
-        float total = 0.0f;
-        for (int w = 0; w < SP_THREADS / 32; ++w) total = __fadd_rn(total, s_part[w]);
-        *cluster.map_shared_rank(&s_cta[rank], 0) = total;
-    }
-    cluster.sync();
-    if (rank == 0 && threadIdx.x == 0) {
-        float total = 0.0f;
-        for (int c = 0; c < SP_CLUSTER; ++c) total = __fadd_rn(total, s_cta[c]);
-        out[r] = total;
-    }
+    dot_sum<CTAS>(acc, s_part, s_cta, out + r);
 }
 
 // out[e] += sum_r M[r] * V[r, j] over the entries (r, j) that address e: one CTA per sub-range of a top-k block
@@ -178,15 +209,22 @@ extern "C" int mab_sparse_rows_dot(int64_t d, int64_t rows, int64_t k, int64_t d
     MAB_REQUIRE((g_dtype == MAB_F32 || g_dtype == MAB_BF16) && (v_dtype == MAB_F32 || v_dtype == MAB_BF16), MAB_ERR_UNSUPPORTED,
                 "sparse_rows_dot: dtypes %d, %d", g_dtype, v_dtype);
     cudaStream_t s = (cudaStream_t)stream;
-    const int grid = (int)rows * SP_CLUSTER, kbs = (int)k_block_size;
-    if (g_dtype == MAB_F32 && v_dtype == MAB_BF16)
-        sparse_rows_dot_kernel<float, uint16_t><<<grid, SP_THREADS, 0, s>>>(k, d_block_size, kbs, nfull, k_few, (const float*)g, I, V, out);
-    else if (g_dtype == MAB_F32)
-        sparse_rows_dot_kernel<float, float><<<grid, SP_THREADS, 0, s>>>(k, d_block_size, kbs, nfull, k_few, (const float*)g, I, V, out);
-    else if (v_dtype == MAB_BF16)
-        sparse_rows_dot_kernel<uint16_t, uint16_t><<<grid, SP_THREADS, 0, s>>>(k, d_block_size, kbs, nfull, k_few, (const uint16_t*)g, I, V, out);
-    else
-        sparse_rows_dot_kernel<uint16_t, float><<<grid, SP_THREADS, 0, s>>>(k, d_block_size, kbs, nfull, k_few, (const uint16_t*)g, I, V, out);
+    const int ctas = k <= SP_ONE_CTA ? 1 : SP_CLUSTER, grid = (int)rows * ctas, kbs = (int)k_block_size;
+    const int blocks = std::max(1, nfull + (k_few > 0 ? 1 : 0)), longest = nfull > 0 ? kbs : k_few;
+    const int parts = std::max(1, std::min(ctas * (SP_THREADS / 32) / blocks, (longest + 31) / 32));
+    const int seg = ((longest + parts - 1) / parts + 31) & ~31;
+#define MAB_LAUNCH_DOT(TG, TV) do { \
+        if (ctas > 1 && parts == 1) { \
+            sparse_rows_dot_kernel<TG, TV><<<grid, SP_THREADS, 0, s>>>(k, d_block_size, kbs, nfull, k_few, (const TG*)g, I, V, out); \
+        } else { \
+            auto kern = ctas == 1 ? sparse_rows_dot_parts_kernel<TG, TV, 1> : sparse_rows_dot_parts_kernel<TG, TV, SP_CLUSTER>; \
+            kern<<<grid, SP_THREADS, 0, s>>>(k, d_block_size, kbs, nfull, k_few, parts, seg, (const TG*)g, I, V, out); \
+        } } while (0)
+    if (g_dtype == MAB_F32 && v_dtype == MAB_BF16) MAB_LAUNCH_DOT(float, uint16_t);
+    else if (g_dtype == MAB_F32) MAB_LAUNCH_DOT(float, float);
+    else if (v_dtype == MAB_BF16) MAB_LAUNCH_DOT(uint16_t, uint16_t);
+    else MAB_LAUNCH_DOT(uint16_t, float);
+#undef MAB_LAUNCH_DOT
     count_launch();
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? MAB_OK : cuda_fail(e, "sparse_rows_dot_kernel launch");

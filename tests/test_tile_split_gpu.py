@@ -89,6 +89,41 @@ def test_sparse_rows_many_blocks(rows):
     assert torch.equal(out.view(torch.int32), out_g.cpu().view(torch.int32))
 
 
+def _rows(d, k_init, rows, seed):
+    """A ring buffer of `rows` rows with random positions, ascending inside every block."""
+    from oracle import microadam_oracle as O
+    geo = O.Geometry.make(d, DBS, k_init, 64)
+    gen = torch.Generator().manual_seed(seed)
+    n_full = geo.topk_full_blocks_count if geo.d_index_topk > 0 else 0
+    parts, at = [], 0
+    while at < d:
+        n = min(geo.d_block_size, d - at)
+        k = geo.k_block_size_many if len(parts) < n_full else geo.k - n_full * geo.k_block_size_many
+        parts.append(torch.rand(rows, n, generator=gen).topk(k, dim=1).indices.sort(dim=1).values)
+        at += n
+    return geo, torch.cat(parts, dim=1).to(torch.int16), torch.randn(rows, geo.k, generator=gen).bfloat16(), gen
+
+
+@pytest.mark.parametrize('g_dtype,v_dtype', [(torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize('d,k', [(40, 1), (33, 33), (DBS, 2048), (DBS, 2049), (2 * DBS + 500, 683), (3 * DBS, 31), (20 * DBS + 777, 300),
+                                 (127 * DBS, 33), (127 * DBS + 64, 33)])
+def test_sparse_rows_dot_of_few_blocks(d, k, g_dtype, v_dtype):
+    """Rows that one CTA takes, rows whose blocks are shared among a cluster's warps in parts, and where the two rules end."""
+    from ista_daslab_optimizers_b200 import _native as N
+    from oracle import microadam_oracle as O
+    rows = 5
+    geo, I, V, gen = _rows(d, (k - 0.5) / min(d, DBS), rows, d)
+    assert geo.k_block_size_many == k
+    g, V, dots = torch.randn(d, generator=gen).to(g_dtype), V.to(v_dtype), torch.zeros(rows, device='cuda')
+    args = (d, rows, geo.k, geo.d_block_size, geo.k_block_size_many)
+    N.sparse_rows_dot(*args, g.cuda(), I.cuda(), V.cuda(), dots)
+    block = torch.arange(geo.k) // geo.k_block_size_many
+    terms = V.double() * g.double()[block * geo.d_block_size + I.long()]
+    # fp32 products and sums: at most k + 1 roundings of 2^-24, each of no more than the sum of the terms' magnitudes
+    bound = (geo.k + 1) * 2.0 ** -24 * terms.abs().sum(dim=1)
+    assert ((dots.cpu().double() - terms.sum(dim=1)).abs() <= bound).all()
+
+
 @pytest.mark.parametrize('dtype,alpha', [(torch.float32, 0.5), (torch.bfloat16, 0.1), (torch.bfloat16, -2)])
 @pytest.mark.parametrize('skip,qbs,offset', [(1, 64, 0.0), (3, 128, 0.0), (4, 8, 0.0), (0, 64, 0.0), (0, 64, 0.2), (2, 32, -1.0)])
 def test_alpha_forms_on_slices_that_start_anywhere(dtype, alpha, skip, qbs, offset):
