@@ -129,10 +129,11 @@ sparse_rows_dot_parts_kernel(int64_t k, int64_t dbs, int kbs, int nfull, int k_f
 
 // out[e] += sum_r M[r] * V[r, j] over the entries (r, j) that address e: one CTA per sub-range of a top-k block
 // with a dense fp32 accumulator in shared memory; rows are added in row order (positions are unique inside a
-// row, so a row needs no atomics, but a barrier).  Bound by the chain of rows: a thread fetches its first entry of
+// row, so a row needs no atomics, but a barrier).  Bound by the chain of rows: a thread fetches its entries of
 // SPR_AHEAD rows at once, so that a row costs a shared-memory update and a barrier (25.6 M elements, 32 rows of 1 %: 232 us
-// with one load latency per row and four walks over a block's entries, 78 now).
-template <typename TO, typename TV>
+// with one load latency per row and four walks over a block's entries, 78 now).  LONG: blocks with more entries than the CTA
+// has threads.
+template <typename TO, typename TV, bool LONG>
 __global__ void __launch_bounds__(SPR_THREADS, 3)
 sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int nfull, int k_few, const float* __restrict__ M,
                            const int16_t* __restrict__ I, const void* __restrict__ V, TO* __restrict__ out, int total_units) {
@@ -149,25 +150,48 @@ sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int
         const int len = min(SPR_SR, n_blk - s0);
         const int64_t row0 = (int64_t)blk * kbs;
         for (int i = t; i < len; i += SPR_THREADS) acc[i] = 0.0f;
-        for (int r0 = 0; r0 < rows; r0 += SPR_AHEAD) {
-            int pos[SPR_AHEAD];
-            float val[SPR_AHEAD];
+        if constexpr (LONG) {
+            // several entries of a row per thread: (row, round) pairs in row order, SPR_AHEAD of them fetched at once
+            const int rounds = (kcnt + SPR_THREADS - 1) / SPR_THREADS, pairs = rows * rounds;
+            int r = 0, c = 0;                                    // the pair to fetch next ...
+            int round_now = 0;                                   // ... and the round of the pair to add next
+            for (int p0 = 0; p0 < pairs; p0 += SPR_AHEAD) {
+                int pos[SPR_AHEAD];
+                float val[SPR_AHEAD];
 #pragma unroll
-            for (int i = 0; i < SPR_AHEAD; ++i) {
-                const bool on = r0 + i < rows && t < kcnt;
-                const int64_t at = (int64_t)(r0 + i) * k + row0 + t;
-                pos[i] = on ? (int)I[at] - s0 : -1;
-                val[i] = on ? __fmul_rn(M[r0 + i], load_value<TV>(V, at)) : 0.0f;
+                for (int i = 0; i < SPR_AHEAD; ++i) {
+                    const int j = c * SPR_THREADS + t;
+                    const bool on = r < rows && j < kcnt;
+                    const int64_t at = (int64_t)r * k + row0 + j;
+                    pos[i] = on ? (int)I[at] - s0 : -1;
+                    val[i] = on ? __fmul_rn(M[r], load_value<TV>(V, at)) : 0.0f;
+                    if (++c == rounds) { c = 0; ++r; }
+                }
+#pragma unroll
+                for (int i = 0; i < SPR_AHEAD; ++i) {
+                    if (p0 + i < pairs) {                        // uniform
+                        if (round_now == 0) __syncthreads();     // the row before (or the clearing) is done
+                        if (pos[i] >= 0 && pos[i] < len) acc[pos[i]] = __fadd_rn(acc[pos[i]], val[i]);
+                        if (++round_now == rounds) round_now = 0;
+                    }
+                }
             }
+        } else {
+            for (int r0 = 0; r0 < rows; r0 += SPR_AHEAD) {
+                int pos[SPR_AHEAD];
+                float val[SPR_AHEAD];
 #pragma unroll
-            for (int i = 0; i < SPR_AHEAD; ++i) {
-                if (r0 + i < rows) {                             // uniform
-                    __syncthreads();                             // the row before (or the clearing) is done
-                    if (pos[i] >= 0 && pos[i] < len) acc[pos[i]] = __fadd_rn(acc[pos[i]], val[i]);
-                    for (int j = t + SPR_THREADS; j < kcnt; j += SPR_THREADS) {
-                        const int64_t at = (int64_t)(r0 + i) * k + row0 + j;
-                        const int p = (int)I[at] - s0;
-                        if (p >= 0 && p < len) acc[p] = __fadd_rn(acc[p], __fmul_rn(M[r0 + i], load_value<TV>(V, at)));
+                for (int i = 0; i < SPR_AHEAD; ++i) {
+                    const bool on = r0 + i < rows && t < kcnt;
+                    const int64_t at = (int64_t)(r0 + i) * k + row0 + t;
+                    pos[i] = on ? (int)I[at] - s0 : -1;
+                    val[i] = on ? __fmul_rn(M[r0 + i], load_value<TV>(V, at)) : 0.0f;
+                }
+#pragma unroll
+                for (int i = 0; i < SPR_AHEAD; ++i) {
+                    if (r0 + i < rows) {                             // uniform
+                        __syncthreads();                             // the row before (or the clearing) is done
+                        if (pos[i] >= 0 && pos[i] < len) acc[pos[i]] = __fadd_rn(acc[pos[i]], val[i]);
                     }
                 }
             }
@@ -249,9 +273,10 @@ extern "C" int mab_sparse_rows_combine(int64_t d, int64_t rows, int64_t k, int64
     const int smem = SPR_SR * (int)sizeof(float);
     cudaStream_t s = (cudaStream_t)stream;
 #define MAB_LAUNCH_COMBINE(TO, TV) do { \
-        MAB_CUDA_TRY(cudaFuncSetAttribute(sparse_rows_combine_kernel<TO, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
-        sparse_rows_combine_kernel<TO, TV><<<grid, SPR_THREADS, smem, s>>>(d, (int)rows, k, dbs, (int)k_block_size, nfull, k_few, \
-                                                                           M, I, V, (TO*)out, (int)units); } while (0)
+        auto kern = std::max<int64_t>(nfull > 0 ? k_block_size : 0, k_few) > SPR_THREADS ? sparse_rows_combine_kernel<TO, TV, true> \
+                                                                                       : sparse_rows_combine_kernel<TO, TV, false>; \
+        MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
+        kern<<<grid, SPR_THREADS, smem, s>>>(d, (int)rows, k, dbs, (int)k_block_size, nfull, k_few, M, I, V, (TO*)out, (int)units); } while (0)
     if (out_dtype == MAB_F32 && v_dtype == MAB_BF16) MAB_LAUNCH_COMBINE(float, uint16_t);
     else if (out_dtype == MAB_F32) MAB_LAUNCH_COMBINE(float, float);
     else if (v_dtype == MAB_BF16) MAB_LAUNCH_COMBINE(uint16_t, uint16_t);

@@ -124,6 +124,22 @@ def test_sparse_rows_dot_of_few_blocks(d, k, g_dtype, v_dtype):
     assert ((dots.cpu().double() - terms.sum(dim=1)).abs() <= bound).all()
 
 
+@pytest.mark.parametrize('out_dtype', [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize('rows', [1, 3, 8])
+@pytest.mark.parametrize('k', [383, 384, 385, 768, 769, 3000, DBS])
+def test_sparse_rows_combine_of_long_rows(k, rows, out_dtype):
+    """Blocks with more entries than a CTA has threads (several per thread and row), and a short last block beside them."""
+    from ista_daslab_optimizers_b200 import _native as N
+    from oracle import microadam_oracle as O
+    d = DBS + 4001
+    geo, I, V, gen = _rows(d, (k - 0.5) / DBS, rows, k)
+    M, out = torch.randn(rows, generator=gen), torch.randn(d, generator=gen).to(out_dtype)
+    out_g, args = out.cuda(), (d, rows, geo.k, geo.d_block_size, geo.k_block_size_many)
+    O.sparse_rows_combine(*args, M, I, V, out)
+    N.sparse_rows_combine(*args, M.cuda(), I.cuda(), V.cuda(), out_g)
+    assert torch.equal(out.view(torch.uint8), out_g.cpu().view(torch.uint8))
+
+
 @pytest.mark.parametrize('dtype,alpha', [(torch.float32, 0.5), (torch.bfloat16, 0.1), (torch.bfloat16, -2)])
 @pytest.mark.parametrize('skip,qbs,offset', [(1, 64, 0.0), (3, 128, 0.0), (4, 8, 0.0), (0, 64, 0.0), (0, 64, 0.2), (2, 32, -1.0)])
 def test_alpha_forms_on_slices_that_start_anywhere(dtype, alpha, skip, qbs, offset):
