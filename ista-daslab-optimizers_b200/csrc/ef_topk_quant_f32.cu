@@ -713,7 +713,13 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
             if (cnt <= 0) return;
             if (T.quant_err != nullptr) {                            // alpha == -2: the residual a also goes to the caller's buffer
                 float* qe = reinterpret_cast<float*>(T.quant_err) + base + o * 8;
-                for (int e = 0; e < min(cnt, 8); ++e) qe[e ^ (hh << 2)] = v[e];
+                if (cnt >= 8 && aligned16(qe)) {
+                    reinterpret_cast<float4*>(qe)[hh] = make_float4(v[0], v[1], v[2], v[3]);
+                    reinterpret_cast<float4*>(qe)[hh ^ 1] = make_float4(v[4], v[5], v[6], v[7]);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) if (e < cnt) qe[e ^ (hh << 2)] = v[e];
+                }
             }
             const uint16_t mn_b = (uint16_t)((st & 0xFFFFu) ^ 0x8000u), mx_b = (uint16_t)(st >> 16);
             if ((o & (lanes_per_qb - 1)) == 0) { mn_g[o >> oshift] = mn_b; mx_g[o >> oshift] = mx_b; }
