@@ -165,3 +165,37 @@ def test_alpha_forms_on_slices_that_start_anywhere(dtype, alpha, skip, qbs, offs
                 assert torch.equal(a[key][:cut].cpu().view(torch.uint8), b[key][:cut].view(torch.uint8)), (n, step, key)
             rtol, atol = cases.param_tolerances(dtype, hyper['lr'])
             torch.testing.assert_close(p.detach().cpu().float(), cpu[i].float(), rtol=rtol, atol=atol)
+
+
+@pytest.mark.parametrize('dtype,alpha', [(torch.float32, 0.5), (torch.bfloat16, 0.25), (torch.bfloat16, -2), (torch.float32, -2)])
+@pytest.mark.parametrize('k,dense', [(3800, True), (3900, False)])
+def test_alpha_forms_with_and_without_room_for_dense_arrays(k, dense, dtype, alpha):
+    """The alpha forms scatter updates into dense arrays of the warps where the window's arrays leave room for them in shared
+    memory, and look them up through the bitmap where they do not: both sides of that line, with a full window of 4 rows."""
+    from ista_daslab_optimizers_b200 import MicroAdam, _native
+    from oracle.microadam_oracle import MicroAdamOracle
+    rows = 4
+    stride = (2 * k + 30 + 15) & ~15                     # window_adam.cu, wt_smem_bytes
+    window = 8 * rows * k + rows * 2 * stride + 6 * 1024 + 2 * rows * k
+    room = 4 * _native.get_max_floats_for_shared_memory_per_thread_block() - 4096
+    assert window <= room and (window + 15 + 8192 <= room) == dense
+    hyper = dict(m=rows, lr=1e-3, quant_block_size=64, k_init=(k - 0.5) / DBS, weight_decay=0.1, alpha=alpha)
+    sizes = (DBS, DBS + 1003)
+    params = [torch.nn.Parameter(S.normal_tensor(90, i, n, 0.02).to(dtype).cuda()) for i, n in enumerate(sizes)]
+    cpu = [p.detach().cpu().clone() for p in params]
+    opt = MicroAdam(params, **hyper)
+    ref = MicroAdamOracle(cpu, d_block_size=opt.d_block_size, **hyper)
+    for step in range(rows + 2):
+        grads = [S.normal_tensor(91 + step, n, n, 1e-3).to(dtype) for n in sizes]
+        for p, g in zip(params, grads):
+            p.grad = g.cuda()
+        opt.step()
+        ref.step([g.clone() for g in grads])
+        for i, (p, n) in enumerate(zip(params, sizes)):
+            a, b, used = opt.state[p], ref.state[i], -(-n // 64)
+            assert a['k_block_size_many'] == k
+            for key, cut in (('error', None), ('min_vals', used), ('max_vals', used)):
+                assert torch.equal(a[key][:cut].cpu().view(torch.uint8), b[key][:cut].view(torch.uint8)), (n, step, key)
+            rtol, atol = cases.param_tolerances(dtype, hyper['lr'])
+            torch.testing.assert_close(p.detach().cpu().float(), cpu[i].float(), rtol=rtol, atol=atol)
+    assert all(e.fused for e in opt._entries) and _native.device_error() == 0
