@@ -36,7 +36,8 @@ constexpr int S_SLOTS = SEL_MAX_TILE / 8 / S_NT;   // octets per thread: 16
 constexpr int S_WPT = SEL_WORDS / S_NT;      // bitmap words per thread: 4
 constexpr int S_CAND_CAP = 2144;             // what three CTAs per SM leave room for ...
 constexpr int S_MAX_K = 1536;                // ... and the largest k it is tried for: c of 3632 octets at the bound hold about
-                                             //     -3632 ln(1 - c / 3632) candidates, 2003 at c = 1536
+                                             //     -3632 ln(1 - c / 3632) candidates, 1997 at c = 1536, 2196 at the most that
+                                             //     is accepted there (1536 + 112); a tile with more than the list holds is bisected
 constexpr int S_WLIST = 384;                 // octets with a candidate, per warp
 constexpr int S_QTAB = 512;                  // quantisation blocks whose constants fit the tables
 constexpr int S_MAX_TENSORS = WIN_MAX_TENSORS;   // one limit for every kernel of a fused launch
@@ -597,7 +598,7 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
         // ---- a = bf16(g + Qinv(e)) in place; per-octet maxima stay in registers ------------------------
         float omax[S_SLOTS];
         // regular tile: blocks of 64, aligned codes, every block with the fast decode.  (While short tiles took the general
-        // route, a step of 120 ragged tensors, 10.2 M elements, spent 78 us in this kernel: 121 us in all, 69 now.)
+        // route, a step of 120 ragged tensors, 10.2 M elements, spent 78 us in this kernel: 121 us in all, 70 now.)
         const bool swz = !LOOSE && tables && ef_al4 && ss.ctrl[slow_slot] == 0;
         if (swz && (n & 7) == 0 && n_oct >= S_FULL * S_NT) dequant_phase_regular<true>(tile4, ss, n, n_oct, cw, omax);
         else if (swz) dequant_phase_regular<false>(tile4, ss, n, n_oct, cw, omax);

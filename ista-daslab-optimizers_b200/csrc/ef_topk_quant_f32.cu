@@ -11,14 +11,14 @@
 // memory is two 16-byte pieces 32 bytes apart from the next lane's: lanes 4-7 of every 8 take the second piece first
 // (`h`), so that a quarter warp's 16-byte accesses cover all banks; the code word is rotated by 16 bits to match.
 //
-// Regular tiles (whole blocks of 64, seven whole octets per thread, aligned buffers, every block with a finite positive
-// step: all but a tensor's last tile) take a leaner route: the decode has no branches and writes a with the sixteen
-// 16-byte pieces of every 256-byte row (= one quantisation block) permuted by the row number (piece c of row r sits at
-// c ^ (r & 7)), so that after the selection a thread owns whole rows, consecutive lanes reading different banks, and
-// computes a block's statistics, constants and 32 code bytes without shuffles.
+// Regular tiles (whole blocks of 64, seven whole octets per thread, codes on a 16-byte boundary, every block with a finite
+// step; the gradient may start anywhere: all but a tensor's last tile) take a leaner route: the decode has no branches and
+// writes a with the sixteen 16-byte pieces of every 256-byte row (= one quantisation block) permuted by the row number
+// (piece c of row r sits at c ^ (r & 7)), so that after the selection a thread owns whole rows, consecutive lanes reading
+// different banks, and computes a block's statistics, constants and 32 code bytes without shuffles.
 //
-// Bound by instruction issue and the phases' barriers, not by memory: a step of one 124.4 M tensor takes 606 us with one
-// tile per SM, 571 with two, 499 with the regular route; 67.1 M with k = 5 % 602, 586 and 556.
+// Bound by instruction issue and the phases' barriers, not by memory: 33.6 M elements take 122 us with one tile per SM, 111
+// with two on the general route (other block sizes), 92 on the regular one; with k = 5 % 141, 133 and 113.
 #include "common.cuh"
 #include "select.cuh"
 #include "codec_fast.cuh"
@@ -122,7 +122,7 @@ __device__ __forceinline__ void add_octet(float (&v)[8], const float (&x)[8]) {
         v[b] = s.x; v[b + 1] = s.y;
     }
 }
-// v <- v + Qinv(codes) with the constants (min, u) of a block whose step is finite and positive; returns the largest |v|.
+// v <- v + Qinv(codes) with the constants (min, u) of a block whose step is finite and not negative; returns the largest |v|.
 __device__ __forceinline__ float accumulate_regular(float (&v)[8], uint32_t codes, float2 mu) {
     const QParams q = {mu.x, mu.y};
     float x[8];
@@ -507,7 +507,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
                         }
                     }
                 }
-                // ... and the octets in shared memory through a list per warp, two of them per lane and round
+                // ... and the octets in shared memory through a list per warp, one of them per lane and round
                 uint16_t* wlist = ss.oct_list + warp * F_WLIST;
                 int n_w = 0;
 #pragma unroll
@@ -840,7 +840,8 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
 
 // Returns 1 (without launching) when two CTAs of its shared memory do not fit an SM (tiles above 29 900 elements or so), or
 // when the selection's candidates would not fit their list: with c of 3632 octets at the bound (k <= c <= k + 192) a tile of
-// independent values holds about -3632 ln(1 - c / 3632) candidates, 3069 at c = 1880 + 192.  The one-tile kernel, whose
+// independent values holds about -3632 ln(1 - c / 3632) candidates, 2648 at c = 1880 and 3069 at c = 1880 + 192 (means: a
+// tile that comes out above the list's 3072 goes to the bisection).  The one-tile kernel, whose
 // list is longer, is the faster one from there on (k = 2325: 1165 us a step of 67 M elements, most of it in kernel B).
 int launch_ef_topk_quant_f32(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, int max_k, cudaStream_t s) {
     int qshift = 0;
