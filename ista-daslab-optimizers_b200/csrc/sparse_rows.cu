@@ -234,7 +234,7 @@ extern "C" int mab_sparse_rows_dot(int64_t d, int64_t rows, int64_t k, int64_t d
                 "sparse_rows_dot: dtypes %d, %d", g_dtype, v_dtype);
     cudaStream_t s = (cudaStream_t)stream;
     const int ctas = k <= SP_ONE_CTA ? 1 : SP_CLUSTER, grid = (int)rows * ctas, kbs = (int)k_block_size;
-    const int blocks = std::max(1, nfull + (k_few > 0 ? 1 : 0)), longest = nfull > 0 ? kbs : k_few;
+    const int blocks = std::max(1, nfull + (k_few > 0 ? 1 : 0)), longest = std::max(nfull > 0 ? kbs : 0, k_few);
     const int parts = std::max(1, std::min(ctas * (SP_THREADS / 32) / blocks, (longest + 31) / 32));
     const int seg = ((longest + parts - 1) / parts + 31) & ~31;
 #define MAB_LAUNCH_DOT(TG, TV) do { \

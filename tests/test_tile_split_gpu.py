@@ -124,6 +124,26 @@ def test_sparse_rows_dot_of_few_blocks(d, k, g_dtype, v_dtype):
     assert ((dots.cpu().double() - terms.sum(dim=1)).abs() <= bound).all()
 
 
+def test_sparse_rows_of_a_last_block_with_the_most_entries():
+    """The last, short block may have more entries than the others."""
+    from ista_daslab_optimizers_b200 import _native as N
+    d, rows, k_many, k_few = DBS + 5000, 3, 40, 4100
+    gen = torch.Generator().manual_seed(7)
+    I = torch.cat([torch.rand(rows, n, generator=gen).topk(k, dim=1).indices.sort(dim=1).values for n, k in ((DBS, k_many), (5000, k_few))], dim=1)
+    V, g, M = torch.randn(rows, k_many + k_few, generator=gen).bfloat16(), torch.randn(d, generator=gen), torch.randn(rows, generator=gen)
+    at = I + torch.tensor([0] * k_many + [DBS] * k_few)
+    dots, out = torch.zeros(rows, device='cuda'), torch.zeros(d, device='cuda')
+    args = (d, rows, k_many + k_few, DBS, k_many)
+    N.sparse_rows_dot(*args, g.cuda(), I.to(torch.int16).cuda(), V.cuda(), dots)
+    N.sparse_rows_combine(*args, M.cuda(), I.to(torch.int16).cuda(), V.cuda(), out)
+    terms = V.double() * g.double()[at]
+    assert ((dots.cpu().double() - terms.sum(dim=1)).abs() <= (k_many + k_few + 1) * 2.0 ** -24 * terms.abs().sum(dim=1)).all()
+    want = torch.zeros(d, dtype=torch.float64)
+    for r in range(rows):
+        want[at[r]] += M[r].double() * V[r].double()
+    torch.testing.assert_close(out.cpu().double(), want, rtol=1e-5, atol=1e-5)     # three fp32 products and sums of unit size
+
+
 @pytest.mark.parametrize('out_dtype', [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize('rows', [1, 3, 8])
 @pytest.mark.parametrize('k', [383, 384, 385, 768, 769, 3000, DBS])
