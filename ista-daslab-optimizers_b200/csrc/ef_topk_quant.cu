@@ -462,10 +462,20 @@ ef_topk_quant_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int 
 
 int units_a_of(const mab_tensor& t) { return t.topk_full_blocks_count + (t.k_block_size_few > 0 ? 1 : 0); }
 
+// Blocks of 64 have two kernels.  The one whose warps own their part of the tile is the faster one in a long run, but finds the
+// first tile's bound more slowly and has no advantage with many candidates or a gradient that has to be staged (us a launch, it
+// and the other one): 134 M elements, 31 tiles per SM, 182 and 200; with k = 0.5 % 170 and 214, 2 % 199 and 220, 5 % 283 and 276;
+// off alignment 244 and 234; 67 M, 16 tiles per SM, 105 and 107; 54.5 M 102 and 98; 2.1 M 16.2 and 12.4.
+constexpr int WARPS_MIN_TILES_PER_SM = 20;
+constexpr int WARPS_MAX_K = 640;             // 2.2 % of a tile
+
 int launch_ef_topk_quant(const mab_tensor* dev_tensors, int n_tensors, int total_units, int grad_dtype,
-                         int qbs, int max_dbs, int max_k, cudaStream_t s, const LooseArgs* loose) {
+                         int qbs, int max_dbs, int max_k, bool wide, cudaStream_t s, const LooseArgs* loose) {
     if (grad_dtype == MAB_BF16) {          // bf16 tiles are small enough for two shared-memory resident CTAs per SM
-        const int rc = launch_ef_topk_quant_bf16(dev_tensors, n_tensors, total_units, qbs, max_dbs, s, loose);
+        const bool warps = loose != nullptr || qbs != 64 ||
+                           (wide && total_units >= WARPS_MIN_TILES_PER_SM * device_sm_count() && max_k <= WARPS_MAX_K);
+        const int rc = warps ? launch_ef_topk_quant_bf16_warps(dev_tensors, n_tensors, total_units, qbs, max_dbs, s, loose)
+                             : launch_ef_topk_quant_bf16(dev_tensors, n_tensors, total_units, max_dbs, s);
         if (rc <= 0) return rc;
     }
     if (grad_dtype == MAB_F32 && loose == nullptr) {   // two CTAs per SM while tile and candidates fit

@@ -1,4 +1,5 @@
-// Kernel A for bf16 gradients: the tile lives in shared memory, three CTAs per SM.
+// Kernel A for bf16 gradients, blocks of 64: the tile lives in shared memory, three CTAs per SM.  (Other block sizes and large
+// launches: ef_topk_quant_bf16_warps.cu; the rule stands in launch_ef_topk_quant.)
 //
 // A bf16 tile (29 056 values) is 58 KB.  Only the tile and 16 KB of selection scratch sit in shared
 // memory (codes and statistics are read from and written to global memory directly, coalesced), so
@@ -10,15 +11,14 @@
 // t, t + 256, ...: consecutive lanes touch consecutive 16-byte pieces of the tile and consecutive
 // code words in global memory) and fetch the constants of an octet's quantisation block from a
 // small table in shared memory.  Statistics walk it block by block (thread t owns quantisation
-// blocks t, t + 256; no shuffles).  For quant_block_size 64 the block tables fit the scratch; other
-// block sizes take general per-block code in the same kernel.
+// blocks t, t + 256; no shuffles).
 //
-// Regular tiles (blocks of 64, aligned codes, all blocks with a finite step) take a leaner route: the decode writes a into the tile with the octets of every
+// Regular tiles (aligned codes, all blocks with a finite step) take a leaner route: the decode writes a into the tile with the octets of every
 // 128-byte row (= one quantisation block) permuted by the row number (octet o sits at o ^ ((o >> 3) & 7)),
 // so that afterwards a thread can own whole blocks - consecutive lanes own consecutive blocks and read
 // different banks - and computes a block's statistics, its constants and its 32 code bytes from
 // registers, with no tables and no shuffles.  The selection addresses the tile through the same
-// permutation.  Everything else (other block sizes, unaligned codes, degenerate blocks) keeps the
+// permutation.  Everything else (unaligned codes, degenerate blocks) keeps the
 // linear layout and the general code.
 //
 // Results are bit-identical to those of the fp32 kernels' arithmetic (ef_topk_quant_f32.cu, ef_topk_quant.cu; same tie rule).
@@ -253,35 +253,17 @@ __device__ __forceinline__ float dequant_octet(uint4* tile4, const uint4& g8, in
 }
 
 // a = bf16(g + Qinv(e)) in place for the thread's octets t, t + S_NT, ...; per-octet maxima to omax.
-// The first FS octets of every thread are promised to exist, to be whole and to find their block in
-// the table, so their code is one branch-free block whose octets the compiler can interleave.
-// loose_qbs != 0: quantisation blocks of that many elements that ignore the tile's borders; the tile starts
-// lrem0 elements into the block mn_g / mx_g point at.
-template <int FS>
-__device__ __forceinline__ void dequant_phase(uint4* tile4, const SmemSel& ss, bool tables, const uint16_t* mn_g, const uint16_t* mx_g,
-                                              int cshift, int n, int n_oct, const uint32_t (&cw)[S_SLOTS], float (&omax)[S_SLOTS],
-                                              int loose_qbs = 0, int lrem0 = 0) {
+__device__ __forceinline__ void dequant_phase(uint4* tile4, const SmemSel& ss, const uint16_t* mn_g, const uint16_t* mx_g, int n, int n_oct,
+                                              const uint32_t (&cw)[S_SLOTS], float (&omax)[S_SLOTS]) {
     const int t = threadIdx.x;
-    const bool big = loose_qbs >= SEL_MAX_TILE;
-    auto block_of = [&](int o) { return loose_qbs ? loose_block(lrem0 + o * 8, loose_qbs, big) : (o >> cshift); };
     uint32_t slow = 0u;                                      // octets whose block needs the defining decode
 #pragma unroll
     for (int j = 0; j < S_SLOTS; ++j) {
         omax[j] = 0.0f;
         const int o = t + j * S_NT;
-        if (j < FS) {
-            if (j % S_GROUP == 0) asm volatile("" ::: "memory");   // octets are interleaved within a group only (register pressure)
-            const float2 c = ss.qt.mu[block_of(o)];
+        if (o < n_oct) {
+            const float2 c = ss.qt.mu[o >> 3];
             const QParams q = {c.x, c.y};
-            const DecodeConsts dc = decode_consts(q);
-            const float m = dequant_octet<true, false>(tile4, tile4[o], o, o, n, cw[j], q, dc, dc.fast);
-            omax[j] = dc.fast ? m : 0.0f;
-            slow |= dc.fast ? 0u : (1u << j);
-        } else if (o < n_oct) {
-            QParams q;
-            const int b = block_of(o);
-            if (tables) { const float2 c = ss.qt.mu[b]; q.mn = c.x; q.u = c.y; }
-            else q = qparams(mn_g[b], mx_g[b]);
             const DecodeConsts dc = decode_consts(q);
             if (!dc.fast) slow |= 1u << j;
             else omax[j] = dequant_octet<true, true>(tile4, tile4[o], o, o, n, cw[j], q, dc, true);
@@ -292,8 +274,7 @@ __device__ __forceinline__ void dequant_phase(uint4* tile4, const SmemSel& ss, b
         for (int j = 0; j < S_SLOTS; ++j) {
             if ((slow >> j) & 1u) {
                 const int o = t + j * S_NT;
-                const int b = block_of(o);
-                const QParams q = qparams(mn_g[b], mx_g[b]);
+                const QParams q = qparams(mn_g[o >> 3], mx_g[o >> 3]);
                 omax[j] = dequant_octet<false, true>(tile4, tile4[o], o, o, n, cw[j], q, decode_consts(q), true);
             }
         }
@@ -458,15 +439,9 @@ __device__ __forceinline__ void encode_phase(const uint4* tile4, const SmemSel& 
     }
 }
 
-// QB64: quant_block_size is 64: the per-block constants fit the shared-memory tables and the loops
-// over a block's 8 octets unroll.
-// LOOSE: quantisation blocks of la.qbs elements that ignore the borders of the top-k blocks; the kernel then ends
-// a tile with the residual written back to the gradient buffer and the extremes of every block it touches merged
-// into la.st_min / la.st_max (requant_loose.cu finishes the job), instead of statistics and codes.
-template <bool QB64, bool LOOSE>
 __global__ void __launch_bounds__(S_NT, S_CTAS)
-ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int qshift, int stage_elems,
-                          LooseArgs la) {
+ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int stage_elems) {
+    constexpr int qshift = 6;                    // quantisation blocks of 64
     extern __shared__ __align__(128) unsigned char smem_raw[];       // [tile][SmemSel]
     __shared__ int s_first[S_MAX_TENSORS + 1];
     __shared__ __align__(8) uint64_t s_bar;
@@ -477,8 +452,8 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
     for (int i = t; i < n_tensors; i += S_NT) s_first[i] = tensors[i].first_unit_a;
     if (t == 0) { s_first[n_tensors] = total_units; mbar_init(&s_bar, 1); ss.ctrl[5] = 0; ss.ctrl[6] = 0; }
     __syncthreads();
-    const int cshift = qshift - 3;              // octets per quantisation block, as a shift
-    const int cpq = 1 << cshift;
+    constexpr int cshift = qshift - 3;          // octets per quantisation block, as a shift
+    constexpr int cpq = 1 << cshift;
     uint32_t parity = 0;
     int guess = 0;
     int tile_no = 0;                            // tiles this CTA has worked on: selects one of two "a block needs the slow decode" flags
@@ -488,7 +463,7 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
 
     for (int unit = blockIdx.x; unit < total_units; unit += gridDim.x) {
         bool issued = false;
-        if (t == 0 && g_next != nullptr && (LOOSE ? (n_next & 7) == 0 : n_next >= 8) && aligned16(g_next)) {   // same test as `staged` below
+        if (t == 0 && g_next != nullptr && n_next >= 8 && aligned16(g_next)) {   // same test as `staged` below
             fence_async_smem();
             mbar_arrive_expect_tx(&s_bar, (uint32_t)(n_next & ~7) * 2u);
             bulk_g2s(smem_raw, g_next, (uint32_t)(n_next & ~7) * 2u, &s_bar);
@@ -504,14 +479,11 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
         const uint16_t* g = reinterpret_cast<const uint16_t*>(T.grad) + base;
         const uint8_t* ef_in = T.error + (base >> 1);
         uint8_t* ef_out = T.error + (base >> 1);
-        const int64_t qb0 = LOOSE ? base / la.qbs : base >> qshift;
-        const int lrem0 = LOOSE ? (int)(base - qb0 * la.qbs) : 0;   // loose: where the tile starts inside its first block
-        // quantisation blocks of the tile; loose ones are at least 72 elements long, so the tables hold those a tile touches
+        const int64_t qb0 = base >> qshift;
         const int n_oct = (n + 7) >> 3;
-        const int n_qb = LOOSE ? loose_block(lrem0 + n - 1, la.qbs, false) + 1 : (n + (1 << qshift) - 1) >> qshift;
-        const bool staged = (LOOSE ? (n & 7) == 0 : n >= 8) && aligned16(g);   // the bulk copy moves whole 16-byte pieces
+        const int n_qb = (n + (1 << qshift) - 1) >> qshift;
+        const bool staged = n >= 8 && aligned16(g);   // the bulk copy moves whole 16-byte pieces
         const bool ef_al4 = (reinterpret_cast<uintptr_t>(ef_in) & 3) == 0;
-        const bool tables = (QB64 || LOOSE) && n_qb <= S_QTAB;
         const uint16_t* mn_g = T.min_vals + qb0;
         const uint16_t* mx_g = T.max_vals + qb0;
         const int64_t row_off = (int64_t)T.ring_index * row_pitch_of(T) + (int64_t)blk * T.k_block_size_many;
@@ -532,13 +504,12 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
                 mbar_arrive_expect_tx(&s_bar, (uint32_t)(n & ~7) * 2u);
                 bulk_g2s(tile, g, (uint32_t)(n & ~7) * 2u, &s_bar);
             }
-            if (!LOOSE && (n & 7) != 0 && t < 8) {           // the last, short octet, zero padded
+            if ((n & 7) != 0 && t < 8) {           // the last, short octet, zero padded
                 const int i = (n & ~7) + t;
                 tile[i] = i < n ? g[i] : (uint16_t)0;
             }
         } else {
-            if constexpr (LOOSE) for (int i = t; i < n_oct * 8; i += S_NT) tile[i] = (i < n) ? g[i] : (uint16_t)0;
-            else load_tile_anywhere(tile, g, n, n_oct);
+            load_tile_anywhere(tile, g, n, n_oct);
         }
         uint32_t cw[S_SLOTS];
         if (ef_al4 && (n & 7) == 0 && n_oct >= S_FULL * S_NT) {  // a full tile: the first S_FULL words of every thread exist and are whole
@@ -554,7 +525,7 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
                 cw[j] = (o < n_oct) ? load_code_word(ef_in, ef_al4, o, n) : 0u;
             }
         }
-        if (tables) {                                        // S_QTAB = 2 * S_NT: a thread's two blocks, their loads issued together
+        {                                                    // S_QTAB = 2 * S_NT: a thread's two blocks, their loads issued together
             const int b0 = t, b1 = t + S_NT;
             const uint16_t mn0 = b0 < n_qb ? mn_g[b0] : (uint16_t)0, mx0 = b0 < n_qb ? mx_g[b0] : (uint16_t)0;
             const uint16_t mn1 = b1 < n_qb ? mn_g[b1] : (uint16_t)0, mx1 = b1 < n_qb ? mx_g[b1] : (uint16_t)0;
@@ -585,7 +556,7 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
             n_next = (int)nn;
             // gradients: 128-byte lines over all threads; codes and statistics: a warp each (they are 4 and 64 times smaller)
             prefetch_l2<S_NT>(reinterpret_cast<uintptr_t>(reinterpret_cast<const uint16_t*>(N.grad) + nbase), nn * 2);
-            if (warp < (LOOSE ? 1 : 3)) {
+            if (warp < 3) {
                 const uintptr_t pb = warp == 0 ? reinterpret_cast<uintptr_t>(N.error + (nbase >> 1))
                                    : reinterpret_cast<uintptr_t>((warp == 1 ? N.min_vals : N.max_vals) + (nbase >> qshift));
                 const int64_t bytes = warp == 0 ? (nn + 1) >> 1 : ((nn >> qshift) + 1) * 2;
@@ -599,12 +570,10 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
         float omax[S_SLOTS];
         // regular tile: blocks of 64, aligned codes, every block with the fast decode.  (While short tiles took the general
         // route, a step of 120 ragged tensors, 10.2 M elements, spent 78 us in this kernel: 121 us in all, 70 now.)
-        const bool swz = !LOOSE && tables && ef_al4 && ss.ctrl[slow_slot] == 0;
+        const bool swz = ef_al4 && ss.ctrl[slow_slot] == 0;
         if (swz && (n & 7) == 0 && n_oct >= S_FULL * S_NT) dequant_phase_regular<true>(tile4, ss, n, n_oct, cw, omax);
         else if (swz) dequant_phase_regular<false>(tile4, ss, n, n_oct, cw, omax);
-        else if (LOOSE && tables && (n & 7) == 0 && n_oct >= S_FULL * S_NT && ef_al4)   // a full tile: branch-free first octets
-            dequant_phase<S_FULL>(tile4, ss, tables, mn_g, mx_g, cshift, n, n_oct, cw, omax, la.qbs, lrem0);
-        else dequant_phase<0>(tile4, ss, tables, mn_g, mx_g, cshift, n, n_oct, cw, omax, LOOSE ? la.qbs : 0, lrem0);
+        else dequant_phase(tile4, ss, mn_g, mx_g, n, n_oct, cw, omax);
 
         MAB_CTICK(1);
         // ---- exact top-k ---------------------------------------------------------------------------
@@ -641,9 +610,8 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
             int lo = 0, hi = kmax + 1, step = 1 << 20;
             int gq = (guess > 0 && guess <= kmax) ? guess : max(1, kmax - (2 << 23));
             bool have_lo = false, have_hi = false, search = true;
-            // no bound from a tile before: the histogram of the maxima gives one (with it, and with the loads above, the loose form
-            // spills more and a step of 218 M elements takes 972 us instead of 947)
-            const bool cold = !LOOSE && (guess <= 0 || guess > kmax);
+            // no bound from a tile before: the histogram of the maxima gives one
+            const bool cold = guess <= 0 || guess > kmax;
             if (cold) {
                 const int c = bound_from_histogram(omax, kmax, k, ss.hist, lo, hi);
                 have_lo = c > 0; have_hi = true;
@@ -889,79 +857,11 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
         // ---- statistics and codes of the residual ----------------------------------------------------------
         uint16_t* mn_out = T.min_vals + qb0;
         uint16_t* mx_out = T.max_vals + qb0;
-        if (LOOSE) {
-            // the residual goes back to the gradient buffer, the extremes of every quantisation block the tile
-            // touches to the scratch arrays
-            uint16_t* g_w = const_cast<uint16_t*>(g);
-            uint32_t* s_qlo = ss.cand;                       // the candidate list is free again
-            uint32_t* s_qhi = ss.cand + LOOSE_MAX_QB;
-            static_assert(2 * LOOSE_MAX_QB <= S_CAND_CAP, "block extremes reuse the candidate list");
-            for (int i = t; i < LOOSE_MAX_QB; i += S_NT) { s_qlo[i] = 0xFFFFFFFFu; s_qhi[i] = 0u; }
-            __syncthreads();
-            if (!staged)
-                for (int i = t; i < n; i += S_NT) g_w[i] = tile[i];
-            MAB_CTICK(6);
-            const bool big = la.qbs >= SEL_MAX_TILE;
-            const int n_whole = n >> 3;                      // octets without padding
-            // a thread's octets are S_NT apart: it keeps the extremes of the block it is in and hands them over
-            // when the block changes (for blocks longer than a tile: at most once)
-            int cur = -1;
-            uint32_t alo = 0x7F807F80u, ahi = 0xFF80FF80u;   // packed bf16 pairs: running minimum from +inf, maximum from -inf
-#pragma unroll
-            for (int j = 0; j < S_SLOTS; ++j) {
-                const int o = t + j * S_NT;
-                if (o < n_whole) {
-                    const uint4 v = tile4[o];
-                    if (staged) reinterpret_cast<uint4*>(g_w)[o] = v;   // whole octets, 16-byte aligned: the residual goes home
-                    const int qi = loose_block(lrem0 + o * 8, la.qbs, big);
-                    if (qi != cur) {
-                        if (cur >= 0) {
-                            alo = min_bf16x2(alo, alo >> 16 | alo << 16); ahi = max_bf16x2(ahi, ahi >> 16 | ahi << 16);
-                            atomicMin(&s_qlo[cur], ord_key(__uint_as_float(alo << 16)));
-                            atomicMax(&s_qhi[cur], ord_key(__uint_as_float(ahi << 16)));
-                        }
-                        cur = qi; alo = 0x7F807F80u; ahi = 0xFF80FF80u;
-                    }
-                    ahi = max_bf16x2(max_bf16x2(ahi, v.x), max_bf16x2(max_bf16x2(v.y, v.z), v.w));
-                    alo = min_bf16x2(min_bf16x2(alo, v.x), min_bf16x2(min_bf16x2(v.y, v.z), v.w));
-                }
-            }
-            if (t == S_NT - 1 && n_whole < n_oct) {           // the tensor's last, short octet: element by element
-                const int qi = loose_block(lrem0 + n_whole * 8, la.qbs, big);
-                for (int e = n_whole * 8; e < n; ++e) {
-                    const float v = __uint_as_float((uint32_t)tile[e] << 16);
-                    if (v != v) continue;                    // (a NaN is in no statistics)
-                    atomicMin(&s_qlo[qi], ord_key(v)); atomicMax(&s_qhi[qi], ord_key(v));
-                }
-            }
-            {
-                alo = min_bf16x2(alo, alo >> 16 | alo << 16); ahi = max_bf16x2(ahi, ahi >> 16 | ahi << 16);
-                uint32_t klo = ord_key(__uint_as_float(alo << 16)), khi = ord_key(__uint_as_float(ahi << 16));
-                const int c_first = __shfl_sync(0xffffffffu, cur, 0);
-                if (__all_sync(0xffffffffu, cur == c_first)) {  // the whole warp ended in one block (or holds nothing)
-                    klo = __reduce_min_sync(0xffffffffu, klo);
-                    khi = __reduce_max_sync(0xffffffffu, khi);
-                    if (lane == 0 && cur >= 0) { atomicMin(&s_qlo[cur], klo); atomicMax(&s_qhi[cur], khi); }
-                } else if (cur >= 0) {
-                    atomicMin(&s_qlo[cur], klo); atomicMax(&s_qhi[cur], khi);
-                }
-            }
-            MAB_CTICK(7);
-            __syncthreads();
-            {
-                const int64_t at = la.qb_first[ti] + qb0;
-                for (int i = t; i < n_qb; i += S_NT) {
-                    atomicMin(la.st_min + at + i, s_qlo[i]);
-                    atomicMax(la.st_max + at + i, s_qhi[i]);
-                }
-            }
-            MAB_CTICK(9);
-            __syncthreads();                                 // the tile is overwritten by the next load
-        } else if (swz) {
+        if (swz) {
             stats_encode_regular(tile4, n >> 6, mn_out, mx_out, ef_out, (reinterpret_cast<uintptr_t>(ef_out) & 15) == 0);
             if ((n & 63) != 0 && warp == S_NT / 32 - 1) stats_encode_short_row(tile4, n >> 6, n, mn_out, mx_out, ef_out);
             __syncthreads();                                 // the tile is overwritten by the next load
-        } else if (tables && (n & 63) == 0) {
+        } else if ((n & 63) == 0) {
             // whole blocks of 64: statistics block by block (a thread's 8 octets, rotated so that a warp's
             // 16-byte reads spread over the banks), constants to the tables, then codes octet by octet
             for (int b = t; b < n_qb; b += S_NT) {
@@ -996,7 +896,7 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
             }
             __syncthreads();                                 // the tile is overwritten by the next load
         } else {
-            // any block size, ragged ends: one thread per quantisation block
+            // ragged ends: one thread per quantisation block
             for (int b = t; b < n_qb; b += S_NT) {
                 uint32_t hi2 = 0xFF80FF80u, lo2 = 0x7F807F80u;
                 const int o_first = b << cshift;
@@ -1043,24 +943,13 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
     }
 }
 
-int launch_ef_topk_quant_bf16(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, cudaStream_t s,
-                              const LooseArgs* loose) {
-    int qshift = 0;
-    if (loose == nullptr) while ((1 << qshift) < qbs) ++qshift;
+int launch_ef_topk_quant_bf16(const mab_tensor* dev_tensors, int n_tensors, int total_units, int max_dbs, cudaStream_t s) {
     const int smem = ((max_dbs * 2 + 127) & ~127) + (int)sizeof(SmemSel);
     const int per_sm = std::min(S_CTAS, (device_max_optin_smem() + 1024) / (smem + 3 * 1024 + 128));
     if (per_sm < 2) return 1;                                // not even two CTAs per SM: the caller uses the other kernel
     const int grid = (int)std::min<int64_t>(total_units, (int64_t)device_sm_count() * per_sm);
-    LooseArgs la = {0, nullptr, nullptr, nullptr};
-    if (loose) la = *loose;
-    auto run = [&](auto kern) -> int {
-        MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        kern<<<grid, S_NT, smem, s>>>(dev_tensors, n_tensors, total_units, qshift, max_dbs, la);
-        return MAB_OK;
-    };
-    const int rc = loose ? run(ef_topk_quant_bf16_kernel<false, true>)
-                 : qshift == 6 ? run(ef_topk_quant_bf16_kernel<true, false>) : run(ef_topk_quant_bf16_kernel<false, false>);
-    if (rc) return rc;
+    MAB_CUDA_TRY(cudaFuncSetAttribute(ef_topk_quant_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    ef_topk_quant_bf16_kernel<<<grid, S_NT, smem, s>>>(dev_tensors, n_tensors, total_units, max_dbs);
     count_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "ef_topk_quant_bf16_kernel launch");

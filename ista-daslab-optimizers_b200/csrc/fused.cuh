@@ -61,18 +61,20 @@ __device__ __forceinline__ int loose_block(int r, int qbs, bool big) {
     return big ? (r >= qbs ? 1 : 0) : (int)((unsigned)r / (unsigned)qbs);
 }
 
-// ef_topk_quant.cu
+// ef_topk_quant.cu; wide: every gradient starts on a 16-byte boundary
 int launch_ef_topk_quant(const mab_tensor* dev_tensors, int n_tensors, int total_units, int grad_dtype,
-                         int qbs, int max_dbs, int max_k, cudaStream_t s, const LooseArgs* loose = nullptr);
+                         int qbs, int max_dbs, int max_k, bool wide, cudaStream_t s, const LooseArgs* loose = nullptr);
 int units_a_of(const mab_tensor& t);
 
 // requant_loose.cu: statistics (bf16) and codes of the residual kernel A left in the gradient buffers
 int launch_requant_loose(const mab_tensor* dev_tensors, int n_tensors, int total_units, int grad_dtype,
                          const LooseArgs& la, cudaStream_t s);
 
-// ef_topk_quant_bf16.cu: returns 1 (without launching) when two CTAs of its shared memory do not fit an SM
-int launch_ef_topk_quant_bf16(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, cudaStream_t s,
-                              const LooseArgs* loose = nullptr);
+// ef_topk_quant_bf16.cu (blocks of 64) and ef_topk_quant_bf16_warps.cu (all others, and large launches): return 1 (without
+// launching) when two CTAs of their shared memory do not fit an SM
+int launch_ef_topk_quant_bf16(const mab_tensor* dev_tensors, int n_tensors, int total_units, int max_dbs, cudaStream_t s);
+int launch_ef_topk_quant_bf16_warps(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, cudaStream_t s,
+                                    const LooseArgs* loose);
 
 // ef_topk_quant_f32.cu: returns 1 (without launching) where the tile or its candidates do not fit
 int launch_ef_topk_quant_f32(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, int max_k, cudaStream_t s);
@@ -82,6 +84,7 @@ int launch_ef_topk_quant_f32(const mab_tensor* dev_tensors, int n_tensors, int t
 int copy_timeout_f32(int* out, bool clear);      // ef_topk_quant.cu
 int copy_timeout_f32_split(int* out, bool clear);   // ef_topk_quant_f32.cu
 int copy_timeout_bf16(int* out, bool clear);     // ef_topk_quant_bf16.cu
+int copy_timeout_bf16_warps(int* out, bool clear);  // ef_topk_quant_bf16_warps.cu
 int copy_timeout_window(int* out, bool clear);   // window_adam.cu
 
 }  // namespace mab
