@@ -171,23 +171,27 @@ __device__ __forceinline__ uint32_t encode_octet(const float (&r)[8], const QPar
     return encode_octet_fast<CLAMP>(r, q, c);
 }
 
-// Codes of one octet by the defining form floor(RN(RN((r - mn) / u) + 0.5)) itself, two elements per
-// instruction and without division or conversion instructions; u in [2^-100, 2^100].  The IEEE quotient
-// comes from the correctly rounded reciprocal r0 = RN(1 / u): q = RN(d * r0) is within 1.5 ulp of d / u, one
-// residual correction q <- RN(q + RN(d - q * u) * r0) (the residual is exact in an FMA) makes it faithful,
-// and a second one makes it the correctly rounded quotient (Markstein's theorem on the final step of a
-// division).  Values far below half a step, where the residual could underflow, get code 0 from any
-// quotient below 0.5.  floor: adding 2^23 with rounding down leaves the integer in the low mantissa bits.
+// Codes of one octet by the defining form floor(RN(RN((r - mn) / u) + 0.5)), two elements per instruction and without division or
+// conversion instructions; u in [2^-100, 2^100].  The quotient is d * r0 + d * r1 with r0 = RN(1 / u) and r1 = RN((1 - u r0) r0),
+// the second product rounded, its sum with the first one rounded once.  That is not always RN(d / u), but floor(RN(q + 0.5))
+// is the same for every mantissa of u and every d within four ulps of a code's threshold (2^23 x 16 x 9 cases, checked
+// on a CPU at the middle and at both ends of the range of u; tests/codec_quotient_check.c goes through a share of them), and farther
+// away an error below an ulp does not matter.  (Two residual corrections of RN(d * r0), which give RN(d / u) itself, took three
+// packed instructions more per pair.)  floor: adding 2^23 with rounding down leaves the integer in the low mantissa bits.
 // CLAMP: values may lie outside [mn, mn + 15 u] (statistics rounded to bf16): s is clamped to [0, 15.5]
 // before the floor, which gives the codes the defining clamp(floor(s), 0, 15) gives, and a NaN the code 0.  Without CLAMP
 // a NaN's bits run into its neighbours' codes: kernel A looks for one first (its block's
 // minimum is then a NaN); the requantisation of loose bf16 blocks does not, NaN being outside the step's contract.
-struct DivConsts { float2 nmn2, r02, nu2; };
+struct DivConsts { float2 nmn2, r02, r12; };
+
+// What RN(1 / u) = r0 leaves of 1 / u.
+__device__ __forceinline__ float rcp_rest(float u, float r0) { return __fmul_rn(__fmaf_rn(-u, r0, 1.0f), r0); }
 
 __device__ __forceinline__ DivConsts div_consts(const QParams& q) {
     DivConsts c;
     const float r0 = (q.u >= CODEC_U_MIN && q.u <= CODEC_U_MAX) ? rcp_rn_normal(q.u) : 0.0f;   // (unused outside that range)
-    c.nmn2 = make_float2(-q.mn, -q.mn); c.r02 = make_float2(r0, r0); c.nu2 = make_float2(-q.u, -q.u);
+    const float r1 = rcp_rest(q.u, r0);
+    c.nmn2 = make_float2(-q.mn, -q.mn); c.r02 = make_float2(r0, r0); c.r12 = make_float2(r1, r1);
     return c;
 }
 
@@ -198,9 +202,7 @@ __device__ __forceinline__ uint32_t encode_octet_div_f32(const float (&r)[8], co
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
         const float2 d = __fadd2_rn(make_float2(r[2 * p], r[2 * p + 1]), c.nmn2);   // r - mn
-        float2 q = __fmul2_rn(d, c.r02);
-        q = __ffma2_rn(__ffma2_rn(q, c.nu2, d), c.r02, q);
-        q = __ffma2_rn(__ffma2_rn(q, c.nu2, d), c.r02, q);                          // RN(d / u)
+        const float2 q = __ffma2_rn(d, c.r02, __fmul2_rn(d, c.r12));
         float2 s = __fadd2_rn(q, half2);
         if (CLAMP) {
             s.x = fminf(fmaxf(s.x, 0.0f), 15.5f);

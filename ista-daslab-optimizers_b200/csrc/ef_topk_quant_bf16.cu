@@ -189,15 +189,10 @@ __device__ __forceinline__ void store_code_word(uint8_t* ef_g, bool aligned4, in
     for (int b = 0; b < 4; ++b) if (o * 8 + 2 * b < n) ef_g[o * 4 + b] = (uint8_t)(w >> (8 * b));
 }
 
-// Codes of one octet of bf16 values r (statistics = their exact block minimum and maximum, u in
-// [2^-100, 2^100]): the defining floor(RN(RN((r - mn) / u) + 0.5)) itself, two elements per instruction and
-// without the division and conversion instructions.  The IEEE quotient comes from the correctly rounded
-// reciprocal r0 = RN(1 / u): q = RN(d * r0) is within 1.5 ulp of d / u, one residual correction
-// q <- RN(q + RN(d - q * u) * r0) (the residual is exact in an FMA) makes it faithful, and a second one
-// makes it the correctly rounded quotient (Markstein's theorem on the final step of a division).  Values far
-// below half a step, where the residual could underflow, get code 0 from any quotient below 0.5.
-// floor: adding 2^23 with rounding down leaves the integer in the low mantissa bits.
-__device__ __forceinline__ uint32_t encode_octet_div(const uint4& v, float2 nmn2, float2 r02, float2 nu2) {
+// Codes of one octet of bf16 values r (statistics = their exact block minimum and maximum, u in [2^-100, 2^100]): the defining
+// form, two elements per instruction, the quotient as in encode_octet_div_f32 (codec_fast.cuh).  floor: adding 2^23 with rounding
+// down leaves the integer in the low mantissa bits.
+__device__ __forceinline__ uint32_t encode_octet_div(const uint4& v, float2 nmn2, float2 r02, float2 r12) {
     const float2 half2 = make_float2(0.5f, 0.5f), magic2 = make_float2(8388608.0f, 8388608.0f);
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     uint32_t y[8];
@@ -205,9 +200,7 @@ __device__ __forceinline__ uint32_t encode_octet_div(const uint4& v, float2 nmn2
     for (int p = 0; p < 4; ++p) {
         const float2 r = make_float2(__uint_as_float(w[p] << 16), __uint_as_float(w[p] & 0xFFFF0000u));
         const float2 d = __fadd2_rn(r, nmn2);                               // r - mn
-        float2 q = __fmul2_rn(d, r02);
-        q = __ffma2_rn(__ffma2_rn(q, nu2, d), r02, q);
-        q = __ffma2_rn(__ffma2_rn(q, nu2, d), r02, q);                      // RN(d / u)
+        const float2 q = __ffma2_rn(d, r02, __fmul2_rn(d, r12));
         const float2 f = __fadd2_rd(__fadd2_rn(q, half2), magic2);          // 2^23 + floor(q + 0.5)
         y[2 * p] = __float_as_uint(f.x); y[2 * p + 1] = __float_as_uint(f.y);
     }
@@ -366,17 +359,17 @@ __device__ __forceinline__ void stats_encode_regular(const uint4* tile4, int n_q
             encode_block_exact(row, key, mn_b, mx_b, mn_out + b, dst);
             continue;
         }
-        const float r0 = rcp_rn_normal(q2.u);
-        const float2 nmn2 = make_float2(-q2.mn, -q2.mn), r02 = make_float2(r0, r0), nu2 = make_float2(-q2.u, -q2.u);
+        const float r0 = rcp_rn_normal(q2.u), r1 = rcp_rest(q2.u, r0);
+        const float2 nmn2 = make_float2(-q2.mn, -q2.mn), r02 = make_float2(r0, r0), r12 = make_float2(r1, r1);
         uint4 lo4, hi4;
-        lo4.x = encode_octet_div(row[0 ^ key], nmn2, r02, nu2);
-        lo4.y = encode_octet_div(row[1 ^ key], nmn2, r02, nu2);
-        lo4.z = encode_octet_div(row[2 ^ key], nmn2, r02, nu2);
-        lo4.w = encode_octet_div(row[3 ^ key], nmn2, r02, nu2);
-        hi4.x = encode_octet_div(row[4 ^ key], nmn2, r02, nu2);
-        hi4.y = encode_octet_div(row[5 ^ key], nmn2, r02, nu2);
-        hi4.z = encode_octet_div(row[6 ^ key], nmn2, r02, nu2);
-        hi4.w = encode_octet_div(row[7 ^ key], nmn2, r02, nu2);
+        lo4.x = encode_octet_div(row[0 ^ key], nmn2, r02, r12);
+        lo4.y = encode_octet_div(row[1 ^ key], nmn2, r02, r12);
+        lo4.z = encode_octet_div(row[2 ^ key], nmn2, r02, r12);
+        lo4.w = encode_octet_div(row[3 ^ key], nmn2, r02, r12);
+        hi4.x = encode_octet_div(row[4 ^ key], nmn2, r02, r12);
+        hi4.y = encode_octet_div(row[5 ^ key], nmn2, r02, r12);
+        hi4.z = encode_octet_div(row[6 ^ key], nmn2, r02, r12);
+        hi4.w = encode_octet_div(row[7 ^ key], nmn2, r02, r12);
         if (ef_al16) {
             reinterpret_cast<uint4*>(dst)[0] = lo4;
             reinterpret_cast<uint4*>(dst)[1] = hi4;

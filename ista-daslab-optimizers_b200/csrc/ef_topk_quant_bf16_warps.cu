@@ -503,13 +503,8 @@ __device__ __noinline__ void decode_unit_scalar(uint16_t* tile, const TileInfo& 
 }
 
 // ---------------------------------------------------------------------------------------------- encode
-// Codes of one octet of bf16 values r (statistics = their exact block minimum and maximum, u in [2^-100, 2^100]): the
-// defining floor(RN(RN((r - mn) / u) + 0.5)), two elements per instruction and without the division and conversion
-// instructions.  The quotient is d * r0 + d * r1 with r0 = RN(1 / u) and r1 = RN((1 - u r0) r0), the product d * r1 rounded and
-// the sum of the other one and it rounded once: not always the correctly rounded quotient, but floor(RN(q + 0.5)) is the
-// same for every mantissa of u and every d within four ulps of a code's threshold (checked exhaustively on a CPU, over
-// 2^23 x 16 x 9 cases, at the middle and at both ends of the range of u; tests/codec_quotient_check.c samples them), and
-// farther away an error below an ulp does not matter.
+// Codes of one octet of bf16 values r (statistics = their exact block minimum and maximum, u in [2^-100, 2^100]): the defining
+// form, two elements per instruction, the quotient as in encode_octet_div_f32 (codec_fast.cuh).
 // floor: adding a power of two with rounding down leaves the integer in the mantissa; 2^23 for the odd elements puts it into
 // bits 0-3, 2^19 for the even ones into bits 4-7, above four bits of fraction that the merge drops.
 __device__ __forceinline__ uint32_t encode_octet_quotient(const uint4& v, const float2& nmn, const float2& r0, const float2& r1) {
@@ -581,7 +576,7 @@ __device__ __forceinline__ void stats_encode(const uint4* tile4, int b, int b1, 
             encode_block_exact(tile4, o0, CPQ, mn_b, mx_b, mn_out + b, dst, al >= 4);
             continue;
         }
-        const float r0 = rcp_rn_normal(q2.u), r1 = __fmul_rn(__fmaf_rn(-q2.u, r0, 1.0f), r0);
+        const float r0 = rcp_rn_normal(q2.u), r1 = rcp_rest(q2.u, r0);
         const float2 nmn = make_float2(-q2.mn, -q2.mn), r02 = make_float2(r0, r0), r12 = make_float2(r1, r1);
         uint32_t w[CPQ];
 #pragma unroll
