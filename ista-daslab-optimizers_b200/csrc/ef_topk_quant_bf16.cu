@@ -442,6 +442,7 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
     uint4* tile4 = reinterpret_cast<uint4*>(smem_raw);
     SmemSel& ss = *reinterpret_cast<SmemSel*>(smem_raw + ((stage_elems * 2 + 127) & ~127));
     const int t = threadIdx.x, lane = lane_id(), warp = warp_id();
+    allow_next_kernel();
     for (int i = t; i < n_tensors; i += S_NT) s_first[i] = tensors[i].first_unit_a;
     if (t == 0) { s_first[n_tensors] = total_units; mbar_init(&s_bar, 1); ss.ctrl[5] = 0; ss.ctrl[6] = 0; }
     __syncthreads();

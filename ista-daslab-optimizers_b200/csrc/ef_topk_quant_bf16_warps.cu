@@ -691,6 +691,7 @@ ef_topk_quant_bf16_warps_kernel(const mab_tensor* __restrict__ tensors, int n_te
     uint4* const tile4 = reinterpret_cast<uint4*>(smem_raw);
     SmemSel& ss = *reinterpret_cast<SmemSel*>(smem_raw + ((stage_elems * 2 + 127) & ~127));
     const int t = threadIdx.x, lane = lane_id(), warp = warp_id();
+    if constexpr (!LOOSE) allow_next_kernel();
     // a CTA's tiles are neighbours: they mostly belong to one tensor, whose bound carries over from tile to tile
     const int unit0 = (int)((int64_t)total_units * blockIdx.x / gridDim.x), unit1 = (int)((int64_t)total_units * (blockIdx.x + 1) / gridDim.x);
     const bool big = LOOSE && la.qbs >= SEL_MAX_TILE;

@@ -278,6 +278,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
     float4* tile4 = reinterpret_cast<float4*>(smem_raw);
     SmemF& ss = *reinterpret_cast<SmemF*>(smem_raw + tile_bytes);
     const int t = threadIdx.x, lane = lane_id(), warp = warp_id();
+    allow_next_kernel();
     for (int i = t; i < n_tensors; i += F_NT) s_first[i] = tensors[i].first_unit_a;
     if (t == 0) { s_first[n_tensors] = total_units; mbar_init(&s_bar, 1); ss.slow = 0; }
     __syncthreads();

@@ -716,6 +716,7 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
     float* const dense = dense_at > 0 ? reinterpret_cast<float*>(smem_raw + dense_at) : nullptr;   // the streams' arrays of the warps
     if (dense != nullptr) for (int i = t; i < NT * 8; i += NT) dense[i] = 0.0f;
     __syncthreads();
+    if (MODE == MODE_STEP) wait_for_kernel_before();
     const float inv_bc1 = 1.0f / a.bc1, inv_bc2 = 1.0f / a.bc2;
     UpdateProbe pr;
     const bool probing = MODE == MODE_STEP && a.probe != nullptr;
@@ -868,6 +869,7 @@ window_resident_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, in
     for (int i = t; i < n_tensors; i += WR_THREADS) s_first[i] = tensors[i].first_unit_a;
     if (t == 0) { s_first[n_tensors] = total_units; mbar_init(&s_bar, 1); }
     __syncthreads();
+    wait_for_kernel_before();
     const float inv_bc1 = 1.0f / a.bc1, inv_bc2 = 1.0f / a.bc2;
     uint32_t parity = 0;
     bool store_in_flight = false;                                               // thread 0 only
@@ -991,6 +993,7 @@ __device__ __forceinline__ void window_wide_body(const mab_tensor* __restrict__ 
     for (int i = threadIdx.x; i < n_tensors; i += WIN_THREADS) s_first[i] = tensors[i].first_unit_b;
     if (threadIdx.x == 0) s_first[n_tensors] = total_units;
     __syncthreads();
+    if (MODE == MODE_STEP) wait_for_kernel_before();
     UpdateProbe pr;
 
     for (int unit = blockIdx.x; unit < total_units; unit += gridDim.x) {
@@ -1053,7 +1056,7 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
         auto run = [&](auto kern, int threads) -> int {
             MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
             if constexpr (MODE == MODE_WRITE_UPDATE) kern<<<grid, threads, smem, s>>>(*single, units_tile, max_k, a);
-            else kern<<<grid, threads, smem, s>>>(dev_tensors, n_tensors, units_tile, max_k, dense_at, a);
+            else MAB_CUDA_TRY(launch_behind_kernel(kern, grid, threads, smem, s, dev_tensors, n_tensors, units_tile, max_k, dense_at, a));
             return MAB_OK;
         };
         int rc;
@@ -1078,7 +1081,7 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
         } else {
             auto kern = window_wide_kernel<TP, MODE, ALPHA>;
             MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WIN_SMEM_BYTES));
-            kern<<<grid, WIN_THREADS, WIN_SMEM_BYTES, s>>>(dev_tensors, n_tensors, units_wide, a);
+            MAB_CUDA_TRY(launch_behind_kernel(kern, grid, WIN_THREADS, WIN_SMEM_BYTES, s, dev_tensors, n_tensors, units_wide, a));
         }
     }
     count_launch();
@@ -1137,7 +1140,7 @@ int launch_window_step(const mab_tensor* dev_tensors, int n_tensors, int units_t
     if (smem > 0) {
         const int grid = (int)std::min<int64_t>(units_tile, (int64_t)device_sm_count() * 2);
         MAB_CUDA_TRY(cudaFuncSetAttribute(window_resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        window_resident_kernel<<<grid, WR_THREADS, smem, s>>>(dev_tensors, n_tensors, units_tile, max_k, tile_bytes, a);
+        MAB_CUDA_TRY(launch_behind_kernel(window_resident_kernel, grid, WR_THREADS, smem, s, dev_tensors, n_tensors, units_tile, max_k, tile_bytes, a));
         count_launch();
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(e, "window_resident_kernel launch");
