@@ -187,13 +187,12 @@ __device__ __forceinline__ void resolve_selection_regs(const uint32_t (&gt)[S_WP
 }
 
 // The whole selection of a tile at a cost that does not depend on the data: bisection on the key bits (all_zero: every key
-// is zero, the k lowest positions win the ties), row written, selected values zeroed.  Starts and ends with a barrier.
+// is zero, the k lowest positions win the ties), row written, selected values zeroed.  The caller has met at a barrier; ends with one.
 __device__ __noinline__ void select_by_bisection(uint16_t* tile, SmemSel& ss, int n, int k, bool all_zero, int16_t* i_out, uint16_t* v_out) {
     const uint4* tile4 = reinterpret_cast<const uint4*>(tile);
     const int t = threadIdx.x, n_oct = (n + 7) >> 3;
     uint32_t gt[S_WPT], tw[S_WPT];
     int need = 0;
-    __syncthreads();
     if (all_zero) {
 #pragma unroll
         for (int i = 0; i < S_WPT; ++i) {
@@ -1037,6 +1036,7 @@ ef_topk_quant_bf16_warps_kernel(const mab_tensor* __restrict__ tensors, int n_te
             }
             __syncwarp();
         } else {
+            if (__syncthreads_or(lost)) return;              // (a tile can come here without having counted candidates)
             select_by_bisection(tile, ss, n, k, zero, I.i_out, I.v_out);
             guess = 0;
         }
