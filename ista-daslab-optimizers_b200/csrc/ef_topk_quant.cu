@@ -448,7 +448,7 @@ ef_topk_quant_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int 
         MAB_TICK(14);
         __syncthreads();   // selection scratch is reused by the next unit
         if (LOOSE) {
-            const int n_qb = loose_block(lrem0 + n - 1, la.qbs, false) + 1;      // blocks the tile touches
+            const int n_qb = loose_blocks_touched(lrem0, n, la.qbs);
             const int64_t at = la.qb_first[ti] + lqb0;
             for (int i = threadIdx.x; i < n_qb; i += SEL_THREADS) {
                 atomicMin(la.st_min + at + i, s_qlo[i]);

@@ -725,7 +725,7 @@ ef_topk_quant_bf16_warps_kernel(const mab_tensor* __restrict__ tensors, int n_te
         };
         ask(N.g, (int64_t)N.n * 2);
         ask(N.ef, ((int64_t)N.n + 1) >> 1);
-        const int64_t nb = LOOSE ? (N.lrem0 + N.n + la.qbs - 1) / la.qbs : ((int64_t)N.n + (1 << QS) - 1) >> QS;
+        const int64_t nb = LOOSE ? loose_blocks_touched(N.lrem0, N.n, la.qbs) : ((int64_t)N.n + (1 << QS) - 1) >> QS;
         ask(N.mn, nb * 2);
         ask(N.mx, nb * 2);
     };

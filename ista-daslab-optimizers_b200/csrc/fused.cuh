@@ -77,8 +77,14 @@ __device__ __forceinline__ float ord_value(uint32_t k) {
 
 // Quantisation block (relative to the tile's first) of the octet that starts `r` elements after that block's start;
 // `big`: the block is at least as long as the longest tile, so the answer is 0 or 1.
-__device__ __forceinline__ int loose_block(int r, int qbs, bool big) {
+__host__ __device__ __forceinline__ int loose_block(int r, int qbs, bool big) {
     return big ? (r >= qbs ? 1 : 0) : (int)((unsigned)r / (unsigned)qbs);
+}
+
+// Quantisation blocks that a tile of n elements touches which starts lrem0 elements into one (lrem0 < qbs <= 2^30: the sum of
+// both and another qbs would not fit 32 bits).
+__host__ __device__ __forceinline__ int loose_blocks_touched(int lrem0, int n, int qbs) {
+    return loose_block(lrem0 + n - 1, qbs, false) + 1;
 }
 
 // ef_topk_quant.cu; wide: every gradient starts on a 16-byte boundary
