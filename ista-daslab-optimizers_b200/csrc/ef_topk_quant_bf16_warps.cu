@@ -944,8 +944,11 @@ ef_topk_quant_bf16_warps_kernel(const mab_tensor* __restrict__ tensors, int n_te
                     n_c += total;
                     const uint16_t* at = tile + phys_oct(2 * u) * 8;
                     const uint16_t* at_odd = tile + phys_oct(2 * u + 1) * 8;
+                    // the warp meets for every value: left to themselves the lanes come apart and take their turns one by one (loose blocks,
+                    // k = 5 %, 29 M elements: this kernel 90 us without, 75 with the vote; 134 M, blocks of 64, k = 1 %: 176 and 168)
 #pragma unroll 1
-                    for (; m; m &= m - 1, ++to) {
+                    for (; __any_sync(0xffffffffu, m != 0u); m &= m - 1, ++to) {
+                        if (m == 0u) continue;
                         const int b = __ffs(m) - 1;
                         const uint32_t v = (b < 8 ? at : at_odd - 8)[b];
                         atomicAdd(&ss.hist[p][min((int)(v & 0x7FFFu) - bound, S_BINS - 1)], 1);
