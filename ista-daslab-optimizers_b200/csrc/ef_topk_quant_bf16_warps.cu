@@ -694,7 +694,8 @@ ef_topk_quant_bf16_warps_kernel(const mab_tensor* __restrict__ tensors, int n_te
     const int t = threadIdx.x, lane = lane_id(), warp = warp_id();
     if constexpr (!LOOSE) allow_next_kernel();
     // a CTA's tiles are neighbours: they mostly belong to one tensor, whose bound carries over from tile to tile
-    const int unit0 = (int)((int64_t)total_units * blockIdx.x / gridDim.x), unit1 = (int)((int64_t)total_units * (blockIdx.x + 1) / gridDim.x);
+    const TileRange range = tiles_of_cta(total_units, gridDim.x, blockIdx.x);
+    const int unit0 = range.first, unit1 = range.end;
     const bool big = LOOSE && la.qbs >= SEL_MAX_TILE;
     uint16_t* const list = ss.w[warp].list;
     const unsigned lower = (1u << lane) - 1u;
