@@ -57,32 +57,102 @@ def test_warp_owned_tiles_match_oracle(kind, qbs, k_init, skip):
     assert _native.device_error() == 0
 
 
-@pytest.mark.parametrize('k_init', [0.005, 0.01, 0.02])
-def test_large_launch_equals_small_ones(k_init):
-    """Blocks of 64: one tensor of 3300 tiles takes one form of the kernel, its thirds the other one."""
+def _kernels_of(step):
+    """Names of the kernels a call launches."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as prof:
+        step()
+        torch.cuda.synchronize()
+    return [e.name for e in prof.events() if e.device_type.name == 'CUDA']
+
+
+def _same(a, b):
+    """Equal bits; a NaN equals every other NaN."""
+    if a.dtype == torch.uint8:
+        return torch.equal(a, b)
+    nan = torch.isnan(a.float()) & torch.isnan(b.float())
+    return torch.equal(a.view(torch.int16)[~nan], b.view(torch.int16)[~nan])
+
+
+# full tiles (the last one: more than 20 a SM together), and between them lengths that end around a unit, a slot or a block and
+# make the warps' parts of the tile change hands
+MANY = (1400 * DBS, 7, DBS - 1, 513, 600 * DBS + 4104, 64, 65 * 64 + 15, 2 * DBS + 8191, 16, 1400 * DBS + 33)
+
+
+@pytest.mark.parametrize('kind,k_init,alpha', [('mixed', 0.005, 0), ('mixed', 0.01, 0), ('mixed', 0.02, 0), ('mixed', 0.01, -2),
+                                               ('nan', 0.01, 0), ('inf', 0.01, 0)])
+def test_large_launch_equals_small_ones(kind, k_init, alpha):
+    """Blocks of 64: a step of more than 20 tiles per SM takes one form of the kernel, its tensors by themselves the other one."""
     from ista_daslab_optimizers_b200 import MicroAdam, _native
-    n, parts = 3300 * DBS, 3
-    hyper = dict(m=2, lr=1e-3, quant_block_size=64, k_init=k_init)
+    hyper = dict(m=2, lr=1e-3, quant_block_size=64, k_init=k_init, alpha=alpha)
     gen = torch.Generator(device='cuda').manual_seed(7)
-    whole = torch.nn.Parameter(torch.zeros(n, dtype=torch.bfloat16, device='cuda'))
-    thirds = [torch.nn.Parameter(whole.detach()[i * (n // parts):(i + 1) * (n // parts)].clone()) for i in range(parts)]
-    opt = MicroAdam([whole], **hyper)
-    opts = [MicroAdam([p], **hyper) for p in thirds]
-    for step in range(2):
-        g = torch.empty(n, dtype=torch.bfloat16, device='cuda').normal_(0.0, 1e-3, generator=gen)
-        blocks = g.view(-1, DBS)
-        blocks[5::97] *= 64.0                            # bounds that do not carry over
-        blocks[6::97] = 0.0
-        blocks[7::97, ::2] = 1e-2 * torch.sign(blocks[7::97, ::2])
-        whole.grad = g
-        opt.step()
-        for i, (p, o) in enumerate(zip(thirds, opts)):
-            p.grad = g[i * (n // parts):(i + 1) * (n // parts)]
-            o.step()
-        a = opt.state[whole]
-        for key in ('I', 'V', 'error', 'min_vals', 'max_vals'):
-            have = a[key][step] if key in 'IV' else a[key]
-            want = torch.cat([o.state[p][key][step] if key in 'IV' else o.state[p][key][:p.numel() // 64 if 'vals' in key else None]
-                              for p, o in zip(thirds, opts)])
-            assert torch.equal(have[:want.numel()].view(torch.uint8), want.view(torch.uint8)), (key, step)
+    whole = [torch.nn.Parameter(torch.zeros(n, dtype=torch.bfloat16, device='cuda')) for n in MANY]
+    alone = [torch.nn.Parameter(p.detach().clone()) for p in whole]
+    opt = MicroAdam(whole, **hyper)
+    opts = [MicroAdam([p], **hyper) for p in alone]
+    for step in range(3):
+        for p, q in zip(whole, alone):
+            n = p.numel()
+            g = torch.empty(n, dtype=torch.bfloat16, device='cuda').normal_(0.0, 1e-3, generator=gen)
+            blocks = g[:n // DBS * DBS].view(-1, DBS)
+            blocks[5::97] *= 64.0                        # bounds that do not carry over
+            blocks[6::97] = 0.0
+            blocks[7::97, ::2] = 1e-2 * torch.sign(blocks[7::97, ::2])
+            if kind == 'nan' and step < 2:
+                g[3::4099] = float('nan')
+                blocks[8::97, 4096:8192] = float('nan')
+                blocks[9::97, :DBS - 1600] = float('nan')
+            if kind == 'inf' and step < 2:
+                g[3::5003] = float('inf')
+                g[9::7001] = float('-inf')
+                blocks[8::97, ::64] = float('inf')       # more than k of them: the residual's statistics are infinite
+            p.grad = g
+            q.grad = g.clone()
+        if step == 0:
+            names = _kernels_of(opt.step)
+            assert any('ef_topk_quant_bf16_warps_kernel<6>' in x.replace('(int)', '') for x in names), names
+        else:
+            opt.step()
+        for i, o in enumerate(opts):
+            if step == 0 and i == 0:
+                names = _kernels_of(o.step)
+                assert any('ef_topk_quant_bf16_kernel' in x for x in names), names
+            else:
+                o.step()
+        for p, q, o in zip(whole, alone, opts):
+            a, b = opt.state[p], o.state[q]
+            used = -(-p.numel() // 64)
+            for key in ('I', 'V', 'error', 'min_vals', 'max_vals') + (('quant_err',) if alpha == -2 else ()):
+                x, y = (t[key][step % 2] if key in ('I', 'V') else t[key][:used] if 'vals' in key else t[key] for t in (a, b))
+                assert _same(x.contiguous(), y.contiguous()), (p.numel(), step, key)
+            assert _same(p.detach(), q.detach()), (p.numel(), step)
+    assert _native.device_error() == 0
+
+
+@pytest.mark.parametrize('qbs', [8, 16, 32, 128, 64, 1000, 100000])
+def test_infinities_match_the_operator_level_kernels(qbs):
+    """Infinite gradients, fewer than k of a tile: selected like any large value, and nothing of them stays in the residual."""
+    from ista_daslab_optimizers_b200 import MicroAdam, _native
+    hyper = dict(m=4, lr=1e-3, quant_block_size=qbs, k_init=0.01)
+    pairs = []
+    for use_fused in (True, False):
+        params = [torch.nn.Parameter(S.normal_tensor(60, i, n, 0.02).bfloat16().cuda()) for i, n in enumerate(SIZES)]
+        pairs.append((params, MicroAdam(params, use_fused=use_fused, **hyper)))
+    for step in range(3):
+        for i, n in enumerate(SIZES):
+            g = _gradient('normal', i, n, step)
+            if step < 2 and n >= 4095:
+                g[11::1500] = float('inf')
+                g[700::3000] = float('-inf')
+            for params, _ in pairs:
+                params[i].grad = g.cuda()
+        for _, opt in pairs:
+            opt.step()
+        for p, q, n in zip(*(params for params, _ in pairs), SIZES):
+            a, b, used = pairs[0][1].state[p], pairs[1][1].state[q], -(-n // qbs)
+            for key in ('I', 'V', 'error', 'min_vals', 'max_vals'):
+                x, y = (t[key][step] if key in ('I', 'V') else t[key][:used] if 'vals' in key else t[key] for t in (a, b))
+                assert torch.equal(x.view(torch.uint8), y.view(torch.uint8)), (n, step, key)
+            assert torch.isfinite(a['max_vals'][:used].float()).all()
+    assert all(e.fused for e in pairs[0][1]._entries) and not any(e.fused for e in pairs[1][1]._entries)
     assert _native.device_error() == 0

@@ -1,5 +1,5 @@
 """The encoder's two-product quotient gives the codes of the defining division: a small C program goes through every 61st
-mantissa of the step (all 2^23 take it some minutes), all code thresholds and their neighbourhood."""
+mantissa of the step (all 2^23 take it about half a minute: argument 1), all code thresholds and their neighbourhood."""
 import os
 import shutil
 import subprocess
