@@ -50,7 +50,7 @@ UNIT = 'Gparams/s'
 # parameter count (traffic grows in proportion to the elements a launch covers).  None = not captured.
 NCU_TRAFFIC_BYTES_PER_PARAM = {
     ('ef_topk_quant', 'bf16'): 3.05, ('window_adam', 'bf16'): 3.98,
-    ('ef_topk_quant', 'f32'): 5.01, ('window_adam', 'f32'): 7.19,
+    ('ef_topk_quant', 'f32'): 5.00, ('window_adam', 'f32'): 7.15,
 }
 
 

@@ -462,10 +462,11 @@ ef_topk_quant_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int 
 
 int units_a_of(const mab_tensor& t) { return t.topk_full_blocks_count + (t.k_block_size_few > 0 ? 1 : 0); }
 
-// Blocks of 64 have two kernels.  The one whose warps own their part of the tile is the faster one in a long run, but finds the
-// first tile's bound more slowly and has no advantage with many candidates or a gradient that has to be staged (us a launch, it
-// and the other one): 134 M elements, 31 tiles per SM, 182 and 200; with k = 0.5 % 170 and 214, 2 % 199 and 220, 5 % 283 and 276;
-// off alignment 244 and 234; 67 M, 16 tiles per SM, 105 and 107; 54.5 M 102 and 98; 2.1 M 16.2 and 12.4.
+// Blocks of 64 have two kernels.  us a launch, the one whose warps own their part of the tile and the other one: k = 1 % with 50, 31,
+// 20, 16, 12 and 6 tiles per SM 255 / 295, 165 / 188, 113 / 129, 91 / 104, 73 / 83 and 41 / 46; 444 tiles in all 20.3 / 20.0, 72
+// 12.1 / 12.2.  31 tiles per SM with k = 0.5 % 164 / 224, 2 % 175 / 205, 5 % 218 / 263; off alignment 220 / 220, with k = 2 % 230 / 237, 5 %
+// 276 / 295.  The line was drawn when the first one lost below 20 tiles per SM, off alignment and above k = 2 % (its lanes took turns at
+// the candidates, its tiles were shared out unevenly); by these times it could lie at 6, whatever k and alignment.
 constexpr int WARPS_MIN_TILES_PER_SM = 20;
 constexpr int WARPS_MAX_K = 640;             // 2.2 % of a tile
 

@@ -20,11 +20,12 @@
 // the histogram of the octet maxima; tiles that defeat this as well (fewer than k values that are not zero, k beyond the octets)
 // fall back to a bisection on the key bits.
 //
-// Bound by instruction issue (23 instructions per element, 64 % of the cycles issue; the first form: 28.5 and 56 %): the codec's
-// half of them runs at the rate of the integer and FMA pipes, the rest is the selection and what every warp does once a tile.
-// 2.05 G elements take 2364 us a launch (the first form 2924), 218 M 278 (322), 134 M 182 (200), 67 M 105 (107); blocks of 32,
-// 33.5 M elements 69 (95), of 128 with k = 5 % 98 (123); loose blocks, 218 M 302 (342).  More registers than 80 a thread would
-// cost the third CTA, and what the compiler spills costs more than it seems: 92 bytes in the inner loops, 20 us at 218 M.
+// Bound by instruction issue (25 instructions per element at 1965 MHz, 62 % of the cycles issue, the ALU pipe 54 % busy): the codec's half
+// of them runs at the rate of the integer and FMA pipes, the rest is the selection and what every warp does once a tile.  us a
+// launch, and the form for small launches: 215 M elements 255 (295), 133 M 165 (188), 69 M 91 (104), 12.9 M 20.3 (20.0).  Against a form of
+// that design for all block sizes, with the quotient it had: blocks of 32, 29 M 53 (89), of 128 with k = 5 % 70 (113); loose blocks,
+// 215 M 291 (331).  More registers than 80 a thread would cost the third CTA, and what the compiler spills costs more than it seems: 92
+// bytes in the inner loops cost 20 us at 218 M.
 //
 // Results are bit-identical to those of the fp32 kernels' arithmetic (ef_topk_quant_f32.cu, ef_topk_quant.cu; same tie rule).
 #include "common.cuh"

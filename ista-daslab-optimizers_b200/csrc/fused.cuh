@@ -33,9 +33,12 @@ __host__ __device__ __forceinline__ TileRange tiles_of_cta(int total, int ctas, 
 
 // The update kernel of a step is launched behind kernel A without the gap between two kernels (programmatic stream
 // serialization): its CTAs read the descriptor table, which neither kernel writes, and wait there for kernel A's end and its
-// results.  A kernel A that leaves half of the SMs free allows it as soon as all its CTAs have started: a step of 7 690 elements
-// 26.6 -> 24.5 us.  With more CTAs the ones that wait take places unevenly among those that work, and the update runs on fewer
-// SMs than it could (254 tiles: 49.8 -> 53.4 us a step, so not there).
+// results.  A kernel A of at most half as many CTAs as a B200 has SMs (148) allows it as soon as all its CTAs have started; with more the
+// ones that wait take places unevenly among those that work, and the update runs on fewer SMs than it could.  us a step with 10 rows,
+// allowed and not: bf16 8 tiles 29.2 / 30.1, 40 tiles 29.6 / 30.6, 74 30.4 / 30.6, 148 30.9 / 30.9; fp32 8 tiles 41.1 / 41.2, 40 41.5 / 41.8, 74
+// 42.2 / 42.3, 90 49.2 / 41.8, 110 49.5 / 42.6, 254 72.8 / 55.5.  Most of what the launch saves is the gap itself (7 690 elements 24.6 -> 22.5 us a
+// step).  Kernel A of loose blocks does not allow it, the requantisation being next; nor do the requantisation and the fp32 kernel with
+// one tile per SM (not tried there).
 constexpr int EARLY_MAX_CTAS = 74;
 __device__ __forceinline__ void allow_next_kernel() { if (gridDim.x <= EARLY_MAX_CTAS) asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
