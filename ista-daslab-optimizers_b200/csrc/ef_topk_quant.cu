@@ -462,19 +462,16 @@ ef_topk_quant_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int 
 
 int units_a_of(const mab_tensor& t) { return t.topk_full_blocks_count + (t.k_block_size_few > 0 ? 1 : 0); }
 
-// Blocks of 64 have two kernels.  us a launch, the one whose warps own their part of the tile and the other one: k = 1 % with 50, 31,
-// 20, 16, 12 and 6 tiles per SM 255 / 295, 165 / 188, 113 / 129, 91 / 104, 73 / 83 and 41 / 46; 444 tiles in all 20.3 / 20.0, 72
-// 12.1 / 12.2.  31 tiles per SM with k = 0.5 % 164 / 224, 2 % 175 / 205, 5 % 218 / 263; off alignment 220 / 220, with k = 2 % 230 / 237, 5 %
-// 276 / 295.  The line was drawn when the first one lost below 20 tiles per SM, off alignment and above k = 2 % (its lanes took turns at
-// the candidates, its tiles were shared out unevenly); by these times it could lie at 6, whatever k and alignment.
-constexpr int WARPS_MIN_TILES_PER_SM = 20;
-constexpr int WARPS_MAX_K = 640;             // 2.2 % of a tile
+// Blocks of 64 have two kernels.  us a launch, the one whose warps own their part of the tile and the other one, from 10 tiles per SM on (1480
+// tiles): k = 0.5 % 63 / 83, 1 % 63 / 72, 2 % 66 / 79, 5 % 82 / 99, 20 % 265 / 266, off alignment 85 / 85, with k = 5 % 106 / 112; 2960 tiles
+// k = 5 % 145 / 181, off alignment 150 / 152; k = 1 % with 31 and 50 tiles per SM 165 / 188 and 255 / 295.  Below, 1000 tiles 47 / 56, 444 tiles
+// 20.3 / 20.0, 72 tiles 12.1 / 12.2: the line could lie lower, at 6 tiles per SM or so.
+constexpr int WARPS_MIN_TILES_PER_SM = 10;
 
 int launch_ef_topk_quant(const mab_tensor* dev_tensors, int n_tensors, int total_units, int grad_dtype,
-                         int qbs, int max_dbs, int max_k, bool wide, cudaStream_t s, const LooseArgs* loose) {
+                         int qbs, int max_dbs, int max_k, cudaStream_t s, const LooseArgs* loose) {
     if (grad_dtype == MAB_BF16) {          // bf16 tiles are small enough for two shared-memory resident CTAs per SM
-        const bool warps = loose != nullptr || qbs != 64 ||
-                           (wide && total_units >= WARPS_MIN_TILES_PER_SM * device_sm_count() && max_k <= WARPS_MAX_K);
+        const bool warps = loose != nullptr || qbs != 64 || total_units >= WARPS_MIN_TILES_PER_SM * device_sm_count();
         const int rc = warps ? launch_ef_topk_quant_bf16_warps(dev_tensors, n_tensors, total_units, qbs, max_dbs, s, loose)
                              : launch_ef_topk_quant_bf16(dev_tensors, n_tensors, total_units, max_dbs, s);
         if (rc <= 0) return rc;

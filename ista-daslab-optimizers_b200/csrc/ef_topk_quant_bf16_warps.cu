@@ -22,7 +22,7 @@
 //
 // Bound by instruction issue (25 instructions per element at 1965 MHz, 62 % of the cycles issue, the ALU pipe 54 % busy): the codec's half
 // of them runs at the rate of the integer and FMA pipes, the rest is the selection and what every warp does once a tile.  us a
-// launch, and the form for small launches: 215 M elements 255 (295), 133 M 165 (188), 69 M 91 (104), 12.9 M 20.3 (20.0).  Against a form of
+// launch, and the form for launches of fewer than ten tiles per SM: 215 M elements 255 (295), 133 M 165 (188), 43 M 63 (72), 12.9 M 20.3 (20.0).  Against a form of
 // that design for all block sizes, with the quotient it had: blocks of 32, 29 M 53 (89), of 128 with k = 5 % 70 (113); loose blocks,
 // 215 M 291 (331).  More registers than 80 a thread would cost the third CTA, and what the compiler spills costs more than it seems: 92
 // bytes in the inner loops cost 20 us at 218 M.

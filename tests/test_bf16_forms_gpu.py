@@ -129,6 +129,39 @@ def test_large_launch_equals_small_ones(kind, k_init, alpha):
     assert _native.device_error() == 0
 
 
+@pytest.mark.parametrize('k_init,skip', [(0.05, 0), (0.01, 3), (0.05, 1), (0.2, 8)])
+def test_line_between_the_forms(k_init, skip):
+    """Blocks of 64: from ten tiles per SM on a launch takes the warp-owned form whatever k and alignment, below the other one;
+    equal results on both sides."""
+    from ista_daslab_optimizers_b200 import MicroAdam, _native
+    from ista_daslab_optimizers_b200.compat import ista_daslab_cuda_tools as tools
+    tiles = 10 * tools.get_sm_count()
+    sizes = ((tiles - 3) * DBS, 2 * DBS + 4104)          # tiles - 3 and three tiles
+    hyper = dict(m=2, lr=1e-3, quant_block_size=64, k_init=k_init)
+    gen = torch.Generator(device='cuda').manual_seed(11)
+    whole = [torch.nn.Parameter(torch.zeros(n, dtype=torch.bfloat16, device='cuda')) for n in sizes]
+    alone = [torch.nn.Parameter(p.detach().clone()) for p in whole]
+    opt, opts = MicroAdam(whole, **hyper), [MicroAdam([p], **hyper) for p in alone]
+    for step in range(2):
+        for p, q in zip(whole, alone):
+            p.grad = torch.empty(p.numel() + skip, dtype=torch.bfloat16, device='cuda')[skip:].normal_(0.0, 1e-3, generator=gen)
+            q.grad = p.grad.clone()
+        for form, o in (('ef_topk_quant_bf16_warps_kernel', opt), ('ef_topk_quant_bf16_kernel', opts[0])):
+            if step == 0:
+                names = _kernels_of(o.step)
+                assert any(form in x for x in names), names
+            else:
+                o.step()
+        opts[1].step()
+        for p, q, o in zip(whole, alone, opts):
+            a, b, used = opt.state[p], o.state[q], -(-p.numel() // 64)
+            for key in ('I', 'V', 'error', 'min_vals', 'max_vals'):
+                x, y = (t[key][step] if key in ('I', 'V') else t[key][:used] if 'vals' in key else t[key] for t in (a, b))
+                assert torch.equal(x.contiguous().view(torch.uint8), y.contiguous().view(torch.uint8)), (p.numel(), step, key)
+            assert torch.equal(p.detach().view(torch.int16), q.detach().view(torch.int16)), (p.numel(), step)
+    assert _native.device_error() == 0
+
+
 @pytest.mark.parametrize('qbs', [8, 16, 32, 128, 64, 1000, 100000])
 def test_infinities_match_the_operator_level_kernels(qbs):
     """Infinite gradients, fewer than k of a tile: selected like any large value, and nothing of them stays in the residual."""
