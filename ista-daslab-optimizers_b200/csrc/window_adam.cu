@@ -3,12 +3,12 @@
 // operator-level compute_microadam_update built on the same code.
 //
 // Two variants share the streaming epilogue:
-//  * tile kernel (the normal case): one CTA of 256 threads per top-k block.  All window entries
+//  * tile kernel (the normal case): one CTA of 256 to 1024 threads per top-k block.  All window entries
 //    of the block are staged in shared memory, the touched positions are numbered through a
 //    bitmap + prefix popcount, the two moments are accumulated in compact arrays (one slot per
 //    touched position, row after row so that the float sums are reproducible), turned into the
 //    update, and the block is then streamed in chunks against a small dense copy of the update.
-//    Shared memory per CTA is ~44 KB for m = 10, k = 1 %, so five CTAs share an SM and one CTA's
+//    Shared memory per CTA is ~48 KB for m = 10, k = 1 %, so two to four CTAs share an SM and one CTA's
 //    window phase overlaps the others' streaming.
 //  * wide kernel (window too large for the compact arrays, e.g. m = 20 with k = 5 %): one CTA per
 //    sub-range of a block with dense accumulators (window.cuh).
@@ -138,15 +138,7 @@ template <> struct RawOctet<uint16_t> {
 };
 
 // Where the streaming loop gets the update of octet o (8 consecutive elements of the range) from.
-struct NoU {                    // no update: the stream only applies the weight decay
-    static constexpr bool has_u = false;
-    __device__ __forceinline__ void load(int, float (&v)[8]) const {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = 0.0f;
-    }
-};
 struct DenseU {                 // a dense float array in shared memory, 16-byte aligned
-    static constexpr bool has_u = true;
     const float* u;
     __device__ __forceinline__ void load(int o, float (&v)[8]) const {
         const float4 a = reinterpret_cast<const float4*>(u + o * 8)[0], b = reinterpret_cast<const float4*>(u + o * 8)[1];
@@ -155,7 +147,6 @@ struct DenseU {                 // a dense float array in shared memory, 16-byte
     __device__ __forceinline__ void load_warp(int o, bool on, float (&v)[8]) const { if (on) load(o, v); }
 };
 struct SparseU {                // touched positions as a bitmap, their updates compact in slot order
-    static constexpr bool has_u = true;
     const uint32_t* bitmap;     // bit i of the range set <=> position i touched
     const uint16_t* prefix;     // touched positions in lower bitmap words
     const float2* mv;           // .x = update of the slot
@@ -177,7 +168,6 @@ struct SparseU {                // touched positions as a bitmap, their updates 
 // consecutive slots, are scattered into a dense array of the warp's own (a look-up per element through the bitmap was
 // a quarter of the streams' instructions).
 struct WarpU {
-    static constexpr bool has_u = true;
     const uint32_t* bitmap;
     const uint16_t* prefix;
     const uint16_t* spos;       // position of each slot
@@ -251,13 +241,6 @@ __device__ __forceinline__ void stream_range(const mab_tensor& T, const WindowAr
     }
     const float decay = T.decay_f32, neg_lr = T.neg_lr_f32;
     const bool do_decay = T.weight_decay > 0.0;
-    if (ALPHA == 0 && !USrc::has_u && !vec) {                // the decay of a misaligned tensor
-        if (do_decay) {
-#pragma unroll 4
-            for (int i = threadIdx.x; i < len; i += NT) Elem<TP>::store(p, i, __fmul_rn(Elem<TP>::load(p, i), decay));
-        }
-        return;
-    }
     if (ALPHA == 0) {
         const float2 decay2 = make_float2(decay, decay), neg_lr2 = make_float2(neg_lr, neg_lr);
         constexpr int B = (sizeof(TP) == 2) ? 4 : 2;          // octets per thread and batch
@@ -280,11 +263,11 @@ __device__ __forceinline__ void stream_range(const mab_tensor& T, const WindowAr
                     float pv[8], u[8];
                     cur[i].unpack(pv);
                     src.load(o, u);
-                    if (USrc::has_u && probing) {
+                    if (probing) {
 #pragma unroll
                         for (int e = 0; e < 8; ++e) { pr.sum_u2 = fmaf(u[e], u[e], pr.sum_u2); pr.zeros_u += (u[e] == 0.0f) ? 1 : 0; }
                     }
-                    update_octet<TP, USrc::has_u>(pv, u, do_decay, decay2, neg_lr2);
+                    update_octet<TP>(pv, u, do_decay, decay2, neg_lr2);
                     Octet<TP>::store(p + o * 8, pv, true, 8);
                 }
             }
@@ -297,11 +280,11 @@ __device__ __forceinline__ void stream_range(const mab_tensor& T, const WindowAr
             float pv[8], u[8];
             Octet<TP>::load(p + o * 8, pv, false, n);
             src.load(o, u);
-            if (USrc::has_u && probing) {
+            if (probing) {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) if (e < n) { pr.sum_u2 = fmaf(u[e], u[e], pr.sum_u2); pr.zeros_u += (u[e] == 0.0f) ? 1 : 0; }
             }
-            update_octet<TP, USrc::has_u>(pv, u, do_decay, decay2, neg_lr2);
+            update_octet<TP>(pv, u, do_decay, decay2, neg_lr2);
             Octet<TP>::store(p + o * 8, pv, false, n);
         }
         return;
@@ -620,14 +603,14 @@ __device__ __forceinline__ int window_tile_moments(const mab_tensor& T, int blk,
     __syncthreads();
     MAB_BTICK(1);
     // 3. number them: prefix[word] = touched positions in words below
-    constexpr int WPT = WT_WORDS / NT;
+    constexpr int WPT = (WT_WORDS + NT - 1) / NT;
     int cnt[WPT], local = 0;
 #pragma unroll
-    for (int i = 0; i < WPT; ++i) { cnt[i] = __popc(w.bitmap[t * WPT + i]); local += cnt[i]; }
+    for (int i = 0; i < WPT; ++i) { cnt[i] = t * WPT + i < WT_WORDS ? __popc(w.bitmap[t * WPT + i]) : 0; local += cnt[i]; }
     int touched;
     int run = block_exclusive_scan(local, s_scan, touched);
 #pragma unroll
-    for (int i = 0; i < WPT; ++i) { w.prefix[t * WPT + i] = (uint16_t)run; run += cnt[i]; }
+    for (int i = 0; i < WPT; ++i) { if (t * WPT + i < WT_WORDS) w.prefix[t * WPT + i] = (uint16_t)run; run += cnt[i]; }
     __syncthreads();
     MAB_BTICK(2);
     // 4. positions -> slots (in place), then accumulate row after row
@@ -700,6 +683,33 @@ __device__ __forceinline__ int window_tile_moments(const mab_tensor& T, int blk,
     return touched;
 }
 
+// p <- round_p(p * decay) on p[0, len), by the NT threads of the CTA.  Out of line: inline, at both places that call it, it cost 360 bytes of spills.
+template <typename TP, int NT>
+__device__ __noinline__ void decay_tile(TP* p, int len, float decay) {
+    const float2 decay2 = make_float2(decay, decay), zero2 = make_float2(0.0f, 0.0f);
+    int done = 0;
+    if (aligned16(p)) {
+        constexpr int B = sizeof(TP) == 2 ? 4 : 2;           // octets a thread has in flight
+        const int full = len >> 3;
+        for (int o0 = threadIdx.x; o0 < full; o0 += NT * B) {
+            RawOctet<TP> x[B];
+#pragma unroll
+            for (int i = 0; i < B; ++i) if (o0 + NT * i < full) x[i].load(p + (o0 + NT * i) * 8);
+#pragma unroll
+            for (int i = 0; i < B; ++i)
+                if (o0 + NT * i < full) {
+                    float v[8], u[8];
+                    x[i].unpack(v);
+                    update_octet<TP, false>(v, u, true, decay2, zero2);
+                    Octet<TP>::store(p + (o0 + NT * i) * 8, v, true, 8);
+                }
+        }
+        done = full * 8;
+    }
+#pragma unroll 4
+    for (int i = done + threadIdx.x; i < len; i += NT) Elem<TP>::store(p, i, __fmul_rn(Elem<TP>::load(p, i), decay));
+}
+
 template <typename TP, int MODE, int ALPHA, int NT>
 __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units,
                                                  int max_k, const WindowArgs& a, int dense_at = 0) {
@@ -736,8 +746,19 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
                 const int nti = nu < s_first[ti + 1] ? ti : find_tensor(s_first, n_tensors, nu);
                 prefetch_window_rows(tensors[nti], nu - s_first[nti], rows, threadIdx.x);
             }
-            // this block's parameters travel to L2 while the window is worked on
-            prefetch_l2<NT>(reinterpret_cast<uintptr_t>(reinterpret_cast<TP*>(T.param) + blk_base), (int64_t)n_blk * sizeof(TP));
+            // This block's bf16 parameters travel to L2 while the window is worked on (windows of 10 rows of 5 %, 58 M elements: 230 us, 240 without).
+            // fp32 tiles are not asked for: they are twice as long, only half of their sectors is touched without decay, and with all CTAs' tiles
+            // in L2 some left it before their turn (us, with and without: 29 M elements 50 and 44, with decay 81 and 73, alpha = 0.5 33.5 M 121
+            // and 115).
+            if (sizeof(TP) == 2) prefetch_l2<NT>(reinterpret_cast<uintptr_t>(reinterpret_cast<TP*>(T.param) + blk_base), (int64_t)n_blk * sizeof(TP));
+        }
+        // The weight decay has a pass of its own; where every CTA has one tile it runs while the window's rows are on their way (500 tiles, fp32:
+        // 49.7 us behind the window phases, 45.6 before them; 4000 tiles 291 and 317: there the other tiles hide its latency, and
+        // parameters read early leave L2 again).
+        const bool decaying = MODE == MODE_STEP && ALPHA == 0 && T.weight_decay > 0.0 && !(sizeof(TP) == 2 && decay_is_identity_bf16(T.decay_f32));
+        const bool one_tile = total_units <= (int)gridDim.x;
+        if constexpr (MODE == MODE_STEP && ALPHA == 0) {
+            if (decaying && one_tile) decay_tile<TP, NT>(reinterpret_cast<TP*>(T.param) + blk_base, n_blk, T.decay_f32);
         }
         const int kcnt = (blk < nfull) ? T.k_block_size_many : T.k_block_size_few;
         const bool g_bf16 = (T.grad_dtype == MAB_BF16);
@@ -752,8 +773,8 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
             //    already final.  A thread has UB of its scattered reads in flight (one at a time, a read that waits for
             //    the write before it: a step of 124.4 M elements 499 -> 493 us,
             //    67.1 M with windows of 10 rows of 5 % 556 -> 504).
-            if (T.weight_decay > 0.0) {
-                stream_range<TP, MODE, NT, ALPHA>(T, a, NoU{}, blk_base, n_blk, pr);
+            if (decaying && !one_tile) {
+                decay_tile<TP, NT>(reinterpret_cast<TP*>(T.param) + blk_base, n_blk, T.decay_f32);
                 __syncthreads();                               // the decayed values are read back below
             }
             MAB_BTICK(6);
@@ -806,10 +827,9 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
     if (probing) pr.flush(a.probe);
 }
 
-// NT threads per CTA: 256 while four CTAs fit an SM; windows whose arrays leave room for two CTAs or one get 512 or
-// 1024 threads instead, so that an SM always has 32 warps to hide the latency of the barrier-separated phases.
+// (threads_of gives NT)
 template <typename TP, int MODE, int ALPHA, int NT>
-__global__ void __launch_bounds__(NT, ALPHA == 0 ? 1024 / NT : 3)
+__global__ void __launch_bounds__(NT, ALPHA != 0 ? 768 / NT : NT == 384 ? 3 : 1024 / NT)
 window_tile_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int max_k,
                    int dense_at, const __grid_constant__ WindowArgs a) {
     window_tile_body<TP, MODE, ALPHA, NT>(tensors, n_tensors, total_units, max_k, a, dense_at);
@@ -1036,6 +1056,21 @@ window_wide_single_kernel(const __grid_constant__ mab_tensor t, int total_units,
 
 // ------------------------------------------------------------------------------------ launch
 
+// Threads of a CTA of the tile kernel; `fit`: how many CTAs' arrays fit an SM.  us of this kernel, fp32, 10 rows; the row loop has its
+// prefetching form while a row's entries do not outnumber the threads, and every tile in flight costs L2.
+//   k = 0.5 % (146 entries), 116 M elements: 256 threads 105, 384 108, 512 120.
+//   k = 1 % (291): 256 / 384 / 512 threads, 100 tiles 12.4 / 9.5 / 8.6, 300 tiles 18.8 / 15.5 / 18.6, 1000 55 / 42 / 44, 1500 77 / 61 / 61, 3000 143 / 124 /
+//   118, 4282 201 / 186 / 166; with weight decay 1000 82 / 70 / 73, 4282 292 / 322 / 268; 120 ragged tensors 33 / 30 / 35.
+//   The alpha forms have 80 registers a thread: 256 threads while three CTAs fit (33.5 M elements 121, 384 threads 127), 384 where two do (bf16, 20
+//   rows, 58 M elements 265 with 256, 209), and 512 where one does or an SM has no more than one tile (100 tiles 29 and 18).
+static int threads_of(bool alpha, int fit, int tiles, int max_k, int sms) {
+    if (alpha) return fit < 2 || tiles <= sms ? 512 : fit < 3 ? 384 : 256;
+    if (fit < 2) return 1024;
+    if (tiles <= 2 * sms || fit < 3) return 512;
+    if (max_k <= 256 && fit >= 4) return 256;
+    return max_k <= 384 && tiles <= 10 * sms ? 384 : 512;
+}
+
 // MODE_WRITE_UPDATE: one tensor, passed by value (`single`); MODE_STEP: n_tensors descriptors in device memory.
 // units_tile / units_wide are the unit counts of the two variants; rows * max_k (the largest
 // k_block_size of the launch) decides which one runs.
@@ -1047,12 +1082,14 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
     const int smem_tile = (int64_t)a.rows * max_k <= WT_MAX_ENTRIES ? wt_smem_bytes(a.rows, max_k) : 0;
     if (smem_tile > 0 && smem_tile + 4096 <= device_max_optin_smem()) {
         // the forms with the alpha term: a dense array of 256 floats per warp behind the window's arrays, if it fits
-        const int dense_at = ALPHA != 0 && ((smem_tile + 15) & ~15) + 8 * 1024 + 4096 <= device_max_optin_smem() ? (smem_tile + 15) & ~15 : 0;
-        const int smem = dense_at > 0 ? dense_at + 8 * 1024 : smem_tile;
-        const int per_sm = std::max(1, std::min(8, (227 * 1024) / (smem + 3072)));
+        const int fit = std::max(1, std::min(8, (227 * 1024) / (smem_tile + (ALPHA != 0 ? 8 * 1024 : 0) + 3072)));   // CTAs per SM by their arrays
+        int nt = threads_of(ALPHA != 0, fit, units_tile, max_k, sms);
+        if (ALPHA != 0 && ((smem_tile + 15) & ~15) + nt * 32 + 4096 > device_max_optin_smem()) nt = 256;
+        const int dense = ALPHA != 0 ? nt * 32 : 0;
+        const int dense_at = ALPHA != 0 && ((smem_tile + 15) & ~15) + dense + 4096 <= device_max_optin_smem() ? (smem_tile + 15) & ~15 : 0;
+        const int smem = dense_at > 0 ? dense_at + dense : smem_tile;
+        const int per_sm = std::max(1, std::min(ALPHA != 0 ? 768 / nt : nt == 384 ? 3 : 1024 / nt, (227 * 1024) / (smem + 3072)));   // (as in __launch_bounds__)
         const int grid = (int)std::min<int64_t>(units_tile, (int64_t)sms * per_sm);
-        // fewer resident CTAs (large windows) get more threads each; the forms with the alpha term keep 256
-        const int nt = (ALPHA != 0 || per_sm >= 4) ? 256 : per_sm >= 2 ? 512 : 1024;
         auto run = [&](auto kern, int threads) -> int {
             MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
             if constexpr (MODE == MODE_WRITE_UPDATE) kern<<<grid, threads, smem, s>>>(*single, units_tile, max_k, a);
@@ -1063,13 +1100,17 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
         if constexpr (MODE == MODE_WRITE_UPDATE) {
             if (nt == 1024) rc = run(window_tile_single_kernel<TP, MODE, 0, 1024>, 1024);
             else if (nt == 512) rc = run(window_tile_single_kernel<TP, MODE, 0, 512>, 512);
+            else if (nt == 384) rc = run(window_tile_single_kernel<TP, MODE, 0, 384>, 384);
             else rc = run(window_tile_single_kernel<TP, MODE, 0, 256>, 256);
         } else if constexpr (ALPHA == 0) {
             if (nt == 1024) rc = run(window_tile_kernel<TP, MODE, 0, 1024>, 1024);
             else if (nt == 512) rc = run(window_tile_kernel<TP, MODE, 0, 512>, 512);
+            else if (nt == 384) rc = run(window_tile_kernel<TP, MODE, 0, 384>, 384);
             else rc = run(window_tile_kernel<TP, MODE, 0, 256>, 256);
         } else {
-            rc = run(window_tile_kernel<TP, MODE, ALPHA, 256>, 256);
+            if (nt == 512) rc = run(window_tile_kernel<TP, MODE, ALPHA, 512>, 512);
+            else if (nt == 384) rc = run(window_tile_kernel<TP, MODE, ALPHA, 384>, 384);
+            else rc = run(window_tile_kernel<TP, MODE, ALPHA, 256>, 256);
         }
         if (rc) return rc;
     } else {
