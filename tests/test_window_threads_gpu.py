@@ -15,7 +15,7 @@ def test_many_tiles_equal_single_tiles(rows, k, per_sm, alpha, weight_decay, dty
     from ista_daslab_optimizers_b200.compat import ista_daslab_cuda_tools as tools
     # as many tiles as the rule's lines lie at, and one more: full ones, and a short one with an element more than whole octets
     sizes = ((per_sm * tools.get_sm_count() - 1) * DBS, DBS, DBS // 2 + 9)
-    hyper = dict(m=rows, lr=1e-3, k_init=(k - 0.5) / DBS, alpha=alpha, weight_decay=weight_decay)
+    hyper = dict(m=rows, lr=1e-3, quant_block_size=64, k_init=(k - 0.5) / DBS, alpha=alpha, weight_decay=weight_decay)
     gen = torch.Generator(device='cuda').manual_seed(k)
     whole = [torch.nn.Parameter(torch.empty(n, dtype=dtype, device='cuda').normal_(0.0, 0.02, generator=gen)) for n in sizes]
     alone = [torch.nn.Parameter(p.detach()[at:at + DBS].clone()) for p in whole[:2] for at in (0, (p.numel() // DBS - 1) * DBS)]
