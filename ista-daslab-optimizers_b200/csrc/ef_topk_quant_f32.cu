@@ -379,7 +379,10 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
             const mab_tensor& N = tensors[nti];
             const int64_t nbase = (int64_t)(nu - s_first[nti]) * N.d_block_size;
             const int64_t nn = min((int64_t)N.d_block_size, N.d - nbase);
-            prefetch_l2<F_NT>(reinterpret_cast<uintptr_t>(reinterpret_cast<const float*>(N.grad) + nbase), nn * 4);
+            // Of the gradient the first three eighths: what the threads load into registers (28 %) and a little more.  The rest is the copy engine's,
+            // whose latency hides; asked for as well, it drove lines out of L2 before their turn (124.4 M elements, us a launch: all of it 274,
+            // 5/8 267, 1/2 267, 3/8 264, 5/16 265, nothing 272; 67 M with k = 5 % 199, 3/8 193).
+            prefetch_l2<F_NT>(reinterpret_cast<uintptr_t>(reinterpret_cast<const float*>(N.grad) + nbase), nn * 3 / 2);
             if (warp < 3) {                                          // codes and statistics: a warp each
                 const uintptr_t pb = warp == 0 ? reinterpret_cast<uintptr_t>(N.error + (nbase >> 1))
                                    : reinterpret_cast<uintptr_t>((warp == 1 ? N.min_vals : N.max_vals) + (nbase >> qshift));
