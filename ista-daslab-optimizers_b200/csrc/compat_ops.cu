@@ -3,7 +3,6 @@
 // geometries faster; these are the general path and the operator-level drop-in surface.
 #include "common.cuh"
 #include "select.cuh"
-#include "select_fast.cuh"
 #include "codec_fast.cuh"
 
 namespace mab {
@@ -256,49 +255,6 @@ quant_stats_kernel(int64_t d, int64_t qbs, int64_t nblocks, uint16_t* __restrict
     }
 }
 
-// One CTA per top-k block: keys to registers, exact k-th key (through the candidates of select_fast.cuh, by
-// bisection where that does not apply), ordered emission.
-template <typename T>
-__global__ void __launch_bounds__(SEL_THREADS, 1)
-block_topk_kernel(int64_t d, int dbs, int nfull, int k_many, int k_few, const T* __restrict__ x,
-                  int16_t* __restrict__ out) {
-    extern __shared__ __align__(16) unsigned char topk_raw[];            // [SelectSmem | FastSelSmem]
-    SelectSmem& sm = *reinterpret_cast<SelectSmem*>(topk_raw);
-    FastSelSmem& fs = *reinterpret_cast<FastSelSmem*>(topk_raw + sizeof(SelectSmem));
-    const int nblocks = nfull + (k_few > 0 ? 1 : 0);
-    int guess = 0;
-    for (int blk = blockIdx.x; blk < nblocks; blk += gridDim.x) {
-        const int64_t base = (int64_t)blk * dbs;
-        const int n = (int)min((int64_t)dbs, d - base);
-        const int k = (blk < nfull) ? k_many : k_few;
-        const bool vec = (reinterpret_cast<uintptr_t>(x + base) & 15) == 0;
-        float key[SEL_OCTETS][8], omax[SEL_OCTETS];
-#pragma unroll
-        for (int j = 0; j < SEL_OCTETS; ++j) {
-            const int o = j * SEL_THREADS + (int)threadIdx.x;
-            if (vec && o * 8 + 8 <= n) {
-                XOctet<T>::load(x + base + o * 8, key[j]);
-            } else {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) key[j][e] = (o * 8 + e < n) ? Elem<T>::load(x, base + o * 8 + e) : 0.0f;
-            }
-            omax[j] = 0.0f;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) omax[j] = fmaxf(omax[j], fabsf(key[j][e]));
-        }
-        int n_cand, oct_slot[SEL_OCTETS];
-        bool compact_octets;
-        if (!fast_select(key, omax, n, k, guess, sm, fs, n_cand, oct_slot, compact_octets, sizeof(T) == 2 ? 16 : 0)) {
-            int need;
-            const int T_key = block_kth_key_bisect(key, k, sm, need);
-            publish_masks(key, T_key, sm);
-            resolve_selection(need, sm);
-        }
-        emit_indices(sm, out + (int64_t)blk * k_many);
-        __syncthreads();
-    }
-}
-
 static int grid_for(int64_t work_items, int threads) {
     int64_t g = ceil_div64(work_items, threads);
     const int64_t cap = (int64_t)device_sm_count() * 16;
@@ -450,16 +406,5 @@ extern "C" int mab_block_topk(int64_t d, int64_t dbs, int64_t k_many, int64_t k_
     if (device_sm_count() < 0) return MAB_ERR_CUDA;
     const int64_t nblocks = nfull + (k_few > 0 ? 1 : 0);
     if (nblocks == 0) return MAB_OK;
-    const int grid = (int)std::min<int64_t>(nblocks, (int64_t)device_sm_count() * 4);
-    cudaStream_t s = (cudaStream_t)stream;
-    const int smem = (int)(sizeof(SelectSmem) + sizeof(FastSelSmem));
-    if (x_dtype == MAB_F32) {
-        MAB_CUDA_TRY(cudaFuncSetAttribute(block_topk_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        block_topk_kernel<float><<<grid, SEL_THREADS, smem, s>>>(d, (int)dbs, (int)nfull, (int)k_many, (int)k_few, (const float*)x, out);
-    } else {
-        MAB_CUDA_TRY(cudaFuncSetAttribute(block_topk_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        block_topk_kernel<uint16_t><<<grid, SEL_THREADS, smem, s>>>(d, (int)dbs, (int)nfull, (int)k_many, (int)k_few, (const uint16_t*)x, out);
-    }
-    MAB_CHECK_LAUNCH("block_topk");
-    return MAB_OK;
+    return launch_block_topk(d, (int)dbs, (int)nfull, (int)k_many, (int)k_few, x, x_dtype, out, (cudaStream_t)stream);
 }

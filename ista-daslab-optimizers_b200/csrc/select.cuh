@@ -155,4 +155,7 @@ __device__ __forceinline__ void emit_indices(const SelectSmem& sm, int16_t* out)
     }
 }
 
+// block_topk.cu
+int launch_block_topk(int64_t d, int dbs, int nfull, int k_many, int k_few, const void* x, int dtype, int16_t* out, cudaStream_t s);
+
 }  // namespace mab

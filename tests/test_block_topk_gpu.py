@@ -1,0 +1,55 @@
+"""block_topk by itself, where its routes change: blocks and one more than there are SMs, blocks around an octet, k around the acceptance window's
+change and beyond the octets, more equal magnitudes than the candidate list or the direct ranking holds, infinities and NaN, x off alignment."""
+import pytest
+import torch
+
+from ista_daslab_optimizers_b200 import synthetic as S
+
+pytestmark = pytest.mark.gpu
+
+DBS = 29056
+
+
+def _expected(x, k_many, k_few):
+    key = x.float().abs()
+    key[key.isnan()] = -1.0
+    rows = []
+    for at in range(0, x.numel(), DBS):
+        n = min(DBS, x.numel() - at)
+        k = k_many if n == DBS else k_few
+        rows.append(torch.sort(key[at:at + n], descending=True, stable=True).indices[:k].sort().values)
+    return torch.cat(rows).to(torch.int16)
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize('kind,k,tail,skip', [
+    ('normal', 291, 0, 0), ('normal', 291, 1, 0), ('normal', 1024, 8191, 1), ('normal', 1025, 8192, 2), ('normal', 3632, 15, 0), ('normal', 3633, 16, 3),
+    ('ties', 1453, 17, 0), ('ties', 33, 4099, 0), ('scales', 291, 777, 4), ('inf', 291, 4096, 0), ('inf', 1, 9, 0), ('nan', 291, 4097, 0),
+    ('zeros', 291, 100, 0), ('cluster', 600, 64, 0)])
+def test_block_topk_routes(dtype, kind, k, tail, skip):
+    from ista_daslab_optimizers_b200 import _native as N
+    for full in (2, N.get_sm_count(), N.get_sm_count() + 1):
+        d, k_few = full * DBS + tail, max(1, tail // 7) if tail else 0
+        x = S.normal_tensor(13, full, d, 1e-3)
+        if kind == 'ties':
+            x = (x * 2000.0).round() / 2000.0
+        elif kind == 'scales':                           # no block's bound fits the next one
+            x *= 2.0 ** ((torch.arange(d) // DBS * 5) % 13 - 6)
+        elif kind == 'inf':
+            x[5::977] = float('inf')
+            x[9::1203] = float('-inf')
+        elif kind == 'nan':
+            x[3::16] = float('nan')
+            x[DBS:DBS + 512] = float('nan')
+        elif kind == 'zeros':
+            x[:DBS] = 0.0
+            x[DBS:2 * DBS] = 0.0
+            x[DBS + 11:2 * DBS:4001] = 1e-3
+        elif kind == 'cluster':
+            x[1000:1000 + k] *= 300.0
+        x = x.to(dtype)
+        g = torch.empty(d + skip, dtype=dtype, device='cuda')[skip:].copy_(x)
+        out = torch.full((full * k + k_few + 8,), -7, dtype=torch.int16, device='cuda')
+        N.block_topk(d, DBS, k, k_few, g, out[:full * k + k_few])
+        assert torch.equal(out[:full * k + k_few].cpu(), _expected(x, k, k_few)), full
+        assert (out[full * k + k_few:] == -7).all()
