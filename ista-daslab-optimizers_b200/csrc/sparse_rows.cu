@@ -15,7 +15,9 @@ namespace mab {
 
 constexpr int SPR_SR = 14592;         // elements of a block one CTA accumulates at a time (57 * 256): a 29 056-element block is two ranges
 constexpr int SPR_THREADS = 384;      // three CTAs of 58 KB of accumulators per SM, 56 registers a thread (512 threads of 40 spill: 98 us, now 78)
-constexpr int SPR_AHEAD = 8;          // rows whose entries a thread has in flight
+// Rows whose entries a thread fetches at once, while it adds those fetched before; (row, round) pairs of long rows (25.6 M elements, 32 rows of
+// 5 %: 6 189 us, 8 198; of 1 %: 6 66.6, 8 65.4).
+template <bool LONG> constexpr int SPR_AHEAD = LONG ? 6 : 8;
 
 constexpr int SP_THREADS = 512;
 constexpr int SP_CLUSTER = 8;         // CTAs per row (the portable cluster size) ...
@@ -127,18 +129,41 @@ sparse_rows_dot_parts_kernel(int64_t k, int64_t dbs, int kbs, int nfull, int k_f
     dot_sum<CTAS>(acc, s_part, s_cta, out + r);
 }
 
+// A thread's entry of a row: its position (negative: none) and its value.
+template <typename TV> struct Entry;
+template <> struct Entry<uint16_t> {
+    uint32_t e;
+    __device__ __forceinline__ void get(const int16_t* I, const void* V, int64_t at, bool on) {
+        e = on ? (uint32_t)(uint16_t)I[at] | ((uint32_t)reinterpret_cast<const uint16_t*>(V)[at] << 16) : 0xFFFFu;
+    }
+    __device__ __forceinline__ int pos() const { return (int16_t)(e & 0xFFFFu); }
+    __device__ __forceinline__ float val() const { return __uint_as_float(e & 0xFFFF0000u); }
+};
+template <> struct Entry<float> {
+    int p;
+    float v;
+    __device__ __forceinline__ void get(const int16_t* I, const void* V, int64_t at, bool on) {
+        p = on ? (int)I[at] : -1;
+        v = on ? reinterpret_cast<const float*>(V)[at] : 0.0f;
+    }
+    __device__ __forceinline__ int pos() const { return p; }
+    __device__ __forceinline__ float val() const { return v; }
+};
+
 // out[e] += sum_r M[r] * V[r, j] over the entries (r, j) that address e: one CTA per sub-range of a top-k block
 // with a dense fp32 accumulator in shared memory; rows are added in row order (positions are unique inside a
-// row, so a row needs no atomics, but a barrier).  Bound by the chain of rows: a thread fetches its entries of
-// SPR_AHEAD rows at once, so that a row costs a shared-memory update and a barrier (25.6 M elements, 32 rows of 1 %: 232 us
-// with one load latency per row and four walks over a block's entries, 78 now).  LONG: blocks with more entries than the CTA
-// has threads.
+// row, so a row needs no atomics, but a barrier).  Bound by the chain of rows: a thread fetches its entries of SPR_AHEAD rows at once,
+// and the next ones before it adds these, so that a row costs a shared-memory update and a barrier (25.6 M elements, 32 rows of 1 %:
+// 232 us with one load latency per row and four walks over a block's entries, 75 with one per eight rows, 65 with the next eight ahead).
+// LONG: blocks with more entries than the CTA has threads.
 template <typename TO, typename TV, bool LONG>
 __global__ void __launch_bounds__(SPR_THREADS, 3)
 sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int nfull, int k_few, const float* __restrict__ M,
                            const int16_t* __restrict__ I, const void* __restrict__ V, TO* __restrict__ out, int total_units) {
     extern __shared__ __align__(16) float acc[];
+    __shared__ float s_M[MAB_MAX_WINDOW];
     const int t = threadIdx.x;
+    for (int i = t; i < rows; i += SPR_THREADS) s_M[i] = M[i];
     const int subs_per_block = (dbs + SPR_SR - 1) / SPR_SR;
     for (int unit = blockIdx.x; unit < total_units; unit += gridDim.x) {
         int blk = unit / subs_per_block, sub = unit - blk * subs_per_block;
@@ -150,55 +175,41 @@ sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int
         const int len = min(SPR_SR, n_blk - s0);
         const int64_t row0 = (int64_t)blk * kbs;
         for (int i = t; i < len; i += SPR_THREADS) acc[i] = 0.0f;
-        if constexpr (LONG) {
-            // several entries of a row per thread: (row, round) pairs in row order, SPR_AHEAD of them fetched at once
-            const int rounds = (kcnt + SPR_THREADS - 1) / SPR_THREADS, pairs = rows * rounds;
-            int r = 0, c = 0;                                    // the pair to fetch next ...
-            int round_now = 0;                                   // ... and the round of the pair to add next
-            for (int p0 = 0; p0 < pairs; p0 += SPR_AHEAD) {
-                int pos[SPR_AHEAD];
-                float val[SPR_AHEAD];
+        // (row, round) pairs in row order, SPR_AHEAD of them fetched at once, and those after them before the current ones are added
+        const int rounds = LONG ? (kcnt + SPR_THREADS - 1) / SPR_THREADS : 1, pairs = rows * rounds;
+        int fr = 0, fc = 0;                                      // the pair to fetch next ...
+        int r = 0, c = 0;                                        // ... and to add next
+        auto fetch = [&](Entry<TV> (&e)[SPR_AHEAD<LONG>]) {
 #pragma unroll
-                for (int i = 0; i < SPR_AHEAD; ++i) {
-                    const int j = c * SPR_THREADS + t;
-                    const bool on = r < rows && j < kcnt;
-                    const int64_t at = (int64_t)r * k + row0 + j;
-                    pos[i] = on ? (int)I[at] - s0 : -1;
-                    val[i] = on ? __fmul_rn(M[r], load_value<TV>(V, at)) : 0.0f;
-                    if (++c == rounds) { c = 0; ++r; }
-                }
+            for (int i = 0; i < SPR_AHEAD<LONG>; ++i) {
+                const int j = fc * SPR_THREADS + t;
+                e[i].get(I, V, (int64_t)fr * k + row0 + j, fr < rows && j < kcnt);
+                if (!LONG || ++fc == rounds) { fc = 0; ++fr; }
+            }
+        };
+        auto add = [&](const Entry<TV> (&e)[SPR_AHEAD<LONG>]) {
 #pragma unroll
-                for (int i = 0; i < SPR_AHEAD; ++i) {
-                    if (p0 + i < pairs) {                        // uniform
-                        if (round_now == 0) __syncthreads();     // the row before (or the clearing) is done
-                        if (pos[i] >= 0 && pos[i] < len) acc[pos[i]] = __fadd_rn(acc[pos[i]], val[i]);
-                        if (++round_now == rounds) round_now = 0;
-                    }
+            for (int i = 0; i < SPR_AHEAD<LONG>; ++i) {
+                if (r < rows) {                                  // uniform
+                    if (c == 0) __syncthreads();                 // the row before (or the clearing) is done
+                    const int pos = e[i].pos() - s0;
+                    if (pos >= 0 && pos < len) acc[pos] = __fadd_rn(acc[pos], __fmul_rn(s_M[r], e[i].val()));
+                    if (!LONG || ++c == rounds) { c = 0; ++r; }
                 }
             }
-        } else {
-            for (int r0 = 0; r0 < rows; r0 += SPR_AHEAD) {
-                int pos[SPR_AHEAD];
-                float val[SPR_AHEAD];
-#pragma unroll
-                for (int i = 0; i < SPR_AHEAD; ++i) {
-                    const bool on = r0 + i < rows && t < kcnt;
-                    const int64_t at = (int64_t)(r0 + i) * k + row0 + t;
-                    pos[i] = on ? (int)I[at] - s0 : -1;
-                    val[i] = on ? __fmul_rn(M[r0 + i], load_value<TV>(V, at)) : 0.0f;
-                }
-#pragma unroll
-                for (int i = 0; i < SPR_AHEAD; ++i) {
-                    if (r0 + i < rows) {                             // uniform
-                        __syncthreads();                             // the row before (or the clearing) is done
-                        if (pos[i] >= 0 && pos[i] < len) acc[pos[i]] = __fadd_rn(acc[pos[i]], val[i]);
-                    }
-                }
-            }
+        };
+        Entry<TV> a[SPR_AHEAD<LONG>], b[SPR_AHEAD<LONG>];
+        fetch(a);
+        for (int p = 0; p < pairs; p += 2 * SPR_AHEAD<LONG>) {
+            fetch(b);
+            add(a);
+            fetch(a);
+            add(b);
         }
         __syncthreads();
         TO* o = out + blk_base + s0;
         const int whole = ((reinterpret_cast<uintptr_t>(o) & 15) == 0) ? len / SPR_VEC<TO> : 0;
+#pragma unroll 4
         for (int i = t; i < whole; i += SPR_THREADS) add_vector(o + i * SPR_VEC<TO>, acc + i * SPR_VEC<TO>);
         for (int i = whole * SPR_VEC<TO> + t; i < len; i += SPR_THREADS)
             Elem<TO>::store(o, i, __fadd_rn(Elem<TO>::load(o, i), acc[i]));
