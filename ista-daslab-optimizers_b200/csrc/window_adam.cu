@@ -757,6 +757,15 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
         // parameters read early leave L2 again).
         const bool decaying = MODE == MODE_STEP && ALPHA == 0 && T.weight_decay > 0.0 && !(sizeof(TP) == 2 && decay_is_identity_bf16(T.decay_f32));
         const bool one_tile = total_units <= (int)gridDim.x;
+        if constexpr (MODE == MODE_WRITE_UPDATE) {
+            // zeros everywhere now, the updates of the touched positions behind the window phases: the stores drain meanwhile (25.6 M fp32
+            // elements 36 us with a look-up through the bitmap for every element at the end, 34.5 so; bf16 30 and 25.5)
+            TP* const p = reinterpret_cast<TP*>(T.param) + blk_base;
+            constexpr int VEC = 16 / (int)sizeof(TP);
+            const int whole = aligned16(p) ? n_blk / VEC : 0;
+            for (int i = threadIdx.x; i < whole; i += NT) reinterpret_cast<uint4*>(p)[i] = make_uint4(0u, 0u, 0u, 0u);
+            for (int i = whole * VEC + threadIdx.x; i < n_blk; i += NT) p[i] = 0;
+        }
         if constexpr (MODE == MODE_STEP && ALPHA == 0) {
             if (decaying && one_tile) decay_tile<TP, NT>(reinterpret_cast<TP*>(T.param) + blk_base, n_blk, T.decay_f32);
         }
@@ -800,6 +809,12 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
                 }
             }
             if (probing && t == 0) pr.zeros_u += n_blk;        // every position without a non-zero update is a zero of u
+        } else if constexpr (MODE == MODE_WRITE_UPDATE) {
+            TP* const p = reinterpret_cast<TP*>(T.param) + blk_base;
+            for (int s = t; s < touched; s += NT) {
+                const float2 acc = w.mv[s];
+                Elem<TP>::store(p, w.spos[s], adam_update_fast(acc.x, acc.y, inv_bc1, inv_bc2, a.eps));
+            }
         } else {
             // 5. moments -> update (rounded to the gradient's element type), slot by slot
             for (int s = t; s < touched; s += NT) {
@@ -809,13 +824,8 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
             __syncthreads();
             MAB_BTICK(5);
             // 6. stream the whole block; each octet finds its updates through the bitmap
-            if constexpr (ALPHA != 0) {
-                const WarpU src{w.bitmap, w.prefix, w.spos, w.mv, touched, dense};
-                stream_range<TP, MODE, NT, ALPHA>(T, a, src, blk_base, n_blk, pr);
-            } else {
-                const SparseU src{w.bitmap, w.prefix, w.mv};
-                stream_range<TP, MODE, NT, ALPHA>(T, a, src, blk_base, n_blk, pr);
-            }
+            const WarpU src{w.bitmap, w.prefix, w.spos, w.mv, touched, dense};
+            stream_range<TP, MODE, NT, ALPHA>(T, a, src, blk_base, n_blk, pr);
         }
         MAB_BTICK(7);
         __syncthreads();                                       // everything is reused by the next unit
@@ -1061,12 +1071,14 @@ window_wide_single_kernel(const __grid_constant__ mab_tensor t, int total_units,
 //   k = 0.5 % (146 entries), 116 M elements: 256 threads 105, 384 108, 512 120.
 //   k = 1 % (291): 256 / 384 / 512 threads, 100 tiles 12.4 / 9.5 / 8.6, 300 tiles 18.8 / 15.5 / 18.6, 1000 55 / 42 / 44, 1500 77 / 61 / 61, 3000 143 / 124 /
 //   118, 4282 201 / 186 / 166; with weight decay 1000 82 / 70 / 73, 4282 292 / 322 / 268; 120 ragged tensors 33 / 30 / 35.
+//   The operator that writes every position's update: 384 (60 M elements k = 1 % 75, 256 and 512 threads 79; 0.5 % 59, 256 73, 512 67).
 //   The alpha forms have 80 registers a thread: 256 threads while three CTAs fit (33.5 M elements 121, 384 threads 127), 384 where two do (bf16, 20
 //   rows, 58 M elements 265 with 256, 209), and 512 where one does or an SM has no more than one tile (100 tiles 29 and 18).
-static int threads_of(bool alpha, int fit, int tiles, int max_k, int sms) {
+static int threads_of(bool write, bool alpha, int fit, int tiles, int max_k, int sms) {
     if (alpha) return fit < 2 || tiles <= sms ? 512 : fit < 3 ? 384 : 256;
     if (fit < 2) return 1024;
     if (tiles <= 2 * sms || fit < 3) return 512;
+    if (write) return 384;
     if (max_k <= 256 && fit >= 4) return 256;
     return max_k <= 384 && tiles <= 10 * sms ? 384 : 512;
 }
@@ -1083,7 +1095,7 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
     if (smem_tile > 0 && smem_tile + 4096 <= device_max_optin_smem()) {
         // the forms with the alpha term: a dense array of 256 floats per warp behind the window's arrays, if it fits
         const int fit = std::max(1, std::min(8, (227 * 1024) / (smem_tile + (ALPHA != 0 ? 8 * 1024 : 0) + 3072)));   // CTAs per SM by their arrays
-        int nt = threads_of(ALPHA != 0, fit, units_tile, max_k, sms);
+        int nt = threads_of(MODE == MODE_WRITE_UPDATE, ALPHA != 0, fit, units_tile, max_k, sms);
         if (ALPHA != 0 && ((smem_tile + 15) & ~15) + nt * 32 + 4096 > device_max_optin_smem()) nt = 256;
         const int dense = ALPHA != 0 ? nt * 32 : 0;
         const int dense_at = ALPHA != 0 && ((smem_tile + 15) & ~15) + dense + 4096 <= device_max_optin_smem() ? (smem_tile + 15) & ~15 : 0;
