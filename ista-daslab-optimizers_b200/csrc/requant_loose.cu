@@ -40,14 +40,18 @@ template <> struct ResidualOctet<uint16_t> {
     }
 };
 
-template <typename TG>
-__global__ void __launch_bounds__(RQ_THREADS, 4)
+// CTAs per SM the registers are sized for, twice that many in the grid.  BIG: blocks at least as long as the longest tile, of which a tile touches two.
+// bf16, 218 M elements, blocks of 100 000: 111 us with four (64 registers), 102 with five (48), 103 with six (40, spills); blocks of 1000, 58 M
+// with kernel A: 154 with four, 156 with five; fp32 spills more: 294, 297.
+template <typename TG, bool BIG> constexpr int rq_ctas = sizeof(TG) == 2 && BIG ? 5 : 4;
+
+template <typename TG, bool BIG>
+__global__ void __launch_bounds__(RQ_THREADS, rq_ctas<TG, BIG>)
 requant_loose_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, LooseArgs la) {
     __shared__ int s_first[WIN_MAX_TENSORS + 1];
     for (int i = threadIdx.x; i < n_tensors; i += RQ_THREADS) s_first[i] = tensors[i].first_unit_a;
     if (threadIdx.x == 0) s_first[n_tensors] = total_units;
     __syncthreads();
-    const bool big = la.qbs >= 32768;
     int ti = 0;
     for (int unit = blockIdx.x; unit < total_units; unit += gridDim.x) {
         if (unit >= s_first[ti + 1] || unit < s_first[ti]) ti = find_tensor(s_first, n_tensors, unit);
@@ -72,7 +76,7 @@ requant_loose_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int 
         // the block's first element
         auto enter_block = [&](int o) {
             const int r = rem0 + o * 8;
-            const int qi = loose_block(r, la.qbs, big);
+            const int qi = loose_block(r, la.qbs, BIG);
             if (qi != cached) {
                 cached = qi;
                 mn_b = f32_to_bf16_bits_rne(ord_value(__ldg(st_min + qi)));
@@ -132,9 +136,13 @@ requant_loose_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int 
 
 int launch_requant_loose(const mab_tensor* dev_tensors, int n_tensors, int total_units, int grad_dtype,
                          const LooseArgs& la, cudaStream_t s) {
-    const int grid = (int)std::min<int64_t>(total_units, (int64_t)device_sm_count() * 8);
-    if (grad_dtype == MAB_F32) requant_loose_kernel<float><<<grid, RQ_THREADS, 0, s>>>(dev_tensors, n_tensors, total_units, la);
-    else requant_loose_kernel<uint16_t><<<grid, RQ_THREADS, 0, s>>>(dev_tensors, n_tensors, total_units, la);
+    auto run = [&](auto kern, int ctas) {
+        const int grid = (int)std::min<int64_t>(total_units, (int64_t)device_sm_count() * ctas);
+        kern<<<grid, RQ_THREADS, 0, s>>>(dev_tensors, n_tensors, total_units, la);
+    };
+    const bool big = la.qbs >= 32768;                    // no block ends twice in a tile
+    if (grad_dtype == MAB_F32) big ? run(requant_loose_kernel<float, true>, 2 * rq_ctas<float, true>) : run(requant_loose_kernel<float, false>, 2 * rq_ctas<float, false>);
+    else big ? run(requant_loose_kernel<uint16_t, true>, 2 * rq_ctas<uint16_t, true>) : run(requant_loose_kernel<uint16_t, false>, 2 * rq_ctas<uint16_t, false>);
     count_launch();
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? MAB_OK : cuda_fail(e, "requant_loose_kernel launch");
