@@ -527,12 +527,11 @@ struct WindowTileSmem {
     }
 };
 
-// Phases 1-4 of a tile, by the NT threads of the CTA: stages the `rows` window rows of block `blk`, numbers
-// the touched positions (slots, in ascending position) and accumulates both moments row after row into
-// w.mv[slot].  Returns the number of touched positions.  Ends with a barrier.
+// Asks for the `rows` window rows of block `blk` (kcnt entries each) in w.raw: every row's slice of I and of V is copied asynchronously in
+// 16-byte pieces from the 16-byte boundary below its first element.  By the NT threads of the CTA; window_tile_moments waits for it.
 template <int NT>
-__device__ __forceinline__ int window_tile_moments(const mab_tensor& T, int blk, int n_blk, int kcnt, const WindowArgs& a,
-                                                   const WindowTileSmem& w, int* s_scan, int* s_pos_off, int* s_val_off) {
+__device__ __forceinline__ void window_tile_stage(const mab_tensor& T, int blk, int kcnt, const WindowArgs& a, const WindowTileSmem& w, int* s_pos_off,
+                                                  int* s_val_off) {
     const int t = threadIdx.x;
     const int rows = a.rows;
     const int64_t koff = (int64_t)blk * T.k_block_size_many;
@@ -540,13 +539,7 @@ __device__ __forceinline__ int window_tile_moments(const mab_tensor& T, int blk,
     const uintptr_t I_blk = reinterpret_cast<uintptr_t>(T.I + koff), V_blk = reinterpret_cast<uintptr_t>(T.V + koff);
     const uintptr_t I_lo = reinterpret_cast<uintptr_t>(T.I), I_hi = reinterpret_cast<uintptr_t>(T.I + (int64_t)a.m * pitch);
     const uintptr_t V_lo = reinterpret_cast<uintptr_t>(T.V), V_hi = reinterpret_cast<uintptr_t>(T.V + (int64_t)a.m * pitch);
-    const int E = rows * kcnt;
-    const uint32_t div_kcnt = kcnt > 1 ? 0xFFFFFFFFu / (uint32_t)kcnt + 1u : 0u;   // i / kcnt == umulhi(i, div_kcnt) while i * kcnt < 2^32
     const int chunks_per_row = w.rstride >> 4;
-    MAB_BTICK_DECL
-    // 1. stage the window entries: every row's slice of I and of V is copied asynchronously in
-    //    16-byte pieces from the 16-byte boundary below its first element; meanwhile clear the
-    //    bitmap and the compact moments
     if (t < rows) {
         s_pos_off[t] = (2 * t) * w.rstride + (int)((I_blk + (uintptr_t)t * pitch * 2) & 15);
         s_val_off[t] = (2 * t + 1) * w.rstride + (int)((V_blk + (uintptr_t)t * pitch * 2) & 15);
@@ -572,6 +565,21 @@ __device__ __forceinline__ int window_tile_moments(const mab_tensor& T, int blk,
         }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// The window phases of a tile, by the NT threads of the CTA: waits for the staged rows, numbers
+// the touched positions (slots, in ascending position) and accumulates both moments row after row into
+// w.mv[slot].  Returns the number of touched positions.  Ends with a barrier, behind which the rows' place is free:
+// the caller stages the next tile's there before it turns to the update.
+template <int NT, bool AHEAD>
+__device__ __forceinline__ int window_tile_moments(int n_blk, int kcnt, const WindowArgs& a, const WindowTileSmem& w, int* s_scan,
+                                                   const int* s_pos_off, const int* s_val_off) {
+    const int t = threadIdx.x;
+    const int rows = a.rows;
+    const int E = rows * kcnt;
+    const uint32_t div_kcnt = kcnt > 1 ? 0xFFFFFFFFu / (uint32_t)kcnt + 1u : 0u;   // i / kcnt == umulhi(i, div_kcnt) while i * kcnt < 2^32
+    MAB_BTICK_DECL
+    // 1. clear the bitmap and the compact moments while the rows are under way
     for (int i = t; i < WT_WORDS; i += NT) w.bitmap[i] = 0u;
     for (int i = t; i < E; i += NT) w.mv[i] = make_float2(0.0f, 0.0f);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -632,8 +640,41 @@ __device__ __forceinline__ int window_tile_moments(const mab_tensor& T, int blk,
     }
     __syncthreads();
     MAB_BTICK(3);
+    constexpr int RE = NT == 256 && AHEAD ? 2 : 1;            // entries a thread looks ahead (291 of a block of 29 056, 1 %: more than 256)
     if ((t & ~31) < kcnt) {                                   // whole warps decide, so that every warp meets the barriers in one piece
-        if (kcnt <= NT) {
+        if (RE > 1 && kcnt <= RE * NT) {
+            // RE entries per thread and row: the next row's slots and values are fetched before the barrier of the current one
+            int slot[RE];
+            uint32_t vbits[RE];
+            auto fetch = [&](int r, int (&sl)[RE], uint32_t (&vb)[RE]) {
+                const uint16_t* slot_r = reinterpret_cast<const uint16_t*>(w.raw + s_pos_off[r]);
+                const uint16_t* val_r = reinterpret_cast<const uint16_t*>(w.raw + s_val_off[r]);
+#pragma unroll
+                for (int i = 0; i < RE; ++i) {
+                    sl[i] = WT_NO_SLOT; vb[i] = 0u;
+                    if (t + i * NT < kcnt) { sl[i] = slot_r[t + i * NT]; vb[i] = val_r[t + i * NT]; }
+                }
+            };
+            fetch(0, slot, vbits);
+            for (int r = 0; r < rows; ++r) {
+                int slot_n[RE];
+                uint32_t vbits_n[RE];
+                if (r + 1 < rows) fetch(r + 1, slot_n, vbits_n);
+                const float w1 = a.w1[r], w2 = a.w2[r];
+#pragma unroll
+                for (int i = 0; i < RE; ++i)
+                    if (slot[i] != WT_NO_SLOT) {
+                        const float val = __uint_as_float(vbits[i] << 16);
+                        float2 acc = w.mv[slot[i]];
+                        acc.x = __fadd_rn(acc.x, __fmul_rn(val, w1));
+                        acc.y = __fadd_rn(acc.y, __fmul_rn(__fmul_rn(val, val), w2));
+                        w.mv[slot[i]] = acc;
+                    }
+                __syncthreads();
+#pragma unroll
+                for (int i = 0; i < RE; ++i) { slot[i] = slot_n[i]; vbits[i] = vbits_n[i]; }
+            }
+        } else if (RE == 1 && kcnt <= NT) {
             // one entry per thread and row: the next row's slot and value are fetched before the barrier of the current one
             const bool on = t < kcnt;
             int slot = WT_NO_SLOT;
@@ -731,7 +772,18 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
     UpdateProbe pr;
     const bool probing = MODE == MODE_STEP && a.probe != nullptr;
 
+    // AHEAD: the next tile's rows travel while this one's elements are updated, and a thread of 256 looks two entries ahead in the row loop.  The
+    // bf16 alpha forms have the registers for it (alpha == -2, 54.5 M elements 152 -> 145 us, alpha = 0.5 with 20 rows 210 -> 203); the others
+    // spill, or hide the rows behind other tiles as it is.
+    constexpr bool AHEAD = sizeof(TP) == 2 && ALPHA != 0;
+    auto stage = [&](const mab_tensor& T, int blk) {
+        window_tile_stage<NT>(T, blk, blk < T.topk_full_blocks_count ? T.k_block_size_many : T.k_block_size_few, a, w, s_pos_off, s_val_off);
+    };
     int ti = 0;
+    if constexpr (AHEAD) {
+        ti = find_tensor(s_first, n_tensors, blockIdx.x);
+        stage(tensors[ti], blockIdx.x - s_first[ti]);
+    }
     for (int unit = blockIdx.x; unit < total_units; unit += gridDim.x) {
         if (unit >= s_first[ti + 1]) ti = find_tensor(s_first, n_tensors, unit);   // (units ascend: mostly the same tensor as before)
         const mab_tensor& T = tensors[ti];
@@ -739,6 +791,12 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
         const int dbs = T.d_block_size, nfull = T.topk_full_blocks_count;
         const int64_t blk_base = (int64_t)blk * dbs;
         const int n_blk = (int)min((int64_t)dbs, T.d - blk_base);
+        auto stage_next = [&]() {                              // the next unit's rows travel while this one's elements are updated
+            const int nu = unit + gridDim.x;
+            if (nu >= total_units) return;
+            const int nti = nu < s_first[ti + 1] ? ti : find_tensor(s_first, n_tensors, nu);
+            stage(tensors[nti], nu - s_first[nti]);
+        };
         if (MODE == MODE_STEP) {
             // the next unit's window rows are small and are asked into L2 now
             if (unit + (int)gridDim.x < total_units && (int)threadIdx.x < 2 * rows) {
@@ -773,7 +831,9 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
         const bool g_bf16 = (T.grad_dtype == MAB_BF16);
 
         MAB_BTICK_DECL
-        const int touched = window_tile_moments<NT>(T, blk, n_blk, kcnt, a, w, s_scan, s_pos_off, s_val_off);
+        if constexpr (!AHEAD) window_tile_stage<NT>(T, blk, kcnt, a, w, s_pos_off, s_val_off);
+        const int touched = window_tile_moments<NT, AHEAD>(n_blk, kcnt, a, w, s_scan, s_pos_off, s_val_off);
+        if constexpr (AHEAD) stage_next();
         MAB_BTICK(9);
         if constexpr (MODE == MODE_STEP && ALPHA == 0) {
             // 5. without the alpha term only the touched positions get an update: stream the block for the
@@ -938,7 +998,8 @@ window_resident_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, in
         }
         const int kcnt = (blk < nfull) ? T.k_block_size_many : T.k_block_size_few;
         const bool g_bf16 = (T.grad_dtype == MAB_BF16);
-        const int touched = window_tile_moments<WR_THREADS>(T, blk, n_blk, kcnt, a, w, s_scan, s_pos_off, s_val_off);
+        window_tile_stage<WR_THREADS>(T, blk, kcnt, a, w, s_pos_off, s_val_off);
+        const int touched = window_tile_moments<WR_THREADS, false>(n_blk, kcnt, a, w, s_scan, s_pos_off, s_val_off);
         MAB_BTICK(9);
 
         // the tile: wait for the bulk copy, or fetch a ragged block (a tensor's last one, an unaligned slice) with plain loads

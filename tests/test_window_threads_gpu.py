@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 DBS = 29056
 
 
-@pytest.mark.parametrize('alpha,weight_decay,dtype', [(0, 0.0, torch.float32), (0, 0.1, torch.float32), (0.5, 0.1, torch.float32), (-2, 0.0, torch.bfloat16)])
+@pytest.mark.parametrize('alpha,weight_decay,dtype', [(0, 0.0, torch.float32), (0, 0.1, torch.float32), (0.5, 0.1, torch.float32), (-2, 0.0, torch.bfloat16), (0.5, 0.0, torch.bfloat16)])
 @pytest.mark.parametrize('rows,k,per_sm', [(3, 256, 1), (3, 257, 2), (3, 384, 3), (3, 385, 3), (10, 256, 3), (10, 291, 10), (10, 385, 1), (20, 291, 3), (3, 2500, 2)])
 def test_many_tiles_equal_single_tiles(rows, k, per_sm, alpha, weight_decay, dtype):
     from ista_daslab_optimizers_b200 import MicroAdam, _native
