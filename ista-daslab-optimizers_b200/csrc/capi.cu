@@ -264,7 +264,7 @@ static int fused_run(mab_tensor* tensors, int n, const mab_step_args* args, void
                                       args->quant_block_size)) return rc;
         wa.probe = args->probe_out;
         for (const Chunk& c : chunks) {
-            if (int rc = launch_window_step(dev + c.first, c.count, c.units_a, c.units_b, c.max_k, c.max_dbs, c.param_dtype, wa, s)) return rc;
+            if (int rc = launch_window_step(dev + c.first, c.count, c.units_a, c.units_b, c.max_k, c.max_dbs, c.param_dtype, wa, (what & RUN_A) && !loose, s)) return rc;
         }
     }
     if (args->probe_out && (what & RUN_A))                     // gradient and final error feedback: after the call's last kernel
@@ -377,7 +377,7 @@ extern "C" int mab_fused_step_static(mab_tensor* tensors, int n, const mab_step_
     wa.probe = args->probe_out;
     for (int first = 0; first < n;) {
         const int end = static_run_end(tensors, n, first, &ua, &ub, &mk, &md);
-        if (int rc = launch_window_step(dev + first, end - first, ua, ub, mk, md, tensors[first].param_dtype, wa, s)) return rc;
+        if (int rc = launch_window_step(dev + first, end - first, ua, ub, mk, md, tensors[first].param_dtype, wa, true, s)) return rc;
         first = end;
     }
     if (args->probe_out)

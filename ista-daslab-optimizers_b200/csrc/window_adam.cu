@@ -528,10 +528,11 @@ struct WindowTileSmem {
 };
 
 // Asks for the `rows` window rows of block `blk` (kcnt entries each) in w.raw: every row's slice of I and of V is copied asynchronously in
-// 16-byte pieces from the 16-byte boundary below its first element.  By the NT threads of the CTA; window_tile_moments waits for it.
+// 16-byte pieces from the 16-byte boundary below its first element (but row `skip`).  By the NT threads of the CTA; window_tile_moments
+// waits for it.
 template <int NT>
 __device__ __forceinline__ void window_tile_stage(const mab_tensor& T, int blk, int kcnt, const WindowArgs& a, const WindowTileSmem& w, int* s_pos_off,
-                                                  int* s_val_off) {
+                                                  int* s_val_off, int skip = -1) {
     const int t = threadIdx.x;
     const int rows = a.rows;
     const int64_t koff = (int64_t)blk * T.k_block_size_many;
@@ -546,6 +547,7 @@ __device__ __forceinline__ void window_tile_stage(const mab_tensor& T, int blk, 
     }
     for (int ra = t >> 6; ra < rows * 2; ra += NT >> 6) {                         // ra = 2 * row + array; 64 threads per slice
         const int r = ra >> 1;
+        if (r == skip) continue;
         const bool isV = ra & 1;
         const uintptr_t seg = (isV ? V_blk : I_blk) + (uintptr_t)r * pitch * 2;
         const uintptr_t seg_end = seg + 2u * kcnt;
@@ -570,10 +572,11 @@ __device__ __forceinline__ void window_tile_stage(const mab_tensor& T, int blk, 
 // The window phases of a tile, by the NT threads of the CTA: waits for the staged rows, numbers
 // the touched positions (slots, in ascending position) and accumulates both moments row after row into
 // w.mv[slot].  Returns the number of touched positions.  Ends with a barrier, behind which the rows' place is free:
-// the caller stages the next tile's there before it turns to the update.
-template <int NT, bool AHEAD>
-__device__ __forceinline__ int window_tile_moments(int n_blk, int kcnt, const WindowArgs& a, const WindowTileSmem& w, int* s_scan,
-                                                   const int* s_pos_off, const int* s_val_off) {
+// the caller stages the next tile's there before it turns to the update.  EARLY: kernel A of this step may still be running; the row that it
+// writes was not staged, and is fetched behind the wait for that kernel, when the others are marked.
+template <int NT, bool AHEAD, bool EARLY>
+__device__ __forceinline__ int window_tile_moments(const mab_tensor& T, int blk, int n_blk, int kcnt, const WindowArgs& a, const WindowTileSmem& w,
+                                                   int* s_scan, const int* s_pos_off, const int* s_val_off) {
     const int t = threadIdx.x;
     const int rows = a.rows;
     const int E = rows * kcnt;
@@ -595,20 +598,40 @@ __device__ __forceinline__ int window_tile_moments(int n_blk, int kcnt, const Wi
     constexpr int KEEP = NT >= 512 ? WT_KEEP : 1;             // (the 256-thread variants have no registers to spare)
     uint16_t* kept_ptr[KEEP];
     uint32_t kept_pos[KEEP];
+    if constexpr (EARLY) {
+        const int ring = T.ring_index;
+        for (int i = t; i < E; i += NT) {
+            const int r = kcnt > 1 ? (int)__umulhi((uint32_t)i, div_kcnt) : i;
+            const uint32_t pos = r != ring ? (uint32_t)*pos_ptr(i) : 0xFFFFFFFFu;
+            if (pos < (uint32_t)n_blk) atomicOr(&w.bitmap[pos >> 5], 1u << (pos & 31));
+        }
+        wait_for_kernel_before();
+        const int64_t at = (int64_t)ring * row_pitch_of(T) + (int64_t)blk * T.k_block_size_many;
+        if (ring < rows)
+            for (int j = t; j < kcnt; j += NT) {
+                const uint16_t pos = __ldcg(reinterpret_cast<const unsigned short*>(T.I + at) + j);
+                *(reinterpret_cast<uint16_t*>(w.raw + s_pos_off[ring]) + j) = pos;
+                *(reinterpret_cast<uint16_t*>(w.raw + s_val_off[ring]) + j) = __ldcg(T.V + at + j);
+                if (pos < n_blk) atomicOr(&w.bitmap[pos >> 5], 1u << (pos & 31));
+            }
+        __syncthreads();
+    }
 #pragma unroll
     for (int it = 0; it < KEEP; ++it) {
         const int i = t + it * NT;
         kept_ptr[it] = pos_ptr(min(i, E - 1));
         kept_pos[it] = i < E ? (uint32_t)*kept_ptr[it] : 0xFFFFFFFFu;
     }
+    if constexpr (!EARLY) {
 #pragma unroll
-    for (int it = 0; it < KEEP; ++it)
-        if (kept_pos[it] < (uint32_t)n_blk) atomicOr(&w.bitmap[kept_pos[it] >> 5], 1u << (kept_pos[it] & 31));
-    for (int i = t + KEEP * NT; i < E; i += NT) {
-        const uint32_t pos = *pos_ptr(i);
-        if (pos < (uint32_t)n_blk) atomicOr(&w.bitmap[pos >> 5], 1u << (pos & 31));
+        for (int it = 0; it < KEEP; ++it)
+            if (kept_pos[it] < (uint32_t)n_blk) atomicOr(&w.bitmap[kept_pos[it] >> 5], 1u << (kept_pos[it] & 31));
+        for (int i = t + KEEP * NT; i < E; i += NT) {
+            const uint32_t pos = *pos_ptr(i);
+            if (pos < (uint32_t)n_blk) atomicOr(&w.bitmap[pos >> 5], 1u << (pos & 31));
+        }
+        __syncthreads();
     }
-    __syncthreads();
     MAB_BTICK(1);
     // 3. number them: prefix[word] = touched positions in words below
     constexpr int WPT = (WT_WORDS + NT - 1) / NT;
@@ -751,7 +774,7 @@ __device__ __noinline__ void decay_tile(TP* p, int len, float decay) {
     for (int i = done + threadIdx.x; i < len; i += NT) Elem<TP>::store(p, i, __fmul_rn(Elem<TP>::load(p, i), decay));
 }
 
-template <typename TP, int MODE, int ALPHA, int NT>
+template <typename TP, int MODE, int ALPHA, int NT, bool EARLY>
 __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units,
                                                  int max_k, const WindowArgs& a, int dense_at = 0) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -767,7 +790,7 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
     float* const dense = dense_at > 0 ? reinterpret_cast<float*>(smem_raw + dense_at) : nullptr;   // the streams' arrays of the warps
     if (dense != nullptr) for (int i = t; i < NT * 8; i += NT) dense[i] = 0.0f;
     __syncthreads();
-    if (MODE == MODE_STEP) wait_for_kernel_before();
+    if (MODE == MODE_STEP && !EARLY) wait_for_kernel_before();
     const float inv_bc1 = 1.0f / a.bc1, inv_bc2 = 1.0f / a.bc2;
     UpdateProbe pr;
     const bool probing = MODE == MODE_STEP && a.probe != nullptr;
@@ -777,7 +800,8 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
     // spill, or hide the rows behind other tiles as it is.
     constexpr bool AHEAD = sizeof(TP) == 2 && ALPHA != 0;
     auto stage = [&](const mab_tensor& T, int blk) {
-        window_tile_stage<NT>(T, blk, blk < T.topk_full_blocks_count ? T.k_block_size_many : T.k_block_size_few, a, w, s_pos_off, s_val_off);
+        window_tile_stage<NT>(T, blk, blk < T.topk_full_blocks_count ? T.k_block_size_many : T.k_block_size_few, a, w, s_pos_off, s_val_off,
+                              EARLY ? T.ring_index : -1);
     };
     int ti = 0;
     if constexpr (AHEAD) {
@@ -808,7 +832,7 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
             // fp32 tiles are not asked for: they are twice as long, only half of their sectors is touched without decay, and with all CTAs' tiles
             // in L2 some left it before their turn (us, with and without: 29 M elements 50 and 44, with decay 81 and 73, alpha = 0.5 33.5 M 121
             // and 115).
-            if (sizeof(TP) == 2) prefetch_l2<NT>(reinterpret_cast<uintptr_t>(reinterpret_cast<TP*>(T.param) + blk_base), (int64_t)n_blk * sizeof(TP));
+            if (sizeof(TP) == 2 || EARLY) prefetch_l2<NT>(reinterpret_cast<uintptr_t>(reinterpret_cast<TP*>(T.param) + blk_base), (int64_t)n_blk * sizeof(TP));
         }
         // The weight decay has a pass of its own; where every CTA has one tile it runs while the window's rows are on their way (500 tiles, fp32:
         // 49.7 us behind the window phases, 45.6 before them; 4000 tiles 291 and 317: there the other tiles hide its latency, and
@@ -831,9 +855,9 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
         const bool g_bf16 = (T.grad_dtype == MAB_BF16);
 
         MAB_BTICK_DECL
-        if constexpr (!AHEAD) window_tile_stage<NT>(T, blk, kcnt, a, w, s_pos_off, s_val_off);
-        const int touched = window_tile_moments<NT, AHEAD>(n_blk, kcnt, a, w, s_scan, s_pos_off, s_val_off);
-        if constexpr (AHEAD) stage_next();
+        if constexpr (!AHEAD) window_tile_stage<NT>(T, blk, kcnt, a, w, s_pos_off, s_val_off, EARLY ? T.ring_index : -1);
+        const int touched = window_tile_moments<NT, AHEAD, EARLY>(T, blk, n_blk, kcnt, a, w, s_scan, s_pos_off, s_val_off);
+        if constexpr (AHEAD && !EARLY) stage_next();
         MAB_BTICK(9);
         if constexpr (MODE == MODE_STEP && ALPHA == 0) {
             // 5. without the alpha term only the touched positions get an update: stream the block for the
@@ -898,11 +922,11 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
 }
 
 // (threads_of gives NT)
-template <typename TP, int MODE, int ALPHA, int NT>
+template <typename TP, int MODE, int ALPHA, int NT, bool EARLY = false>
 __global__ void __launch_bounds__(NT, ALPHA != 0 ? 768 / NT : NT == 384 ? 3 : 1024 / NT)
 window_tile_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int max_k,
                    int dense_at, const __grid_constant__ WindowArgs a) {
-    window_tile_body<TP, MODE, ALPHA, NT>(tensors, n_tensors, total_units, max_k, a, dense_at);
+    window_tile_body<TP, MODE, ALPHA, NT, EARLY>(tensors, n_tensors, total_units, max_k, a, dense_at);
 }
 
 // Single tensor whose descriptor travels as a kernel argument (operator-level entry point).
@@ -910,7 +934,7 @@ template <typename TP, int MODE, int ALPHA, int NT>
 __global__ void __launch_bounds__(NT)
 window_tile_single_kernel(const __grid_constant__ mab_tensor t, int total_units, int max_k,
                           const __grid_constant__ WindowArgs a) {
-    window_tile_body<TP, MODE, ALPHA, NT>(&t, 1, total_units, max_k, a);
+    window_tile_body<TP, MODE, ALPHA, NT, false>(&t, 1, total_units, max_k, a);
 }
 
 // ------------------------------------------------------------------------------------ resident-tile kernel
@@ -942,6 +966,7 @@ __device__ __noinline__ void update_in_place(uint16_t* p, const uint16_t* spos, 
     }
 }
 
+template <bool EARLY>
 __global__ void __launch_bounds__(WR_THREADS, 2)
 window_resident_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int max_k, int tile_bytes,
                        const __grid_constant__ WindowArgs a) {
@@ -959,7 +984,7 @@ window_resident_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, in
     for (int i = t; i < n_tensors; i += WR_THREADS) s_first[i] = tensors[i].first_unit_a;
     if (t == 0) { s_first[n_tensors] = total_units; mbar_init(&s_bar, 1); }
     __syncthreads();
-    wait_for_kernel_before();
+    if (!EARLY) wait_for_kernel_before();
     const float inv_bc1 = 1.0f / a.bc1, inv_bc2 = 1.0f / a.bc2;
     uint32_t parity = 0;
     bool store_in_flight = false;                                               // thread 0 only
@@ -998,8 +1023,8 @@ window_resident_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, in
         }
         const int kcnt = (blk < nfull) ? T.k_block_size_many : T.k_block_size_few;
         const bool g_bf16 = (T.grad_dtype == MAB_BF16);
-        window_tile_stage<WR_THREADS>(T, blk, kcnt, a, w, s_pos_off, s_val_off);
-        const int touched = window_tile_moments<WR_THREADS, false>(n_blk, kcnt, a, w, s_scan, s_pos_off, s_val_off);
+        window_tile_stage<WR_THREADS>(T, blk, kcnt, a, w, s_pos_off, s_val_off, EARLY ? T.ring_index : -1);
+        const int touched = window_tile_moments<WR_THREADS, false, EARLY>(T, blk, n_blk, kcnt, a, w, s_scan, s_pos_off, s_val_off);
         MAB_BTICK(9);
 
         // the tile: wait for the bulk copy, or fetch a ragged block (a tensor's last one, an unaligned slice) with plain loads
@@ -1149,7 +1174,7 @@ static int threads_of(bool write, bool alpha, int fit, int tiles, int max_k, int
 // k_block_size of the launch) decides which one runs.
 template <typename TP, int MODE, int ALPHA>
 static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* single, int n_tensors, int units_tile,
-                              int units_wide, int max_k, const WindowArgs& a, cudaStream_t s) {
+                              int units_wide, int max_k, const WindowArgs& a, bool early, cudaStream_t s) {
     const int sms = device_sm_count();
     // the tile variant while its compact arrays fit one CTA's shared memory (next to the kernel's static arrays)
     const int smem_tile = (int64_t)a.rows * max_k <= WT_MAX_ENTRIES ? wt_smem_bytes(a.rows, max_k) : 0;
@@ -1177,11 +1202,13 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
             else rc = run(window_tile_single_kernel<TP, MODE, 0, 256>, 256);
         } else if constexpr (ALPHA == 0) {
             if (nt == 1024) rc = run(window_tile_kernel<TP, MODE, 0, 1024>, 1024);
+            else if (nt == 512 && early) rc = run(window_tile_kernel<TP, MODE, 0, 512, true>, 512);
             else if (nt == 512) rc = run(window_tile_kernel<TP, MODE, 0, 512>, 512);
             else if (nt == 384) rc = run(window_tile_kernel<TP, MODE, 0, 384>, 384);
             else rc = run(window_tile_kernel<TP, MODE, 0, 256>, 256);
         } else {
-            if (nt == 512) rc = run(window_tile_kernel<TP, MODE, ALPHA, 512>, 512);
+            if (nt == 512 && early) rc = run(window_tile_kernel<TP, MODE, ALPHA, 512, true>, 512);
+            else if (nt == 512) rc = run(window_tile_kernel<TP, MODE, ALPHA, 512>, 512);
             else if (nt == 384) rc = run(window_tile_kernel<TP, MODE, ALPHA, 384>, 384);
             else rc = run(window_tile_kernel<TP, MODE, ALPHA, 256>, 256);
         }
@@ -1206,12 +1233,12 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
 
 template <typename TP, int MODE>
 static int launch_window(const mab_tensor* dev_tensors, const mab_tensor* single, int n_tensors, int units_tile,
-                         int units_wide, int max_k, const WindowArgs& a, cudaStream_t s) {
+                         int units_wide, int max_k, const WindowArgs& a, bool early, cudaStream_t s) {
     if constexpr (MODE == MODE_STEP) {
-        if (a.alpha == -2.0f) return launch_window_impl<TP, MODE, 2>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, s);
-        if (a.alpha != 0.0f) return launch_window_impl<TP, MODE, 1>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, s);
+        if (a.alpha == -2.0f) return launch_window_impl<TP, MODE, 2>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, early, s);
+        if (a.alpha != 0.0f) return launch_window_impl<TP, MODE, 1>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, early, s);
     }
-    return launch_window_impl<TP, MODE, 0>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, s);
+    return launch_window_impl<TP, MODE, 0>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, early, s);
 }
 
 int fill_window_args(WindowArgs& a, int64_t steps, int m, double beta1, double beta2, double eps, float alpha, int qbs) {
@@ -1246,21 +1273,23 @@ static int resident_smem_bytes(int rows, int max_k, int max_dbs, int* tile_bytes
 }
 
 int launch_window_step(const mab_tensor* dev_tensors, int n_tensors, int units_tile, int units_wide, int max_k, int max_dbs,
-                       int param_dtype, const WindowArgs& a, cudaStream_t s) {
+                       int param_dtype, const WindowArgs& a, bool behind_a, cudaStream_t s) {
+    const bool early = behind_a && units_tile <= EARLY_MAX_CTAS;
     if (param_dtype == MAB_F32)
-        return launch_window<float, MODE_STEP>(dev_tensors, nullptr, n_tensors, units_tile, units_wide, max_k, a, s);
+        return launch_window<float, MODE_STEP>(dev_tensors, nullptr, n_tensors, units_tile, units_wide, max_k, a, early, s);
     int tile_bytes = 0;
     const int smem = (a.alpha == 0.0f) ? resident_smem_bytes(a.rows, max_k, max_dbs, &tile_bytes) : 0;
     if (smem > 0) {
         const int grid = (int)std::min<int64_t>(units_tile, (int64_t)device_sm_count() * 2);
-        MAB_CUDA_TRY(cudaFuncSetAttribute(window_resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        MAB_CUDA_TRY(launch_behind_kernel(window_resident_kernel, grid, WR_THREADS, smem, s, dev_tensors, n_tensors, units_tile, max_k, tile_bytes, a));
+        auto kern = early ? window_resident_kernel<true> : window_resident_kernel<false>;
+        MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        MAB_CUDA_TRY(launch_behind_kernel(kern, grid, WR_THREADS, smem, s, dev_tensors, n_tensors, units_tile, max_k, tile_bytes, a));
         count_launch();
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_fail(e, "window_resident_kernel launch");
         return MAB_OK;
     }
-    return launch_window<uint16_t, MODE_STEP>(dev_tensors, nullptr, n_tensors, units_tile, units_wide, max_k, a, s);
+    return launch_window<uint16_t, MODE_STEP>(dev_tensors, nullptr, n_tensors, units_tile, units_wide, max_k, a, early, s);
 }
 
 // The give-up path of the bounded waits, exercised without any fault: the barrier is told to expect
@@ -1340,6 +1369,6 @@ extern "C" int mab_compute_microadam_update(int blocks, int threads, int carveou
     if (units_tile == 0) return MAB_OK;
     const int max_k = std::max(t.k_block_size_many, t.k_block_size_few);
     cudaStream_t s = (cudaStream_t)stream;
-    if (out_dtype == MAB_F32) return launch_window<float, MODE_WRITE_UPDATE>(nullptr, &t, 1, units_tile, units_wide, max_k, a, s);
-    return launch_window<uint16_t, MODE_WRITE_UPDATE>(nullptr, &t, 1, units_tile, units_wide, max_k, a, s);
+    if (out_dtype == MAB_F32) return launch_window<float, MODE_WRITE_UPDATE>(nullptr, &t, 1, units_tile, units_wide, max_k, a, false, s);
+    return launch_window<uint16_t, MODE_WRITE_UPDATE>(nullptr, &t, 1, units_tile, units_wide, max_k, a, false, s);
 }
