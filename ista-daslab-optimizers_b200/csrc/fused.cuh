@@ -33,17 +33,16 @@ __host__ __device__ __forceinline__ TileRange tiles_of_cta(int total, int ctas, 
 
 // The update kernel of a step is launched behind kernel A without the gap between two kernels (programmatic stream
 // serialization): its CTAs read the descriptor table, which neither kernel writes, and wait there for kernel A's end and its
-// results.  A kernel A of at most half as many CTAs as a B200 has SMs (148) allows it as soon as all its CTAs have started; with more the
-// ones that wait take places unevenly among those that work, and the update runs on fewer SMs than it could.  us a step with 10 rows,
-// allowed and not: bf16 8 tiles 29.2 / 30.1, 40 tiles 29.6 / 30.6, 74 30.4 / 30.6, 148 30.9 / 30.9; fp32 8 tiles 41.1 / 41.2, 40 41.5 / 41.8, 74
-// 42.2 / 42.3, 90 49.2 / 41.8, 110 49.5 / 42.6, 254 72.8 / 55.5.  Most of what the launch saves is the gap itself (7 690 elements 24.6 -> 22.5 us a
-// step).  Kernel A of loose blocks does not allow it, the requantisation being next; nor do the requantisation and the fp32 kernel with
-// one tile per SM (not tried there).
+// results.  A kernel A of at most as many CTAs as a B200 has SMs (148) allows it as soon as all its CTAs have started; with more the
+// ones that wait take places unevenly among those that work, and the update runs on fewer SMs than it could (fp32, 254 tiles 72.8 us a step
+// allowed, 55.5 not).  Kernel A of loose blocks does not allow it, the requantisation being next; nor do the requantisation and the fp32 kernel
+// with one tile per SM (not tried there).
 // What does not depend on kernel A comes before that wait where every CTA of the update has one tile (template flag EARLY): the other rows of
 // the window are staged and marked, the weight decay is applied, or the bf16 parameters are on their way into shared memory; the row
-// that kernel A writes follows behind the wait.  Kernel A itself is an ordinary launch, so everything before it is complete.  us a step: 7 690 fp32
-// elements 20.5 -> 18.5, 40 tiles fp32 24.6 -> 22.6, with weight decay 28 -> 22.6, bf16 22.6 -> 20.9.
-constexpr int EARLY_MAX_CTAS = 74;
+// that kernel A writes follows behind the wait.  Kernel A itself is an ordinary launch, so everything before it is complete.  us a step, everything
+// behind the wait and so: 7 690 fp32 elements 20.5 / 18.5, 40 tiles fp32 24.6 / 22.6, with weight decay 28 / 22.6, bf16 22.6 / 20.9; not allowed
+// and so: 80 tiles bf16 22.6 / 21.9, 100 fp32 with weight decay 28.7 / 26.7, 110 with 20 rows 28.7 / 27.1, 148 fp32 26.5 / 25.5, bf16 22.7 / 22.6.
+constexpr int EARLY_MAX_CTAS = 148;
 __device__ __forceinline__ void allow_next_kernel() { if (gridDim.x <= EARLY_MAX_CTAS) asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
