@@ -5,7 +5,7 @@
 // tile's first 1024 octets in registers (two per thread, 32 KB) and the other 2608 in shared memory (83 KB), next to
 // 26 KB of selection scratch, so that two CTAs share an SM and one tile's chain of dependent phases overlaps the
 // other's arithmetic.  The shared-memory part is staged by the bulk copy engine and turned into a = g + Qinv(e) in
-// place; the tile after this one is asked into L2 meanwhile.
+// place; the beginning of the tile after this one is asked into L2 meanwhile.
 //
 // Thread t owns octets 2 t and 2 t + 1 (registers) and 1024 + t, 1024 + t + 512, ... (shared memory).  An octet in shared
 // memory is two 16-byte pieces 32 bytes apart from the next lane's: lanes 4-7 of every 8 take the second piece first

@@ -595,7 +595,7 @@ __device__ __forceinline__ int window_tile_moments(const mab_tensor& T, int blk,
     };
     // 2. mark touched positions (an index outside the block - only a damaged checkpoint can hold one - is
     //    ignored, here and below).  A thread's first entries stay in registers for step 4.
-    constexpr int KEEP = NT >= 512 ? WT_KEEP : 1;             // (the 256-thread variants have no registers to spare)
+    constexpr int KEEP = NT >= 512 ? WT_KEEP : 1;             // (with fewer threads there are no registers to spare)
     uint16_t* kept_ptr[KEEP];
     uint32_t kept_pos[KEEP];
     if constexpr (EARLY) {
