@@ -15,8 +15,9 @@ namespace mab {
 
 constexpr int SPR_SR = 14592;         // elements of a block one CTA accumulates at a time (57 * 256): a 29 056-element block is two ranges
 constexpr int SPR_THREADS = 384;      // three CTAs of 58 KB of accumulators per SM, 56 registers a thread (512 threads of 40 spill: 98 us, now 78)
+static_assert(MAB_MAX_WINDOW <= SPR_THREADS, "a thread brings one row's multiplier");
 // Rows whose entries a thread fetches at once, while it adds those fetched before; (row, round) pairs of long rows (25.6 M elements, 32 rows of
-// 5 %: 6 189 us, 8 198; of 1 %: 6 66.6, 8 65.4).
+// 5 %: 6 189 us, 8 198; of 1 %: 6 66.6, 8 65.4, products behind the barriers).
 template <bool LONG> constexpr int SPR_AHEAD = LONG ? 6 : 8;
 
 constexpr int SP_THREADS = 512;
@@ -155,7 +156,9 @@ template <> struct Entry<float> {
 // row, so a row needs no atomics, but a barrier).  Bound by the chain of rows: a thread fetches its entries of SPR_AHEAD rows at once,
 // and the next ones before it adds these, so that a row costs a shared-memory update and a barrier (25.6 M elements, 32 rows of 1 %:
 // 232 us with one load latency per row and four walks over a block's entries, 75 with one per eight rows, 65 with the next eight ahead).
-// LONG: blocks with more entries than the CTA has threads.
+// The products of eight rows are made before the first of their barriers, off that chain (64 us; 1.28 M elements, bf16, 64 rows of 0.5 %: 14.4
+// behind the barriers, 11.6 so; 60 M the same 217 / 202).  LONG, blocks with more entries than the CTA has threads: behind them, as the
+// registers do not hold the products too (25.6 M, 32 rows of 5 %: 188, 206 before them).
 template <typename TO, typename TV, bool LONG>
 __global__ void __launch_bounds__(SPR_THREADS, 3)
 sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int nfull, int k_few, const float* __restrict__ M,
@@ -163,7 +166,6 @@ sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int
     extern __shared__ __align__(16) float acc[];
     __shared__ float s_M[MAB_MAX_WINDOW];
     const int t = threadIdx.x;
-    for (int i = t; i < rows; i += SPR_THREADS) s_M[i] = M[i];
     const int subs_per_block = (dbs + SPR_SR - 1) / SPR_SR;
     for (int unit = blockIdx.x; unit < total_units; unit += gridDim.x) {
         int blk = unit / subs_per_block, sub = unit - blk * subs_per_block;
@@ -188,18 +190,30 @@ sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int
             }
         };
         auto add = [&](const Entry<TV> (&e)[SPR_AHEAD<LONG>]) {
+            int pos[SPR_AHEAD<LONG>];
+            float val[SPR_AHEAD<LONG>];
+            if constexpr (!LONG) {
+#pragma unroll
+                for (int i = 0; i < SPR_AHEAD<LONG>; ++i) {
+                    pos[i] = e[i].pos() - s0;
+                    val[i] = __fmul_rn(s_M[min(r + i, rows - 1)], e[i].val());
+                }
+            }
 #pragma unroll
             for (int i = 0; i < SPR_AHEAD<LONG>; ++i) {
                 if (r < rows) {                                  // uniform
                     if (c == 0) __syncthreads();                 // the row before (or the clearing) is done
-                    const int pos = e[i].pos() - s0;
-                    if (pos >= 0 && pos < len) acc[pos] = __fadd_rn(acc[pos], __fmul_rn(s_M[r], e[i].val()));
+                    if constexpr (LONG) { pos[i] = e[i].pos() - s0; val[i] = __fmul_rn(s_M[r], e[i].val()); }
+                    if (pos[i] >= 0 && pos[i] < len) acc[pos[i]] = __fadd_rn(acc[pos[i]], val[i]);
                     if (!LONG || ++c == rounds) { c = 0; ++r; }
                 }
             }
         };
         Entry<TV> a[SPR_AHEAD<LONG>], b[SPR_AHEAD<LONG>];
+        const float factor = t < rows ? M[t] : 0.0f;
         fetch(a);
+        if (t < rows) s_M[t] = factor;
+        if constexpr (!LONG) __syncthreads();                    // the first products are made before the first row's barrier
         for (int p = 0; p < pairs; p += 2 * SPR_AHEAD<LONG>) {
             fetch(b);
             add(a);
