@@ -42,7 +42,7 @@ __host__ __device__ __forceinline__ TileRange tiles_of_cta(int total, int ctas, 
 // that kernel A writes follows behind the wait.  Kernel A itself is an ordinary launch, so everything before it is complete.  us a step, everything
 // behind the wait and so: 7 690 fp32 elements 20.5 / 18.5, 40 tiles fp32 24.6 / 22.6, with weight decay 28 / 22.6, bf16 22.6 / 20.9; not allowed
 // and so: 80 tiles bf16 22.6 / 21.9, 100 fp32 with weight decay 28.7 / 26.7, 110 with 20 rows 28.7 / 27.1, 148 fp32 26.5 / 25.5, bf16 22.7 / 22.6.
-constexpr int EARLY_MAX_CTAS = 148;
+constexpr int EARLY_MAX_CTAS = 148;            // (how many CTAs kernel A may have; the update's own grid decides as well: early_form)
 __device__ __forceinline__ void allow_next_kernel() { if (gridDim.x <= EARLY_MAX_CTAS) asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

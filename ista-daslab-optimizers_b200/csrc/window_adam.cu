@@ -14,6 +14,7 @@
 //    sub-range of a block with dense accumulators (window.cuh).
 #include "common.cuh"
 #include "window.cuh"
+#include "window_launch.cuh"
 #include "codec_fast.cuh"
 #include "fused.cuh"
 #include "async_copy.cuh"
@@ -32,7 +33,6 @@ __device__ unsigned long long g_stats_b[16];
 
 enum : int { MODE_WRITE_UPDATE = 0, MODE_STEP = 1 };
 
-constexpr int WT_WORDS = 1024;            // bitmap words of a tile (32768 positions)
 
 // 8 consecutive elements of a buffer as floats; vector access when `full`, else element-wise
 // up to `n` (the tensor's last, short octet).
@@ -477,18 +477,8 @@ __device__ __forceinline__ void stream_range(const mab_tensor& T, const WindowAr
 
 // ------------------------------------------------------------------------------------ tile kernel
 
-constexpr int WT_MAX_ENTRIES = 16384;     // window entries of one block the compact arrays may hold
 constexpr int WT_KEEP = 6;                // window entries a thread keeps in registers between marking and numbering
 constexpr int WT_NO_SLOT = 0xFFFF;        // slot of a window entry whose index lies outside the block (slots stay below 32768)
-
-// Bytes one row's slice of I (or V) occupies in the raw staging area: the slice is copied from the
-// 16-byte boundary below its first element, in whole 16-byte pieces.
-__host__ __device__ constexpr int wt_row_stride(int max_k) { return ((max_k * 2 + 30) + 15) & ~15; }
-
-__host__ __device__ constexpr int wt_smem_bytes(int rows, int max_k) {
-    const int e = (rows * max_k + 3) & ~3;
-    return 8 * e + rows * 2 * wt_row_stride(max_k) + 4 * WT_WORDS + 2 * WT_WORDS + 2 * e;
-}
 
 // Asks L2 for one unit's slices of the valid window rows: one thread per row slice of I or V.
 // `who` = index of the calling thread among those that ask (the first 2 * rows of them do).
@@ -1153,46 +1143,20 @@ window_wide_single_kernel(const __grid_constant__ mab_tensor t, int total_units,
 
 // ------------------------------------------------------------------------------------ launch
 
-// Threads of a CTA of the tile kernel; `fit`: how many CTAs' arrays fit an SM.  us of this kernel, fp32, 10 rows; the row loop has its
-// prefetching form while a row's entries do not outnumber the threads, and every tile in flight costs L2.
-//   k = 0.5 % (146 entries), 116 M elements: 256 threads 105, 384 108, 512 120.
-//   k = 1 % (291): 256 / 384 / 512 threads, 100 tiles 12.4 / 9.5 / 8.6, 300 tiles 18.8 / 15.5 / 18.6, 1000 55 / 42 / 44, 1500 77 / 61 / 61, 3000 143 / 124 /
-//   118, 4282 201 / 186 / 166; with weight decay 1000 82 / 70 / 73, 4282 292 / 322 / 268; 120 ragged tensors 33 / 30 / 35.
-//   The operator that writes every position's update: 384 (60 M elements k = 1 % 75, 256 and 512 threads 79; 0.5 % 59, 256 73, 512 67).
-//   The alpha forms have 80 registers a thread: 256 threads while three CTAs fit (33.5 M elements 121, 384 threads 127), 384 where two do (bf16, 20
-//   rows, 58 M elements 265 with 256, 209), and 512 where one does or an SM has no more than one tile (100 tiles 29 and 18).
-static int threads_of(bool write, bool alpha, int fit, int tiles, int max_k, int sms) {
-    if (alpha) return fit < 2 || tiles <= sms ? 512 : fit < 3 ? 384 : 256;
-    if (fit < 2) return 1024;
-    if (tiles <= 2 * sms || fit < 3) return 512;
-    if (write) return 384;
-    if (max_k <= 256 && fit >= 4) return 256;
-    return max_k <= 384 && tiles <= 10 * sms ? 384 : 512;
-}
-
 // MODE_WRITE_UPDATE: one tensor, passed by value (`single`); MODE_STEP: n_tensors descriptors in device memory.
 // units_tile / units_wide are the unit counts of the two variants; rows * max_k (the largest
 // k_block_size of the launch) decides which one runs.
 template <typename TP, int MODE, int ALPHA>
 static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* single, int n_tensors, int units_tile,
-                              int units_wide, int max_k, const WindowArgs& a, bool early, cudaStream_t s) {
+                              int units_wide, int max_k, const WindowArgs& a, bool behind_a, cudaStream_t s) {
     const int sms = device_sm_count();
-    // the tile variant while its compact arrays fit one CTA's shared memory (next to the kernel's static arrays)
-    const int smem_tile = (int64_t)a.rows * max_k <= WT_MAX_ENTRIES ? wt_smem_bytes(a.rows, max_k) : 0;
-    if (smem_tile > 0 && smem_tile + 4096 <= device_max_optin_smem()) {
-        // the forms with the alpha term: a dense array of 256 floats per warp behind the window's arrays, if it fits
-        const int fit = std::max(1, std::min(8, (227 * 1024) / (smem_tile + (ALPHA != 0 ? 8 * 1024 : 0) + 3072)));   // CTAs per SM by their arrays
-        int nt = threads_of(MODE == MODE_WRITE_UPDATE, ALPHA != 0, fit, units_tile, max_k, sms);
-        if (ALPHA != 0 && ((smem_tile + 15) & ~15) + nt * 32 + 4096 > device_max_optin_smem()) nt = 256;
-        const int dense = ALPHA != 0 ? nt * 32 : 0;
-        const int dense_at = ALPHA != 0 && ((smem_tile + 15) & ~15) + dense + 4096 <= device_max_optin_smem() ? (smem_tile + 15) & ~15 : 0;
-        const int smem = dense_at > 0 ? dense_at + dense : smem_tile;
-        const int per_sm = std::max(1, std::min(ALPHA != 0 ? 768 / nt : nt == 384 ? 3 : 1024 / nt, (227 * 1024) / (smem + 3072)));   // (as in __launch_bounds__)
-        const int grid = (int)std::min<int64_t>(units_tile, (int64_t)sms * per_sm);
+    const TileLaunch L = plan_tile_launch(MODE == MODE_WRITE_UPDATE, ALPHA != 0, a.rows, max_k, units_tile, behind_a, sms, device_max_optin_smem());
+    if (L.smem > 0) {
+        const int nt = L.threads;
         auto run = [&](auto kern, int threads) -> int {
-            MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-            if constexpr (MODE == MODE_WRITE_UPDATE) kern<<<grid, threads, smem, s>>>(*single, units_tile, max_k, a);
-            else MAB_CUDA_TRY(launch_behind_kernel(kern, grid, threads, smem, s, dev_tensors, n_tensors, units_tile, max_k, dense_at, a));
+            MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.smem));
+            if constexpr (MODE == MODE_WRITE_UPDATE) kern<<<L.grid, threads, L.smem, s>>>(*single, units_tile, max_k, a);
+            else MAB_CUDA_TRY(launch_behind_kernel(kern, L.grid, threads, L.smem, s, dev_tensors, n_tensors, units_tile, max_k, L.dense_at, a));
             return MAB_OK;
         };
         int rc;
@@ -1203,12 +1167,12 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
             else rc = run(window_tile_single_kernel<TP, MODE, 0, 256>, 256);
         } else if constexpr (ALPHA == 0) {
             if (nt == 1024) rc = run(window_tile_kernel<TP, MODE, 0, 1024>, 1024);
-            else if (nt == 512 && early) rc = run(window_tile_kernel<TP, MODE, 0, 512, true>, 512);
+            else if (nt == 512 && L.early) rc = run(window_tile_kernel<TP, MODE, 0, 512, true>, 512);
             else if (nt == 512) rc = run(window_tile_kernel<TP, MODE, 0, 512>, 512);
             else if (nt == 384) rc = run(window_tile_kernel<TP, MODE, 0, 384>, 384);
             else rc = run(window_tile_kernel<TP, MODE, 0, 256>, 256);
         } else {
-            if (nt == 512 && early) rc = run(window_tile_kernel<TP, MODE, ALPHA, 512, true>, 512);
+            if (nt == 512 && L.early) rc = run(window_tile_kernel<TP, MODE, ALPHA, 512, true>, 512);
             else if (nt == 512) rc = run(window_tile_kernel<TP, MODE, ALPHA, 512>, 512);
             else if (nt == 384) rc = run(window_tile_kernel<TP, MODE, ALPHA, 384>, 384);
             else rc = run(window_tile_kernel<TP, MODE, ALPHA, 256>, 256);
@@ -1234,12 +1198,12 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
 
 template <typename TP, int MODE>
 static int launch_window(const mab_tensor* dev_tensors, const mab_tensor* single, int n_tensors, int units_tile,
-                         int units_wide, int max_k, const WindowArgs& a, bool early, cudaStream_t s) {
+                         int units_wide, int max_k, const WindowArgs& a, bool behind_a, cudaStream_t s) {
     if constexpr (MODE == MODE_STEP) {
-        if (a.alpha == -2.0f) return launch_window_impl<TP, MODE, 2>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, early, s);
-        if (a.alpha != 0.0f) return launch_window_impl<TP, MODE, 1>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, early, s);
+        if (a.alpha == -2.0f) return launch_window_impl<TP, MODE, 2>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, behind_a, s);
+        if (a.alpha != 0.0f) return launch_window_impl<TP, MODE, 1>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, behind_a, s);
     }
-    return launch_window_impl<TP, MODE, 0>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, early, s);
+    return launch_window_impl<TP, MODE, 0>(dev_tensors, single, n_tensors, units_tile, units_wide, max_k, a, behind_a, s);
 }
 
 int fill_window_args(WindowArgs& a, int64_t steps, int m, double beta1, double beta2, double eps, float alpha, int qbs) {
@@ -1275,14 +1239,13 @@ static int resident_smem_bytes(int rows, int max_k, int max_dbs, int* tile_bytes
 
 int launch_window_step(const mab_tensor* dev_tensors, int n_tensors, int units_tile, int units_wide, int max_k, int max_dbs,
                        int param_dtype, const WindowArgs& a, bool behind_a, cudaStream_t s) {
-    const bool early = behind_a && units_tile <= EARLY_MAX_CTAS;
     if (param_dtype == MAB_F32)
-        return launch_window<float, MODE_STEP>(dev_tensors, nullptr, n_tensors, units_tile, units_wide, max_k, a, early, s);
+        return launch_window<float, MODE_STEP>(dev_tensors, nullptr, n_tensors, units_tile, units_wide, max_k, a, behind_a, s);
     int tile_bytes = 0;
     const int smem = (a.alpha == 0.0f) ? resident_smem_bytes(a.rows, max_k, max_dbs, &tile_bytes) : 0;
     if (smem > 0) {
         const int grid = (int)std::min<int64_t>(units_tile, (int64_t)device_sm_count() * 2);
-        auto kern = early ? window_resident_kernel<true> : window_resident_kernel<false>;
+        auto kern = behind_a && early_form(units_tile, grid) ? window_resident_kernel<true> : window_resident_kernel<false>;
         MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         MAB_CUDA_TRY(launch_behind_kernel(kern, grid, WR_THREADS, smem, s, dev_tensors, n_tensors, units_tile, max_k, tile_bytes, a));
         count_launch();
@@ -1290,7 +1253,7 @@ int launch_window_step(const mab_tensor* dev_tensors, int n_tensors, int units_t
         if (e != cudaSuccess) return cuda_fail(e, "window_resident_kernel launch");
         return MAB_OK;
     }
-    return launch_window<uint16_t, MODE_STEP>(dev_tensors, nullptr, n_tensors, units_tile, units_wide, max_k, a, early, s);
+    return launch_window<uint16_t, MODE_STEP>(dev_tensors, nullptr, n_tensors, units_tile, units_wide, max_k, a, behind_a, s);
 }
 
 // The give-up path of the bounded waits, exercised without any fault: the barrier is told to expect

@@ -1,0 +1,66 @@
+// How the update kernel's tile form is launched: threads, CTAs and shared memory by the window, the tiles and the GPU.  Host side only, so that
+// the choice can be checked without a GPU.
+#pragma once
+#include "window.cuh"
+#include "fused.cuh"
+
+namespace mab {
+
+constexpr int WT_WORDS = 1024;            // bitmap words of a tile (32768 positions)
+constexpr int WT_MAX_ENTRIES = 16384;     // window entries of one block the compact arrays may hold
+
+// Bytes one row's slice of I (or V) occupies in the raw staging area: the slice is copied from the
+// 16-byte boundary below its first element, in whole 16-byte pieces.
+__host__ __device__ constexpr int wt_row_stride(int max_k) { return ((max_k * 2 + 30) + 15) & ~15; }
+
+__host__ __device__ constexpr int wt_smem_bytes(int rows, int max_k) {
+    const int e = (rows * max_k + 3) & ~3;
+    return 8 * e + rows * 2 * wt_row_stride(max_k) + 4 * WT_WORDS + 2 * WT_WORDS + 2 * e;
+}
+
+// Threads of a CTA of the tile kernel; `fit`: how many CTAs' arrays fit an SM.  us of this kernel, fp32, 10 rows; the row loop has its
+// prefetching form while a row's entries do not outnumber the threads, and every tile in flight costs L2.
+//   k = 0.5 % (146 entries), 116 M elements: 256 threads 105, 384 108, 512 120.
+//   k = 1 % (291): 256 / 384 / 512 threads, 100 tiles 12.4 / 9.5 / 8.6, 300 tiles 18.8 / 15.5 / 18.6, 1000 55 / 42 / 44, 1500 77 / 61 / 61, 3000 143 / 124 /
+//   118, 4282 201 / 186 / 166; with weight decay 1000 82 / 70 / 73, 4282 292 / 322 / 268; 120 ragged tensors 33 / 30 / 35.
+//   The operator that writes every position's update: 384 (60 M elements k = 1 % 75, 256 and 512 threads 79; 0.5 % 59, 256 73, 512 67).
+//   The alpha forms have 80 registers a thread: 256 threads while three CTAs fit (33.5 M elements 121, 384 threads 127), 384 where two do (bf16, 20
+//   rows, 58 M elements 265 with 256, 209), and 512 where one does or an SM has no more than one tile (100 tiles 29 and 18).
+static inline int threads_of(bool write, bool alpha, int fit, int tiles, int max_k, int sms) {
+    if (alpha) return fit < 2 || tiles <= sms ? 512 : fit < 3 ? 384 : 256;
+    if (fit < 2) return 1024;
+    if (tiles <= 2 * sms || fit < 3) return 512;
+    if (write) return 384;
+    if (max_k <= 256 && fit >= 4) return 256;
+    return max_k <= 384 && tiles <= 10 * sms ? 384 : 512;
+}
+
+// The EARLY form (see wait_for_kernel_before): every CTA has one tile.  Not a matter of the tiles alone, and not of the chip's 148 SMs: a CTA that an
+// SM has to itself gets two tiles as soon as there are more tiles than the device shows SMs, a part of a GPU for instance.
+static inline bool early_form(int tiles, int grid) { return tiles <= grid && tiles <= EARLY_MAX_CTAS; }
+
+struct TileLaunch {
+    int  threads, grid, smem;             // smem 0: the window is too large for the compact arrays, the wide form takes it
+    int  dense_at;                        // the alpha forms' dense arrays of the warps in shared memory (0: they do not fit)
+    bool early;
+};
+
+static inline TileLaunch plan_tile_launch(bool write, bool alpha, int rows, int max_k, int tiles, bool behind_a, int sms, int optin_smem) {
+    TileLaunch L = {0, 0, 0, 0, false};
+    // while the compact arrays fit one CTA's shared memory (next to the kernel's static arrays)
+    const int smem_tile = (int64_t)rows * max_k <= WT_MAX_ENTRIES ? wt_smem_bytes(rows, max_k) : 0;
+    if (smem_tile == 0 || smem_tile + 4096 > optin_smem) return L;
+    // the forms with the alpha term: a dense array of 256 floats per warp behind the window's arrays, if it fits
+    const int fit = std::max(1, std::min(8, (227 * 1024) / (smem_tile + (alpha ? 8 * 1024 : 0) + 3072)));   // CTAs per SM by their arrays
+    L.threads = threads_of(write, alpha, fit, tiles, max_k, sms);
+    if (alpha && ((smem_tile + 15) & ~15) + L.threads * 32 + 4096 > optin_smem) L.threads = 256;
+    const int nt = L.threads, dense = alpha ? nt * 32 : 0;
+    L.dense_at = alpha && ((smem_tile + 15) & ~15) + dense + 4096 <= optin_smem ? (smem_tile + 15) & ~15 : 0;
+    L.smem = L.dense_at > 0 ? L.dense_at + dense : smem_tile;
+    const int per_sm = std::max(1, std::min(alpha ? 768 / nt : nt == 384 ? 3 : 1024 / nt, (227 * 1024) / (L.smem + 3072)));   // (as in __launch_bounds__)
+    L.grid = (int)std::min<int64_t>(tiles, (int64_t)sms * per_sm);
+    L.early = behind_a && nt == 512 && early_form(tiles, L.grid);
+    return L;
+}
+
+}  // namespace mab

@@ -1,0 +1,28 @@
+// plan_tile_launch (csrc/window_launch.cuh) on the host, over windows, tiles and GPUs with 148 SMs and fewer.  Prints the number of violations; exit
+// status 0 when there are none.
+#include "window_launch.cuh"
+
+int main() {
+    const int optin = 227 * 1024;
+    long long plans = 0, bad_early = 0;
+    int early_at_148 = 0;
+    for (int sms : {16, 37, 74, 132, 148, 160})
+        for (int rows : {1, 2, 3, 5, 10, 20, 32, 128})
+            for (int max_k = 1; max_k <= 16384 / rows; max_k += max_k < 400 ? 1 : 37)
+                for (int tiles : {1, 2, 15, 16, 17, 37, 38, 74, 75, 111, 132, 133, 147, 148, 149, 296, 297, 444, 445, 5000})
+                    for (int form = 0; form < 3; ++form) {
+                        const mab::TileLaunch L = mab::plan_tile_launch(form == 2, form == 1, rows, max_k, tiles, form != 2, sms, optin);
+                        if (L.smem == 0) continue;
+                        ++plans;
+                        // the form that starts before kernel A ends stages one tile's rows: a CTA must not get a second one
+                        bad_early += L.early && tiles > L.grid;
+                        early_at_148 += L.early && sms == 148 && rows == 10 && max_k == 291 && tiles == 148;
+                    }
+    for (int sms : {16, 37, 74, 132, 148})                   // the resident form, two CTAs per SM
+        for (int tiles = 1; tiles <= 400; ++tiles) {
+            const int grid = std::min(tiles, 2 * sms);
+            bad_early += mab::early_form(tiles, grid) && tiles > grid;
+        }
+    printf("plans %lld, early forms with more tiles than CTAs %lld\n", plans, bad_early);
+    return plans > 100000 && early_at_148 == 2 && bad_early == 0 ? 0 : 1;
+}
