@@ -1,5 +1,5 @@
 // Block top-k by itself (micro_adam.py:193-200): the positions of the k largest magnitudes of every block, ascending, ties to the lower
-// position.
+// position; NaN last.
 //
 // A block is not held anywhere: one pass over it leaves the maxima of its octets in registers (sixteen a thread), a bound of the k-th
 // magnitude is searched on them, and only the octets that reach the bound, one in eight or so, are read again, from L2.  Their values that
@@ -109,8 +109,17 @@ __device__ __forceinline__ int kth_bin(const int* hist, int& k_rem, int& size) {
     return bin;
 }
 
+// The `keep` lowest of the set bits (none where it is not positive).
+__device__ __forceinline__ uint32_t lowest_bits(uint32_t bits, int keep) {
+    if (keep <= 0) return 0u;
+    while (__popc(bits) > keep) bits &= ~(0x80000000u >> __clz(bits));
+    return bits;
+}
+
 // The selection at a cost that does not depend on the data (zeros, infinities, equal magnitudes, k beyond the octets, more candidates than the list
-// holds): the k-th key by digits of eight bits over the whole block, read anew every time, then masks of the larger and equal keys.
+// holds): the k-th key by digits of eight bits over the whole block, read anew every time, then masks of the larger and equal keys.  A NaN is
+// selected only where the block holds fewer than k numbers: a row has k different positions of its block always (left short, it would keep the end of
+// the row it replaces, whose positions may be the same again).
 // Every thread of the CTA calls.
 template <typename T, int NT>
 __device__ __noinline__ void select_general(const T* x, int n, int k, bool vec, Smem& ss, int16_t* out) {
@@ -132,7 +141,7 @@ __device__ __noinline__ void select_general(const T* x, int n, int k, bool vec, 
         }
         __syncthreads();
         int size;
-        const int bin = kth_bin(ss.hist, rem, size);         // (-1: fewer than k numbers; the smallest digit then, all zeros are taken)
+        const int bin = kth_bin(ss.hist, rem, size);         // (-1: fewer than k numbers; the smallest digit then, and all of them are taken)
         kth = (kth << width) | max(bin, 0);
     }
     for (int o = t; o < SEL_MAX_TILE / 8; o += NT) {
@@ -158,15 +167,32 @@ __device__ __noinline__ void select_general(const T* x, int n, int k, bool vec, 
     __syncthreads();
     const int larger = [&] { int all; block_exclusive_scan(cnt, ss.scan, all); return all; }();
     __syncthreads();
+    const int missing = k - larger - total;                  // > 0: fewer than k numbers, and every one of them is in a mask
     cnt = 0;
 #pragma unroll
     for (int i = 0; i < K_WPT; ++i) {
         const int keep = k - larger - before;                // the lowest positions among the equal ones
         before += __popc(tw[i]);
-        if (keep <= 0) tw[i] = 0u;
-        else while (__popc(tw[i]) > keep) tw[i] &= ~(0x80000000u >> __clz(tw[i]));
-        sel[i] |= tw[i];
+        sel[i] |= lowest_bits(tw[i], keep);
         cnt += __popc(sel[i]);
+    }
+    if (missing > 0) {                                       // uniform; the lowest positions that hold a NaN complete the row
+        int nans = 0;
+#pragma unroll
+        for (int i = 0; i < K_WPT; ++i) {
+            const int left = n - (t * K_WPT + i) * 32;
+            tw[i] = left >= 32 ? ~sel[i] : left > 0 ? ~sel[i] & ((1u << left) - 1u) : 0u;
+            nans += __popc(tw[i]);
+        }
+        before = block_exclusive_scan(nans, ss.scan, total);
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < K_WPT; ++i) {
+            const uint32_t add = lowest_bits(tw[i], missing - before);
+            before += __popc(tw[i]);
+            sel[i] |= add;
+            cnt += __popc(add);
+        }
     }
     int to = block_exclusive_scan(cnt, ss.scan, total);
 #pragma unroll

@@ -1,5 +1,6 @@
 """block_topk by itself, where its routes change: blocks and one more than there are SMs, blocks around an octet, k around the acceptance window's
-change and beyond the octets, more equal magnitudes than the candidate list or the direct ranking holds, infinities and NaN, x off alignment."""
+change and beyond the octets, more equal magnitudes than the candidate list or the direct ranking holds, infinities and NaN, fewer than k numbers in a
+block (NaN fill the row up, at the lowest positions), x off alignment."""
 import pytest
 import torch
 
@@ -25,7 +26,7 @@ def _expected(x, k_many, k_few):
 @pytest.mark.parametrize('kind,k,tail,skip', [
     ('normal', 291, 0, 0), ('normal', 291, 1, 0), ('normal', 1024, 8191, 1), ('normal', 1025, 8192, 2), ('normal', 3632, 15, 0), ('normal', 3633, 16, 3),
     ('ties', 1453, 17, 0), ('ties', 33, 4099, 0), ('scales', 291, 777, 4), ('inf', 291, 4096, 0), ('inf', 1, 9, 0), ('nan', 291, 4097, 0),
-    ('zeros', 291, 100, 0), ('cluster', 600, 64, 0)])
+    ('zeros', 291, 100, 0), ('cluster', 600, 64, 0), ('all_nan', 291, 33, 0), ('short', 291, 300, 1), ('short', 7264, 9, 0)])
 def test_block_topk_routes(dtype, kind, k, tail, skip):
     from ista_daslab_optimizers_b200 import _native as N
     for full in (2, N.get_sm_count(), N.get_sm_count() + 1):
@@ -45,11 +46,18 @@ def test_block_topk_routes(dtype, kind, k, tail, skip):
             x[:DBS] = 0.0
             x[DBS:2 * DBS] = 0.0
             x[DBS + 11:2 * DBS:4001] = 1e-3
+        elif kind == 'all_nan':                          # nothing else in the blocks, and in the short one behind them
+            x[DBS:] = float('nan')
+        elif kind == 'short':                            # one number fewer than k, zeros among them, and none
+            x[:DBS][torch.arange(DBS) % (DBS // (k - 1)) != 2] = float('nan')
+            x[:DBS][2 + DBS // (k - 1) * (k - 1):] = float('nan')
+            x[2:DBS // 2:DBS // (k - 1)] *= 0.0
+            x[DBS:2 * DBS] = float('nan')
         elif kind == 'cluster':
             x[1000:1000 + k] *= 300.0
         x = x.to(dtype)
         g = torch.empty(d + skip, dtype=dtype, device='cuda')[skip:].copy_(x)
-        out = torch.full((full * k + k_few + 8,), -7, dtype=torch.int16, device='cuda')
+        out = torch.full((full * k + k_few + 8,), -7, dtype=torch.int16, device='cuda')      # (what a row held before must not stay in it)
         N.block_topk(d, DBS, k, k_few, g, out[:full * k + k_few])
         assert torch.equal(out[:full * k + k_few].cpu(), _expected(x, k, k_few)), full
         assert (out[full * k + k_few:] == -7).all()
