@@ -463,15 +463,18 @@ ef_topk_quant_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int 
 int units_a_of(const mab_tensor& t) { return t.topk_full_blocks_count + (t.k_block_size_few > 0 ? 1 : 0); }
 
 // Blocks of 64 have two kernels.  us a launch, the one whose warps own their part of the tile and the other one, from 10 tiles per SM on (1480
-// tiles): k = 0.5 % 63 / 83, 1 % 63 / 72, 2 % 66 / 79, 5 % 82 / 99, 20 % 265 / 266, off alignment 85 / 85, with k = 5 % 106 / 112; 2960 tiles
-// k = 5 % 145 / 181, off alignment 150 / 152; k = 1 % with 31 and 50 tiles per SM 165 / 188 and 255 / 295.  Below, 1000 tiles 47 / 56, 444 tiles
-// 20.3 / 20.0, 72 tiles 12.1 / 12.2: the line could lie lower, at 6 tiles per SM or so.
+// tiles): k = 0.5 % 63 / 83, 1 % 63 / 72, 2 % 66 / 79, 5 % 82 / 99, 20 % 265 / 266; 2960 tiles k = 5 % 145 / 181; k = 1 % with 31 and 50 tiles per
+// SM 165 / 188 and 255 / 295.  Below, 1000 tiles 47 / 56, 444 tiles 20.3 / 20.0, 72 tiles 12.1 / 12.2: the line could lie lower, at 6 tiles per SM
+// or so.
+// A tile whose gradient the copy engine cannot move (off a 16-byte boundary) costs the first one more, the other one little: k = 1 %, 1480, 2960,
+// 4588 and 7400 tiles 95 / 84, 166 / 153, 248 / 222 and 391 / 349; 5 % 118 / 112, 206 / 201, 301 / 293, 467 / 475; 0.5 % 96 / 93, 166 / 169, 250 / 255,
+// 388 / 399 (a step of 7400 tiles all the same 497 / 481).  So a launch with more of those tiles than others takes the other one.
 constexpr int WARPS_MIN_TILES_PER_SM = 10;
 
 int launch_ef_topk_quant(const mab_tensor* dev_tensors, int n_tensors, int total_units, int grad_dtype,
-                         int qbs, int max_dbs, int max_k, cudaStream_t s, const LooseArgs* loose) {
+                         int qbs, int max_dbs, int max_k, int units_off, cudaStream_t s, const LooseArgs* loose) {
     if (grad_dtype == MAB_BF16) {          // bf16 tiles are small enough for two shared-memory resident CTAs per SM
-        const bool warps = loose != nullptr || qbs != 64 || total_units >= WARPS_MIN_TILES_PER_SM * device_sm_count();
+        const bool warps = loose != nullptr || qbs != 64 || (total_units >= WARPS_MIN_TILES_PER_SM * device_sm_count() && units_off <= total_units / 2);
         const int rc = warps ? launch_ef_topk_quant_bf16_warps(dev_tensors, n_tensors, total_units, qbs, max_dbs, s, loose)
                              : launch_ef_topk_quant_bf16(dev_tensors, n_tensors, total_units, max_dbs, s);
         if (rc <= 0) return rc;

@@ -82,7 +82,7 @@ MANY = (1400 * DBS, 7, DBS - 1, 513, 600 * DBS + 4104, 64, 65 * 64 + 15, 2 * DBS
 @pytest.mark.parametrize('kind,k_init,alpha', [('mixed', 0.005, 0), ('mixed', 0.01, 0), ('mixed', 0.02, 0), ('mixed', 0.01, -2),
                                                ('nan', 0.01, 0), ('inf', 0.01, 0)])
 def test_large_launch_equals_small_ones(kind, k_init, alpha):
-    """Blocks of 64: a step of more than 20 tiles per SM takes one form of the kernel, its tensors by themselves the other one."""
+    """Blocks of 64: a step of more than ten tiles per SM takes one form of the kernel, its tensors by themselves the other one."""
     from ista_daslab_optimizers_b200 import MicroAdam, _native
     hyper = dict(m=2, lr=1e-3, quant_block_size=64, k_init=k_init, alpha=alpha)
     gen = torch.Generator(device='cuda').manual_seed(7)
@@ -129,10 +129,10 @@ def test_large_launch_equals_small_ones(kind, k_init, alpha):
     assert _native.device_error() == 0
 
 
-@pytest.mark.parametrize('k_init,skip', [(0.05, 0), (0.01, 3), (0.05, 1), (0.2, 8)])
+@pytest.mark.parametrize('k_init,skip', [(0.05, 0), (0.01, 3), (0.05, 1), (0.2, 8), (0.01, 8), (0.01, -3)])
 def test_line_between_the_forms(k_init, skip):
-    """Blocks of 64: from ten tiles per SM on a launch takes the warp-owned form whatever k and alignment, below the other one;
-    equal results on both sides."""
+    """Blocks of 64: from ten tiles per SM on a launch takes the warp-owned form whatever k, but where most of the
+    gradients are off alignment (skip < 0: those of the short tensor only); below, the other one; equal results on both sides."""
     from ista_daslab_optimizers_b200 import MicroAdam, _native
     from ista_daslab_optimizers_b200.compat import ista_daslab_cuda_tools as tools
     tiles = 10 * tools.get_sm_count()
@@ -144,9 +144,10 @@ def test_line_between_the_forms(k_init, skip):
     opt, opts = MicroAdam(whole, **hyper), [MicroAdam([p], **hyper) for p in alone]
     for step in range(2):
         for p, q in zip(whole, alone):
-            p.grad = torch.empty(p.numel() + skip, dtype=torch.bfloat16, device='cuda')[skip:].normal_(0.0, 1e-3, generator=gen)
+            off = skip if skip >= 0 else -skip if p is whole[1] else 0
+            p.grad = torch.empty(p.numel() + off, dtype=torch.bfloat16, device='cuda')[off:].normal_(0.0, 1e-3, generator=gen)
             q.grad = p.grad.clone()
-        for form, o in (('ef_topk_quant_bf16_warps_kernel', opt), ('ef_topk_quant_bf16_kernel', opts[0])):
+        for form, o in (('ef_topk_quant_bf16_warps_kernel' if skip % 8 == 0 or skip < 0 else 'ef_topk_quant_bf16_kernel', opt), ('ef_topk_quant_bf16_kernel', opts[0])):
             if step == 0:
                 names = _kernels_of(o.step)
                 assert any(form in x for x in names), names
