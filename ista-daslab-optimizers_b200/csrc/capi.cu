@@ -248,7 +248,7 @@ static int fused_run(mab_tensor* tensors, int n, const mab_step_args* args, void
         for (const Chunk& c : chunks) {
             const LooseArgs la = {qbs, reinterpret_cast<uint32_t*>(ws + L.off_min), reinterpret_cast<uint32_t*>(ws + L.off_max),
                                   reinterpret_cast<const int64_t*>(ws + L.off_first) + c.first};
-            if (int rc = launch_ef_topk_quant(dev + c.first, c.count, c.units_a, c.grad_dtype, qbs, c.max_dbs, c.max_k, c.units_off, s, &la)) return rc;
+            if (int rc = launch_ef_topk_quant(dev + c.first, c.count, c.units_a, c.grad_dtype, qbs, c.max_dbs, c.max_k, c.units_off, 0, s, &la)) return rc;
         }
         for (const Chunk& c : chunks) {
             const LooseArgs la = {qbs, reinterpret_cast<uint32_t*>(ws + L.off_min), reinterpret_cast<uint32_t*>(ws + L.off_max),
@@ -256,8 +256,11 @@ static int fused_run(mab_tensor* tensors, int n, const mab_step_args* args, void
             if (int rc = launch_requant_loose(dev + c.first, c.count, c.units_a, c.grad_dtype, la, s)) return rc;
         }
     } else if (what & RUN_A) {
+        // (what follows the last kernel A is the first update, if this call runs it)
+        const Chunk& b = chunks[0];
+        const int allowing = (what & RUN_B) ? allowing_ctas(b.units_a, (int)std::min<int64_t>(args->steps, args->m), b.max_k, b.max_dbs, b.param_dtype, args->alpha) : 0;
         for (const Chunk& c : chunks)
-            if (int rc = launch_ef_topk_quant(dev + c.first, c.count, c.units_a, c.grad_dtype, args->quant_block_size, c.max_dbs, c.max_k, c.units_off, s)) return rc;
+            if (int rc = launch_ef_topk_quant(dev + c.first, c.count, c.units_a, c.grad_dtype, args->quant_block_size, c.max_dbs, c.max_k, c.units_off, allowing, s)) return rc;
     }
     if (what & RUN_B) {
         WindowArgs wa;
@@ -370,10 +373,12 @@ extern "C" int mab_fused_step_static(mab_tensor* tensors, int n, const mab_step_
     for (int first = 0; first < n;) first = static_run_end(tensors, n, first, &ua, &ub, &mk, &md, &off);
     MAB_CUDA_TRY(cudaMemcpyAsync(table, tensors, (size_t)n * sizeof(mab_tensor), cudaMemcpyHostToDevice, s));
     const mab_tensor* dev = reinterpret_cast<const mab_tensor*>(table);
-    // kernel A over every run, then kernel B over every run (the runs are recomputed, not stored)
+    // kernel A over every run, then kernel B over every run (the runs are recomputed, not stored); the first update follows the last kernel A
+    static_run_end(tensors, n, 0, &ua, &ub, &mk, &md, &off);
+    const int allowing = allowing_ctas(ua, wa.rows, mk, md, tensors[0].param_dtype, wa.alpha);
     for (int first = 0; first < n;) {
         const int end = static_run_end(tensors, n, first, &ua, &ub, &mk, &md, &off);
-        if (int rc = launch_ef_topk_quant(dev + first, end - first, ua, tensors[first].grad_dtype, args->quant_block_size, md, mk, off, s)) return rc;
+        if (int rc = launch_ef_topk_quant(dev + first, end - first, ua, tensors[first].grad_dtype, args->quant_block_size, md, mk, off, allowing, s)) return rc;
         first = end;
     }
     wa.probe = args->probe_out;

@@ -472,15 +472,15 @@ int units_a_of(const mab_tensor& t) { return t.topk_full_blocks_count + (t.k_blo
 constexpr int WARPS_MIN_TILES_PER_SM = 10;
 
 int launch_ef_topk_quant(const mab_tensor* dev_tensors, int n_tensors, int total_units, int grad_dtype,
-                         int qbs, int max_dbs, int max_k, int units_off, cudaStream_t s, const LooseArgs* loose) {
+                         int qbs, int max_dbs, int max_k, int units_off, int allowing, cudaStream_t s, const LooseArgs* loose) {
     if (grad_dtype == MAB_BF16) {          // bf16 tiles are small enough for two shared-memory resident CTAs per SM
         const bool warps = loose != nullptr || qbs != 64 || (total_units >= WARPS_MIN_TILES_PER_SM * device_sm_count() && units_off <= total_units / 2);
-        const int rc = warps ? launch_ef_topk_quant_bf16_warps(dev_tensors, n_tensors, total_units, qbs, max_dbs, s, loose)
-                             : launch_ef_topk_quant_bf16(dev_tensors, n_tensors, total_units, max_dbs, s);
+        const int rc = warps ? launch_ef_topk_quant_bf16_warps(dev_tensors, n_tensors, total_units, qbs, max_dbs, allowing, s, loose)
+                             : launch_ef_topk_quant_bf16(dev_tensors, n_tensors, total_units, max_dbs, allowing, s);
         if (rc <= 0) return rc;
     }
     if (grad_dtype == MAB_F32 && loose == nullptr) {   // two CTAs per SM while tile and candidates fit
-        const int rc = launch_ef_topk_quant_f32(dev_tensors, n_tensors, total_units, qbs, max_dbs, max_k, s);
+        const int rc = launch_ef_topk_quant_f32(dev_tensors, n_tensors, total_units, qbs, max_dbs, max_k, allowing, s);
         if (rc <= 0) return rc;
     }
     const int grid = (int)std::min<int64_t>(total_units, (int64_t)device_sm_count());

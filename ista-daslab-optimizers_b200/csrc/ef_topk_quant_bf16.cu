@@ -433,7 +433,7 @@ __device__ __forceinline__ void encode_phase(const uint4* tile4, const SmemSel& 
 }
 
 __global__ void __launch_bounds__(S_NT, S_CTAS)
-ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int stage_elems) {
+ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int stage_elems, int allowing) {
     constexpr int qshift = 6;                    // quantisation blocks of 64
     extern __shared__ __align__(128) unsigned char smem_raw[];       // [tile][SmemSel]
     __shared__ int s_first[S_MAX_TENSORS + 1];
@@ -442,7 +442,7 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
     uint4* tile4 = reinterpret_cast<uint4*>(smem_raw);
     SmemSel& ss = *reinterpret_cast<SmemSel*>(smem_raw + ((stage_elems * 2 + 127) & ~127));
     const int t = threadIdx.x, lane = lane_id(), warp = warp_id();
-    allow_next_kernel();
+    allow_next_kernel(allowing);
     for (int i = t; i < n_tensors; i += S_NT) s_first[i] = tensors[i].first_unit_a;
     if (t == 0) { s_first[n_tensors] = total_units; mbar_init(&s_bar, 1); ss.ctrl[5] = 0; ss.ctrl[6] = 0; }
     __syncthreads();
@@ -937,13 +937,13 @@ ef_topk_quant_bf16_kernel(const mab_tensor* __restrict__ tensors, int n_tensors,
     }
 }
 
-int launch_ef_topk_quant_bf16(const mab_tensor* dev_tensors, int n_tensors, int total_units, int max_dbs, cudaStream_t s) {
+int launch_ef_topk_quant_bf16(const mab_tensor* dev_tensors, int n_tensors, int total_units, int max_dbs, int allowing, cudaStream_t s) {
     const int smem = ((max_dbs * 2 + 127) & ~127) + (int)sizeof(SmemSel);
     const int per_sm = std::min(S_CTAS, (device_max_optin_smem() + 1024) / (smem + 3 * 1024 + 128));
     if (per_sm < 2) return 1;                                // not even two CTAs per SM: the caller uses the other kernel
     const int grid = (int)std::min<int64_t>(total_units, (int64_t)device_sm_count() * per_sm);
     MAB_CUDA_TRY(cudaFuncSetAttribute(ef_topk_quant_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    ef_topk_quant_bf16_kernel<<<grid, S_NT, smem, s>>>(dev_tensors, n_tensors, total_units, max_dbs);
+    ef_topk_quant_bf16_kernel<<<grid, S_NT, smem, s>>>(dev_tensors, n_tensors, total_units, max_dbs, allowing);
     count_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "ef_topk_quant_bf16_kernel launch");

@@ -683,7 +683,7 @@ __device__ __forceinline__ void residual_and_extremes(const uint16_t* tile, int 
 // every block it touches merged into la.st_min / la.st_max (requant_loose.cu finishes the job).
 template <int QS>
 __global__ void __launch_bounds__(S_NT, S_CTAS)
-ef_topk_quant_bf16_warps_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int stage_elems, LooseArgs la) {
+ef_topk_quant_bf16_warps_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int stage_elems, int allowing, LooseArgs la) {
     constexpr bool LOOSE = QS == 0;
     constexpr bool TABLE = LOOSE || QS >= 6;                 // constants of the warp's blocks from a table, else per unit
     extern __shared__ __align__(128) unsigned char smem_raw[];       // [tile][SmemSel]
@@ -693,7 +693,7 @@ ef_topk_quant_bf16_warps_kernel(const mab_tensor* __restrict__ tensors, int n_te
     uint4* const tile4 = reinterpret_cast<uint4*>(smem_raw);
     SmemSel& ss = *reinterpret_cast<SmemSel*>(smem_raw + ((stage_elems * 2 + 127) & ~127));
     const int t = threadIdx.x, lane = lane_id(), warp = warp_id();
-    if constexpr (!LOOSE) allow_next_kernel();
+    if constexpr (!LOOSE) allow_next_kernel(allowing);
     // a CTA's tiles are neighbours: they mostly belong to one tensor, whose bound carries over from tile to tile
     const TileRange range = tiles_of_cta(total_units, gridDim.x, blockIdx.x);
     const int unit0 = range.first, unit1 = range.end;
@@ -1086,7 +1086,7 @@ ef_topk_quant_bf16_warps_kernel(const mab_tensor* __restrict__ tensors, int n_te
 
 }  // namespace warps
 
-int launch_ef_topk_quant_bf16_warps(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, cudaStream_t s,
+int launch_ef_topk_quant_bf16_warps(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, int allowing, cudaStream_t s,
                               const LooseArgs* loose) {
     using namespace warps;
     const int smem = ((max_dbs * 2 + 127) & ~127) + (int)sizeof(SmemSel);
@@ -1097,7 +1097,7 @@ int launch_ef_topk_quant_bf16_warps(const mab_tensor* dev_tensors, int n_tensors
     if (loose) la = *loose;
     auto run = [&](auto kern) -> int {
         MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        kern<<<grid, S_NT, smem, s>>>(dev_tensors, n_tensors, total_units, max_dbs, la);
+        kern<<<grid, S_NT, smem, s>>>(dev_tensors, n_tensors, total_units, max_dbs, allowing, la);
         return MAB_OK;
     };
     const int rc = loose ? run(ef_topk_quant_bf16_warps_kernel<0>)

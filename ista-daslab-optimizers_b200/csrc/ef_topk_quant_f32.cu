@@ -270,7 +270,7 @@ __device__ __forceinline__ void f32_resolve(uint32_t (&sel)[F_WPT], uint32_t (&t
 }
 
 __global__ void __launch_bounds__(F_NT, F_CTAS)
-ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int qshift, int tile_bytes) {
+ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int qshift, int tile_bytes, int allowing) {
     extern __shared__ __align__(128) unsigned char smem_raw[];       // [tile elements from F_REG_ELEMS on][SmemF]
     __shared__ int s_first[WIN_MAX_TENSORS + 1];
     __shared__ __align__(8) uint64_t s_bar;
@@ -278,7 +278,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
     float4* tile4 = reinterpret_cast<float4*>(smem_raw);
     SmemF& ss = *reinterpret_cast<SmemF*>(smem_raw + tile_bytes);
     const int t = threadIdx.x, lane = lane_id(), warp = warp_id();
-    allow_next_kernel();
+    allow_next_kernel(allowing);
     for (int i = t; i < n_tensors; i += F_NT) s_first[i] = tensors[i].first_unit_a;
     if (t == 0) { s_first[n_tensors] = total_units; mbar_init(&s_bar, 1); ss.slow = 0; }
     __syncthreads();
@@ -847,7 +847,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
 // independent values holds about -3632 ln(1 - c / 3632) candidates, 2648 at c = 1880 and 3069 at c = 1880 + 192 (means: a
 // tile that comes out above the list's 3072 goes to the bisection).  The one-tile kernel, whose
 // list is longer, is the faster one from there on (k = 2325: 1165 us a step of 67 M elements, most of it in kernel B).
-int launch_ef_topk_quant_f32(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, int max_k, cudaStream_t s) {
+int launch_ef_topk_quant_f32(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, int max_k, int allowing, cudaStream_t s) {
     int qshift = 0;
     while ((1 << qshift) < qbs) ++qshift;
     const int tile_bytes = (std::max(0, ((max_dbs + 7) & ~7) - F_REG_ELEMS) * 4 + 127) & ~127;
@@ -856,7 +856,7 @@ int launch_ef_topk_quant_f32(const mab_tensor* dev_tensors, int n_tensors, int t
     if (max_k > F_MAX_K || F_CTAS * (smem + fixed) > device_max_optin_smem() + 1024) return 1;
     const int grid = (int)std::min<int64_t>(total_units, (int64_t)device_sm_count() * F_CTAS);
     MAB_CUDA_TRY(cudaFuncSetAttribute(ef_topk_quant_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    ef_topk_quant_f32_kernel<<<grid, F_NT, smem, s>>>(dev_tensors, n_tensors, total_units, qshift, tile_bytes);
+    ef_topk_quant_f32_kernel<<<grid, F_NT, smem, s>>>(dev_tensors, n_tensors, total_units, qshift, tile_bytes, allowing);
     count_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "ef_topk_quant_f32_kernel launch");

@@ -33,17 +33,17 @@ __host__ __device__ __forceinline__ TileRange tiles_of_cta(int total, int ctas, 
 
 // The update kernel of a step is launched behind kernel A without the gap between two kernels (programmatic stream
 // serialization): its CTAs read the descriptor table, which neither kernel writes, and wait there for kernel A's end and its
-// results.  A kernel A of at most as many CTAs as a B200 has SMs (148) allows it as soon as all its CTAs have started; with more the
-// ones that wait take places unevenly among those that work, and the update runs on fewer SMs than it could (fp32, 254 tiles 72.8 us a step
-// allowed, 55.5 not).  Kernel A of loose blocks does not allow it, the requantisation being next; nor do the requantisation and the fp32 kernel
-// with one tile per SM (not tried there).
+// results.  A kernel A allows it as soon as all its CTAs have started, if it has no more CTAs than there are SMs and the update is of the form below, or
+// no more than half as many; with more the ones that wait take places unevenly among those that work, and the update runs on fewer SMs than it
+// could (us a step, allowed and not: fp32, 254 tiles 72.8 and 55.5; the wide form of the update behind 100 tiles, 20 rows of 5 %, bf16 73.3 and
+// 63.6, fp32 65.5 and 55.4).  Kernel A of loose blocks does not allow it, the requantisation being next; nor do the requantisation and the fp32
+// kernel with one tile per SM (not tried there).
 // What does not depend on kernel A comes before that wait where every CTA of the update has one tile (template flag EARLY): the other rows of
 // the window are staged and marked, the weight decay is applied, or the bf16 parameters are on their way into shared memory; the row
 // that kernel A writes follows behind the wait.  Kernel A itself is an ordinary launch, so everything before it is complete.  us a step, everything
 // behind the wait and so: 7 690 fp32 elements 20.5 / 18.5, 40 tiles fp32 24.6 / 22.6, with weight decay 28 / 22.6, bf16 22.6 / 20.9; not allowed
 // and so: 80 tiles bf16 22.6 / 21.9, 100 fp32 with weight decay 28.7 / 26.7, 110 with 20 rows 28.7 / 27.1, 148 fp32 26.5 / 25.5, bf16 22.7 / 22.6.
-constexpr int EARLY_MAX_CTAS = 148;            // (how many CTAs kernel A may have; the update's own grid decides as well: early_form)
-__device__ __forceinline__ void allow_next_kernel() { if (gridDim.x <= EARLY_MAX_CTAS) asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void allow_next_kernel(int most_ctas) { if ((int)gridDim.x <= most_ctas) asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... P, typename... A>
@@ -61,6 +61,7 @@ static inline cudaError_t launch_behind_kernel(void (*kern)(P...), int grid, int
 int fill_window_args(WindowArgs& a, int64_t steps, int m, double beta1, double beta2, double eps, float alpha, int qbs);
 int launch_window_step(const mab_tensor* dev_tensors, int n_tensors, int units_tile, int units_wide, int max_k, int max_dbs,
                        int param_dtype, const WindowArgs& a, bool behind_a, cudaStream_t s);
+int allowing_ctas(int units_tile, int rows, int max_k, int max_dbs, int param_dtype, float alpha);   // most CTAs of a kernel A that allows such an update
 int units_b_of(const mab_tensor& t);
 int launch_wait_selftest(int probe_limit, cudaStream_t s);
 
@@ -103,9 +104,9 @@ __host__ __device__ __forceinline__ int loose_blocks_touched(int lrem0, int n, i
     return loose_block(lrem0 + n - 1, qbs, false) + 1;
 }
 
-// ef_topk_quant.cu; units_off: tiles of gradients that start off a 16-byte boundary
+// ef_topk_quant.cu; units_off: tiles of gradients that start off a 16-byte boundary; allowing: see allow_next_kernel
 int launch_ef_topk_quant(const mab_tensor* dev_tensors, int n_tensors, int total_units, int grad_dtype,
-                         int qbs, int max_dbs, int max_k, int units_off, cudaStream_t s, const LooseArgs* loose = nullptr);
+                         int qbs, int max_dbs, int max_k, int units_off, int allowing, cudaStream_t s, const LooseArgs* loose = nullptr);
 int units_a_of(const mab_tensor& t);
 
 // requant_loose.cu: statistics (bf16) and codes of the residual kernel A left in the gradient buffers
@@ -114,12 +115,12 @@ int launch_requant_loose(const mab_tensor* dev_tensors, int n_tensors, int total
 
 // ef_topk_quant_bf16.cu (blocks of 64) and ef_topk_quant_bf16_warps.cu (all others, and large launches): return 1 (without
 // launching) when two CTAs of their shared memory do not fit an SM
-int launch_ef_topk_quant_bf16(const mab_tensor* dev_tensors, int n_tensors, int total_units, int max_dbs, cudaStream_t s);
-int launch_ef_topk_quant_bf16_warps(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, cudaStream_t s,
+int launch_ef_topk_quant_bf16(const mab_tensor* dev_tensors, int n_tensors, int total_units, int max_dbs, int allowing, cudaStream_t s);
+int launch_ef_topk_quant_bf16_warps(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, int allowing, cudaStream_t s,
                                     const LooseArgs* loose);
 
 // ef_topk_quant_f32.cu: returns 1 (without launching) where the tile or its candidates do not fit
-int launch_ef_topk_quant_f32(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, int max_k, cudaStream_t s);
+int launch_ef_topk_quant_f32(const mab_tensor* dev_tensors, int n_tensors, int total_units, int qbs, int max_dbs, int max_k, int allowing, cudaStream_t s);
 
 // Each kernel file keeps its own "a bounded wait gave up" flag (no relocatable device code): these read
 // it into *out and optionally clear it.

@@ -1228,13 +1228,9 @@ int fill_window_args(WindowArgs& a, int64_t steps, int m, double beta1, double b
     return MAB_OK;
 }
 
-// Shared memory of one CTA of the resident-tile kernel, or 0 when two such CTAs do not fit an SM.
-static int resident_smem_bytes(int rows, int max_k, int max_dbs, int* tile_bytes) {
-    *tile_bytes = (max_dbs * 2 + 127) & ~127;
-    if ((int64_t)rows * max_k > WT_MAX_ENTRIES) return 0;
-    const int smem = *tile_bytes + wt_smem_bytes(rows, max_k);
-    const int static_and_reserved = 6 * 1024;                 // the kernel's static arrays + the per-CTA reservation
-    return 2 * (smem + static_and_reserved) <= device_max_optin_smem() + 1024 ? smem : 0;
+int allowing_ctas(int units_tile, int rows, int max_k, int max_dbs, int param_dtype, float alpha) {
+    const int sms = device_sm_count();
+    return update_is_early(units_tile, rows, max_k, max_dbs, param_dtype == MAB_BF16, alpha != 0.0f, sms, device_max_optin_smem()) ? sms : sms / 2;
 }
 
 int launch_window_step(const mab_tensor* dev_tensors, int n_tensors, int units_tile, int units_wide, int max_k, int max_dbs,
@@ -1242,10 +1238,10 @@ int launch_window_step(const mab_tensor* dev_tensors, int n_tensors, int units_t
     if (param_dtype == MAB_F32)
         return launch_window<float, MODE_STEP>(dev_tensors, nullptr, n_tensors, units_tile, units_wide, max_k, a, behind_a, s);
     int tile_bytes = 0;
-    const int smem = (a.alpha == 0.0f) ? resident_smem_bytes(a.rows, max_k, max_dbs, &tile_bytes) : 0;
+    const int smem = (a.alpha == 0.0f) ? resident_smem_bytes(a.rows, max_k, max_dbs, device_max_optin_smem(), &tile_bytes) : 0;
     if (smem > 0) {
-        const int grid = (int)std::min<int64_t>(units_tile, (int64_t)device_sm_count() * 2);
-        auto kern = behind_a && early_form(units_tile, grid) ? window_resident_kernel<true> : window_resident_kernel<false>;
+        const int sms = device_sm_count(), grid = std::min(units_tile, sms * 2);
+        auto kern = behind_a && early_form(units_tile, grid, sms) ? window_resident_kernel<true> : window_resident_kernel<false>;
         MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         MAB_CUDA_TRY(launch_behind_kernel(kern, grid, WR_THREADS, smem, s, dev_tensors, n_tensors, units_tile, max_k, tile_bytes, a));
         count_launch();

@@ -35,9 +35,9 @@ static inline int threads_of(bool write, bool alpha, int fit, int tiles, int max
     return max_k <= 384 && tiles <= 10 * sms ? 384 : 512;
 }
 
-// The EARLY form (see wait_for_kernel_before): every CTA has one tile.  Not a matter of the tiles alone, and not of the chip's 148 SMs: a CTA that an
-// SM has to itself gets two tiles as soon as there are more tiles than the device shows SMs, a part of a GPU for instance.
-static inline bool early_form(int tiles, int grid) { return tiles <= grid && tiles <= EARLY_MAX_CTAS; }
+// The EARLY form (see wait_for_kernel_before): every CTA has one tile, and kernel A no more CTAs than there are SMs.  Not a matter of the tiles alone: a
+// CTA that an SM has to itself gets two tiles as soon as there are more tiles than the device shows SMs, a part of a GPU for instance.
+static inline bool early_form(int tiles, int grid, int sms) { return tiles <= grid && tiles <= sms; }
 
 struct TileLaunch {
     int  threads, grid, smem;             // smem 0: the window is too large for the compact arrays, the wide form takes it
@@ -59,8 +59,24 @@ static inline TileLaunch plan_tile_launch(bool write, bool alpha, int rows, int 
     L.smem = L.dense_at > 0 ? L.dense_at + dense : smem_tile;
     const int per_sm = std::max(1, std::min(alpha ? 768 / nt : nt == 384 ? 3 : 1024 / nt, (227 * 1024) / (L.smem + 3072)));   // (as in __launch_bounds__)
     L.grid = (int)std::min<int64_t>(tiles, (int64_t)sms * per_sm);
-    L.early = behind_a && nt == 512 && early_form(tiles, L.grid);
+    L.early = behind_a && nt == 512 && early_form(tiles, L.grid, sms);
     return L;
+}
+
+// Shared memory of one CTA of the resident-tile kernel, or 0 when two such CTAs do not fit an SM.
+static inline int resident_smem_bytes(int rows, int max_k, int max_dbs, int optin_smem, int* tile_bytes) {
+    *tile_bytes = (max_dbs * 2 + 127) & ~127;
+    if ((int64_t)rows * max_k > WT_MAX_ENTRIES) return 0;
+    const int smem = *tile_bytes + wt_smem_bytes(rows, max_k);
+    const int static_and_reserved = 6 * 1024;                 // the kernel's static arrays + the per-CTA reservation
+    return 2 * (smem + static_and_reserved) <= optin_smem + 1024 ? smem : 0;
+}
+
+// Whether the update of a step on such tensors takes the EARLY form.
+static inline bool update_is_early(int tiles, int rows, int max_k, int max_dbs, bool bf16, bool alpha, int sms, int optin_smem) {
+    int tile_bytes;
+    if (bf16 && !alpha && resident_smem_bytes(rows, max_k, max_dbs, optin_smem, &tile_bytes) > 0) return early_form(tiles, std::min(tiles, 2 * sms), sms);
+    return plan_tile_launch(false, alpha, rows, max_k, tiles, true, sms, optin_smem).early;
 }
 
 }  // namespace mab

@@ -21,8 +21,23 @@ int main() {
     for (int sms : {16, 37, 74, 132, 148})                   // the resident form, two CTAs per SM
         for (int tiles = 1; tiles <= 400; ++tiles) {
             const int grid = std::min(tiles, 2 * sms);
-            bad_early += mab::early_form(tiles, grid) && tiles > grid;
+            bad_early += mab::early_form(tiles, grid, sms) && tiles > grid;
         }
-    printf("plans %lld, early forms with more tiles than CTAs %lld\n", plans, bad_early);
-    return plans > 100000 && early_at_148 == 2 && bad_early == 0 ? 0 : 1;
+    // what kernel A may let start early with up to a CTA per SM: tile and resident forms with a tile per CTA, neither the wide form (20 rows of 5 %) nor
+    // one CTA of 1024 threads per SM
+    const int dbs = 29056;
+    bool form_ok = true;
+    for (int sms : {74, 132, 148})
+        for (int tiles : {sms / 2, sms, sms + 1}) {
+            const bool one = tiles <= sms;
+            form_ok = form_ok && mab::update_is_early(tiles, 10, 291, dbs, true, false, sms, optin) == one;
+            form_ok = form_ok && mab::update_is_early(tiles, 10, 291, dbs, false, false, sms, optin) == one;
+            form_ok = form_ok && mab::update_is_early(tiles, 10, 291, dbs, true, true, sms, optin) == one;
+            for (bool bf16 : {false, true}) {
+                form_ok = form_ok && !mab::update_is_early(tiles, 20, 1453, dbs, bf16, false, sms, optin) && !mab::update_is_early(tiles, 5, 14528, dbs, bf16, true, sms, optin);
+                form_ok = form_ok && !mab::update_is_early(tiles, 10, 1453, dbs, bf16, false, sms, optin);
+            }
+        }
+    printf("plans %lld, early forms with more tiles than CTAs %lld, what may start early %s\n", plans, bad_early, form_ok ? "right" : "wrong");
+    return form_ok && plans > 100000 && early_at_148 == 2 && bad_early == 0 ? 0 : 1;
 }
