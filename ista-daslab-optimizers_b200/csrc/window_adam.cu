@@ -12,6 +12,7 @@
 //    window phase overlaps the others' streaming.
 //  * wide kernel (window too large for the compact arrays, e.g. m = 20 with k = 5 %): one CTA per
 //    sub-range of a block with dense accumulators (window.cuh).
+#include <type_traits>
 #include "common.cuh"
 #include "window.cuh"
 #include "window_launch.cuh"
@@ -92,8 +93,7 @@ __device__ __forceinline__ bool decay_is_identity_bf16(float decay) {
 
 // p <- round_p(round_p(p * decay) - lr * u) for 8 values, two per instruction (packed f32x2
 // operations round each component like the scalar ones).
-// HAS_U = false: only the decay (the caller updates the few touched elements afterwards).
-template <typename TP, bool HAS_U = true>
+template <typename TP>
 __device__ __forceinline__ void update_octet(float (&pv)[8], const float (&u)[8], bool do_decay, float2 decay2, float2 neg_lr2) {
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
@@ -105,7 +105,7 @@ __device__ __forceinline__ void update_octet(float (&pv)[8], const float (&u)[8]
                 x = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
             }
         }
-        if (HAS_U) x = __ffma2_rn(neg_lr2, make_float2(u[2 * b], u[2 * b + 1]), x);
+        x = __ffma2_rn(neg_lr2, make_float2(u[2 * b], u[2 * b + 1]), x);
         pv[2 * b] = x.x; pv[2 * b + 1] = x.y;
     }
 }
@@ -738,31 +738,36 @@ __device__ __forceinline__ int window_tile_moments(const mab_tensor& T, int blk,
     return touched;
 }
 
-// p <- round_p(p * decay) on p[0, len), by the NT threads of the CTA.  Out of line: inline, at both places that call it, it cost 360 bytes of spills.
+// 16 bytes of parameters times the decay.
+__device__ __forceinline__ float4 decayed(float4 x, float decay) {
+    return make_float4(__fmul_rn(x.x, decay), __fmul_rn(x.y, decay), __fmul_rn(x.z, decay), __fmul_rn(x.w, decay));
+}
+__device__ __forceinline__ uint4 decayed(uint4 x, float decay) {
+    auto pair = [&](uint32_t w) { return pack_bf16x2_rne(__fmul_rn(__uint_as_float(w << 16), decay), __fmul_rn(__uint_as_float(w & 0xFFFF0000u), decay)); };
+    return make_uint4(pair(x.x), pair(x.y), pair(x.z), pair(x.w));
+}
+
+// p <- round_p(p * decay) on p[0, len), by the NT threads of the CTA: 16 bytes a lane from the first 16-byte boundary on, the elements around them one
+// by one, read before.  us a step of 63.9 M elements, fp32 with bf16 gradients, windows of 10 rows of 5 %: 428, with 32 bytes a lane 451; 10 rows of
+// 1 % on a shard that starts 4 bytes off such a boundary 250, element by element from end to end 315 (296 where all of it was asked into L2 before).
+// Out of line: inline, at both places that call it, it cost 360 bytes of spills.
 template <typename TP, int NT>
 __device__ __noinline__ void decay_tile(TP* p, int len, float decay) {
-    const float2 decay2 = make_float2(decay, decay), zero2 = make_float2(0.0f, 0.0f);
-    int done = 0;
-    if (aligned16(p)) {
-        constexpr int B = sizeof(TP) == 2 ? 4 : 2;           // octets a thread has in flight
-        const int full = len >> 3;
-        for (int o0 = threadIdx.x; o0 < full; o0 += NT * B) {
-            RawOctet<TP> x[B];
+    using V = typename std::conditional<sizeof(TP) == 4, float4, uint4>::type;
+    constexpr int N = 16 / (int)sizeof(TP), B = 4;           // elements of a vector, vectors a thread has in flight
+    const int head = min(len, (int)((0u - (uint32_t)reinterpret_cast<uintptr_t>(p)) & 15u) / (int)sizeof(TP));
+    const int whole = (len - head) / N, around = len - whole * N;   // (around: fewer than 16, a thread each)
+    V* const q = reinterpret_cast<V*>(p + head);
+    TP* const edge = (int)threadIdx.x < head ? p + threadIdx.x : p + whole * N + threadIdx.x;
+    const float edge_v = (int)threadIdx.x < around ? Elem<TP>::load(edge, 0) : 0.0f;
+    for (int o0 = threadIdx.x; o0 < whole; o0 += NT * B) {
+        V x[B];
 #pragma unroll
-            for (int i = 0; i < B; ++i) if (o0 + NT * i < full) x[i].load(p + (o0 + NT * i) * 8);
+        for (int i = 0; i < B; ++i) if (o0 + NT * i < whole) x[i] = q[o0 + NT * i];
 #pragma unroll
-            for (int i = 0; i < B; ++i)
-                if (o0 + NT * i < full) {
-                    float v[8], u[8];
-                    x[i].unpack(v);
-                    update_octet<TP, false>(v, u, true, decay2, zero2);
-                    Octet<TP>::store(p + (o0 + NT * i) * 8, v, true, 8);
-                }
-        }
-        done = full * 8;
+        for (int i = 0; i < B; ++i) if (o0 + NT * i < whole) q[o0 + NT * i] = decayed(x[i], decay);
     }
-#pragma unroll 4
-    for (int i = done + threadIdx.x; i < len; i += NT) Elem<TP>::store(p, i, __fmul_rn(Elem<TP>::load(p, i), decay));
+    if ((int)threadIdx.x < around) Elem<TP>::store(edge, 0, __fmul_rn(edge_v, decay));
 }
 
 template <typename TP, int MODE, int ALPHA, int NT, bool EARLY>

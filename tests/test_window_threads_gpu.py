@@ -32,3 +32,28 @@ def test_many_tiles_equal_single_tiles(rows, k, per_sm, alpha, weight_decay, dty
             assert opt.state[whole[0]]['k_block_size_many'] == k
             assert torch.equal(whole[i].detach()[at:at + q.numel()].view(torch.uint8), q.detach().view(torch.uint8)), (step, i, at)
     assert _native.device_error() == 0
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize('skip', [0, 1, 2, 3, 5, 7])
+def test_decay_of_slices_that_start_anywhere(dtype, skip):
+    """The weight decay alone (zero gradients): parameters that start anywhere in a buffer, shorter than the elements before the first vector and longer
+    than a block.  Exact: one rounded product per step, and what lies around the slices stays.  (bf16 windows of more than a few rows of 5 %
+    leave the form that keeps the block in shared memory.)"""
+    from ista_daslab_optimizers_b200 import MicroAdam, _native
+    sizes = (1, 2, 3, 7, 8, 9, 15, 16, 17, 250, DBS - 1, DBS, DBS + 1, 3 * DBS + 21)
+    gen = torch.Generator(device='cuda').manual_seed(skip)
+    buffers = [torch.empty(n + skip + 9, dtype=dtype, device='cuda').normal_(0.0, 0.02, generator=gen) for n in sizes]
+    params = [torch.nn.Parameter(b[skip:skip + n]) for b, n in zip(buffers, sizes)]
+    expected = [b.clone() for b in buffers]
+    opt = MicroAdam(params, m=10, lr=1e-2, quant_block_size=64, k_init=0.05, weight_decay=1.0)
+    decay = torch.tensor(1.0 - 1e-2, dtype=torch.float32, device='cuda')
+    for step in range(11):
+        for p in params:
+            p.grad = torch.zeros_like(p)
+        opt.step()
+        for e, n in zip(expected, sizes):
+            e[skip:skip + n] = (e[skip:skip + n].float() * decay).to(dtype)
+        for b, e in zip(buffers, expected):
+            assert torch.equal(b.view(torch.uint8), e.view(torch.uint8)), (step, b.numel())
+    assert _native.device_error() == 0
