@@ -38,21 +38,23 @@ struct __align__(16) Smem {
     };
     unsigned long long member[32];
     int hist[256];
-    int rot[64];
+    int rot[64];                             // octets at each threshold of the search; [63]: candidates above a tied bound
     int scan[36];
     int n_member, n_cand, kmax;
 };
 
-template <typename T> struct Octet;
+template <typename T> struct Octet;           // eight values as they are in memory
 template <> struct Octet<float> {
-    __device__ __forceinline__ static void load(const float* p, float (&v)[8]) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    float4 a, b;
+    __device__ __forceinline__ void load(const float* p) { a = __ldg(reinterpret_cast<const float4*>(p)); b = __ldg(reinterpret_cast<const float4*>(p) + 1); }
+    __device__ __forceinline__ void values(float (&v)[8]) const {
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     }
 };
 template <> struct Octet<uint16_t> {
-    __device__ __forceinline__ static void load(const uint16_t* p, float (&v)[8]) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4*>(p));
+    uint4 a;
+    __device__ __forceinline__ void load(const uint16_t* p) { a = __ldg(reinterpret_cast<const uint4*>(p)); }
+    __device__ __forceinline__ void values(float (&v)[8]) const {
         v[0] = __uint_as_float(a.x << 16); v[1] = __uint_as_float(a.x & 0xFFFF0000u);
         v[2] = __uint_as_float(a.y << 16); v[3] = __uint_as_float(a.y & 0xFFFF0000u);
         v[4] = __uint_as_float(a.z << 16); v[5] = __uint_as_float(a.z & 0xFFFF0000u);
@@ -64,7 +66,9 @@ template <> struct Octet<uint16_t> {
 template <typename T>
 __device__ __forceinline__ void load_octet(const T* x, int o, int n, bool vec, float (&v)[8]) {
     if (vec && o * 8 + 8 <= n) {
-        Octet<T>::load(x + o * 8, v);
+        Octet<T> r;
+        r.load(x + o * 8);
+        r.values(v);
     } else {
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = o * 8 + e < n ? Elem<T>::load(x, o * 8 + e) : 0.0f;
@@ -116,48 +120,68 @@ __device__ __forceinline__ uint32_t lowest_bits(uint32_t bits, int keep) {
     return bits;
 }
 
-// The selection at a cost that does not depend on the data (zeros, infinities, equal magnitudes, k beyond the octets, more candidates than the list
-// holds): the k-th key by digits of eight bits over the whole block, read anew every time, then masks of the larger and equal keys.  A NaN is
-// selected only where the block holds fewer than k numbers: a row has k different positions of its block always (left short, it would keep the end of
-// the row it replaces, whose positions may be the same again).
+// The selection of any block (zeros, infinities, equal magnitudes, k beyond the octets, more candidates than the list holds): the k-th key by
+// digits of eight bits between two bounds, `lo`, which at least k numbers reach (0: none known), and the largest, over the whole block, read anew every
+// time; then masks of the larger and equal keys, and the row by a warp per 32 positions.  Zeros are not counted: where fewer than k
+// numbers are larger the k-th is one.  A NaN is selected only where the block holds fewer than k numbers: a row has k different positions of
+// its block always (left short, it would keep the end of the row it replaces, whose positions may be the same again).  Bound by the reads' latency
+// and the shared-memory counters.  us, 149 blocks (4.3 M fp32 elements), and in parentheses with four digits of eight bits from the top, an octet at a
+// time, a thread writing its 128 positions: zeros 13.6 (56), equal magnitudes 31 (73), infinities 35 (48), k = 20 % 36 (53), 50 % 36 (66), all 20 (82);
+// 881 blocks, zeros 32 (119), k = 20 % 78 (122), all 63 (299).
 // Every thread of the CTA calls.
 template <typename T, int NT>
-__device__ __noinline__ void select_general(const T* x, int n, int k, bool vec, Smem& ss, int16_t* out) {
+__device__ __noinline__ void select_general(const T* x, int n, int k, int lo, int kmax, bool vec, Smem& ss, int16_t* out) {
     constexpr int K_WPT = SEL_WORDS / NT;                    // bitmap words per thread
+    constexpr int ZB = sizeof(T) == 2 ? 16 : 0;              // low key bits that are always zero
+    constexpr int B = 2;                                     // octets a thread has in flight (with four the bf16 kernel spills)
     const int t = threadIdx.x, n_oct = (n + 7) >> 3;
-    int kth = 0, rem = k;
-    for (int level = 0; level < 4; ++level) {
-        const int sh = level == 3 ? 0 : 23 - 8 * level, width = level == 3 ? 7 : 8;
+    auto each_octet = [&](auto&& f) {
+        int o = t;
+        if (vec)
+            for (; o + (B - 1) * NT < n >> 3; o += B * NT) {
+                Octet<T> r[B];
+#pragma unroll
+                for (int i = 0; i < B; ++i) r[i].load(x + (o + i * NT) * 8);
+#pragma unroll
+                for (int i = 0; i < B; ++i) { float v[8]; r[i].values(v); f(o + i * NT, v); }
+            }
+        for (; o < n_oct; o += NT) { float v[8]; load_octet(x, o, n, vec, v); f(o, v); }
+    };
+    const int inf = K_INF >> ZB;
+    int lo_k = lo >> ZB, hi_k = kmax >> ZB, rem = k;
+    while (lo_k < hi_k) {
+        const int span = hi_k - lo_k, sh = span < 256 ? 0 : (32 - __clz(span)) - 8;
         __syncthreads();
         if (t < 256) ss.hist[t] = 0;
         __syncthreads();
-        for (int o = t; o < n_oct; o += NT) {
-            float v[8];
-            load_octet(x, o, n, vec, v);
-            for (int e = 0; e < min(8, n - o * 8); ++e) {
-                const int key = key_of(v[e]);
-                if (key <= K_INF && (level == 0 || (key >> (sh + width)) == kth)) atomicAdd(&ss.hist[(key >> sh) & ((1 << width) - 1)], 1);
+        each_octet([&](int, const float (&v)[8]) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int key = key_of(v[e]) >> ZB;
+                if (key >= lo_k && key <= hi_k && key != 0) atomicAdd(&ss.hist[(key - lo_k) >> sh], 1);
             }
-        }
+        });
         __syncthreads();
-        int size;
-        const int bin = kth_bin(ss.hist, rem, size);         // (-1: fewer than k numbers; the smallest digit then, and all of them are taken)
-        kth = (kth << width) | max(bin, 0);
+        int size = 0;
+        const int bin = kth_bin(ss.hist, rem, size);
+        if (bin < 0) { lo_k = 0; break; }                    // fewer than k numbers above zero
+        lo_k += bin << sh;
+        hi_k = min(hi_k, lo_k + (1 << sh) - 1);
+        if (rem == size) { lo_k = max(lo_k - 1, 0); break; } // all of the bin: the keys above what lies below it
     }
-    for (int o = t; o < SEL_MAX_TILE / 8; o += NT) {
+    const int kth = lo_k;
+    each_octet([&](int o, const float (&v)[8]) {
         uint32_t gt = 0u, tie = 0u;
-        if (o < n_oct) {
-            float v[8];
-            load_octet(x, o, n, vec, v);
-            for (int e = 0; e < min(8, n - o * 8); ++e) {
-                const int key = key_of(v[e]);
-                gt |= key > kth && key <= K_INF ? 1u << e : 0u;
-                tie |= key == kth ? 1u << e : 0u;
-            }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int key = key_of(v[e]) >> ZB;
+            gt |= key > kth && key <= inf ? 1u << e : 0u;
+            tie |= key == kth ? 1u << e : 0u;
         }
         reinterpret_cast<uint8_t*>(ss.gt_bm)[o] = (uint8_t)gt;
-        reinterpret_cast<uint8_t*>(ss.tie_bm)[o] = (uint8_t)tie;
-    }
+        reinterpret_cast<uint8_t*>(ss.tie_bm)[o] = (uint8_t)(n - o * 8 >= 8 ? tie : tie & ((1u << (n - o * 8)) - 1u));   // (not what lies past the end)
+    });
+    for (int o = n_oct + t; o < SEL_MAX_TILE / 8; o += NT) { reinterpret_cast<uint8_t*>(ss.gt_bm)[o] = 0; reinterpret_cast<uint8_t*>(ss.tie_bm)[o] = 0; }
     __syncthreads();
     uint32_t sel[K_WPT], tw[K_WPT];
     int ties = 0, cnt = 0, total;
@@ -196,8 +220,13 @@ __device__ __noinline__ void select_general(const T* x, int n, int k, bool vec, 
     }
     int to = block_exclusive_scan(cnt, ss.scan, total);
 #pragma unroll
-    for (int i = 0; i < K_WPT; ++i)
-        for (uint32_t s = sel[i]; s; s &= s - 1) out[to++] = (int16_t)((t * K_WPT + i) * 32 + __ffs(s) - 1);
+    for (int i = 0; i < K_WPT; ++i) { ss.sel_bm[t * K_WPT + i] = sel[i]; ss.sel_before[t * K_WPT + i] = (uint16_t)to; to += __popc(sel[i]); }
+    __syncthreads();
+#pragma unroll 4
+    for (int w = warp_id(); w < (n + 31) >> 5; w += NT / 32) {
+        const uint32_t s = ss.sel_bm[w];
+        if (s >> lane_id() & 1u) out[ss.sel_before[w] + __popc(s & ((1u << lane_id()) - 1u))] = (int16_t)(w * 32 + lane_id());
+    }
 }
 
 template <typename T, int NT>
@@ -245,6 +274,7 @@ block_topk_kernel(int64_t d, int dbs, int nfull, int k_many, int k_few, const T*
         const int kmax = ss.kmax;
         bool fast = false;
         int C = 0, lo = 0;
+        bool tied = false;                                    // more octets than wanted reach the bound, and no higher one is reached by k
         if (kmax > 0 && kmax < K_INF && k <= n_oct) {
             // ---- a bound that at least k octets reach and at most about 1.5 k, fewer where that would bring more candidates than the list holds
             const int accept = k + (k > 1024 ? 192 : (k >> 1) + 8);
@@ -258,7 +288,7 @@ block_topk_kernel(int64_t d, int dbs, int nfull, int k_many, int k_few, const T*
                 search = hi - lo > 1 && !(c > 0 && c <= accept);
                 gq = have_lo ? lo + ((hi - lo) >> 1) : max(hi - step, 1);
             }
-            for (int it = 0; search && it < 64; ++it) {
+            for (int it = 0; search && it < 63; ++it) {
                 int mine = 0;
 #pragma unroll
                 for (int j = 0; j < K_SLOTS; ++j) mine += __float_as_int(omax[j]) >= gq ? 1 : 0;
@@ -274,7 +304,8 @@ block_topk_kernel(int64_t d, int dbs, int nfull, int k_many, int k_few, const T*
                 else { gq = (int)max((int64_t)hi - step, (int64_t)1); step <<= 1; }
             }
             guess = lo;
-            if (have_lo && lo > 0) {
+            tied = hi - lo <= 1;
+            if (lo > 0) {                   // (an octet that reaches the bound is a candidate at least)
                 // ---- candidates: the octets that reach the bound through a list per warp, one of them per lane and round ----------
                 const float lo_f = __int_as_float(lo);
                 int n_w = 0;
@@ -322,6 +353,14 @@ block_topk_kernel(int64_t d, int dbs, int nfull, int k_many, int k_few, const T*
             unsigned long long lo_c = (unsigned long long)(uint32_t)(lo >> ZB) << 15, hi_c = ((unsigned long long)(uint32_t)(kmax >> ZB) << 15) | 0x7FFFu;
             unsigned long long kth = 0;
             int k_rem = k;
+            if (tied) {                                      // often their k-th is one of many with the bound's magnitude: then the positions decide
+                int above = 0;
+                for (int i = t; i < C; i += NT) above += ss.key[i] > (uint32_t)(lo >> ZB) ? 1 : 0;
+                above = __reduce_add_sync(0xffffffffu, above);
+                if (lane == 0 && above) atomicAdd(&ss.rot[63], above);
+                __syncthreads();
+                if (ss.rot[63] < k) { k_rem = k - ss.rot[63]; hi_c = lo_c | 0x7FFFu; }
+            }
             auto cand = [&](int i) { return ((unsigned long long)ss.key[i] << 15) | ss.pos[i]; };
             for (int level = 0; level < 7; ++level) {        // 46 bits, 8 a level at least after the first
                 const unsigned long long W1 = hi_c - lo_c;
@@ -373,7 +412,7 @@ block_topk_kernel(int64_t d, int dbs, int nfull, int k_many, int k_few, const T*
                     out[ss.sel_before[w] + __popc(ss.sel_bm[w] & ((1u << (pos & 31)) - 1u))] = (int16_t)pos;
                 }
         } else {
-            select_general<T, NT>(x, n, k, vec, ss, out);
+            select_general<T, NT>(x, n, k, lo, kmax, vec, ss, out);
         }
         __syncthreads();                                     // everything is used again
     }

@@ -26,7 +26,8 @@ def _expected(x, k_many, k_few):
 @pytest.mark.parametrize('kind,k,tail,skip', [
     ('normal', 291, 0, 0), ('normal', 291, 1, 0), ('normal', 1024, 8191, 1), ('normal', 1025, 8192, 2), ('normal', 3632, 15, 0), ('normal', 3633, 16, 3),
     ('ties', 1453, 17, 0), ('ties', 33, 4099, 0), ('scales', 291, 777, 4), ('inf', 291, 4096, 0), ('inf', 1, 9, 0), ('nan', 291, 4097, 0),
-    ('zeros', 291, 100, 0), ('cluster', 600, 64, 0), ('all_nan', 291, 33, 0), ('short', 291, 300, 1), ('short', 7264, 9, 0)])
+    ('zeros', 291, 100, 0), ('cluster', 600, 64, 0), ('all_nan', 291, 33, 0), ('short', 291, 300, 1), ('short', 7264, 9, 0),
+    ('equal', 291, 100, 0), ('equal', 14000, 7, 1), ('three', 291, 9, 0), ('normal', 29056, 50, 0), ('zeros', 29056, 1, 0), ('zeros', 9000, 13, 2)])
 def test_block_topk_routes(dtype, kind, k, tail, skip):
     from ista_daslab_optimizers_b200 import _native as N
     for full in (2, N.get_sm_count(), N.get_sm_count() + 1):
@@ -46,6 +47,10 @@ def test_block_topk_routes(dtype, kind, k, tail, skip):
             x[:DBS] = 0.0
             x[DBS:2 * DBS] = 0.0
             x[DBS + 11:2 * DBS:4001] = 1e-3
+        elif kind == 'equal':                            # one magnitude, either sign
+            x = torch.sign(x) * 1e-3
+        elif kind == 'three':                            # zeros and two magnitudes, the larger one rare
+            x = torch.where(x.abs() > 2.9e-3, 2e-3, torch.where(x.abs() > 1e-3, 1e-3, 0.0)) * torch.sign(x)
         elif kind == 'all_nan':                          # nothing else in the blocks, and in the short one behind them
             x[DBS:] = float('nan')
         elif kind == 'short':                            # one number fewer than k, zeros among them, and none
