@@ -16,9 +16,9 @@ namespace mab {
 constexpr int SPR_SR = 14592;         // elements of a block one CTA accumulates at a time (57 * 256): a 29 056-element block is two ranges
 constexpr int SPR_THREADS = 384;      // three CTAs of 58 KB of accumulators per SM, 56 registers a thread (512 threads of 40 spill: 98 us, now 78)
 static_assert(MAB_MAX_WINDOW <= SPR_THREADS, "a thread brings one row's multiplier");
-// Rows whose entries a thread fetches at once, while it adds those fetched before; (row, round) pairs of long rows (25.6 M elements, 32 rows of
-// 5 %: 6 189 us, 8 198; of 1 %: 6 66.6, 8 65.4, products behind the barriers).
-template <bool LONG> constexpr int SPR_AHEAD = LONG ? 6 : 8;
+// Rows whose entries a thread fetches at once; (row, round) pairs of long rows (bf16 values, 25.6 M elements, 32 rows of 5 %: 6 189 us, 8 198; of
+// 1 %: 6 66.6, 8 65.4, products behind the barriers).
+template <typename TV, bool LONG> constexpr int SPR_AHEAD = LONG && sizeof(TV) == 2 ? 6 : 8;
 
 constexpr int SP_THREADS = 512;
 constexpr int SP_CLUSTER = 8;         // CTAs per row (the portable cluster size) ...
@@ -134,19 +134,14 @@ sparse_rows_dot_parts_kernel(int64_t k, int64_t dbs, int kbs, int nfull, int k_f
 template <typename TV> struct Entry;
 template <> struct Entry<uint16_t> {
     uint32_t e;
-    __device__ __forceinline__ void get(const int16_t* I, const void* V, int64_t at, bool on) {
-        e = on ? (uint32_t)(uint16_t)I[at] | ((uint32_t)reinterpret_cast<const uint16_t*>(V)[at] << 16) : 0xFFFFu;
-    }
+    __device__ __forceinline__ void get(const int16_t* i, const uint16_t* v, bool on) { e = on ? (uint32_t)(uint16_t)*i | ((uint32_t)*v << 16) : 0xFFFFu; }
     __device__ __forceinline__ int pos() const { return (int16_t)(e & 0xFFFFu); }
     __device__ __forceinline__ float val() const { return __uint_as_float(e & 0xFFFF0000u); }
 };
 template <> struct Entry<float> {
     int p;
     float v;
-    __device__ __forceinline__ void get(const int16_t* I, const void* V, int64_t at, bool on) {
-        p = on ? (int)I[at] : -1;
-        v = on ? reinterpret_cast<const float*>(V)[at] : 0.0f;
-    }
+    __device__ __forceinline__ void get(const int16_t* i, const float* x, bool on) { p = on ? (int)*i : -1; v = on ? *x : 0.0f; }
     __device__ __forceinline__ int pos() const { return p; }
     __device__ __forceinline__ float val() const { return v; }
 };
@@ -154,11 +149,14 @@ template <> struct Entry<float> {
 // out[e] += sum_r M[r] * V[r, j] over the entries (r, j) that address e: one CTA per sub-range of a top-k block
 // with a dense fp32 accumulator in shared memory; rows are added in row order (positions are unique inside a
 // row, so a row needs no atomics, but a barrier).  Bound by the chain of rows: a thread fetches its entries of SPR_AHEAD rows at once,
-// and the next ones before it adds these, so that a row costs a shared-memory update and a barrier (25.6 M elements, 32 rows of 1 %:
-// 232 us with one load latency per row and four walks over a block's entries, 75 with one per eight rows, 65 with the next eight ahead).
+// and, while the values are bf16, the next ones before it adds these, so that a row costs a shared-memory update and a barrier (25.6 M elements, 32
+// rows of 1 %: 232 us with one load latency per row and four walks over a block's entries, 75 with one per eight rows, 65 with the next eight
+// ahead; fp32 values have no registers for a second eight: 12 to 60 bytes of spills, bf16 out 73 against 54).
 // The products of eight rows are made before the first of their barriers, off that chain (64 us; 1.28 M elements, bf16, 64 rows of 0.5 %: 14.4
 // behind the barriers, 11.6 so; 60 M the same 217 / 202).  LONG, blocks with more entries than the CTA has threads: behind them, as the
-// registers do not hold the products too (25.6 M, 32 rows of 5 %: 188, 206 before them).
+// registers do not hold the products too (25.6 M, 32 rows of 5 %: 188, 206 before them).  Where a row has fewer entries a warp without one takes part in
+// the barriers only, and groups behind the last row are not walked: with both in every warp one row of 1 % took,
+// bf16 out, 28.2 us, 21.3 so.
 template <typename TO, typename TV, bool LONG>
 __global__ void __launch_bounds__(SPR_THREADS, 3)
 sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int nfull, int k_few, const float* __restrict__ M,
@@ -167,6 +165,7 @@ sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int
     __shared__ float s_M[MAB_MAX_WINDOW];
     const int t = threadIdx.x;
     const int subs_per_block = (dbs + SPR_SR - 1) / SPR_SR;
+    const float factor = t < rows ? M[t] : 0.0f;
     for (int unit = blockIdx.x; unit < total_units; unit += gridDim.x) {
         int blk = unit / subs_per_block, sub = unit - blk * subs_per_block;
         if (blk > nfull) { sub += (blk - nfull) * subs_per_block; blk = nfull; }
@@ -177,30 +176,33 @@ sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int
         const int len = min(SPR_SR, n_blk - s0);
         const int64_t row0 = (int64_t)blk * kbs;
         for (int i = t; i < len; i += SPR_THREADS) acc[i] = 0.0f;
-        // (row, round) pairs in row order, SPR_AHEAD of them fetched at once, and those after them before the current ones are added
+        // (row, round) pairs in row order, A of them fetched at once, and with bf16 values those after them before the current ones are added
+        constexpr int A = SPR_AHEAD<TV, LONG>;
         const int rounds = LONG ? (kcnt + SPR_THREADS - 1) / SPR_THREADS : 1, pairs = rows * rounds;
         int fr = 0, fc = 0;                                      // the pair to fetch next ...
+        const int16_t* fI = I + row0 + t;                        // ... from here
+        const TV* fV = static_cast<const TV*>(V) + row0 + t;
         int r = 0, c = 0;                                        // ... and to add next
-        auto fetch = [&](Entry<TV> (&e)[SPR_AHEAD<LONG>]) {
+        auto fetch = [&](Entry<TV> (&e)[A]) {
 #pragma unroll
-            for (int i = 0; i < SPR_AHEAD<LONG>; ++i) {
-                const int j = fc * SPR_THREADS + t;
-                e[i].get(I, V, (int64_t)fr * k + row0 + j, fr < rows && j < kcnt);
-                if (!LONG || ++fc == rounds) { fc = 0; ++fr; }
+            for (int i = 0; i < A; ++i) {
+                const int j = LONG ? fc * SPR_THREADS : 0;
+                e[i].get(fI + j, fV + j, fr < rows && j + t < kcnt);
+                if (!LONG || ++fc == rounds) { fc = 0; ++fr; fI += k; fV += k; }
             }
         };
-        auto add = [&](const Entry<TV> (&e)[SPR_AHEAD<LONG>]) {
-            int pos[SPR_AHEAD<LONG>];
-            float val[SPR_AHEAD<LONG>];
+        auto add = [&](const Entry<TV> (&e)[A]) {
+            int pos[A];
+            float val[A];
             if constexpr (!LONG) {
 #pragma unroll
-                for (int i = 0; i < SPR_AHEAD<LONG>; ++i) {
+                for (int i = 0; i < A; ++i) {
                     pos[i] = e[i].pos() - s0;
                     val[i] = __fmul_rn(s_M[min(r + i, rows - 1)], e[i].val());
                 }
             }
 #pragma unroll
-            for (int i = 0; i < SPR_AHEAD<LONG>; ++i) {
+            for (int i = 0; i < A; ++i) {
                 if (r < rows) {                                  // uniform
                     if (c == 0) __syncthreads();                 // the row before (or the clearing) is done
                     if constexpr (LONG) { pos[i] = e[i].pos() - s0; val[i] = __fmul_rn(s_M[r], e[i].val()); }
@@ -209,16 +211,28 @@ sparse_rows_combine_kernel(int64_t d, int rows, int64_t k, int dbs, int kbs, int
                 }
             }
         };
-        Entry<TV> a[SPR_AHEAD<LONG>], b[SPR_AHEAD<LONG>];
-        const float factor = t < rows ? M[t] : 0.0f;
-        fetch(a);
-        if (t < rows) s_M[t] = factor;
-        if constexpr (!LONG) __syncthreads();                    // the first products are made before the first row's barrier
-        for (int p = 0; p < pairs; p += 2 * SPR_AHEAD<LONG>) {
-            fetch(b);
-            add(a);
-            fetch(a);
-            add(b);
+        const bool mine = LONG || (t & ~31) < kcnt;              // a warp without entries only keeps step at the barriers
+        Entry<TV> a[A];
+        if (mine) fetch(a);
+        if (unit == (int)blockIdx.x) {
+            if (t < rows) s_M[t] = factor;
+            if constexpr (!LONG) __syncthreads();                // the first products are made before the first row's barrier
+        }
+        if (!mine) {
+            for (int i = 0; i < rows; ++i) __syncthreads();
+        } else if constexpr (sizeof(TV) == 2) {
+            Entry<TV> b[A];
+            for (int p = 0; p < pairs; p += 2 * A) {
+                if (p + A < pairs) fetch(b);
+                add(a);
+                if (p + 2 * A < pairs) fetch(a);
+                if (p + A < pairs) add(b);
+            }
+        } else {
+            for (int p = 0; p < pairs; p += A) {
+                add(a);
+                if (p + A < pairs) fetch(a);
+            }
         }
         __syncthreads();
         TO* o = out + blk_base + s0;

@@ -168,6 +168,33 @@ def test_sparse_rows_dot_and_combine(N, gdtype, vdtype):
             assert torch.equal(bits(out), bits(outg)), (d, rows)    # same operations in the same order: bit-exact
 
 
+@pytest.mark.parametrize('odtype', [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('vdtype', [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('rows,kbs,k_few,blocks,dbs', [
+    (1, 1, 0, 3, 4096), (3, 31, 5, 2, 4096), (7, 32, 1, 2, 4096), (8, 33, 0, 2, 4096), (9, 352, 33, 2, 4096), (16, 383, 100, 1, 4096),
+    (17, 384, 64, 2, 29056), (6, 385, 7, 2, 29056), (13, 385, 100, 1, 4096), (25, 800, 0, 2, 16000), (33, 291, 1, 1, 29056), (9, 33, 11, 1000, 512)])
+def test_sparse_rows_combine_shapes(N, rows, kbs, k_few, blocks, dbs, vdtype, odtype):
+    """Rows around the number fetched at once, entries of a row around a warp's and the CTA's threads, a short block with and without entries, more
+    blocks than CTAs: the rows are added in their order whatever the shape, so the result is exact."""
+    tail = 100
+    d, k = blocks * dbs + tail, blocks * kbs + k_few
+    gen = torch.Generator().manual_seed(rows * 1000 + kbs)
+    I = torch.empty(rows, k, dtype=torch.int16)
+    for r in range(rows):
+        full = torch.rand(blocks, dbs, generator=gen).topk(kbs, dim=1).indices.sort(dim=1).values
+        few = torch.rand(tail, generator=gen).topk(k_few).indices.sort().values
+        I[r] = torch.cat([full.reshape(-1), few]).to(torch.int16)
+    V = torch.randn(rows, k, generator=gen).to(vdtype)
+    M, out = torch.randn(rows, generator=gen), torch.randn(d, generator=gen).to(odtype)
+    acc = torch.zeros(d)
+    base = torch.cat([torch.arange(blocks).repeat_interleave(kbs), torch.full((k_few,), blocks)]) * dbs
+    for r in range(rows):
+        acc[base + I[r].long()] += M[r] * V[r].float()
+    got = out.cuda()
+    N.sparse_rows_combine(d, rows, k, dbs, kbs, M.cuda(), I.cuda(), V.cuda(), got)
+    assert torch.equal(bits((out.float() + acc).to(odtype)), bits(got))
+
+
 def test_device_queries(N):
     assert N.get_sm_count() == torch.cuda.get_device_properties(0).multi_processor_count
     floats = N.get_max_floats_for_shared_memory_per_thread_block()
