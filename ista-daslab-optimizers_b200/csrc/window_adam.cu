@@ -770,7 +770,7 @@ __device__ __noinline__ void decay_tile(TP* p, int len, float decay) {
     if ((int)threadIdx.x < around) Elem<TP>::store(edge, 0, __fmul_rn(edge_v, decay));
 }
 
-template <typename TP, int MODE, int ALPHA, int NT, bool EARLY>
+template <typename TP, int MODE, int ALPHA, int NT, bool EARLY, bool AHEAD>
 __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units,
                                                  int max_k, const WindowArgs& a, int dense_at = 0) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -791,10 +791,9 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
     UpdateProbe pr;
     const bool probing = MODE == MODE_STEP && a.probe != nullptr;
 
-    // AHEAD: the next tile's rows travel while this one's elements are updated, and a thread of 256 looks two entries ahead in the row loop.  The
-    // bf16 alpha forms have the registers for it (alpha == -2, 54.5 M elements 152 -> 145 us, alpha = 0.5 with 20 rows 210 -> 203); the others
-    // spill, or hide the rows behind other tiles as it is.
-    constexpr bool AHEAD = sizeof(TP) == 2 && ALPHA != 0;
+    // AHEAD: the next tile's rows travel while this one's elements are updated, and a thread of 256 looks two entries ahead in the row loop
+    // (rows_ahead gives it).
+    static_assert(!(EARLY && AHEAD), "an EARLY launch has no next tile, and stages without the row that kernel A writes");
     auto stage = [&](const mab_tensor& T, int blk) {
         window_tile_stage<NT>(T, blk, blk < T.topk_full_blocks_count ? T.k_block_size_many : T.k_block_size_few, a, w, s_pos_off, s_val_off,
                               EARLY ? T.ring_index : -1);
@@ -853,7 +852,7 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
         MAB_BTICK_DECL
         if constexpr (!AHEAD) window_tile_stage<NT>(T, blk, kcnt, a, w, s_pos_off, s_val_off, EARLY ? T.ring_index : -1);
         const int touched = window_tile_moments<NT, AHEAD, EARLY>(T, blk, n_blk, kcnt, a, w, s_scan, s_pos_off, s_val_off);
-        if constexpr (AHEAD && !EARLY) stage_next();
+        if constexpr (AHEAD) stage_next();
         MAB_BTICK(9);
         if constexpr (MODE == MODE_STEP && ALPHA == 0) {
             // 5. without the alpha term only the touched positions get an update: stream the block for the
@@ -918,11 +917,11 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
 }
 
 // (threads_of gives NT)
-template <typename TP, int MODE, int ALPHA, int NT, bool EARLY = false>
+template <typename TP, int MODE, int ALPHA, int NT, bool EARLY = false, bool AHEAD = false>
 __global__ void __launch_bounds__(NT, ALPHA != 0 ? 768 / NT : NT == 384 ? 3 : 1024 / NT)
 window_tile_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units, int max_k,
                    int dense_at, const __grid_constant__ WindowArgs a) {
-    window_tile_body<TP, MODE, ALPHA, NT, EARLY>(tensors, n_tensors, total_units, max_k, a, dense_at);
+    window_tile_body<TP, MODE, ALPHA, NT, EARLY, AHEAD>(tensors, n_tensors, total_units, max_k, a, dense_at);
 }
 
 // Single tensor whose descriptor travels as a kernel argument (operator-level entry point).
@@ -930,7 +929,7 @@ template <typename TP, int MODE, int ALPHA, int NT>
 __global__ void __launch_bounds__(NT)
 window_tile_single_kernel(const __grid_constant__ mab_tensor t, int total_units, int max_k,
                           const __grid_constant__ WindowArgs a) {
-    window_tile_body<TP, MODE, ALPHA, NT, false>(&t, 1, total_units, max_k, a);
+    window_tile_body<TP, MODE, ALPHA, NT, false, false>(&t, 1, total_units, max_k, a);
 }
 
 // ------------------------------------------------------------------------------------ resident-tile kernel
@@ -1155,7 +1154,7 @@ template <typename TP, int MODE, int ALPHA>
 static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* single, int n_tensors, int units_tile,
                               int units_wide, int max_k, const WindowArgs& a, bool behind_a, cudaStream_t s) {
     const int sms = device_sm_count();
-    const TileLaunch L = plan_tile_launch(MODE == MODE_WRITE_UPDATE, ALPHA != 0, a.rows, max_k, units_tile, behind_a, sms, device_max_optin_smem());
+    const TileLaunch L = plan_tile_launch(MODE == MODE_WRITE_UPDATE, ALPHA, sizeof(TP) == 2, a.rows, max_k, units_tile, behind_a, sms, device_max_optin_smem());
     if (L.smem > 0) {
         const int nt = L.threads;
         auto run = [&](auto kern, int threads) -> int {
@@ -1177,7 +1176,11 @@ static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* s
             else if (nt == 384) rc = run(window_tile_kernel<TP, MODE, 0, 384>, 384);
             else rc = run(window_tile_kernel<TP, MODE, 0, 256>, 256);
         } else {
+            constexpr bool BF16 = sizeof(TP) == 2;            // (only its launches are ahead)
             if (nt == 512 && L.early) rc = run(window_tile_kernel<TP, MODE, ALPHA, 512, true>, 512);
+            else if (nt == 512 && L.ahead) rc = run(window_tile_kernel<TP, MODE, ALPHA, 512, false, BF16>, 512);
+            else if (nt == 384 && L.ahead) rc = run(window_tile_kernel<TP, MODE, ALPHA, 384, false, BF16>, 384);
+            else if (L.ahead) rc = run(window_tile_kernel<TP, MODE, ALPHA, 256, false, BF16>, 256);
             else if (nt == 512) rc = run(window_tile_kernel<TP, MODE, ALPHA, 512>, 512);
             else if (nt == 384) rc = run(window_tile_kernel<TP, MODE, ALPHA, 384>, 384);
             else rc = run(window_tile_kernel<TP, MODE, ALPHA, 256>, 256);
@@ -1235,7 +1238,7 @@ int fill_window_args(WindowArgs& a, int64_t steps, int m, double beta1, double b
 
 int allowing_ctas(int units_tile, int rows, int max_k, int max_dbs, int param_dtype, float alpha) {
     const int sms = device_sm_count();
-    return update_is_early(units_tile, rows, max_k, max_dbs, param_dtype == MAB_BF16, alpha != 0.0f, sms, device_max_optin_smem()) ? sms : sms / 2;
+    return update_is_early(units_tile, rows, max_k, max_dbs, param_dtype == MAB_BF16, alpha == -2.0f ? 2 : alpha != 0.0f ? 1 : 0, sms, device_max_optin_smem()) ? sms : sms / 2;
 }
 
 int launch_window_step(const mab_tensor* dev_tensors, int n_tensors, int units_tile, int units_wide, int max_k, int max_dbs,

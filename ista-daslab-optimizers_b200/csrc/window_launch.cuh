@@ -39,20 +39,29 @@ static inline int threads_of(bool write, bool alpha, int fit, int tiles, int max
 // CTA that an SM has to itself gets two tiles as soon as there are more tiles than the device shows SMs, a part of a GPU for instance.
 static inline bool early_form(int tiles, int grid, int sms) { return tiles <= grid && tiles <= sms; }
 
+// The AHEAD form of the alpha forms on bf16 parameters; fp32 spills.  It pays where a CTA has tiles enough or a row more entries than 256 threads.  us a
+// step, ahead and not (alpha == -2, 444 CTAs): k = 0.5 % 444 tiles 55.5 / 54.3, 740 108.4 / 106.4, 1000 141.5 / 143.9, 2000 219.9 / 221.7; k = 1 %
+// 200 tiles 43.1 / 45.0, 445 85.9 / 87.4, 2000 238.5 / 246.4; 20 rows (296 CTAs) 445 90.4 / 90.2, 600 115.8 / 118.3; k = 5 % (148) 600 181.7 / 185.4.
+// alpha = 0.5, k = 0.5 %: 1000 143.1 / 143.9, 1500 183.9 / 183.1, 2000 228.4 / 226.2.
+static inline bool rows_ahead(bool bf16, int alpha, int threads, int grid, int tiles, int max_k) {
+    if (!bf16 || alpha == 0) return false;
+    return threads != 256 ? tiles > grid : max_k > 256 || (alpha == 2 && tiles > 2 * grid);
+}
+
 struct TileLaunch {
     int  threads, grid, smem;             // smem 0: the window is too large for the compact arrays, the wide form takes it
     int  dense_at;                        // the alpha forms' dense arrays of the warps in shared memory (0: they do not fit)
-    bool early;
+    bool early, ahead;
 };
 
-static inline TileLaunch plan_tile_launch(bool write, bool alpha, int rows, int max_k, int tiles, bool behind_a, int sms, int optin_smem) {
-    TileLaunch L = {0, 0, 0, 0, false};
+static inline TileLaunch plan_tile_launch(bool write, int alpha, bool bf16, int rows, int max_k, int tiles, bool behind_a, int sms, int optin_smem) {
+    TileLaunch L = {0, 0, 0, 0, false, false};
     // while the compact arrays fit one CTA's shared memory (next to the kernel's static arrays)
     const int smem_tile = (int64_t)rows * max_k <= WT_MAX_ENTRIES ? wt_smem_bytes(rows, max_k) : 0;
     if (smem_tile == 0 || smem_tile + 4096 > optin_smem) return L;
     // the forms with the alpha term: a dense array of 256 floats per warp behind the window's arrays, if it fits
     const int fit = std::max(1, std::min(8, (227 * 1024) / (smem_tile + (alpha ? 8 * 1024 : 0) + 3072)));   // CTAs per SM by their arrays
-    L.threads = threads_of(write, alpha, fit, tiles, max_k, sms);
+    L.threads = threads_of(write, alpha != 0, fit, tiles, max_k, sms);
     if (alpha && ((smem_tile + 15) & ~15) + L.threads * 32 + 4096 > optin_smem) L.threads = 256;
     const int nt = L.threads, dense = alpha ? nt * 32 : 0;
     L.dense_at = alpha && ((smem_tile + 15) & ~15) + dense + 4096 <= optin_smem ? (smem_tile + 15) & ~15 : 0;
@@ -60,6 +69,7 @@ static inline TileLaunch plan_tile_launch(bool write, bool alpha, int rows, int 
     const int per_sm = std::max(1, std::min(alpha ? 768 / nt : nt == 384 ? 3 : 1024 / nt, (227 * 1024) / (L.smem + 3072)));   // (as in __launch_bounds__)
     L.grid = (int)std::min<int64_t>(tiles, (int64_t)sms * per_sm);
     L.early = behind_a && nt == 512 && early_form(tiles, L.grid, sms);
+    L.ahead = !L.early && rows_ahead(bf16, alpha, nt, L.grid, tiles, max_k);
     return L;
 }
 
@@ -73,10 +83,10 @@ static inline int resident_smem_bytes(int rows, int max_k, int max_dbs, int opti
 }
 
 // Whether the update of a step on such tensors takes the EARLY form.
-static inline bool update_is_early(int tiles, int rows, int max_k, int max_dbs, bool bf16, bool alpha, int sms, int optin_smem) {
+static inline bool update_is_early(int tiles, int rows, int max_k, int max_dbs, bool bf16, int alpha, int sms, int optin_smem) {
     int tile_bytes;
-    if (bf16 && !alpha && resident_smem_bytes(rows, max_k, max_dbs, optin_smem, &tile_bytes) > 0) return early_form(tiles, std::min(tiles, 2 * sms), sms);
-    return plan_tile_launch(false, alpha, rows, max_k, tiles, true, sms, optin_smem).early;
+    if (bf16 && alpha == 0 && resident_smem_bytes(rows, max_k, max_dbs, optin_smem, &tile_bytes) > 0) return early_form(tiles, std::min(tiles, 2 * sms), sms);
+    return plan_tile_launch(false, alpha, bf16, rows, max_k, tiles, true, sms, optin_smem).early;
 }
 
 }  // namespace mab

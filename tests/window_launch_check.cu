@@ -4,18 +4,21 @@
 
 int main() {
     const int optin = 227 * 1024;
-    long long plans = 0, bad_early = 0;
+    long long plans = 0, bad_early = 0, bad_ahead = 0;
     int early_at_148 = 0;
     for (int sms : {16, 37, 74, 132, 148, 160})
         for (int rows : {1, 2, 3, 5, 10, 20, 32, 128})
             for (int max_k = 1; max_k <= 16384 / rows; max_k += max_k < 400 ? 1 : 37)
                 for (int tiles : {1, 2, 15, 16, 17, 37, 38, 74, 75, 111, 132, 133, 147, 148, 149, 296, 297, 444, 445, 5000})
-                    for (int form = 0; form < 3; ++form) {
-                        const mab::TileLaunch L = mab::plan_tile_launch(form == 2, form == 1, rows, max_k, tiles, form != 2, sms, optin);
+                    for (int form = 0; form < 7; ++form) {   // the update with alpha 0, in (0, 1) and -2, fp32 and bf16; the operator
+                        const int alpha = form < 6 ? form % 3 : 0;
+                        const mab::TileLaunch L = mab::plan_tile_launch(form == 6, alpha, form >= 3, rows, max_k, tiles, form != 6, sms, optin);
                         if (L.smem == 0) continue;
                         ++plans;
                         // the form that starts before kernel A ends stages one tile's rows: a CTA must not get a second one
-                        bad_early += L.early && tiles > L.grid;
+                        bad_early += L.early && (tiles > L.grid || L.ahead);
+                        // rows staged ahead: bf16 alpha forms only, and not without a next tile unless the row loop is the one with two entries
+                        bad_ahead += L.ahead && (form < 4 || form > 5 || (tiles <= L.grid && (L.threads != 256 || max_k <= 256)));
                         early_at_148 += L.early && sms == 148 && rows == 10 && max_k == 291 && tiles == 148;
                     }
     for (int sms : {16, 37, 74, 132, 148})                   // the resident form, two CTAs per SM
@@ -30,14 +33,14 @@ int main() {
     for (int sms : {74, 132, 148})
         for (int tiles : {sms / 2, sms, sms + 1}) {
             const bool one = tiles <= sms;
-            form_ok = form_ok && mab::update_is_early(tiles, 10, 291, dbs, true, false, sms, optin) == one;
-            form_ok = form_ok && mab::update_is_early(tiles, 10, 291, dbs, false, false, sms, optin) == one;
-            form_ok = form_ok && mab::update_is_early(tiles, 10, 291, dbs, true, true, sms, optin) == one;
+            form_ok = form_ok && mab::update_is_early(tiles, 10, 291, dbs, true, 0, sms, optin) == one;
+            form_ok = form_ok && mab::update_is_early(tiles, 10, 291, dbs, false, 0, sms, optin) == one;
+            form_ok = form_ok && mab::update_is_early(tiles, 10, 291, dbs, true, 1, sms, optin) == one;
             for (bool bf16 : {false, true}) {
-                form_ok = form_ok && !mab::update_is_early(tiles, 20, 1453, dbs, bf16, false, sms, optin) && !mab::update_is_early(tiles, 5, 14528, dbs, bf16, true, sms, optin);
-                form_ok = form_ok && !mab::update_is_early(tiles, 10, 1453, dbs, bf16, false, sms, optin);
+                form_ok = form_ok && !mab::update_is_early(tiles, 20, 1453, dbs, bf16, 0, sms, optin) && !mab::update_is_early(tiles, 5, 14528, dbs, bf16, 1, sms, optin);
+                form_ok = form_ok && !mab::update_is_early(tiles, 10, 1453, dbs, bf16, 0, sms, optin);
             }
         }
-    printf("plans %lld, early forms with more tiles than CTAs %lld, what may start early %s\n", plans, bad_early, form_ok ? "right" : "wrong");
-    return form_ok && plans > 100000 && early_at_148 == 2 && bad_early == 0 ? 0 : 1;
+    printf("plans %lld, early forms with more tiles than CTAs %lld, rows ahead of nothing %lld, what may start early %s\n", plans, bad_early, bad_ahead, form_ok ? "right" : "wrong");
+    return form_ok && bad_ahead == 0 && plans > 100000 && early_at_148 == 6 && bad_early == 0 ? 0 : 1;
 }
