@@ -625,13 +625,14 @@ __device__ __forceinline__ int window_tile_moments(const mab_tensor& T, int blk,
     MAB_BTICK(1);
     // 3. number them: prefix[word] = touched positions in words below
     constexpr int WPT = (WT_WORDS + NT - 1) / NT;
+    constexpr bool EVEN = WT_WORDS % NT == 0;                 // (else the last threads have fewer words; the check costs the wide accesses)
     int cnt[WPT], local = 0;
 #pragma unroll
-    for (int i = 0; i < WPT; ++i) { cnt[i] = t * WPT + i < WT_WORDS ? __popc(w.bitmap[t * WPT + i]) : 0; local += cnt[i]; }
+    for (int i = 0; i < WPT; ++i) { cnt[i] = EVEN || t * WPT + i < WT_WORDS ? __popc(w.bitmap[t * WPT + i]) : 0; local += cnt[i]; }
     int touched;
     int run = block_exclusive_scan(local, s_scan, touched);
 #pragma unroll
-    for (int i = 0; i < WPT; ++i) { if (t * WPT + i < WT_WORDS) w.prefix[t * WPT + i] = (uint16_t)run; run += cnt[i]; }
+    for (int i = 0; i < WPT; ++i) { if (EVEN || t * WPT + i < WT_WORDS) w.prefix[t * WPT + i] = (uint16_t)run; run += cnt[i]; }
     __syncthreads();
     MAB_BTICK(2);
     // 4. positions -> slots (in place), then accumulate row after row
