@@ -773,7 +773,7 @@ __device__ __noinline__ void decay_tile(TP* p, int len, float decay) {
 
 template <typename TP, int MODE, int ALPHA, int NT, bool EARLY, bool AHEAD>
 __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ tensors, int n_tensors, int total_units,
-                                                 int max_k, const WindowArgs& a, int dense_at = 0) {
+                                                 int max_k, const WindowArgs& a, int dense_at, bool zeros_late = false) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ int s_first[WIN_MAX_TENSORS + 1];
     __shared__ int s_scan[36];
@@ -835,15 +835,17 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
         // parameters read early leave L2 again).
         const bool decaying = MODE == MODE_STEP && ALPHA == 0 && T.weight_decay > 0.0 && !(sizeof(TP) == 2 && decay_is_identity_bf16(T.decay_f32));
         const bool one_tile = total_units <= (int)gridDim.x;
-        if constexpr (MODE == MODE_WRITE_UPDATE) {
-            // zeros everywhere now, the updates of the touched positions behind the window phases: the stores drain meanwhile (25.6 M fp32
-            // elements 36 us with a look-up through the bitmap for every element at the end, 34.5 so; bf16 30 and 25.5)
+        // The operator: zeros everywhere before the window phases, the updates of the touched positions behind them, so that the stores drain
+        // meanwhile (25.6 M fp32 elements 36 us with a look-up through the bitmap for every element at the end, 34.5 so; bf16 30 and 25.5).
+        // zeros_late: behind them too, where an output larger than L2 would lose its zeros to memory before their updates (write_mode).
+        auto zero_tile = [&]() {
             TP* const p = reinterpret_cast<TP*>(T.param) + blk_base;
             constexpr int VEC = 16 / (int)sizeof(TP);
             const int whole = aligned16(p) ? n_blk / VEC : 0;
             for (int i = threadIdx.x; i < whole; i += NT) reinterpret_cast<uint4*>(p)[i] = make_uint4(0u, 0u, 0u, 0u);
             for (int i = whole * VEC + threadIdx.x; i < n_blk; i += NT) p[i] = 0;
-        }
+        };
+        if constexpr (MODE == MODE_WRITE_UPDATE) { if (!zeros_late) zero_tile(); }
         if constexpr (MODE == MODE_STEP && ALPHA == 0) {
             if (decaying && one_tile) decay_tile<TP, NT>(reinterpret_cast<TP*>(T.param) + blk_base, n_blk, T.decay_f32);
         }
@@ -890,6 +892,7 @@ __device__ __forceinline__ void window_tile_body(const mab_tensor* __restrict__ 
             }
             if (probing && t == 0) pr.zeros_u += n_blk;        // every position without a non-zero update is a zero of u
         } else if constexpr (MODE == MODE_WRITE_UPDATE) {
+            if (zeros_late) { zero_tile(); __syncthreads(); }
             TP* const p = reinterpret_cast<TP*>(T.param) + blk_base;
             for (int s = t; s < touched; s += NT) {
                 const float2 acc = w.mv[s];
@@ -925,12 +928,13 @@ window_tile_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, int to
     window_tile_body<TP, MODE, ALPHA, NT, EARLY, AHEAD>(tensors, n_tensors, total_units, max_k, a, dense_at);
 }
 
-// Single tensor whose descriptor travels as a kernel argument (operator-level entry point).
+// Single tensor whose descriptor travels as a kernel argument (operator-level entry point).  (The compiler gives 256 threads 32 registers by itself, and
+// spills; told of three CTAs of 384 it makes them 2 to 5 % slower.)
 template <typename TP, int MODE, int ALPHA, int NT>
-__global__ void __launch_bounds__(NT)
-window_tile_single_kernel(const __grid_constant__ mab_tensor t, int total_units, int max_k,
+__global__ void __launch_bounds__(NT, NT == 256 ? 4 : 0)
+window_tile_single_kernel(const __grid_constant__ mab_tensor t, int total_units, int max_k, bool zeros_late,
                           const __grid_constant__ WindowArgs a) {
-    window_tile_body<TP, MODE, ALPHA, NT, false, false>(&t, 1, total_units, max_k, a);
+    window_tile_body<TP, MODE, ALPHA, NT, false, false>(&t, 1, total_units, max_k, a, 0, zeros_late);
 }
 
 // ------------------------------------------------------------------------------------ resident-tile kernel
@@ -1155,12 +1159,13 @@ template <typename TP, int MODE, int ALPHA>
 static int launch_window_impl(const mab_tensor* dev_tensors, const mab_tensor* single, int n_tensors, int units_tile,
                               int units_wide, int max_k, const WindowArgs& a, bool behind_a, cudaStream_t s) {
     const int sms = device_sm_count();
-    const TileLaunch L = plan_tile_launch(MODE == MODE_WRITE_UPDATE, ALPHA, sizeof(TP) == 2, a.rows, max_k, units_tile, behind_a, sms, device_max_optin_smem());
+    const int write = MODE == MODE_WRITE_UPDATE ? write_mode(single->d * (int64_t)sizeof(TP), sizeof(TP) == 2) : 0;
+    const TileLaunch L = plan_tile_launch(write, ALPHA, sizeof(TP) == 2, a.rows, max_k, units_tile, behind_a, sms, device_max_optin_smem());
     if (L.smem > 0) {
         const int nt = L.threads;
         auto run = [&](auto kern, int threads) -> int {
             MAB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L.smem));
-            if constexpr (MODE == MODE_WRITE_UPDATE) kern<<<L.grid, threads, L.smem, s>>>(*single, units_tile, max_k, a);
+            if constexpr (MODE == MODE_WRITE_UPDATE) kern<<<L.grid, threads, L.smem, s>>>(*single, units_tile, max_k, write == 2, a);
             else MAB_CUDA_TRY(launch_behind_kernel(kern, L.grid, threads, L.smem, s, dev_tensors, n_tensors, units_tile, max_k, L.dense_at, a));
             return MAB_OK;
         };

@@ -23,17 +23,25 @@ __host__ __device__ constexpr int wt_smem_bytes(int rows, int max_k) {
 //   k = 0.5 % (146 entries), 116 M elements: 256 threads 105, 384 108, 512 120.
 //   k = 1 % (291): 256 / 384 / 512 threads, 100 tiles 12.4 / 9.5 / 8.6, 300 tiles 18.8 / 15.5 / 18.6, 1000 55 / 42 / 44, 1500 77 / 61 / 61, 3000 143 / 124 /
 //   118, 4282 201 / 186 / 166; with weight decay 1000 82 / 70 / 73, 4282 292 / 322 / 268; 120 ragged tensors 33 / 30 / 35.
-//   The operator that writes every position's update: 384 (60 M elements k = 1 % 75, 256 and 512 threads 79; 0.5 % 59, 256 73, 512 67).
+//   The operator that writes every position's update: 384 (60 M elements k = 1 % 75, 256 and 512 threads 79; 0.5 % 59, 256 73, 512 67); with late zeros
+//   256 for many short rows (232 M elements, 0.5 %, 10 and 20 rows 202 and 270, 384 threads 219 and 298; 1 and 3 rows 161 and 173, 155 and 164).
 //   The alpha forms have 80 registers a thread: 256 threads while three CTAs fit (33.5 M elements 121, 384 threads 127), 384 where two do (bf16, 20
 //   rows, 58 M elements 265 with 256, 209), and 512 where one does or an SM has no more than one tile (100 tiles 29 and 18).
-static inline int threads_of(bool write, bool alpha, int fit, int tiles, int max_k, int sms) {
+static inline int threads_of(int write, bool alpha, int fit, int tiles, int rows, int max_k, int sms) {
     if (alpha) return fit < 2 || tiles <= sms ? 512 : fit < 3 ? 384 : 256;
     if (fit < 2) return 1024;
     if (tiles <= 2 * sms || fit < 3) return 512;
-    if (write) return 384;
+    if (write == 1) return 384;
+    if (write == 2) return max_k <= 256 && fit >= 4 && rows >= 8 ? 256 : 384;
     if (max_k <= 256 && fit >= 4) return 256;
     return max_k <= 384 && tiles <= 10 * sms ? 384 : 512;
 }
+
+// When the operator that writes every position's update stores the zeros: 1 before the window phases, 2 behind them.  (0: a step.)  Where the output does
+// not fit the 126 MB of L2, zeros stored before are written to memory and brought back for their updates.  us, before / behind, fp32, 10 rows of 1 %:
+// 25.6 M elements 35.3 / 35.4, 34.9 M 47.6 / 46.2, 58 M 78 / 72, 116 M 168 / 140, 232 M 342 / 274 (288 with a look-up for every element); bf16, half
+// as long, 58 M 56 / 57, 232 M 215 / 220.
+static inline int write_mode(int64_t bytes, bool bf16) { return !bf16 && bytes > ((int64_t)1 << 27) ? 2 : 1; }
 
 // The EARLY form (see wait_for_kernel_before): every CTA has one tile, and kernel A no more CTAs than there are SMs.  Not a matter of the tiles alone: a
 // CTA that an SM has to itself gets two tiles as soon as there are more tiles than the device shows SMs, a part of a GPU for instance.
@@ -54,14 +62,14 @@ struct TileLaunch {
     bool early, ahead;
 };
 
-static inline TileLaunch plan_tile_launch(bool write, int alpha, bool bf16, int rows, int max_k, int tiles, bool behind_a, int sms, int optin_smem) {
+static inline TileLaunch plan_tile_launch(int write, int alpha, bool bf16, int rows, int max_k, int tiles, bool behind_a, int sms, int optin_smem) {
     TileLaunch L = {0, 0, 0, 0, false, false};
     // while the compact arrays fit one CTA's shared memory (next to the kernel's static arrays)
     const int smem_tile = (int64_t)rows * max_k <= WT_MAX_ENTRIES ? wt_smem_bytes(rows, max_k) : 0;
     if (smem_tile == 0 || smem_tile + 4096 > optin_smem) return L;
     // the forms with the alpha term: a dense array of 256 floats per warp behind the window's arrays, if it fits
     const int fit = std::max(1, std::min(8, (227 * 1024) / (smem_tile + (alpha ? 8 * 1024 : 0) + 3072)));   // CTAs per SM by their arrays
-    L.threads = threads_of(write, alpha != 0, fit, tiles, max_k, sms);
+    L.threads = threads_of(write, alpha != 0, fit, tiles, rows, max_k, sms);
     if (alpha && ((smem_tile + 15) & ~15) + L.threads * 32 + 4096 > optin_smem) L.threads = 256;
     const int nt = L.threads, dense = alpha ? nt * 32 : 0;
     L.dense_at = alpha && ((smem_tile + 15) & ~15) + dense + 4096 <= optin_smem ? (smem_tile + 15) & ~15 : 0;
@@ -86,7 +94,7 @@ static inline int resident_smem_bytes(int rows, int max_k, int max_dbs, int opti
 static inline bool update_is_early(int tiles, int rows, int max_k, int max_dbs, bool bf16, int alpha, int sms, int optin_smem) {
     int tile_bytes;
     if (bf16 && alpha == 0 && resident_smem_bytes(rows, max_k, max_dbs, optin_smem, &tile_bytes) > 0) return early_form(tiles, std::min(tiles, 2 * sms), sms);
-    return plan_tile_launch(false, alpha, bf16, rows, max_k, tiles, true, sms, optin_smem).early;
+    return plan_tile_launch(0, alpha, bf16, rows, max_k, tiles, true, sms, optin_smem).early;
 }
 
 }  // namespace mab

@@ -137,6 +137,33 @@ def test_compute_microadam_update(N, dtype, m, k_init):
             assert ((out == 0) == (outg.cpu() == 0)).all()
 
 
+@pytest.mark.parametrize('rows,k', [(10, 146), (10, 291), (2, 30), (10, 1453)])
+def test_update_of_an_output_larger_than_l2(N, rows, k):
+    """compute_microadam_update on an fp32 output that L2 does not hold stores its zeros at another time and with other threads: the same bits as
+    pieces of it, over what the buffers held before."""
+    blocks, tail, k_tail = 1160, 1003, 17
+    d, total = blocks * DBS + tail, blocks * k + k_tail
+    gen = torch.Generator(device='cuda').manual_seed(k)
+    I = torch.empty(rows, total, dtype=torch.int16, device='cuda')
+    for r in range(rows):
+        I[r, :blocks * k] = torch.rand(blocks, DBS, device='cuda', generator=gen).topk(k, dim=1).indices.sort(dim=1).values.reshape(-1).to(torch.int16)
+        I[r, blocks * k:] = torch.rand(tail, device='cuda', generator=gen).topk(k_tail).indices.sort().values.to(torch.int16)
+    V = torch.empty(rows, total, dtype=torch.bfloat16, device='cuda').normal_(0.0, 1e-3, generator=gen)
+    whole, parts = (torch.full((d,), float('nan'), device='cuda') for _ in range(2))
+
+    def update(n, total, I, V, out):
+        N.compute_microadam_update(148, 512, 100, rows + 3, 0.9, 0.999, 1e-8, DBS, k, n, rows, total, I, V, out)
+
+    update(d, total, I, V, whole)
+    for b0, b1 in ((0, 500), (500, 1000), (1000, blocks)):
+        last = b1 == blocks
+        at, end = b0 * k, total if last else b1 * k
+        piece = parts[b0 * DBS:d if last else b1 * DBS]
+        update(piece.numel(), end - at, I[:, at:end].contiguous(), V[:, at:end].contiguous(), piece)
+    assert torch.equal(whole.view(torch.int32), parts.view(torch.int32))
+    assert int((whole != 0).sum()) > 0
+
+
 @pytest.mark.parametrize('vdtype', [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize('gdtype', [torch.float32, torch.bfloat16])
 def test_sparse_rows_dot_and_combine(N, gdtype, vdtype):

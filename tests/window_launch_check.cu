@@ -12,7 +12,7 @@ int main() {
                 for (int tiles : {1, 2, 15, 16, 17, 37, 38, 74, 75, 111, 132, 133, 147, 148, 149, 296, 297, 444, 445, 5000})
                     for (int form = 0; form < 7; ++form) {   // the update with alpha 0, in (0, 1) and -2, fp32 and bf16; the operator
                         const int alpha = form < 6 ? form % 3 : 0;
-                        const mab::TileLaunch L = mab::plan_tile_launch(form == 6, alpha, form >= 3, rows, max_k, tiles, form != 6, sms, optin);
+                        const mab::TileLaunch L = mab::plan_tile_launch(form == 6 ? 1 + (rows & 1) : 0, alpha, form >= 3, rows, max_k, tiles, form != 6, sms, optin);
                         if (L.smem == 0) continue;
                         ++plans;
                         // the form that starts before kernel A ends stages one tile's rows: a CTA must not get a second one
