@@ -18,7 +18,7 @@ __host__ __device__ constexpr int wt_smem_bytes(int rows, int max_k) {
     return 8 * e + rows * 2 * wt_row_stride(max_k) + 4 * WT_WORDS + 2 * WT_WORDS + 2 * e;
 }
 
-// Threads of a CTA of the tile kernel; `fit`: how many CTAs' arrays fit an SM.  us of this kernel, fp32, 10 rows; the row loop has its
+// Threads of a CTA of the tile kernel; `fit`: how many CTAs' arrays fit an SM (`fit_384`: with 384 threads, the alpha forms' dense arrays grow with them).  us of this kernel, fp32, 10 rows; the row loop has its
 // prefetching form while a row's entries do not outnumber the threads, and every tile in flight costs L2.
 //   k = 0.5 % (146 entries), 116 M elements: 256 threads 105, 384 108, 512 120.
 //   k = 1 % (291): 256 / 384 / 512 threads, 100 tiles 12.4 / 9.5 / 8.6, 300 tiles 18.8 / 15.5 / 18.6, 1000 55 / 42 / 44, 1500 77 / 61 / 61, 3000 143 / 124 /
@@ -26,9 +26,9 @@ __host__ __device__ constexpr int wt_smem_bytes(int rows, int max_k) {
 //   The operator that writes every position's update: 384 (60 M elements k = 1 % 75, 256 and 512 threads 79; 0.5 % 59, 256 73, 512 67); with late zeros
 //   256 for many short rows (232 M elements, 0.5 %, 10 and 20 rows 202 and 270, 384 threads 219 and 298; 1 and 3 rows 161 and 173, 155 and 164).
 //   The alpha forms have 80 registers a thread: 256 threads while three CTAs fit (33.5 M elements 121, 384 threads 127), 384 where two do (bf16, 20
-//   rows, 58 M elements 265 with 256, 209), and 512 where one does or an SM has no more than one tile (100 tiles 29 and 18).
-static inline int threads_of(int write, bool alpha, int fit, int tiles, int rows, int max_k, int sms) {
-    if (alpha) return fit < 2 || tiles <= sms ? 512 : fit < 3 ? 384 : 256;
+//   rows, 58 M elements 265 with 256, 209; one CTA of 384 alone 415, two of 256 373), and 512 where one does or an SM has no more than one tile (100 tiles 29 and 18).
+static inline int threads_of(int write, bool alpha, int fit, int fit_384, int tiles, int rows, int max_k, int sms) {
+    if (alpha) return fit < 2 || tiles <= sms ? 512 : fit < 3 && fit_384 >= 2 ? 384 : 256;
     if (fit < 2) return 1024;
     if (tiles <= 2 * sms || fit < 3) return 512;
     if (write == 1) return 384;
@@ -56,6 +56,13 @@ static inline bool rows_ahead(bool bf16, int alpha, int threads, int grid, int t
     return threads != 256 ? tiles > grid : max_k > 256 || (alpha == 2 && tiles > 2 * grid);
 }
 
+// CTAs of `dynamic` bytes of shared memory an SM holds, next to the kernel's static arrays (the tensors' first units, the scan's scratch, the rows'
+// offsets) and the 1024 bytes that every CTA costs.  One CTA too many is a second wave of them, and threads chosen for what does not fit (us a step,
+// 58 M elements, 10 rows, reckoned too small by 1280 bytes and right: alpha = 0.5, bf16, 419 entries a row 356 and 271, 670 411 and 345; fp32, alpha 0,
+// 757 entries 342 and 298).
+constexpr int WT_STATIC_BYTES = (4 * (WIN_MAX_TENSORS + 1 + 36 + 2 * MAB_MAX_WINDOW) + 127) & ~127;
+static inline int ctas_of_sm(int dynamic, int optin_smem) { return (optin_smem + 1024) / (dynamic + WT_STATIC_BYTES + 1024); }
+
 struct TileLaunch {
     int  threads, grid, smem;             // smem 0: the window is too large for the compact arrays, the wide form takes it
     int  dense_at;                        // the alpha forms' dense arrays of the warps in shared memory (0: they do not fit)
@@ -68,13 +75,13 @@ static inline TileLaunch plan_tile_launch(int write, int alpha, bool bf16, int r
     const int smem_tile = (int64_t)rows * max_k <= WT_MAX_ENTRIES ? wt_smem_bytes(rows, max_k) : 0;
     if (smem_tile == 0 || smem_tile + 4096 > optin_smem) return L;
     // the forms with the alpha term: a dense array of 256 floats per warp behind the window's arrays, if it fits
-    const int fit = std::max(1, std::min(8, (227 * 1024) / (smem_tile + (alpha ? 8 * 1024 : 0) + 3072)));   // CTAs per SM by their arrays
-    L.threads = threads_of(write, alpha != 0, fit, tiles, rows, max_k, sms);
+    const int fit = std::max(1, std::min(8, ctas_of_sm(smem_tile + (alpha ? 8 * 1024 : 0), optin_smem)));
+    L.threads = threads_of(write, alpha != 0, fit, ctas_of_sm(smem_tile + 12 * 1024, optin_smem), tiles, rows, max_k, sms);
     if (alpha && ((smem_tile + 15) & ~15) + L.threads * 32 + 4096 > optin_smem) L.threads = 256;
     const int nt = L.threads, dense = alpha ? nt * 32 : 0;
     L.dense_at = alpha && ((smem_tile + 15) & ~15) + dense + 4096 <= optin_smem ? (smem_tile + 15) & ~15 : 0;
     L.smem = L.dense_at > 0 ? L.dense_at + dense : smem_tile;
-    const int per_sm = std::max(1, std::min(alpha ? 768 / nt : nt == 384 ? 3 : 1024 / nt, (227 * 1024) / (L.smem + 3072)));   // (as in __launch_bounds__)
+    const int per_sm = std::max(1, std::min(alpha ? 768 / nt : nt == 384 ? 3 : 1024 / nt, ctas_of_sm(L.smem, optin_smem)));   // (as in __launch_bounds__)
     L.grid = (int)std::min<int64_t>(tiles, (int64_t)sms * per_sm);
     L.early = behind_a && nt == 512 && early_form(tiles, L.grid, sms);
     L.ahead = !L.early && rows_ahead(bf16, alpha, nt, L.grid, tiles, max_k);

@@ -4,7 +4,7 @@
 
 int main() {
     const int optin = 227 * 1024;
-    long long plans = 0, bad_early = 0, bad_ahead = 0;
+    long long plans = 0, bad_early = 0, bad_ahead = 0, bad_fit = 0;
     int early_at_148 = 0;
     for (int sms : {16, 37, 74, 132, 148, 160})
         for (int rows : {1, 2, 3, 5, 10, 20, 32, 128})
@@ -15,6 +15,10 @@ int main() {
                         const mab::TileLaunch L = mab::plan_tile_launch(form == 6 ? 1 + (rows & 1) : 0, alpha, form >= 3, rows, max_k, tiles, form != 6, sms, optin);
                         if (L.smem == 0) continue;
                         ++plans;
+                        // no more CTAs than an SM holds (228 KB, 1 KB for each of them), which a second, nearly empty wave would follow, and 384
+                        // threads only where two CTAs have room
+                        const int held = (228 * 1024) / (L.smem + mab::WT_STATIC_BYTES + 1024);
+                        bad_fit += L.grid > (int64_t)sms * held || held < 1 || (alpha && L.threads == 384 && L.grid < std::min(tiles, 2 * sms));
                         // the form that starts before kernel A ends stages one tile's rows: a CTA must not get a second one
                         bad_early += L.early && (tiles > L.grid || L.ahead);
                         // rows staged ahead: bf16 alpha forms only, and not without a next tile unless the row loop is the one with two entries
@@ -41,6 +45,6 @@ int main() {
                 form_ok = form_ok && !mab::update_is_early(tiles, 10, 1453, dbs, bf16, 0, sms, optin);
             }
         }
-    printf("plans %lld, early forms with more tiles than CTAs %lld, rows ahead of nothing %lld, what may start early %s\n", plans, bad_early, bad_ahead, form_ok ? "right" : "wrong");
-    return form_ok && bad_ahead == 0 && plans > 100000 && early_at_148 == 6 && bad_early == 0 ? 0 : 1;
+    printf("plans %lld, early forms with more tiles than CTAs %lld, rows ahead of nothing %lld, CTAs without room %lld, what may start early %s\n", plans, bad_early, bad_ahead, bad_fit, form_ok ? "right" : "wrong");
+    return form_ok && bad_ahead == 0 && bad_fit == 0 && plans > 100000 && early_at_148 == 6 && bad_early == 0 ? 0 : 1;
 }
