@@ -77,16 +77,6 @@ __device__ __forceinline__ void load_octet(const T* x, int o, int n, bool vec, f
 
 __device__ __forceinline__ int key_of(float v) { return __float_as_int(fabsf(v)); }
 
-// First free slot behind *counter for each lane's `cnt` entries (one atomic per warp).  All 32 lanes call.
-__device__ __forceinline__ int warp_alloc(int cnt, int* counter) {
-    int inc = cnt;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) { const int v = __shfl_up_sync(0xffffffffu, inc, d); if (lane_id() >= d) inc += v; }
-    int base = 0;
-    if (lane_id() == 31 && inc) base = atomicAdd(counter, inc);
-    return __shfl_sync(0xffffffffu, base, 31) + inc - cnt;
-}
-
 // A level of the radix search, every warp for itself: the bin of the k_rem-th largest entry (hist[b]: entries of bin b); k_rem then counts
 // within that bin, whose size is returned in `size`.  -1: there are fewer entries.
 __device__ __forceinline__ int kth_bin(const int* hist, int& k_rem, int& size) {

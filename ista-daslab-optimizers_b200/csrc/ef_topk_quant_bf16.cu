@@ -87,18 +87,6 @@ __device__ __forceinline__ void unpack8(const uint4& a, float (&v)[8]) {
     v[6] = __uint_as_float(a.w << 16); v[7] = __uint_as_float(a.w & 0xFFFF0000u);
 }
 
-// Reserves `cnt` consecutive slots behind *counter for every lane (one atomic per warp); returns the
-// lane's first slot.  All 32 lanes must call.
-__device__ __forceinline__ int warp_alloc(int cnt, int* counter) {
-    int inc = cnt;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) { const int v = __shfl_up_sync(0xffffffffu, inc, d); if (lane_id() >= d) inc += v; }
-    int base = 0;
-    if (lane_id() == 31 && inc) base = atomicAdd(counter, inc);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    return base + inc - cnt;
-}
-
 // Where octet o of the tile sits: rows of 8 octets are permuted by the row number on regular tiles.
 __device__ __forceinline__ int phys_oct(int o, bool swz) { return swz ? (o ^ ((o >> 3) & 7)) : o; }
 __device__ __forceinline__ int phys_pos(int pos, bool swz) { return (phys_oct(pos >> 3, swz) << 3) | (pos & 7); }

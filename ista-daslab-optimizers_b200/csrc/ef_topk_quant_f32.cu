@@ -68,17 +68,6 @@ struct __align__(16) SmemF {
 constexpr int F_QTAB = F_CAND_CAP * 6 / 8;   // quantisation blocks whose constants fit the table: 2304 (all of a tile's when they have 16 elements or more)
 static_assert(sizeof(uint16_t) * (F_NT / 32) * F_WLIST <= (4 + 2) * SEL_WORDS, "the octet lists reuse the bitmap");
 
-// First free slot behind *counter for each lane's `cnt` entries (one atomic per warp).  All 32 lanes must call.
-__device__ __forceinline__ int f32_warp_alloc(int cnt, int* counter) {
-    int inc = cnt;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) { const int v = __shfl_up_sync(0xffffffffu, inc, d); if (lane_id() >= d) inc += v; }
-    int base = 0;
-    if (lane_id() == 31 && inc) base = atomicAdd(counter, inc);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    return base + inc - cnt;
-}
-
 // The octet thread t owns in slot j.
 __device__ __forceinline__ int f32_oct(int j) { return j < F_REG ? F_REG * (int)threadIdx.x + j : j * F_NT + (int)threadIdx.x; }
 
@@ -491,7 +480,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
                     for (int j = 0; j < F_REG; ++j)
 #pragma unroll
                         for (int e = 0; e < 8; ++e) mask |= (fabsf(a[j][e]) >= lo_f) ? (1u << (8 * j + e)) : 0u;
-                    int slot = f32_warp_alloc(__popc(mask), &ss.n_cand);
+                    int slot = warp_alloc(__popc(mask), &ss.n_cand);
                     if (mask) {
 #pragma unroll
                         for (int j = 0; j < F_REG; ++j) {
@@ -534,7 +523,7 @@ ef_topk_quant_f32_kernel(const mab_tensor* __restrict__ tensors, int n_tensors, 
 #pragma unroll
                         for (int e = 0; e < 8; ++e) mask |= (fabsf(v[e]) >= lo_f) ? (1u << e) : 0u;
                     }
-                    int slot = f32_warp_alloc(__popc(mask), &ss.n_cand);
+                    int slot = warp_alloc(__popc(mask), &ss.n_cand);
                     while (mask) {
                         const uint32_t pos = (o << 3) + (__ffs(mask) - 1);
                         mask &= mask - 1;

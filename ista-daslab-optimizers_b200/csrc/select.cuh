@@ -30,6 +30,16 @@ struct SelectSmem {
     int      sel_before[SEL_WORDS];   // selected positions in lower words
 };
 
+// First free slot behind *counter for each lane's `cnt` entries (one atomic per warp).  All 32 lanes call.
+__device__ __forceinline__ int warp_alloc(int cnt, int* counter) {
+    int inc = cnt;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) { const int v = __shfl_up_sync(0xffffffffu, inc, d); if (lane_id() >= d) inc += v; }
+    int base = 0;
+    if (lane_id() == 31 && inc) base = atomicAdd(counter, inc);
+    return __shfl_sync(0xffffffffu, base, 31) + inc - cnt;
+}
+
 // Number of keys >= thr (key bits) over the whole tile.  `counter` must be zero on entry and is
 // left dirty.  A threshold above the bit pattern of infinity compares false everywhere.
 __device__ __forceinline__ int block_count_ge(const float (&a)[SEL_OCTETS][8], int thr, int* counter) {
