@@ -625,7 +625,7 @@ __device__ __forceinline__ int window_tile_moments(const mab_tensor& T, int blk,
     MAB_BTICK(1);
     // 3. number them: prefix[word] = touched positions in words below
     constexpr int WPT = (WT_WORDS + NT - 1) / NT;
-    constexpr bool EVEN = WT_WORDS % NT == 0;                 // (else the last threads have fewer words; the check costs the wide accesses)
+    constexpr bool EVEN = WT_WORDS % NT == 0 && WPT >= 4;     // (else the last threads may have fewer words; the check costs the 16-byte accesses)
     int cnt[WPT], local = 0;
 #pragma unroll
     for (int i = 0; i < WPT; ++i) { cnt[i] = EVEN || t * WPT + i < WT_WORDS ? __popc(w.bitmap[t * WPT + i]) : 0; local += cnt[i]; }
@@ -751,11 +751,13 @@ __device__ __forceinline__ uint4 decayed(uint4 x, float decay) {
 // p <- round_p(p * decay) on p[0, len), by the NT threads of the CTA: 16 bytes a lane from the first 16-byte boundary on, the elements around them one
 // by one, read before.  us a step of 63.9 M elements, fp32 with bf16 gradients, windows of 10 rows of 5 %: 428, with 32 bytes a lane 451; 10 rows of
 // 1 % on a shard that starts 4 bytes off such a boundary 250, element by element from end to end 315 (296 where all of it was asked into L2 before).
+// (us of the kernel with two, four and eight vectors in flight: 384 threads, 600 tiles of 1 % 44.2, 52.4 and 43.9, 1480 tiles 91.9, 107.4 and 93; 512
+// threads, 2200 tiles 138.5, 127.4 and 136; 256 threads, 600 tiles of 0.5 % 43.9, 38.1 and 39.5.)
 // Out of line: inline, at both places that call it, it cost 360 bytes of spills.
 template <typename TP, int NT>
 __device__ __noinline__ void decay_tile(TP* p, int len, float decay) {
     using V = typename std::conditional<sizeof(TP) == 4, float4, uint4>::type;
-    constexpr int N = 16 / (int)sizeof(TP), B = 4;           // elements of a vector, vectors a thread has in flight
+    constexpr int N = 16 / (int)sizeof(TP), B = NT == 384 ? 2 : 4;   // elements of a vector, vectors a thread has in flight
     const int head = min(len, (int)((0u - (uint32_t)reinterpret_cast<uintptr_t>(p)) & 15u) / (int)sizeof(TP));
     const int whole = (len - head) / N, around = len - whole * N;   // (around: fewer than 16, a thread each)
     V* const q = reinterpret_cast<V*>(p + head);
