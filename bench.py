@@ -49,8 +49,8 @@ UNIT = 'Gparams/s'
 # 134 217 728-element (bf16) / 67 108 864-element (fp32) flat tensor and scaled to the workload by its
 # parameter count (traffic grows in proportion to the elements a launch covers).  None = not captured.
 NCU_TRAFFIC_BYTES_PER_PARAM = {
-    ('ef_topk_quant', 'bf16'): 3.05, ('window_adam', 'bf16'): 3.98,
-    ('ef_topk_quant', 'f32'): 5.00, ('window_adam', 'f32'): 7.15,
+    ('ef_topk_quant', 'bf16'): 3.02, ('window_adam', 'bf16'): 3.98,
+    ('ef_topk_quant', 'f32'): 5.00, ('window_adam', 'f32'): 6.03,
 }
 
 
