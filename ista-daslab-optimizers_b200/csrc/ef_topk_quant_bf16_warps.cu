@@ -721,14 +721,16 @@ ef_topk_quant_bf16_warps_kernel(const mab_tensor* __restrict__ tensors, int n_te
         I.qb_at = LOOSE ? la.qb_first[ti] + qb0 : 0;
     };
 
-    // a tile's codes and statistics into L2; one thread.  (Not its gradient, which the copy engine brings a warp's part at a time: 215 M elements
-    // 259 us a launch, 262 with it; loose blocks with the requantisation 395 and 398; 58 M with k = 5 % 104 and 105.)
+    // a tile's codes and statistics into L2; one thread.  (Its gradient only where plain loads fetch it; the copy engine brings a warp's part at a
+    // time: 215 M elements 259 us a launch, 262 with it; loose blocks with the requantisation 395 and 398; 58 M with k = 5 % 104 and 105.  Off alignment 43 M 82
+    // with it and 95 without, 133 M 220 and 249, blocks of 32, 116 M 210 and 232.)
     auto ask_tile = [&](const TileInfo& N) {
         auto ask = [](const void* at, int64_t bytes) {
             const uintptr_t from = reinterpret_cast<uintptr_t>(at) & ~(uintptr_t)15;
             const uint32_t len = (uint32_t)((reinterpret_cast<uintptr_t>(at) + bytes - from + 15) & ~(uintptr_t)15);
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(from), "r"(len) : "memory");
         };
+        if (!aligned16(N.g) || (reinterpret_cast<uintptr_t>(N.ef) & 7) != 0) ask(N.g, (int64_t)N.n * 2);   // (`staged` below)
         ask(N.ef, ((int64_t)N.n + 1) >> 1);
         const int64_t nb = LOOSE ? loose_blocks_touched(N.lrem0, N.n, la.qbs) : ((int64_t)N.n + (1 << QS) - 1) >> QS;
         ask(N.mn, nb * 2);
