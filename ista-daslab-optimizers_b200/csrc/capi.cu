@@ -198,14 +198,14 @@ static int fused_run(mab_tensor* tensors, int n, const mab_step_args* args, void
     auto key = [&](int i) { return tensors[i].grad_dtype * 2 + tensors[i].param_dtype; };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return key(x) < key(y); });
 
-    struct Chunk { int first, count, units_a, units_b, grad_dtype, param_dtype, max_k, max_dbs, units_off; };
+    struct Chunk { int first, count, units_a, units_b, grad_dtype, param_dtype, max_k, max_dbs; };
     std::vector<Chunk> chunks;
     static thread_local std::vector<mab_tensor> staged;
     staged.resize(n);
     const int max_tensors = WIN_MAX_TENSORS;              // kernels A and B size their unit-prefix tables by it
     const int64_t unit_cap = (int64_t)1 << 30;
     for (int pos = 0; pos < n;) {
-        Chunk c = {pos, 0, 0, 0, tensors[order[pos]].grad_dtype, tensors[order[pos]].param_dtype, 0, 0, 0};
+        Chunk c = {pos, 0, 0, 0, tensors[order[pos]].grad_dtype, tensors[order[pos]].param_dtype, 0, 0};
         int64_t ua = 0, ub = 0;
         while (pos < n && c.count < max_tensors && key(order[pos]) == c.grad_dtype * 2 + c.param_dtype) {
             mab_tensor& t = tensors[order[pos]];
@@ -220,7 +220,6 @@ static int fused_run(mab_tensor* tensors, int n, const mab_step_args* args, void
             ua += na; ub += nb;
             c.max_k = std::max(c.max_k, std::max(t.k_block_size_many, t.k_block_size_few));
             c.max_dbs = std::max(c.max_dbs, t.d_block_size);
-            if (!aligned_to(t.grad, 16)) c.units_off += (int)na;
             ++c.count; ++pos;
         }
         c.units_a = (int)ua; c.units_b = (int)ub;
@@ -248,7 +247,7 @@ static int fused_run(mab_tensor* tensors, int n, const mab_step_args* args, void
         for (const Chunk& c : chunks) {
             const LooseArgs la = {qbs, reinterpret_cast<uint32_t*>(ws + L.off_min), reinterpret_cast<uint32_t*>(ws + L.off_max),
                                   reinterpret_cast<const int64_t*>(ws + L.off_first) + c.first};
-            if (int rc = launch_ef_topk_quant(dev + c.first, c.count, c.units_a, c.grad_dtype, qbs, c.max_dbs, c.max_k, c.units_off, 0, s, &la)) return rc;
+            if (int rc = launch_ef_topk_quant(dev + c.first, c.count, c.units_a, c.grad_dtype, qbs, c.max_dbs, c.max_k, 0, s, &la)) return rc;
         }
         for (const Chunk& c : chunks) {
             const LooseArgs la = {qbs, reinterpret_cast<uint32_t*>(ws + L.off_min), reinterpret_cast<uint32_t*>(ws + L.off_max),
@@ -260,7 +259,7 @@ static int fused_run(mab_tensor* tensors, int n, const mab_step_args* args, void
         const Chunk& b = chunks[0];
         const int allowing = (what & RUN_B) ? allowing_ctas(b.units_a, (int)std::min<int64_t>(args->steps, args->m), b.max_k, b.max_dbs, b.param_dtype, args->alpha) : 0;
         for (const Chunk& c : chunks)
-            if (int rc = launch_ef_topk_quant(dev + c.first, c.count, c.units_a, c.grad_dtype, args->quant_block_size, c.max_dbs, c.max_k, c.units_off, allowing, s)) return rc;
+            if (int rc = launch_ef_topk_quant(dev + c.first, c.count, c.units_a, c.grad_dtype, args->quant_block_size, c.max_dbs, c.max_k, allowing, s)) return rc;
     }
     if (what & RUN_B) {
         WindowArgs wa;
@@ -319,12 +318,12 @@ static int static_table_address(void** out) {
 
 // End (exclusive) of the run of tensors starting at `first` that one launch can take: same element
 // types, at most 512 tensors, unit counts within the kernels' 32-bit prefix.  Fills the library-owned
-// fields of those tensors and reports the run's totals (units_off: tiles of gradients off a 16-byte boundary).
-static int static_run_end(mab_tensor* tensors, int n, int first, int* units_a, int* units_b, int* max_k, int* max_dbs, int* units_off) {
+// fields of those tensors and reports the run's totals.
+static int static_run_end(mab_tensor* tensors, int n, int first, int* units_a, int* units_b, int* max_k, int* max_dbs) {
     const int gd = tensors[first].grad_dtype, pd = tensors[first].param_dtype;
     const int64_t unit_cap = (int64_t)1 << 30;
     int64_t ua = 0, ub = 0;
-    int i = first, mk = 0, md = 0, off = 0;
+    int i = first, mk = 0, md = 0;
     while (i < n && i - first < WIN_MAX_TENSORS && tensors[i].grad_dtype == gd && tensors[i].param_dtype == pd) {
         mab_tensor& t = tensors[i];
         const int64_t na = units_a_of(t), nb = units_b_of(t);
@@ -336,10 +335,9 @@ static int static_run_end(mab_tensor* tensors, int n, int first, int* units_a, i
         ua += na; ub += nb;
         mk = std::max(mk, std::max(t.k_block_size_many, t.k_block_size_few));
         md = std::max(md, t.d_block_size);
-        if (!aligned_to(t.grad, 16)) off += (int)na;
         ++i;
     }
-    *units_a = (int)ua; *units_b = (int)ub; *max_k = mk; *max_dbs = md; *units_off = off;
+    *units_a = (int)ua; *units_b = (int)ub; *max_k = mk; *max_dbs = md;
     return i;
 }
 
@@ -369,27 +367,27 @@ extern "C" int mab_fused_step_static(mab_tensor* tensors, int n, const mab_step_
                                   args->quant_block_size)) return rc;
 
     // first pass: fill the library-owned fields of every run, then ship the table
-    int ua, ub, mk, md, off;
-    for (int first = 0; first < n;) first = static_run_end(tensors, n, first, &ua, &ub, &mk, &md, &off);
+    int ua, ub, mk, md;
+    for (int first = 0; first < n;) first = static_run_end(tensors, n, first, &ua, &ub, &mk, &md);
     MAB_CUDA_TRY(cudaMemcpyAsync(table, tensors, (size_t)n * sizeof(mab_tensor), cudaMemcpyHostToDevice, s));
     const mab_tensor* dev = reinterpret_cast<const mab_tensor*>(table);
     // kernel A over every run, then kernel B over every run (the runs are recomputed, not stored); the first update follows the last kernel A
-    static_run_end(tensors, n, 0, &ua, &ub, &mk, &md, &off);
+    static_run_end(tensors, n, 0, &ua, &ub, &mk, &md);
     const int allowing = allowing_ctas(ua, wa.rows, mk, md, tensors[0].param_dtype, wa.alpha);
     for (int first = 0; first < n;) {
-        const int end = static_run_end(tensors, n, first, &ua, &ub, &mk, &md, &off);
-        if (int rc = launch_ef_topk_quant(dev + first, end - first, ua, tensors[first].grad_dtype, args->quant_block_size, md, mk, off, allowing, s)) return rc;
+        const int end = static_run_end(tensors, n, first, &ua, &ub, &mk, &md);
+        if (int rc = launch_ef_topk_quant(dev + first, end - first, ua, tensors[first].grad_dtype, args->quant_block_size, md, mk, allowing, s)) return rc;
         first = end;
     }
     wa.probe = args->probe_out;
     for (int first = 0; first < n;) {
-        const int end = static_run_end(tensors, n, first, &ua, &ub, &mk, &md, &off);
+        const int end = static_run_end(tensors, n, first, &ua, &ub, &mk, &md);
         if (int rc = launch_window_step(dev + first, end - first, ua, ub, mk, md, tensors[first].param_dtype, wa, true, s)) return rc;
         first = end;
     }
     if (args->probe_out)
         for (int first = 0; first < n;) {
-            const int end = static_run_end(tensors, n, first, &ua, &ub, &mk, &md, &off);
+            const int end = static_run_end(tensors, n, first, &ua, &ub, &mk, &md);
             if (int rc = launch_probe(dev + first, end - first, ua, args->quant_block_size, args->probe_out, s)) return rc;
             first = end;
         }

@@ -466,15 +466,14 @@ int units_a_of(const mab_tensor& t) { return t.topk_full_blocks_count + (t.k_blo
 // tiles): k = 0.5 % 63 / 83, 1 % 63 / 72, 2 % 66 / 79, 5 % 82 / 99, 20 % 265 / 266; 2960 tiles k = 5 % 145 / 181; k = 1 % with 31 and 50 tiles per
 // SM 165 / 188 and 255 / 295.  Below, 1000 tiles 47 / 56, 444 tiles 20.3 / 20.0, 72 tiles 12.1 / 12.2: the line could lie lower, at 6 tiles per SM
 // or so.
-// A tile whose gradient the copy engine cannot move (off a 16-byte boundary) costs the first one more, the other one little: k = 1 %, 1480, 2960,
-// 4588 and 7400 tiles 95 / 84, 166 / 153, 248 / 222 and 391 / 349; 5 % 118 / 112, 206 / 201, 301 / 293, 467 / 475; 0.5 % 96 / 93, 166 / 169, 250 / 255,
-// 388 / 399 (a step of 7400 tiles all the same 497 / 481).  So a launch with more of those tiles than others takes the other one.
+// Off a 16-byte boundary, k = 0.5, 1 and 5 %: 1480 tiles 84 / 93, 82 / 84 and 106 / 111; 2960 tiles 149 / 170, 150 / 153 and 189 / 202; 4588 tiles
+// 217 / 257, 220 / 222 and 277 / 293 (that form with the gradient not asked into L2: 1 % 95, 166 and 249).
 constexpr int WARPS_MIN_TILES_PER_SM = 10;
 
 int launch_ef_topk_quant(const mab_tensor* dev_tensors, int n_tensors, int total_units, int grad_dtype,
-                         int qbs, int max_dbs, int max_k, int units_off, int allowing, cudaStream_t s, const LooseArgs* loose) {
+                         int qbs, int max_dbs, int max_k, int allowing, cudaStream_t s, const LooseArgs* loose) {
     if (grad_dtype == MAB_BF16) {          // bf16 tiles are small enough for two shared-memory resident CTAs per SM
-        const bool warps = loose != nullptr || qbs != 64 || (total_units >= WARPS_MIN_TILES_PER_SM * device_sm_count() && units_off <= total_units / 2);
+        const bool warps = loose != nullptr || qbs != 64 || total_units >= WARPS_MIN_TILES_PER_SM * device_sm_count();
         const int rc = warps ? launch_ef_topk_quant_bf16_warps(dev_tensors, n_tensors, total_units, qbs, max_dbs, allowing, s, loose)
                              : launch_ef_topk_quant_bf16(dev_tensors, n_tensors, total_units, max_dbs, allowing, s);
         if (rc <= 0) return rc;

@@ -104,9 +104,9 @@ __host__ __device__ __forceinline__ int loose_blocks_touched(int lrem0, int n, i
     return loose_block(lrem0 + n - 1, qbs, false) + 1;
 }
 
-// ef_topk_quant.cu; units_off: tiles of gradients that start off a 16-byte boundary; allowing: see allow_next_kernel
+// ef_topk_quant.cu; allowing: see allow_next_kernel
 int launch_ef_topk_quant(const mab_tensor* dev_tensors, int n_tensors, int total_units, int grad_dtype,
-                         int qbs, int max_dbs, int max_k, int units_off, int allowing, cudaStream_t s, const LooseArgs* loose = nullptr);
+                         int qbs, int max_dbs, int max_k, int allowing, cudaStream_t s, const LooseArgs* loose = nullptr);
 int units_a_of(const mab_tensor& t);
 
 // requant_loose.cu: statistics (bf16) and codes of the residual kernel A left in the gradient buffers

@@ -131,8 +131,8 @@ def test_large_launch_equals_small_ones(kind, k_init, alpha):
 
 @pytest.mark.parametrize('k_init,skip', [(0.05, 0), (0.01, 3), (0.05, 1), (0.2, 8), (0.01, 8), (0.01, -3)])
 def test_line_between_the_forms(k_init, skip):
-    """Blocks of 64: from ten tiles per SM on a launch takes the warp-owned form whatever k, but where most of the
-    gradients are off alignment (skip < 0: those of the short tensor only); below, the other one; equal results on both sides."""
+    """Blocks of 64: from ten tiles per SM on a launch takes the warp-owned form whatever k and alignment (skip < 0:
+    the short tensor's gradient only), below it the other one; equal results on both sides."""
     from ista_daslab_optimizers_b200 import MicroAdam, _native
     from ista_daslab_optimizers_b200.compat import ista_daslab_cuda_tools as tools
     tiles = 10 * tools.get_sm_count()
@@ -147,7 +147,7 @@ def test_line_between_the_forms(k_init, skip):
             off = skip if skip >= 0 else -skip if p is whole[1] else 0
             p.grad = torch.empty(p.numel() + off, dtype=torch.bfloat16, device='cuda')[off:].normal_(0.0, 1e-3, generator=gen)
             q.grad = p.grad.clone()
-        for form, o in (('ef_topk_quant_bf16_warps_kernel' if skip % 8 == 0 or skip < 0 else 'ef_topk_quant_bf16_kernel', opt), ('ef_topk_quant_bf16_kernel', opts[0])):
+        for form, o in (('ef_topk_quant_bf16_warps_kernel', opt), ('ef_topk_quant_bf16_kernel', opts[0])):
             if step == 0:
                 names = _kernels_of(o.step)
                 assert any(form in x for x in names), names
