@@ -51,9 +51,12 @@ static inline bool early_form(int tiles, int grid, int sms) { return tiles <= gr
 // step, ahead and not (alpha == -2, 444 CTAs): k = 0.5 % 444 tiles 55.5 / 54.3, 740 108.4 / 106.4, 1000 141.5 / 143.9, 2000 219.9 / 221.7; k = 1 %
 // 200 tiles 43.1 / 45.0, 445 85.9 / 87.4, 2000 238.5 / 246.4; 20 rows (296 CTAs) 445 90.4 / 90.2, 600 115.8 / 118.3; k = 5 % (148) 600 181.7 / 185.4.
 // alpha = 0.5, k = 0.5 %: 1000 143.1 / 143.9, 1500 183.9 / 183.1, 2000 228.4 / 226.2.
-static inline bool rows_ahead(bool bf16, int alpha, int threads, int grid, int tiles, int max_k) {
+// Two entries a thread: rows of up to 512, and four of them at least (alpha == -2, 300 tiles of 1 %, 1, 2 and 3 rows 43.1 / 42.7, 44.9 / 43.9 and 44.3 / 43.8,
+// 5 rows 45.7 / 45.8; alpha = 0.5, 2000 tiles, 1 row 212.7 / 210.4, 5 rows 225.9 / 227.6).
+static inline bool rows_ahead(bool bf16, int alpha, int threads, int grid, int tiles, int rows, int max_k) {
     if (!bf16 || alpha == 0) return false;
-    return threads != 256 ? tiles > grid : max_k > 256 || (alpha == 2 && tiles > 2 * grid);
+    if (threads != 256) return tiles > grid;
+    return (max_k > 256 && max_k <= 512 && rows >= 4) || (alpha == 2 && tiles > 2 * grid);
 }
 
 // CTAs of `dynamic` bytes of shared memory an SM holds, next to the kernel's static arrays (the tensors' first units, the scan's scratch, the rows'
@@ -84,7 +87,7 @@ static inline TileLaunch plan_tile_launch(int write, int alpha, bool bf16, int r
     const int per_sm = std::max(1, std::min(alpha ? 768 / nt : nt == 384 ? 3 : 1024 / nt, ctas_of_sm(L.smem, optin_smem)));   // (as in __launch_bounds__)
     L.grid = (int)std::min<int64_t>(tiles, (int64_t)sms * per_sm);
     L.early = behind_a && nt == 512 && early_form(tiles, L.grid, sms);
-    L.ahead = !L.early && rows_ahead(bf16, alpha, nt, L.grid, tiles, max_k);
+    L.ahead = !L.early && rows_ahead(bf16, alpha, nt, L.grid, tiles, rows, max_k);
     return L;
 }
 

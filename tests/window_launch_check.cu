@@ -22,7 +22,7 @@ int main() {
                         // the form that starts before kernel A ends stages one tile's rows: a CTA must not get a second one
                         bad_early += L.early && (tiles > L.grid || L.ahead);
                         // rows staged ahead: bf16 alpha forms only, and not without a next tile unless the row loop is the one with two entries
-                        bad_ahead += L.ahead && (form < 4 || form > 5 || (tiles <= L.grid && (L.threads != 256 || max_k <= 256)));
+                        bad_ahead += L.ahead && (form < 4 || form > 5 || (tiles <= L.grid && (L.threads != 256 || max_k <= 256 || max_k > 512 || rows < 4)));
                         early_at_148 += L.early && sms == 148 && rows == 10 && max_k == 291 && tiles == 148;
                     }
     for (int sms : {16, 37, 74, 132, 148})                   // the resident form, two CTAs per SM
